@@ -229,6 +229,7 @@ static void scene_free(kdop_scene* s) {
   dfree(s, &s->cand, kdop::kCandCols * s->cand_cap);
   dfree(s, &s->contacts, s->contact_cap);
   dfree(s, &s->records, s->cand_cap);
+  dfree(s, &s->seeds, s->seeds_cap);
   dfree(s, &s->q_items, s->queue_cap);
   dfree(s, &s->q_tags, s->queue_cap);
   dfree(s, &s->ctl, 1);
@@ -307,9 +308,12 @@ static int grow_pairs(kdop_scene* s, int64_t n) {
   drop_graph(s);
   dfree(s, &s->pairs, s->pairs_cap);
   dfree(s, &s->pair_order, s->pairs_cap);
-  s->pairs_cap = 0;
+  dfree(s, &s->seeds, s->seeds_cap);
+  s->pairs_cap = s->seeds_cap = 0;
   KDOP_CUDA(s->ctx, dalloc(s, &s->pair_order, n));
   KDOP_CUDA(s->ctx, dalloc(s, &s->pairs, n));
+  KDOP_CUDA(s->ctx, dalloc(s, &s->seeds, kdop::seed_entries(s->ctx->sm_count, n)));
+  s->seeds_cap = kdop::seed_entries(s->ctx->sm_count, n);
   s->pairs_cap = n;
   return KDOP_OK;
 }
@@ -712,7 +716,8 @@ int kdop_resolve_traverse_opts(const kdop_scene* s, const kdop_traverse_opts* o,
   if (p.block_warps > 16 || (p.stack_cap & (p.stack_cap - 1)) || p.stack_cap < 64 || p.init_chunk > 32)
     return KDOP_ERR_INVALID;
   if (p.load_group != 1 && p.load_group != 2 && p.load_group != 4 && p.load_group != 8) return KDOP_ERR_INVALID;
-  if (kdop::traverse_smem_bytes(p.block_warps, p.stack_cap) > s->ctx->smem_optin) return KDOP_ERR_INVALID;
+  // 12 bytes per deque entry (an entry takes 8)
+  if ((size_t)p.block_warps * p.stack_cap * 12 > s->ctx->smem_optin) return KDOP_ERR_INVALID;
   return KDOP_OK;
 }
 

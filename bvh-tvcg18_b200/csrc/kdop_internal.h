@@ -35,7 +35,7 @@ struct TravCtl {
   unsigned int n_contacts;           // contacts emitted (may exceed capacity)
   unsigned int n_init;               // root pairs in this launch
   unsigned int pair_base;            // pair index of the first root pair
-  unsigned int max_stack;            // deepest warp stack seen
+  unsigned int n_seed;               // node pairs the first seed pass left for the second
   unsigned int n_surv;               // candidates past the contact pre-filter
   unsigned int n_mid;                // candidates past the face axes of the SAT test
   unsigned int pad0[21];
@@ -129,6 +129,8 @@ struct kdop_scene {
   kdop_contact* contacts = nullptr;
   int4* records = nullptr;  // per candidate: faces, candidate codes, count, first contact
   int64_t contact_cap = 0;
+  uint4* seeds = nullptr;  // frontiers of the seed pass: seed_entries(pairs_cap)
+  int64_t seeds_cap = 0;
   uint4* q_items = nullptr;
   uint32_t* q_tags = nullptr;
   int64_t queue_cap = 0;
@@ -150,6 +152,10 @@ struct kdop_scene {
 };
 
 namespace kdop {
+
+// Entries (16 bytes each) the traversal's seed pass can leave for any list of
+// at most n pairs (kdop_traverse.cu).
+int64_t seed_entries(int sm_count, int64_t n);
 
 // fn(0 .. n-1) on up to 64 host threads
 template <typename F>

@@ -23,8 +23,9 @@
 //   * ballot compaction: prefix sums over per-lane push counts pack the kept
 //     pairs into the deque, and emitted leaf pairs reserve rows with one
 //     atomic per warp;
-//   * load balance: root pairs are claimed from the pair list (largest first),
-//     and a warp whose deque is deep while other warps wait gives its oldest
+//   * load balance: a seed pass expands the pairs (largest first) breadth first
+//     into thousands of node pairs, which the warps claim a few at a time; a
+//     warp whose deque is deep while other warps wait gives its oldest
 //     (largest) entries to a global queue -- any deque with work gives half
 //     while many warps wait; a deque overflow spills there too;
 //   * termination: a global count of outstanding work units reaches zero;
@@ -60,6 +61,8 @@ struct TravArgs {
   unsigned n_meshes;
   const uint32_t* __restrict__ order;  // root pair i -> pair index (NULL: identity)
   const uint4* __restrict__ entries;   // when set: initial work = these deque entries (A, B, pair)
+  int seeded;          // entries come from the seed pass (their count is known on the device only)
+  int stuck;           // test hook: outstanding work units nobody completes
   unsigned poll_mask;  // queue counters polled on steps with (step & poll_mask) == 0
 };
 
@@ -75,6 +78,7 @@ struct TravBuffers {
   uint32_t* q_tags;
   int64_t q_cap;
   TravCtl* ctl;
+  uint4* seeds = nullptr;  // room for the seed pass's entries (seed_entries), or NULL: start from the root pairs
 };
 
 __device__ __forceinline__ unsigned long long global_ns() {
@@ -146,6 +150,141 @@ struct Coop {
   static constexpr int PM = (4 + Q - 1) / Q;   // child pairs per lane
 };
 
+// The slab tests of one lane: on the lane's chunks of both children of each
+// side, separation of child pairs (0,0), (0,1), (1,0), (1,1) in s, and word 0
+// of the four children (A0, A1, B0, B1) in t on the lane holding the topology
+// chunk.
+template <int K, int C>
+__device__ __forceinline__ void test_twins(const float4 (&A0)[C], const float4 (&A1)[C], const float4 (&B0)[C],
+                                           const float4 (&B1)[C], int gq, bool (&s)[4], uint32_t (&t)[4]) {
+  using L = NodeLayout<K>;
+  constexpr int Q = Coop<K, C>::Q, TR = L::TOPO_CHUNK / Q;
+#pragma unroll
+  for (int c = 0; c < 4; ++c) {
+    s[c] = false;
+    t[c] = 0u;
+  }
+#pragma unroll
+  for (int r = 0; r < C; ++r) {
+    const int j = gq + Q * r;
+    const float4 a0 = A0[r], a1 = A1[r], b0 = B0[r], b1 = B1[r];
+    if (2 * j < L::NS) {
+      s[0] = s[0] || (a0.y < b0.x) || (b0.y < a0.x);
+      s[1] = s[1] || (a0.y < b1.x) || (b1.y < a0.x);
+      s[2] = s[2] || (a1.y < b0.x) || (b0.y < a1.x);
+      s[3] = s[3] || (a1.y < b1.x) || (b1.y < a1.x);
+    }
+    if (2 * j + 1 < L::NS) {
+      s[0] = s[0] || (a0.w < b0.z) || (b0.w < a0.z);
+      s[1] = s[1] || (a0.w < b1.z) || (b1.w < a0.z);
+      s[2] = s[2] || (a1.w < b0.z) || (b0.w < a1.z);
+      s[3] = s[3] || (a1.w < b1.z) || (b1.w < a1.z);
+    }
+    if (r == TR) {
+      t[0] = L::word0(a0);
+      t[1] = L::word0(a1);
+      t[2] = L::word0(b0);
+      t[3] = L::word0(b1);
+    }
+  }
+}
+
+// What becomes of a lane's child pairs c = gq + Q r (c = 2 i + k: child i of
+// A, child k of B) of the entry (xa, xb): pushed, emitted, counted.  A single
+// side is the node itself, which is side (x & 1) of the twin loaded: the
+// pairs with the other side are absent.  The verdicts of the entry's lanes
+// come together by one ballot per child pair (a shuffle would go through the
+// L1 data pipe, the kernel's busiest unit).  Called by whole warps.
+template <int K, int C>
+__device__ __forceinline__ void child_pairs(uint32_t xa, uint32_t xb, bool valid, const bool (&s)[4],
+                                            const uint32_t (&t)[4], int ge, int gq, unsigned group_mask, uint32_t need,
+                                            bool* push, bool* emit, uint32_t* pushA, uint32_t* pushB,
+                                            unsigned& tests32, unsigned& lo32) {
+  using L = NodeLayout<K>;
+  using CP = Coop<K, C>;
+  constexpr int Q = CP::Q, PM = CP::PM;
+  constexpr int TQ = L::TOPO_CHUNK % Q;  // lane holding topology
+  const unsigned m0 = __ballot_sync(0xffffffffu, s[0]), m1 = __ballot_sync(0xffffffffu, s[1]);
+  const unsigned m2 = __ballot_sync(0xffffffffu, s[2]), m3 = __ballot_sync(0xffffffffu, s[3]);
+  // word 0 of the four children, from the lane holding the topology chunk
+  const int src = ge * Q + TQ;
+  const uint32_t wA0 = __shfl_sync(0xffffffffu, t[0], src);
+  const uint32_t wA1 = __shfl_sync(0xffffffffu, t[1], src);
+  uint32_t wB0, wB1;
+  if (Q == 2) {
+    // lane gq only handles child gq of B: the topology lane keeps its own
+    // word, the other lane gets the other child's
+    const uint32_t wo = __shfl_sync(0xffffffffu, TQ ? t[2] : t[3], src);
+    wB0 = wB1 = (gq == TQ) ? (TQ ? t[3] : t[2]) : wo;
+  } else {
+    wB0 = __shfl_sync(0xffffffffu, t[2], src);
+    wB1 = __shfl_sync(0xffffffffu, t[3], src);
+  }
+  const bool singleA = (xa & LEAF_BIT) != 0, singleB = (xb & LEAF_BIT) != 0;
+#pragma unroll
+  for (int r = 0; r < PM; ++r) {
+    const int c = gq + Q * r;
+    const int ci = (Q == 2) ? r : (c >> 1), ck = (Q == 2) ? gq : (c & 1);
+    const uint32_t wa = ci ? wA1 : wA0, wb = ck ? wB1 : wB0;
+    const unsigned mc = ci ? (ck ? m3 : m2) : (ck ? m1 : m0);
+    const bool there = valid && (Q * r + Q - 1 < 4 || c < 4) && !(singleA && (int)(xa & 1u) != ci) &&
+                       !(singleB && (int)(xb & 1u) != ck);
+    const bool ok = there && (mc & group_mask) == 0u;
+    const uint32_t both = wa & wb;
+    const bool leaf = ok && (both & LEAF_BIT);
+    if (there) tests32 += 1u;
+    if (leaf) lo32 += 1u;
+    push[r] = ok && !(both & LEAF_BIT);
+    emit[r] = leaf && (both & need) == need;
+    pushA[r] = wa;
+    pushB[r] = wb;
+  }
+}
+
+// A candidate row for the leaves of words wa, wb at position `at`.
+template <int K>
+__device__ __forceinline__ void put_candidate(const TravArgs& a, unsigned at, uint32_t wa, uint32_t wb, uint32_t pid) {
+  if (at < a.cand_cap) {
+    a.candA[at] = leaf_tet<K>(a.nodes, wa);
+    a.candB[at] = leaf_tet<K>(a.nodes, wb);
+    a.candP[at] = pid;
+  }
+}
+
+// Root test of mesh pair pid (kdop_tandem_traversal.h:164), then the
+// traversal's own test of the root pair (:42), both counted as the reference
+// does.  True when the pair is to be expanded (wa, wb its entry).
+template <int K>
+__device__ __forceinline__ bool root_pair(const TravArgs& a, uint32_t pid, bool count, uint32_t& wa, uint32_t& wb,
+                                          unsigned& tests32, unsigned& lo32) {
+  const uint2 mp = a.pairs[pid];
+  if (mp.x >= a.n_meshes || mp.y >= a.n_meshes) {
+    if (count) atomicOr(&a.ctl->error, DEV_ERR_BAD_INDEX);
+    return false;
+  }
+  const uint32_t ra = a.root[mp.x], rb = a.root[mp.y];
+  if (ra == NO_NODE || rb == NO_NODE) return false;
+  const bool ov = node_overlap<K>(a.nodes, ra, rb, wa, wb);
+  if (count) tests32 += ov ? 2u : 1u;
+  if (!ov || !(wa & wb & LEAF_BIT)) return ov;
+  if (count) {
+    lo32 += 1u;
+    if (!a.surface_filter || (wa & wb & SURF_BIT)) put_candidate<K>(a, atomicAdd(&a.ctl->n_cand, 1u), wa, wb, pid);
+  }
+  return false;
+}
+
+// Claims of the seed pass's entries: this many at most per claim (a deque
+// takes them in one go), fewer towards the end (guided self-scheduling).
+// Claims of one entry cost small launches an atomic per expansion (a pair of
+// 6,000 tets: 114 us, 81 us with up to 4), claims of up to 16 leave long tails
+// (256 touching pairs: 500 against 435 us; a pair of 1.6 M tets: 979 against
+// 886 us).
+constexpr unsigned kMaxClaim = 4;
+__device__ __forceinline__ unsigned claim_size(unsigned left, unsigned warps) {
+  return min(max(left / (2u * warps), 1u), kMaxClaim);
+}
+
 // Deque entries (X, Y, pair): X and Y overlap and their children are to be
 // tested.  A side with LEAF_BIT is the single node X & NODE_MASK (a leaf);
 // otherwise X is the first child of an internal node, whose children X, X + 1
@@ -156,9 +295,15 @@ struct Coop {
 // children of each side, one 256-bit load per chunk and side (twin records
 // interleave the siblings' chunks), so the lanes of an entry read whole
 // 128-byte lines (k = 14) and a warp-wide load touches E lines instead of 32.
-// The lane tests its slabs for the four child pairs; a butterfly OR over the
+// The lane tests its slabs for the four child pairs; a ballot over the
 // entry's lanes combines the verdicts; the lane holding the topology chunk
 // broadcasts the children's word 0; lane q then handles child pairs q, q + Q.
+// Bound: instruction issue and the L1 data pipe.  A deque holding one pair
+// only (no pair index beside its entries: 8 instead of 12 bytes of shared
+// memory, the rest of the array caches records), verdicts combined by ballots
+// instead of shuffles, and the refill, root test and donation polls outside
+// the step took the batched workload (1.96 G tests, k = 14) from 11.28 to 9.6
+// ms.
 // S sub-batches are loaded together per step, and one compaction per step
 // packs the pushes of all of them.
 template <int K, int C, int S>
@@ -168,24 +313,22 @@ __global__ void __launch_bounds__(512, (C * S >= 4) ? 1 : 2) traverse_kernel(Tra
   constexpr int NW = L::NW;
   constexpr int Q = CP::Q, E = CP::E, PM = CP::PM;
   constexpr int SLOTS = PM * S;                     // pushes per lane per step
-  constexpr int TQ = L::TOPO_CHUNK % Q, TR = L::TOPO_CHUNK / Q;  // lane and round holding topology
   constexpr int CBITS = SLOTS <= 1 ? 1 : SLOTS <= 3 ? 2 : 3;  // bits of a lane's push count
   extern __shared__ uint32_t smem[];
+  __shared__ uint2 s_claim[16];  // per warp: claimed initial work not yet taken [x, y)
   const int lane = threadIdx.x & 31;
   const int wib = threadIdx.x >> 5;
   const int ge = lane / Q, gq = lane % Q;  // entry and chunk lane of this lane
   const float4* __restrict__ nodes_q = a.nodes + 2 * gq;  // chunk gq of twin 0
   const unsigned lt_mask = (1u << lane) - 1u;
+  const unsigned group_mask = ((1u << Q) - 1u) << (ge * Q);  // lanes of this lane's entry
   const int CAP = a.stack_cap;
   const int MASK = CAP - 1;
-  // this warp's deque: CAP entries of (A, B) words, then CAP pair indices
-  // (written and read only while the deque mixes pairs, see curP below)
-  uint32_t* wbase = smem + (size_t)wib * 3 * CAP;
-  uint2* sAB = reinterpret_cast<uint2*>(wbase);
-  uint32_t* sP = wbase + 2 * CAP;
+  uint2* sAB = reinterpret_cast<uint2*>(smem) + (size_t)wib * CAP;  // this warp's deque
   TravCtl* ctl = a.ctl;
-  const unsigned n_init = ctl->n_init;
-  const unsigned pair_base = ctl->pair_base;
+  if (a.seeded && ctl->n_init == 0u && a.stuck == 0) return;  // the seed pass finished every pair
+  if (lane == 0) s_claim[wib] = make_uint2(0u, 0u);
+  __syncwarp();
 
   int top = 0, bot = 0;  // deque [bot, top) in virtual positions
   int release = 0;       // work units taken and not yet released
@@ -207,33 +350,14 @@ __global__ void __launch_bounds__(512, (C * S >= 4) ? 1 : 2) traverse_kernel(Tra
     }
     tests32 = lo32 = 0;
   };
-  unsigned max_depth = 0;
-  bool failed = false;
-  // Pair index of the deque's entries.  A deque filled from one root pair or
-  // one queue item holds a single pair (entries inherit their parent's pair),
-  // kept in curP; only a claim of several root pairs or frontier entries at
-  // once mixes pairs, and then each entry's pair is kept in sP (warp-uniform).
+  // Pair index of the deque's entries.  A deque is filled from one root pair,
+  // one queue item or frontier entries of one pair, and entries inherit their
+  // parent's pair, so it holds a single pair at any time (warp-uniform).
   uint32_t curP = 0;
-  bool mixed = false;
+  const uint32_t need = a.surface_filter ? SURF_BIT : 0u;  // word bits an emitted leaf pair has to share
 
   unsigned step = 0;
   for (;;) {
-    // Queue counters for the donation check, read early so that their
-    // latency overlaps the node loads of this step.
-    unsigned q_h = 0, q_t = 0;
-    ++step;
-    if ((step & 1023u) == 0u) fold_counts();
-    // warp-uniform: poll the queue counters on every (poll_mask + 1)-th step
-    // with work
-    const bool polled = top - bot >= 2 && (step & a.poll_mask) == 0u;
-    if (lane == 0 && polled) {
-      q_h = ld_volatile(&ctl->q_head);
-      q_t = ld_volatile(&ctl->q_tail);
-    }
-    // this step's pushes (entry words) and emitted leaf pairs (node words)
-    unsigned push_mask = 0, emit_mask = 0;
-    uint32_t pushA[SLOTS], pushB[SLOTS], slotP[SLOTS];
-
     if (top == bot) {
       // Work handed to the queue was counted before it was published, so the
       // release needs no fence.
@@ -241,125 +365,117 @@ __global__ void __launch_bounds__(512, (C * S >= 4) ? 1 : 2) traverse_kernel(Tra
         if (lane == 0) atomicSub(&ctl->work, release);
         release = 0;
       }
-      bool have = false;
-      mixed = false;  // the deque is empty
       if (!init_done) {
-        unsigned base = 0;
-        if (lane == 0) base = atomicAdd(&ctl->init_head, (unsigned)a.init_chunk);
-        base = __shfl_sync(0xffffffffu, base, 0);
-        if (base < n_init) {
-          int n = (int)min((unsigned)a.init_chunk, n_init - base);
-          release += n;
-          have = true;
-          uint32_t p0 = 0;
-          if (lane < n && a.entries) {
-            // a pending node pair of a frontier (its tests are counted already)
-            const uint4 e = a.entries[base + lane];
-            pushA[0] = e.x;
-            pushB[0] = e.y;
-            slotP[0] = e.z;
-            p0 = e.z;
-            push_mask = 1;
-          } else if (lane < n) {
-            // root test (kdop_tandem_traversal.h:164), then the traversal's own
-            // test of the root pair (:42), both counted as the reference does.
-            uint32_t pid = pair_base + base + lane;
+        uint2 r = s_claim[wib];
+        __syncwarp();
+        if (r.x == r.y) {
+          // a warp's first claim of seeded entries is its own share, later
+          // ones (and all claims of root pairs) come off the common counter
+          const unsigned n_init = ctl->n_init, warps = gridDim.x * (blockDim.x >> 5);
+          const unsigned first = a.seeded ? max(claim_size(n_init, warps), (unsigned)a.init_chunk) : 0u;
+          unsigned base, chunk;
+          if (a.seeded && r.y == 0u) {
+            chunk = first;
+            base = min((blockIdx.x * (blockDim.x >> 5) + wib) * first, n_init);
+          } else {
+            chunk = (unsigned)a.init_chunk;
+            if (a.seeded) chunk = max(chunk, claim_size(n_init - min(n_init, max(r.y, warps * first)), warps));
+            base = 0;
+            if (lane == 0) base = atomicAdd(&ctl->init_head, chunk);
+            base = min(__shfl_sync(0xffffffffu, base, 0) + warps * first, n_init);
+          }
+          init_done = base >= n_init;
+          r = make_uint2(base, min(base + chunk, n_init));
+        }
+        if (!init_done) {
+          if (a.entries) {
+            // pending node pairs of a frontier (their tests are counted
+            // already): the claim's leading run of one pair
+            const bool in = r.x + lane < r.y;
+            uint4 e = make_uint4(0u, 0u, 0u, 0u);
+            if (in) e = a.entries[r.x + lane];
+            curP = __shfl_sync(0xffffffffu, e.z, 0);
+            const unsigned same = __ballot_sync(0xffffffffu, in && e.z == curP);
+            const int run = (same == 0xffffffffu) ? 32 : __ffs(~same) - 1;
+            if (lane < run) sAB[(top + lane) & MASK] = make_uint2(e.x, e.y);
+            top += run;
+            release += run;
+            r.x += (unsigned)run;
+          } else {
+            // a root pair: the whole warp tests it, lane 0 counts and writes
+            uint32_t pid = ctl->pair_base + r.x;
             if (a.order) pid = a.order[pid];
-            p0 = pid;
-            uint2 mp = a.pairs[pid];
-            uint32_t ra = NO_NODE, rb = NO_NODE;
-            if (mp.x < a.n_meshes && mp.y < a.n_meshes) {
-              ra = a.root[mp.x];
-              rb = a.root[mp.y];
-            } else {
-              atomicOr(&ctl->error, DEV_ERR_BAD_INDEX);
-            }
-            if (ra != NO_NODE && rb != NO_NODE) {
-              uint32_t wa, wb;
-              bool ov = node_overlap<K>(a.nodes, ra, rb, wa, wb);
-              tests32 += 1u;
-              if (ov) {
-                tests32 += 1u;
-                pushA[0] = wa;
-                pushB[0] = wb;
-                slotP[0] = pid;
-                if (wa & wb & LEAF_BIT) {
-                  lo32 += 1u;
-                  if (!a.surface_filter || (wa & wb & SURF_BIT)) emit_mask = 1;
-                } else {
-                  push_mask = 1;
-                }
-              }
+            uint32_t wa = 0, wb = 0;
+            const bool expand = root_pair<K>(a, pid, lane == 0, wa, wb, tests32, lo32);
+            curP = pid;
+            release += 1;
+            r.x += 1u;
+            if (expand) {
+              if (lane == 0) sAB[top & MASK] = make_uint2(wa, wb);
+              top += 1;
             }
           }
-          if (n > 1)
-            mixed = true;  // entries of several pairs
-          else
-            curP = __shfl_sync(0xffffffffu, p0, 0);
-        } else {
-          init_done = true;
+          if (lane == 0) s_claim[wib] = r;
+          __syncwarp();
+          continue;
         }
       }
-      if (!have) {
-        // wait for a queue item or the end of all work
-        if (claim == 0xFFFFFFFFu) {
-          unsigned c = 0;
-          if (lane == 0) c = atomicAdd(&ctl->q_head, 1u);
-          claim = __shfl_sync(0xffffffffu, c, 0);
-        }
-        unsigned long long t0 = global_ns();
-        unsigned backoff = 64;
-        int got = 0;
-        for (unsigned it = 0;; ++it) {
-          if (claim < a.q_cap && ld_volatile(&a.q_tags[claim]) != 0u) {
-            got = 1;
-            break;
-          }
-          // the end-of-work counter is polled by every waiting warp: every
-          // 4th round only, to keep its line free for the workers' atomics
-          if ((it & 3u) == 0u && ld_volatile(&ctl->work) == 0) break;
-          if ((long long)(global_ns() - t0) > a.timeout_ns) {
-            failed = true;
-            break;
-          }
-          __nanosleep(backoff);
-          backoff = min(backoff * 2u, 2048u);
-        }
-        got = __shfl_sync(0xffffffffu, got, 0);
-        if (__shfl_sync(0xffffffffu, (int)failed, 0)) {
-          failed = true;
+      // wait for a queue item or the end of all work
+      if (claim == 0xFFFFFFFFu) {
+        unsigned c = 0;
+        if (lane == 0) c = atomicAdd(&ctl->q_head, 1u);
+        claim = __shfl_sync(0xffffffffu, c, 0);
+      }
+      unsigned long long t0 = global_ns();
+      unsigned backoff = 64;
+      int got = 0, failed = 0;
+      for (unsigned it = 0;; ++it) {
+        if (claim < a.q_cap && ld_volatile(&a.q_tags[claim]) != 0u) {
+          got = 1;
           break;
         }
-        if (!got) break;
-        __threadfence();
-        uint4 it = __ldcg(a.q_items + claim);
-        if (lane == 0) {
-          a.q_tags[claim] = 0u;
-          sAB[top & MASK] = make_uint2(it.x, it.y);
+        // the end-of-work counter is polled by every waiting warp: every
+        // 4th round only, to keep its line free for the workers' atomics
+        if ((it & 3u) == 0u && ld_volatile(&ctl->work) == 0) break;
+        if ((long long)(global_ns() - t0) > a.timeout_ns) {
+          failed = 1;
+          break;
         }
-        curP = it.z;  // the deque was empty: one pair
-        top += 1;
-        release += 1;
-        claim = 0xFFFFFFFFu;
-        __syncwarp();
-        continue;
+        __nanosleep(backoff);
+        backoff = min(backoff * 2u, 2048u);
       }
-    } else {
+      got = __shfl_sync(0xffffffffu, got, 0);
+      failed = __shfl_sync(0xffffffffu, failed, 0);
+      if (failed && lane == 0) atomicOr(&ctl->error, DEV_ERR_TIMEOUT);
+      if (failed || !got) break;
+      __threadfence();
+      uint4 it = __ldcg(a.q_items + claim);
+      if (lane == 0) {
+        a.q_tags[claim] = 0u;
+        sAB[top & MASK] = make_uint2(it.x, it.y);
+      }
+      curP = it.z;  // the deque was empty: one pair
+      top += 1;
+      release += 1;
+      claim = 0xFFFFFFFFu;
+      __syncwarp();
+      continue;
+    }
+
+    // ---- one step: expand up to E * S entries from the top of the deque ----
+    // this step's pushes (entry words) and emitted leaf pairs (node words)
+    bool push[SLOTS], emit[SLOTS];
+    uint32_t pushA[SLOTS], pushB[SLOTS];
+    {
       const int n = min(E * S, top - bot);
       top -= n;
       uint2 eab[S];
-      uint32_t ep[S];
       float4 A0[S][C], A1[S][C], B0[S][C], B1[S][C];
 #pragma unroll
       for (int b = 0; b < S; ++b) {
         const int i = b * E + ge;
         eab[b] = make_uint2(0u, 0u);
-        ep[b] = 0;
-        if (i < n) {
-          const int at = (top + i) & MASK;
-          eab[b] = sAB[at];
-          ep[b] = mixed ? sP[at] : curP;
-        }
+        if (i < n) eab[b] = sAB[(top + i) & MASK];
         const float4* pa = nodes_q + (size_t)((eab[b].x & NODE_MASK) >> 1) * (2 * NW);
         const float4* pb = nodes_q + (size_t)((eab[b].y & NODE_MASK) >> 1) * (2 * NW);
 #pragma unroll
@@ -378,101 +494,29 @@ __global__ void __launch_bounds__(512, (C * S >= 4) ? 1 : 2) traverse_kernel(Tra
       for (int b = 0; b < S; ++b) {
         const bool valid = b * E + ge < n;
         const uint32_t xa = eab[b].x, xb = eab[b].y;
-        const bool singleA = (xa & LEAF_BIT) != 0, singleB = (xb & LEAF_BIT) != 0;
-        // Separation of child pairs (0,0), (0,1), (1,0), (1,1).  A single
-        // side is the node itself, which is side (x & 1) of the twin just
-        // loaded: the pairs with the other side of that twin are absent and
-        // count as separated.
-        const bool noA0 = singleA && (xa & 1u), noA1 = singleA && !(xa & 1u);
-        const bool noB0 = singleB && (xb & 1u), noB1 = singleB && !(xb & 1u);
-        bool s0 = noA0 || noB0, s1 = noA0 || noB1, s2 = noA1 || noB0, s3 = noA1 || noB1;
-        uint32_t t0 = 0, t1 = 0, t2 = 0, t3 = 0;
-#pragma unroll
-        for (int r = 0; r < C; ++r) {
-          const int j = gq + Q * r;
-          const float4 a0 = A0[b][r], a1 = A1[b][r], b0 = B0[b][r], b1 = B1[b][r];
-          if (2 * j < L::NS) {
-            s0 = s0 || (a0.y < b0.x) || (b0.y < a0.x);
-            s1 = s1 || (a0.y < b1.x) || (b1.y < a0.x);
-            s2 = s2 || (a1.y < b0.x) || (b0.y < a1.x);
-            s3 = s3 || (a1.y < b1.x) || (b1.y < a1.x);
-          }
-          if (2 * j + 1 < L::NS) {
-            s0 = s0 || (a0.w < b0.z) || (b0.w < a0.z);
-            s1 = s1 || (a0.w < b1.z) || (b1.w < a0.z);
-            s2 = s2 || (a1.w < b0.z) || (b0.w < a1.z);
-            s3 = s3 || (a1.w < b1.z) || (b1.w < a1.z);
-          }
-          if (r == TR) {
-            t0 = L::word0(a0);
-            t1 = L::word0(a1);
-            t2 = L::word0(b0);
-            t3 = L::word0(b1);
-          }
-        }
-        unsigned sep = (s0 ? 1u : 0u) | (s1 ? 2u : 0u) | (s2 ? 4u : 0u) | (s3 ? 8u : 0u);
-#pragma unroll
-        for (int o = 1; o < Q; o <<= 1) sep |= __shfl_xor_sync(0xffffffffu, sep, o);
-        // word 0 of the four children, from the lane holding the topology chunk
-        const int src = ge * Q + TQ;
-        const uint32_t wA0 = __shfl_sync(0xffffffffu, t0, src);
-        const uint32_t wA1 = __shfl_sync(0xffffffffu, t1, src);
-        uint32_t wB0, wB1;
-        if (Q == 2) {
-          // lane gq only handles child gq of B (see below): the topology lane
-          // keeps its own word, the other lane gets the other child's
-          const uint32_t wo = __shfl_sync(0xffffffffu, TQ ? t2 : t3, src);
-          wB0 = wB1 = (gq == TQ) ? (TQ ? t3 : t2) : wo;
-        } else {
-          wB0 = __shfl_sync(0xffffffffu, t2, src);
-          wB1 = __shfl_sync(0xffffffffu, t3, src);
-        }
-        if (valid) {
-          if (gq == 0) tests32 += (singleA ? 1u : 2u) * (singleB ? 1u : 2u);
-          // the lane's child pairs c = gq + Q r (c = 2 i + k: child i of A,
-          // child k of B) as bit masks: overlapping, both leaves, both on
-          // the surface
-          unsigned alive = 0, leaf = 0, surf = 0;
-#pragma unroll
-          for (int r = 0; r < PM; ++r) {
-            const int c = gq + Q * r;
-            const int ci = (Q == 2) ? r : (c >> 1), ck = (Q == 2) ? gq : (c & 1);
-            const uint32_t wa = ci ? wA1 : wA0, wb = ck ? wB1 : wB0;
-            const uint32_t both = wa & wb;
-            const int k = b * PM + r;
-            pushA[k] = wa;
-            pushB[k] = wb;
-            slotP[k] = ep[b];
-            const bool ok = (Q * r + Q - 1 < 4 || c < 4) && !((sep >> c) & 1u);
-            alive |= (ok ? 1u : 0u) << r;
-            leaf |= (both >> 31) << r;
-            surf |= ((both >> 30) & 1u) << r;
-          }
-          if (!a.surface_filter) surf = ~0u;
-          lo32 += __popc(alive & leaf);  // both leaves
-          emit_mask |= (alive & leaf & surf) << (b * PM);
-          push_mask |= (alive & ~leaf & ((1u << PM) - 1u)) << (b * PM);
-        }
+        bool sep[4];
+        uint32_t words[4];
+        test_twins<K, C>(A0[b], A1[b], B0[b], B1[b], gq, sep, words);
+        child_pairs<K, C>(xa, xb, valid, sep, words, ge, gq, group_mask, need, push + b * PM, emit + b * PM,
+                          pushA + b * PM, pushB + b * PM, tests32, lo32);
       }
     }
 
     // ---- emits (rare): leaf pairs to candidate rows, one atomic per warp ----
-    if (__any_sync(0xffffffffu, emit_mask != 0u)) {
-      int tot_e = 0, off_e = 0;
-      warp_prefix<CBITS>(__popc(emit_mask), lt_mask, tot_e, off_e);
+    bool any_emit = false;
+#pragma unroll
+    for (int k = 0; k < SLOTS; ++k) any_emit |= emit[k];
+    if (__any_sync(0xffffffffu, any_emit)) {
+      int ne = 0, tot_e = 0, off_e = 0;
+#pragma unroll
+      for (int k = 0; k < SLOTS; ++k) ne += emit[k] ? 1 : 0;
+      warp_prefix<CBITS>(ne, lt_mask, tot_e, off_e);
       unsigned base = 0;
       if (lane == 0) base = atomicAdd(&ctl->n_cand, (unsigned)tot_e);
       base = __shfl_sync(0xffffffffu, base, 0) + (unsigned)off_e;
 #pragma unroll
       for (int k = 0; k < SLOTS; ++k) {
-        if (emit_mask & (1u << k)) {
-          if (base < a.cand_cap) {
-            a.candA[base] = leaf_tet<K>(a.nodes, pushA[k]);
-            a.candB[base] = leaf_tet<K>(a.nodes, pushB[k]);
-            a.candP[base] = slotP[k];
-          }
-          ++base;
-        }
+        if (emit[k]) put_candidate<K>(a, base++, pushA[k], pushB[k], curP);
       }
     }
     // ---- pushes: deque (or the global queue), slot-major: every lane's
@@ -484,76 +528,76 @@ __global__ void __launch_bounds__(512, (C * S >= 4) ? 1 : 2) traverse_kernel(Tra
       int tot_p = 0;
 #pragma unroll
       for (int k = 0; k < SLOTS; ++k) {
-        pm[k] = __ballot_sync(0xffffffffu, (push_mask >> k) & 1u);
+        pm[k] = __ballot_sync(0xffffffffu, push[k]);
         pbase[k] = tot_p;
         tot_p += __popc(pm[k]);
       }
-      if (tot_p) {
-        if (top - bot + tot_p <= CAP) {
+      if (top - bot + tot_p <= CAP) {
 #pragma unroll
-          for (int k = 0; k < SLOTS; ++k) {
-            if (push_mask & (1u << k)) {
-              const int at = (top + pbase[k] + __popc(pm[k] & lt_mask)) & MASK;
-              sAB[at] = make_uint2(pushA[k], pushB[k]);
-              if (mixed) sP[at] = slotP[k];
-            }
-          }
-          top += tot_p;
-        } else {
-          // deque full: the new entries go to the global queue
-          unsigned t0 = 0;
-          if (lane == 0) t0 = atomicAdd(&ctl->q_tail, (unsigned)tot_p);
-          t0 = __shfl_sync(0xffffffffu, t0, 0);
-          int room = (int)min((unsigned long long)tot_p,
-                              (t0 < a.q_cap) ? (unsigned long long)(a.q_cap - t0) : 0ull);
-          if (room < tot_p && lane == 0) atomicOr(&ctl->error, DEV_ERR_QUEUE_FULL);
-          if (room > 0 && lane == 0) atomicAdd(&ctl->work, room);
-          __syncwarp();
-#pragma unroll
-          for (int k = 0; k < SLOTS; ++k) {
-            const unsigned slot = t0 + (unsigned)(pbase[k] + __popc(pm[k] & lt_mask));
-            if ((push_mask & (1u << k)) && slot < t0 + (unsigned)room)
-              a.q_items[slot] = make_uint4(pushA[k], pushB[k], slotP[k], 0u);
-          }
-          __threadfence();
-          __syncwarp();
-#pragma unroll
-          for (int k = 0; k < SLOTS; ++k) {
-            const unsigned slot = t0 + (unsigned)(pbase[k] + __popc(pm[k] & lt_mask));
-            if ((push_mask & (1u << k)) && slot < t0 + (unsigned)room) atomicExch(&a.q_tags[slot], 1u);
-          }
-        }
-      }
-    }
-    int depth = top - bot;
-    if (polled && (unsigned)depth > max_depth) max_depth = (unsigned)depth;
-
-    // ---- donation: give the oldest entries to waiting warps ----
-    // A deep deque gives to any waiting warp; while many warps wait (the
-    // tail of the traversal) any deque with two or more entries gives half.
-    if (polled && depth >= 2) {
-      int waiting = 0;
-      if (lane == 0) waiting = (q_h > q_t) ? (int)min(q_h - q_t, 1024u) : 0;
-      waiting = __shfl_sync(0xffffffffu, waiting, 0);
-      int d = (depth >= a.donate_min || waiting >= kTailWaiting) ? min(min(waiting, 32), depth / 2) : 0;
-      if (d > 0) {
+        for (int k = 0; k < SLOTS; ++k)
+          if (push[k])
+            sAB[(top + pbase[k] + __popc(pm[k] & lt_mask)) & MASK] = make_uint2(pushA[k], pushB[k]);
+        top += tot_p;
+      } else {
+        // deque full: the new entries go to the global queue
         unsigned t0 = 0;
-        if (lane == 0) t0 = atomicAdd(&ctl->q_tail, (unsigned)d);
+        if (lane == 0) t0 = atomicAdd(&ctl->q_tail, (unsigned)tot_p);
         t0 = __shfl_sync(0xffffffffu, t0, 0);
-        int room = (int)min((unsigned long long)d, (t0 < a.q_cap) ? (unsigned long long)(a.q_cap - t0) : 0ull);
-        if (room < d && lane == 0) atomicOr(&ctl->error, DEV_ERR_QUEUE_FULL);
+        int room = (int)min((unsigned long long)tot_p,
+                            (t0 < a.q_cap) ? (unsigned long long)(a.q_cap - t0) : 0ull);
+        if (room < tot_p && lane == 0) atomicOr(&ctl->error, DEV_ERR_QUEUE_FULL);
         if (room > 0 && lane == 0) atomicAdd(&ctl->work, room);
         __syncwarp();
-        if (lane < room) {
-          int at = (bot + lane) & MASK;
-          uint2 ab = sAB[at];
-          a.q_items[t0 + lane] = make_uint4(ab.x, ab.y, mixed ? sP[at] : curP, 0u);
+#pragma unroll
+        for (int k = 0; k < SLOTS; ++k) {
+          const unsigned slot = t0 + (unsigned)(pbase[k] + __popc(pm[k] & lt_mask));
+          if (push[k] && slot < t0 + (unsigned)room) a.q_items[slot] = make_uint4(pushA[k], pushB[k], curP, 0u);
         }
         __threadfence();
         __syncwarp();
-        if (lane < room) atomicExch(&a.q_tags[t0 + lane], 1u);
-        // entries that found no room stay lost only with DEV_ERR_QUEUE_FULL set
-        bot += d;
+#pragma unroll
+        for (int k = 0; k < SLOTS; ++k) {
+          const unsigned slot = t0 + (unsigned)(pbase[k] + __popc(pm[k] & lt_mask));
+          if (push[k] && slot < t0 + (unsigned)room) atomicExch(&a.q_tags[slot], 1u);
+        }
+      }
+    }
+
+    // ---- donation: give the oldest entries to waiting warps ----
+    // The queue counters are polled on every (poll_mask + 1)-th step.  A deep
+    // deque gives to any waiting warp; while many warps wait (the tail of the
+    // traversal) any deque with two or more entries gives half.
+    ++step;
+    if ((step & a.poll_mask) == 0u) {
+      if ((step & 1023u) == 0u) fold_counts();
+      const int depth = top - bot;
+      if (depth >= 2) {
+        int waiting = 0;
+        if (lane == 0) {
+          const unsigned q_h = ld_volatile(&ctl->q_head), q_t = ld_volatile(&ctl->q_tail);
+          waiting = (q_h > q_t) ? (int)min(q_h - q_t, 1024u) : 0;
+        }
+        waiting = __shfl_sync(0xffffffffu, waiting, 0);
+        int d = (depth >= a.donate_min || waiting >= kTailWaiting) ? min(min(waiting, 32), depth / 2) : 0;
+        if (d > 0) {
+          __syncwarp();  // this step's pushes, before other lanes read them
+          unsigned t0 = 0;
+          if (lane == 0) t0 = atomicAdd(&ctl->q_tail, (unsigned)d);
+          t0 = __shfl_sync(0xffffffffu, t0, 0);
+          int room = (int)min((unsigned long long)d, (t0 < a.q_cap) ? (unsigned long long)(a.q_cap - t0) : 0ull);
+          if (room < d && lane == 0) atomicOr(&ctl->error, DEV_ERR_QUEUE_FULL);
+          if (room > 0 && lane == 0) atomicAdd(&ctl->work, room);
+          __syncwarp();
+          if (lane < room) {
+            uint2 ab = sAB[(bot + lane) & MASK];
+            a.q_items[t0 + lane] = make_uint4(ab.x, ab.y, curP, 0u);
+          }
+          __threadfence();
+          __syncwarp();
+          if (lane < room) atomicExch(&a.q_tags[t0 + lane], 1u);
+          // entries that found no room stay lost only with DEV_ERR_QUEUE_FULL set
+          bot += d;
+        }
       }
     }
     __syncwarp();
@@ -561,9 +605,168 @@ __global__ void __launch_bounds__(512, (C * S >= 4) ? 1 : 2) traverse_kernel(Tra
 
   // ---- totals ----
   fold_counts();
+}
+
+// ---- seed pass ----------------------------------------------------------------
+// Breadth-first expansion of the top of the node-pair trees, so that the
+// persistent traversal starts from thousands of node pairs instead of the root
+// pairs.  Starting from few roots, the traversal hands work on through the
+// global queue one donation at a time, a chain of atomics, polls and record
+// loads per generation: a launch of one pair of 6,000 tets spent most of its
+// 149 us on that, with 4,700 of its 4,736 warps waiting.  Here a block takes
+// `group` pairs (their root tests one per thread) or, in the second pass,
+// an even share of the first pass's node pairs, and expands them level by
+// level in shared memory until at least kSeedStop are pending, which it
+// appends to the frontier; a block whose pairs end earlier leaves nothing.
+// The traversal claims the frontier's entries in order.  Tests, leaf pairs
+// and candidates are those of the same expansions done by the traversal.
+// Measured, whole traversal call without -> with this pass and the loop below:
+// one pair of 6,000 tets 149 -> 81 us, of 24,576 tets in touch 138 -> 51 us,
+// 64 deforming pairs of 384 k tets 1,027 -> 477 us, 256 touching pairs of 48 k
+// tets 668 -> 435 us.  Stopping at 128 or 1024 pending pairs instead of 512:
+// 537 and 578 us on the 64 pairs, 490 and 472 us on the 256.
+constexpr unsigned kSeedStop = 512;
+constexpr unsigned kSeedCap = 4 * kSeedStop;  // most a level of fewer than kSeedStop pairs leaves
+constexpr int kSeedThreads = 512;
+constexpr int64_t kSeedTwiceMax = 64;
+
+// Pairs per block of the first pass: four blocks per SM until a group fills
+// a block's list.
+static int64_t seed_group(int sm_count, int64_t n_pairs) {
+  const int64_t blocks = 4 * (int64_t)sm_count;
+  return std::min<int64_t>(std::max<int64_t>((n_pairs + blocks - 1) / blocks, 1), kSeedCap);
+}
+// Few pairs leave too few node pairs for 4,736 warps after one pass: they are
+// expanded once more, over two blocks per SM (one pair of 1.6 M tets 1,250 us
+// with one pass, 1,022 with two; 64 pairs 601 and 560 us, 256 pairs 455 and
+// 471 us, each against the same loop).
+static int seed_blocks2(int sm_count, int64_t n_pairs) { return n_pairs <= kSeedTwiceMax ? 2 * sm_count : 0; }
+
+// Entries the first pass can leave: kSeedCap per group of pairs.
+static int64_t seed_entries1(int sm_count, int64_t n) {
+  return std::max(std::min<int64_t>(n, 4 * (int64_t)sm_count), (n + kSeedCap - 1) / kSeedCap) * kSeedCap;
+}
+int64_t seed_entries(int sm_count, int64_t n) {
+  return seed_entries1(sm_count, n) + (int64_t)seed_blocks2(sm_count, 1) * kSeedCap;
+}
+
+template <int K>
+__global__ void __launch_bounds__(kSeedThreads) seed_kernel(TravArgs a, unsigned n_pairs, unsigned group,
+                                                            const uint4* __restrict__ in,
+                                                            const unsigned* __restrict__ in_count, uint4* out,
+                                                            unsigned* out_count) {
+  constexpr int C = 2;
+  using CP = Coop<K, C>;
+  constexpr int NW = NodeLayout<K>::NW, Q = CP::Q, E = CP::E, PM = CP::PM;
+  extern __shared__ uint32_t smem[];
+  __shared__ unsigned cnt[2], flush_at;
+  // two lists of (A, B) words and of pair indices, read and written in turn
+  uint2* const AB = reinterpret_cast<uint2*>(smem);
+  uint32_t* const P = smem + 4 * kSeedCap;
+  const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5, nw = blockDim.x >> 5;
+  const unsigned lt_mask = (1u << lane) - 1u;
+  const int ge = lane / Q, gq = lane % Q;
+  const unsigned group_mask = ((1u << Q) - 1u) << (ge * Q);
+  const float4* __restrict__ nodes_q = a.nodes + 2 * gq;
+  const uint32_t need = a.surface_filter ? SURF_BIT : 0u;
+  TravCtl* ctl = a.ctl;
+  unsigned tests32 = 0, lo32 = 0;
+  unsigned n_src = n_pairs;
+  if (in) {
+    n_src = *in_count;
+    group = min((n_src + gridDim.x - 1) / gridDim.x, kSeedCap);
+  }
+  for (unsigned long long base = (unsigned long long)blockIdx.x * group; base < n_src;
+       base += (unsigned long long)gridDim.x * group) {
+    const unsigned n = (unsigned)min((unsigned long long)group, n_src - base);
+    if (threadIdx.x < 2) cnt[threadIdx.x] = (in && threadIdx.x == 0) ? n : 0u;
+    __syncthreads();
+    for (unsigned i = threadIdx.x; i < n; i += blockDim.x) {
+      if (in) {
+        const uint4 e = in[base + i];
+        AB[i] = make_uint2(e.x, e.y);
+        P[i] = e.z;
+      } else {
+        const uint32_t pid = a.order[base + i];
+        uint32_t wa = 0, wb = 0;
+        if (root_pair<K>(a, pid, true, wa, wb, tests32, lo32)) {
+          const unsigned at = atomicAdd(&cnt[0], 1u);
+          AB[at] = make_uint2(wa, wb);
+          P[at] = pid;
+        }
+      }
+    }
+    __syncthreads();
+    unsigned cur = 0, c = cnt[0];
+    while (c > 0 && c < kSeedStop) {
+      const unsigned nx = cur ^ 1u;
+      for (unsigned i0 = wib * E; i0 < c; i0 += nw * E) {
+        const unsigned i = i0 + ge;
+        const bool valid = i < c;
+        const uint2 x = valid ? AB[cur * kSeedCap + i] : make_uint2(0u, 0u);
+        const uint32_t pid = valid ? P[cur * kSeedCap + i] : 0u;
+        const float4* pa = nodes_q + (size_t)((x.x & NODE_MASK) >> 1) * (2 * NW);
+        const float4* pb = nodes_q + (size_t)((x.y & NODE_MASK) >> 1) * (2 * NW);
+        float4 A0[C], A1[C], B0[C], B1[C];
+#pragma unroll
+        for (int r = 0; r < C; ++r)
+          if (gq + Q * r < NW) {
+            ldg256(pa + 2 * Q * r, A0[r], A1[r]);
+            ldg256(pb + 2 * Q * r, B0[r], B1[r]);
+          }
+        bool sep[4], push[PM], emit[PM];
+        uint32_t words[4], pa_w[PM], pb_w[PM];
+        test_twins<K, C>(A0, A1, B0, B1, gq, sep, words);
+        child_pairs<K, C>(x.x, x.y, valid, sep, words, ge, gq, group_mask, need, push, emit, pa_w, pb_w, tests32,
+                          lo32);
+#pragma unroll
+        for (int r = 0; r < PM; ++r) {
+          const unsigned pm = __ballot_sync(0xffffffffu, push[r]);
+          if (pm) {
+            unsigned at = 0;
+            if (lane == 0) at = atomicAdd(&cnt[nx], (unsigned)__popc(pm));
+            at = __shfl_sync(0xffffffffu, at, 0) + __popc(pm & lt_mask);
+            if (push[r]) {
+              AB[nx * kSeedCap + at] = make_uint2(pa_w[r], pb_w[r]);
+              P[nx * kSeedCap + at] = pid;
+            }
+          }
+          const unsigned em = __ballot_sync(0xffffffffu, emit[r]);
+          if (em) {
+            unsigned at = 0;
+            if (lane == 0) at = atomicAdd(&ctl->n_cand, (unsigned)__popc(em));
+            at = __shfl_sync(0xffffffffu, at, 0) + __popc(em & lt_mask);
+            if (emit[r]) put_candidate<K>(a, at, pa_w[r], pb_w[r], pid);
+          }
+        }
+      }
+      __syncthreads();
+      cur = nx;
+      c = cnt[cur];
+      if (threadIdx.x == 0) cnt[cur ^ 1u] = 0;
+      __syncthreads();
+    }
+    if (c > 0) {
+      if (threadIdx.x == 0) {
+        flush_at = atomicAdd(out_count, c);
+        if (out_count == &ctl->n_init) atomicAdd(&ctl->work, (int)c);  // the traversal's work units
+      }
+      __syncthreads();
+      for (unsigned i = threadIdx.x; i < c; i += blockDim.x) {
+        const uint2 x = AB[cur * kSeedCap + i];
+        out[flush_at + i] = make_uint4(x.x, x.y, P[cur * kSeedCap + i], 0u);
+      }
+    }
+    __syncthreads();
+  }
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) {
+    tests32 += __shfl_down_sync(0xffffffffu, tests32, o);
+    lo32 += __shfl_down_sync(0xffffffffu, lo32, o);
+  }
   if (lane == 0) {
-    atomicMax(&ctl->max_stack, max_depth);
-    if (failed) atomicOr(&ctl->error, DEV_ERR_TIMEOUT);
+    if (tests32) atomicAdd(&ctl->tests, (unsigned long long)tests32);
+    if (lo32) atomicAdd(&ctl->leaf_overlaps, (unsigned long long)lo32);
   }
 }
 
@@ -574,7 +777,7 @@ __global__ void trav_init_kernel(TravCtl* c, unsigned n_init, unsigned pair_base
     c->leaf_overlaps = 0;
     c->n_cand = 0;
     c->error = 0;
-    c->max_stack = 0;
+    c->n_seed = 0;
     c->n_contacts = 0;
   }
   c->init_head = 0;
@@ -587,7 +790,7 @@ __global__ void trav_init_kernel(TravCtl* c, unsigned n_init, unsigned pair_base
 
 int traverse_block_threads(int block_warps) { return 32 * block_warps; }
 size_t traverse_smem_bytes(int block_warps, int stack_cap) {
-  return (size_t)block_warps * 3 * (size_t)stack_cap * sizeof(uint32_t);
+  return (size_t)block_warps * (size_t)stack_cap * sizeof(uint2);
 }
 
 template <int K>
@@ -621,7 +824,7 @@ static cudaError_t traverse_impl(kdop_scene* s, int64_t n_pairs, const TravBuffe
   cudaStream_t st = s->ctx->stream;
   int threads = traverse_block_threads(p.block_warps);
   size_t smem = traverse_smem_bytes(p.block_warps, p.stack_cap);
-  cudaError_t e = prepare_k<K>(smem);
+  cudaError_t e = cudaFuncSetAttribute(traverse_kernel<K, C, S>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   if (e != cudaSuccess) return e;
   e = cudaFuncSetAttribute(traverse_kernel<K, C, S>, cudaFuncAttributePreferredSharedMemoryCarveout,
                            p.smem_carveout > 0 ? p.smem_carveout : -1);
@@ -658,6 +861,29 @@ static cudaError_t traverse_impl(kdop_scene* s, int64_t n_pairs, const TravBuffe
   // waiting for donations and polls every 4th step (config 3, one launch per
   // pair: 88 ms vs 103 ms every 16th).
   a.poll_mask = plain ? 3u : 15u;
+  a.seeded = 0;
+  a.stuck = p.stuck_work;
+  if (b.seeds && !plain && p.wave_pairs <= 0 && n_pairs > 0) {
+    const int sms = s->ctx->sm_count;
+    const int64_t group = seed_group(sms, n_pairs), groups = (n_pairs + group - 1) / group;
+    const unsigned blocks2 = (unsigned)seed_blocks2(sms, n_pairs);
+    constexpr size_t seed_smem = kSeedCap * 24;
+    e = cudaFuncSetAttribute(seed_kernel<K>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)seed_smem);
+    if (e != cudaSuccess) return e;
+    uint4* seeds2 = b.seeds + seed_entries1(sms, n_pairs);
+    trav_init_kernel<<<1, 32, 0, st>>>(b.ctl, 0u, 0u, 1, p.stuck_work);
+    seed_kernel<K><<<(unsigned)std::min<int64_t>(groups, 4 * sms), kSeedThreads, seed_smem, st>>>(
+        a, (unsigned)n_pairs, (unsigned)group, nullptr, nullptr, b.seeds,
+        blocks2 ? &b.ctl->n_seed : &b.ctl->n_init);
+    if (blocks2)
+      seed_kernel<K><<<blocks2, kSeedThreads, seed_smem, st>>>(a, 0u, 0u, b.seeds, &b.ctl->n_seed, seeds2,
+                                                              &b.ctl->n_init);
+    a.entries = blocks2 ? seeds2 : b.seeds;
+    a.seeded = 1;
+    traverse_kernel<K, C, S><<<grid, threads, smem, st>>>(a);
+    s->ctx->launches += blocks2 ? 4 : 3;
+    return cudaGetLastError();
+  }
   if (b.entries) {
     // seeded by a frontier: its tests and leaf pairs are in the totals already
     trav_init_kernel<<<1, 32, 0, st>>>(b.ctl, (unsigned)n_pairs, 0u, 0, p.stuck_work);
@@ -723,6 +949,7 @@ cudaError_t launch_traverse(kdop_scene* s, int64_t n_pairs, const uint2* pairs, 
   TravBuffers b;
   b.pairs = pairs;
   b.order = s->pair_order;
+  b.seeds = s->seeds;
   b.cand = s->cand;
   b.cand_cap = s->cand_cap;
   b.q_items = s->q_items;
