@@ -20,7 +20,7 @@
 #include <cstring>
 
 #include "kdop_device.cuh"
-#include "kdop_sort.h"
+#include "kdop_sort.cuh"
 
 namespace kdop {
 
@@ -107,28 +107,34 @@ __device__ __forceinline__ uint64_t spread3(uint64_t x) {
   return x;
 }
 
-// code = interleave(x, y, z) with x on bit 3k, y on 3k + 1, z on 3k + 2
-__global__ void codes_kernel(const uint4* __restrict__ tets, const float4* __restrict__ rest, int64_t nt,
-                             const MortonParam* __restrict__ prm, uint64_t* codes, uint64_t* keys, uint32_t* vals) {
-  int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (t >= nt) return;
-  uint4 q = __ldg(tets + t);
-  MortonParam p = prm[mesh_of(rest, q.x)];
-  f3 c = centroid(rest, q);
-  uint64_t x = (uint64_t)(float)__float2int_rz(fmul(fsub(c.x, p.mn[0]), p.scale));
-  uint64_t y = (uint64_t)(float)__float2int_rz(fmul(fsub(c.y, p.mn[1]), p.scale));
-  uint64_t z = (uint64_t)(float)__float2int_rz(fmul(fsub(c.z, p.mn[2]), p.scale));
-  uint64_t code = spread3(x) | (spread3(y) << 1) | (spread3(z) << 2);
-  codes[t] = code;
-  keys[t] = code;
-  vals[t] = (uint32_t)t;
-}
-
-__global__ void mesh_keys_kernel(const uint4* __restrict__ tets, const float4* __restrict__ rest,
-                                 const uint32_t* __restrict__ vals, int64_t nt, uint64_t* keys) {
-  int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (i < nt) keys[i] = (uint64_t)(uint32_t)mesh_of(rest, __ldg(tets + vals[i]).x);
-}
+// Sort key of a tet: code = interleave(x, y, z) with x on bit 3k, y on 3k + 1,
+// z on 3k + 2; the codes also go to an array of their own.
+struct CodeGen {
+  const uint4* tets;
+  const float4* rest;
+  const MortonParam* prm;
+  uint64_t* codes;
+  __device__ uint64_t key(int64_t t) const {
+    uint4 q = __ldg(tets + t);
+    MortonParam p = prm[mesh_of(rest, q.x)];
+    f3 c = centroid(rest, q);
+    uint64_t x = (uint64_t)(float)__float2int_rz(fmul(fsub(c.x, p.mn[0]), p.scale));
+    uint64_t y = (uint64_t)(float)__float2int_rz(fmul(fsub(c.y, p.mn[1]), p.scale));
+    uint64_t z = (uint64_t)(float)__float2int_rz(fmul(fsub(c.z, p.mn[2]), p.scale));
+    uint64_t code = spread3(x) | (spread3(y) << 1) | (spread3(z) << 2);
+    codes[t] = code;
+    return code;
+  }
+  __device__ uint32_t val(int64_t t) const { return (uint32_t)t; }
+};
+// Mesh of a tet in code order: the second, stable sort groups the meshes.
+struct MeshGen {
+  const uint4* tets;
+  const float4* rest;
+  const uint32_t* order;
+  __device__ uint64_t key(int64_t i) const { return (uint64_t)(uint32_t)mesh_of(rest, __ldg(tets + order[i]).x); }
+  __device__ uint32_t val(int64_t i) const { return order[i]; }
+};
 
 // equal neighbouring codes within a mesh
 __global__ void ties_kernel(const uint4* __restrict__ tets, const float4* __restrict__ rest,
@@ -248,7 +254,7 @@ cudaError_t device_morton_perm(kdop_scene* s, uint32_t* perm, std::vector<char>&
   const int nm = s->n_meshes;
   need_host.assign((size_t)nm, 0);
   if (nt <= 0) return cudaSuccess;
-  // scratch: mm (6 nm words) | tied (nm) | params (nm) | codes, keys, keys_tmp (nt u64) | vals_tmp (nt) | radix
+  // scratch: mm (6 nm words) | tied (nm), error word | params (nm) | codes, keys, keys_tmp (nt u64) | vals_tmp (nt) | radix
   const size_t radix_words = radix_scratch_words(nt);
   size_t bytes = 0;
   auto take = [&](size_t b) {
@@ -256,7 +262,7 @@ cudaError_t device_morton_perm(kdop_scene* s, uint32_t* perm, std::vector<char>&
     bytes += (b + 255) & ~(size_t)255;
     return o;
   };
-  const size_t o_mm = take((size_t)6 * nm * 4), o_tied = take((size_t)nm * 4),
+  const size_t o_mm = take((size_t)6 * nm * 4), o_tied = take((size_t)nm * 4 + 4),
                o_prm = take((size_t)nm * sizeof(MortonParam)), o_codes = take((size_t)nt * 8),
                o_keys = take((size_t)nt * 8), o_ktmp = take((size_t)nt * 8), o_vtmp = take((size_t)nt * 4),
                o_rad = take(radix_words * 4);
@@ -267,10 +273,9 @@ cudaError_t device_morton_perm(kdop_scene* s, uint32_t* perm, std::vector<char>&
   uint32_t* tied = reinterpret_cast<uint32_t*>(w + o_tied);
   MortonParam* prm = reinterpret_cast<MortonParam*>(w + o_prm);
   uint64_t* codes = reinterpret_cast<uint64_t*>(w + o_codes);
-  uint64_t* keys = reinterpret_cast<uint64_t*>(w + o_keys);
-  uint64_t* ktmp = reinterpret_cast<uint64_t*>(w + o_ktmp);
-  uint32_t* vtmp = reinterpret_cast<uint32_t*>(w + o_vtmp);
-  uint32_t* rad = reinterpret_cast<uint32_t*>(w + o_rad);
+  SortBuffers b{reinterpret_cast<uint64_t*>(w + o_keys), reinterpret_cast<uint64_t*>(w + o_ktmp),
+                perm, reinterpret_cast<uint32_t*>(w + o_vtmp)};
+  unsigned* err = tied + nm;
   const unsigned g = (unsigned)((nt + 255) / 256);
   do {
     bounds_init_kernel<<<(6 * nm + 255) / 256, 256, 0, st>>>(mm, nm);
@@ -296,19 +301,24 @@ cudaError_t device_morton_perm(kdop_scene* s, uint32_t* perm, std::vector<char>&
     if ((e = cudaMemcpyAsync(prm, hp.data(), (size_t)nm * sizeof(MortonParam), cudaMemcpyHostToDevice, st)) !=
         cudaSuccess)
       break;
-    codes_kernel<<<g, 256, 0, st>>>(s->tets, s->rest, nt, prm, codes, keys, perm);
-    if ((e = radix_sort_pairs(keys, perm, ktmp, vtmp, nt, rad, st)) != cudaSuccess) break;
-    mesh_keys_kernel<<<g, 256, 0, st>>>(s->tets, s->rest, perm, nt, keys);
-    if ((e = radix_sort_pairs(keys, perm, ktmp, vtmp, nt, rad, st)) != cudaSuccess) break;
-    if ((e = cudaMemsetAsync(tied, 0, (size_t)nm * 4, st)) != cudaSuccess) break;
+    if ((e = cudaMemsetAsync(tied, 0, (size_t)nm * 4 + 4, st)) != cudaSuccess) break;
+    if ((e = radix_sort(CodeGen{s->tets, s->rest, prm, codes}, nt, 63, b, w + o_rad, err, st, s->ctx->launches)) !=
+        cudaSuccess)
+      break;
+    if ((e = radix_sort(MeshGen{s->tets, s->rest, b.vals}, nt, bits_of(nm - 1), b, w + o_rad, err, st,
+                        s->ctx->launches)) != cudaSuccess)
+      break;
+    if (b.vals != perm &&
+        (e = cudaMemcpyAsync(perm, b.vals, (size_t)nt * 4, cudaMemcpyDeviceToDevice, st)) != cudaSuccess)
+      break;
     ties_kernel<<<g, 256, 0, st>>>(s->tets, s->rest, perm, codes, nt, tied);
-    std::vector<uint32_t> ht((size_t)nm);
-    if ((e = cudaMemcpyAsync(ht.data(), tied, (size_t)nm * 4, cudaMemcpyDeviceToHost, st)) != cudaSuccess) break;
+    std::vector<uint32_t> ht((size_t)nm + 1);
+    if ((e = cudaMemcpyAsync(ht.data(), tied, (size_t)nm * 4 + 4, cudaMemcpyDeviceToHost, st)) != cudaSuccess) break;
     if ((e = cudaStreamSynchronize(st)) != cudaSuccess) break;
     for (int m = 0; m < nm; ++m)
       if (ht[m]) need_host[m] = 1;
-    s->ctx->launches += 7;
-    e = cudaGetLastError();
+    s->ctx->launches += 3;
+    e = ht[nm] ? cudaErrorLaunchTimeout : cudaGetLastError();
   } while (0);
   cudaStreamSynchronize(st);
   cudaFree(w);

@@ -84,6 +84,7 @@ struct kdop_scene_ext {
   std::vector<uint32_t> order_host;  // their order of processing
   int64_t graph_kernels = 0;
   int graph_refit_mode = 0;  // refit mode of the captured step
+  int64_t graph_pairs = 0;   // pairs of the captured step
   kdop_traverse_opts tuned{};
   bool has_tuned = false;
 };
@@ -219,6 +220,7 @@ static void scene_free(kdop_scene* s) {
   dfree(s, &s->nodes, s->nn * s->NW);
   if (s->root_dev) cudaFree(s->root_dev);
   s->root_dev = nullptr;
+  dfree(s, &s->t_off_dev, s->n_meshes + 1);
   dfree(s, &s->quat, s->n_meshes);
   dfree(s, &s->pos, s->n_meshes);
   dfree(s, &s->lin_vel, s->n_meshes);
@@ -439,6 +441,9 @@ int kdop_scene_create_ex(kdop_ctx* ctx, int K, int n_meshes, const kdop_mesh_des
     size_t root_bytes = (size_t)n_meshes * 4;
     SC_TRY(cudaMalloc((void**)&s->root_dev, std::max<size_t>(root_bytes, 8)));
     s->device_bytes += (int64_t)root_bytes;
+    SC_TRY(dalloc(s, &s->t_off_dev, n_meshes + 1));
+    std::vector<uint32_t> toff(s->t_off.begin(), s->t_off.end());
+    SC_TRY(cudaMemcpyAsync(s->t_off_dev, toff.data(), toff.size() * 4, cudaMemcpyHostToDevice, st));
     SC_TRY(dalloc(s, &s->quat, n_meshes));
     SC_TRY(dalloc(s, &s->pos, n_meshes));
     SC_TRY(dalloc(s, &s->lin_vel, n_meshes));
@@ -771,6 +776,7 @@ static int upload_pairs(kdop_scene* s, int64_t n, const uint32_t* pairs, int mem
   kdop_scene_ext* x = ext(s);
   int rc = grow_pairs(s, std::max<int64_t>(n, 1));
   if (rc != KDOP_OK) return rc;
+  s->pairs_current = false;  // until a traversal of this list is enqueued
   if (n == 0) {
     x->pairs_host.clear();
     return KDOP_OK;
@@ -816,7 +822,8 @@ int kdop_traverse(kdop_scene* s, int64_t n_pairs, const uint32_t* pairs, int mem
   KDOP_CUDA(s->ctx, kdop::launch_traverse(s, n_pairs, s->pairs, p, mode == KDOP_TRAVERSE_PLAIN));
   s->traversed = true;
   s->contacted = false;
-  s->last_pairs = n_pairs;
+  s->last_pairs = s->result_pairs = n_pairs;
+  s->pairs_current = true;
   s->last_mode = mode;
   s->last_params = p;
   return KDOP_OK;
@@ -894,7 +901,8 @@ int kdop_traverse_shard(kdop_scene* s, int64_t n_pairs, const uint32_t* pairs, i
   if (e != cudaSuccess) return cuda_fail(s->ctx, e, "kdop_traverse_shard");
   s->traversed = true;
   s->contacted = false;
-  s->last_pairs = n_pairs;
+  s->last_pairs = s->result_pairs = n_pairs;
+  s->pairs_current = true;
   s->last_mode = mode;
   s->last_params = p;
   return KDOP_OK;
@@ -1020,7 +1028,9 @@ int kdop_sort_results(kdop_scene* s) {
     s->device_bytes += (int64_t)need;
   }
   KDOP_CUDA(s->ctx, kdop::sort_results(s, n, nc, x->sort_work, s->ctx->stream));
+  KDOP_CUDA(s->ctx, cudaMemcpyAsync(s->ctl_host, s->ctl, sizeof(TravCtl), cudaMemcpyDeviceToHost, s->ctx->stream));
   KDOP_CUDA(s->ctx, cudaStreamSynchronize(s->ctx->stream));
+  if (s->ctl_host->error & kdop::DEV_ERR_TIMEOUT) return fail(s->ctx, KDOP_ERR_TIMEOUT, "sort wait timed out");
   return KDOP_OK;
 }
 
@@ -1079,15 +1089,16 @@ static size_t reduce_rows_bytes(int64_t n) {
 // Reduces n device rows with their device bodies in `buf` (reduce_rows_bytes(n)
 // bytes), then copies the kept rows (and bodies) to the caller's buffers
 // (host or device).
-static int reduce_rows(kdop_ctx* ctx, const kdop_contact* rows, const uint2* bodies, int64_t n, char* buf,
-                       kdop_contact* out, uint32_t* out_bodies, int64_t cap, int64_t* n_out) {
+// n_bodies: bound of the body numbers, 0 when unknown.
+static int reduce_rows(kdop_ctx* ctx, const kdop_contact* rows, const uint2* bodies, int64_t n, int64_t n_bodies,
+                       char* buf, kdop_contact* out, uint32_t* out_bodies, int64_t cap, int64_t* n_out) {
   const size_t m = (size_t)std::max<int64_t>(n, 1);
   const size_t wb = align256(kdop::reduce_work_bytes(n));
   const size_t rb = align256(m * sizeof(kdop_contact));
   kdop_contact* kept_rows = reinterpret_cast<kdop_contact*>(buf + wb);
   uint2* kept_bodies = reinterpret_cast<uint2*>(buf + wb + rb);
   int64_t kept = 0;
-  cudaError_t e = kdop::reduce_contact_rows(ctx, rows, bodies, n, buf, kept_rows, kept_bodies, &kept);
+  cudaError_t e = kdop::reduce_contact_rows(ctx, rows, bodies, n, n_bodies, buf, kept_rows, kept_bodies, &kept);
   *n_out = kept;
   if (e != cudaSuccess) return cuda_fail(ctx, e, "reduce_contact_rows");
   if (kept > cap) return fail(ctx, KDOP_ERR_CAPACITY, "reduced contact buffer too small");
@@ -1120,7 +1131,7 @@ int kdop_reduce_contact_rows(kdop_ctx* ctx, const kdop_contact* rows, const uint
     cudaStreamSynchronize(ctx->stream);  // a started copy may still read the caller's rows
     return cuda_fail(ctx, e, "reduce input copy");
   }
-  return reduce_rows(ctx, reinterpret_cast<kdop_contact*>(in), reinterpret_cast<uint2*>(in + rb), n, in + rb + bb,
+  return reduce_rows(ctx, reinterpret_cast<kdop_contact*>(in), reinterpret_cast<uint2*>(in + rb), n, 0, in + rb + bb,
                      out, out_bodies, cap, n_out);
 }
 
@@ -1140,7 +1151,7 @@ int kdop_reduce_contacts(kdop_scene* s, kdop_contact* out, uint32_t* out_bodies,
   uint2* bodies = reinterpret_cast<uint2*>(buf);
   cudaError_t e = kdop::scene_contact_bodies(s, n, bodies);
   if (e != cudaSuccess) return cuda_fail(s->ctx, e, "scene_contact_bodies");
-  return reduce_rows(s->ctx, s->contacts, bodies, n, buf + bb, out, out_bodies, cap, n_out);
+  return reduce_rows(s->ctx, s->contacts, bodies, n, s->n_meshes, buf + bb, out, out_bodies, cap, n_out);
 }
 
 int kdop_contacts_adjoint(kdop_scene* s, const float* dd, const float* dn, float* grad, int memory) {
@@ -1229,6 +1240,7 @@ int kdop_graph_capture(kdop_scene* s, int refit_mode, int64_t n_pairs, const uin
   cudaGraphGetNodes(g, nullptr, &n_nodes);
   ext(s)->graph_kernels = (int64_t)n_nodes;
   ext(s)->graph_refit_mode = refit_mode;
+  ext(s)->graph_pairs = n_pairs;
   s->refit_mode = refit_mode;
   // capturing runs nothing: the posed array holds no step of this graph yet
   s->posed_valid = false;
@@ -1249,6 +1261,8 @@ int kdop_graph_launch(kdop_scene* s) {
   // the step just enqueued refits in the graph's mode: the contacts, the
   // adjoint and read-backs follow it, whatever direct refit ran in between
   s->refit_mode = ext(s)->graph_refit_mode;
+  s->result_pairs = ext(s)->graph_pairs;
+  s->pairs_current = true;
   if (s->refit_mode != KDOP_REFIT_VERTICES) s->posed_valid = true;
   return KDOP_OK;
 }
@@ -1292,6 +1306,9 @@ int kdop_autotune(kdop_scene* s, int64_t n_pairs, const uint32_t* pairs, int mem
   repeats = std::max(repeats, 5) | 1;
   int rc = upload_pairs(s, n_pairs, pairs, memory);
   if (rc != KDOP_OK) return rc;
+  // the timed traversals leave their results in the scene
+  s->result_pairs = n_pairs;
+  s->pairs_current = true;
   std::vector<cudaEvent_t> ev((size_t)repeats + 1, nullptr);
   for (auto& e : ev) {
     cudaError_t ce = cudaEventCreate(&e);

@@ -111,6 +111,7 @@ struct kdop_scene {
   uint8_t* surf = nullptr;
   float4* nodes = nullptr;
   uint32_t* root_dev = nullptr;
+  uint32_t* t_off_dev = nullptr;  // first tet of each mesh (n_meshes + 1)
   float4* quat = nullptr;
   float4* pos = nullptr;
   float4* lin_vel = nullptr;
@@ -142,6 +143,8 @@ struct kdop_scene {
   bool traversed = false;
   bool contacted = false;
   int64_t last_pairs = 0;
+  int64_t result_pairs = 0;    // pairs the last results' pair indices run over
+  bool pairs_current = false;  // `pairs` is the list the last results came from
   int last_mode = 0;
   kdop::TravParams last_params{};
 
@@ -230,8 +233,8 @@ cudaError_t launch_traverse_shard(kdop_scene* s, int64_t n_pairs, const uint2* p
 cudaError_t launch_contacts(kdop_scene* s);
 // contact reduction (kdop_reduce.cu)
 size_t reduce_work_bytes(int64_t n);
-cudaError_t reduce_contact_rows(kdop_ctx* ctx, const kdop_contact* rows, const uint2* bodies, int64_t n, void* work,
-                                kdop_contact* out, uint2* out_bodies, int64_t* n_out);
+cudaError_t reduce_contact_rows(kdop_ctx* ctx, const kdop_contact* rows, const uint2* bodies, int64_t n,
+                                int64_t n_bodies, void* work, kdop_contact* out, uint2* out_bodies, int64_t* n_out);
 cudaError_t scene_contact_bodies(kdop_scene* s, int64_t n, uint2* bodies);
 cudaError_t launch_adjoint(kdop_scene* s, const float* dd, const float* dn, float* grad);
 cudaError_t launch_motion(kdop_scene* s);

@@ -10,24 +10,37 @@
 // FOUNDATION/TINY/TINY/include/tiny_precision.h:21-24), which keeps a row
 // only when it differs from the last row kept.
 //
-// Here: five stable LSD radix sorts of 64-bit keys build the order (the least
-// significant field pair first; floats mapped to integers that order like
-// float `<`, -0 folded onto +0).  The unique is sequential by definition (a
-// row is compared with the last row kept, not with its predecessor, and the
-// tolerance is not transitive), but a row whose p.y exceeds its
-// predecessor's by more than the tolerance, or whose bodies differ, can equal
-// no earlier row (rounded subtraction is monotonic, so every earlier p.y is
-// further away), so the sorted rows split into independent segments there;
-// one thread walks each segment.  A scan of the keep flags compacts them.
+// Here: one stable radix sort by (body i, body j, p.y), whose width follows
+// from the bodies' numbers (50 bits for 512 bodies), then the rows that tie in
+// it -- runs of equal keys -- are ranked among themselves by the other six
+// fields, a thread per row counting the run's rows before its own.  Runs
+// longer than kRankMax are ordered by three more stable radix sorts of their
+// rows alone and a fourth by run.  (Sorting all rows by all nine fields, five
+// 64-bit sorts of up to eight passes each, moved every row's key 32 times: of
+// the 3.6 M rows of 256 touching pairs 40 % are in runs of one or two rows and
+// 17 % in runs of more than 32, the longest 371.)  Floats are mapped to
+// integers that order like float `<`, -0 folded onto +0.
+//
+// The unique is sequential by definition (a row is compared with the last row
+// kept, not with its predecessor, and the tolerance is not transitive), but it
+// splits into independent segments: a row whose p.y exceeds its predecessor's
+// by more than the tolerance, or whose bodies differ, can equal no earlier row
+// (rounded subtraction is monotonic, so every earlier p.y is further away).
+// Within a run of equal p.y that itself starts a segment the same holds for a
+// gap in p.x, by which such a run is sorted.  The thread of a segment's first
+// row walks it; a one-pass scan of the keep flags compacts the rows.
 #include <algorithm>
 
 #include "kdop_device.cuh"
 #include "kdop_internal.h"
-#include "kdop_sort.h"
+#include "kdop_sort.cuh"
 
 namespace kdop {
 
 namespace {
+
+constexpr float kEps = 1.19209290e-07f * 10.0f;  // working_precision<float>()
+constexpr uint32_t kRankMax = 512;               // longest run ranked row by row
 
 // Integer image of a float that orders like float `<` (NaN aside); -0 and +0
 // map to the same value.
@@ -36,95 +49,265 @@ __device__ __forceinline__ uint32_t ord_key(float f) {
   if ((u << 1) == 0u) u = 0u;
   return (u & 0x80000000u) ? ~u : (u | 0x80000000u);
 }
+__device__ __forceinline__ uint64_t two_keys(float hi, float lo) { return ((uint64_t)ord_key(hi) << 32) | ord_key(lo); }
 
-__global__ void red_iota_kernel(uint32_t* perm, int64_t n) {
-  int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (i < n) perm[i] = (uint32_t)i;
+// One row in registers: p, n.x | n.y, n.z, depth, cand.
+struct Row {
+  float4 a, b;
+};
+__device__ __forceinline__ Row load_row(const kdop_contact* rows, int64_t r) {
+  const float4* p = reinterpret_cast<const float4*>(rows) + 2 * r;
+  return Row{p[0], p[1]};
 }
 
-// Key of one LSD pass for the row at perm[i]; pass 0 is the least significant
-// (n.z, depth), pass 4 the most (body i, body j).
-__global__ void red_keys_kernel(const kdop_contact* __restrict__ rows, const uint2* __restrict__ bodies,
-                                const uint32_t* __restrict__ perm, int64_t n, int pass, uint64_t* keys) {
-  int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= n) return;
-  const uint32_t r = perm[i];
-  const kdop_contact c = rows[r];
-  uint64_t hi = 0, lo = 0;
-  switch (pass) {
-    case 0: hi = ord_key(c.n[2]); lo = ord_key(c.depth); break;
-    case 1: hi = ord_key(c.n[1]); lo = ord_key(c.n[0]); break;
-    case 2: hi = ord_key(c.p[0]); lo = ord_key(c.p[2]); break;
-    case 3: lo = ord_key(c.p[1]); break;
-    default: {
-      const uint2 b = bodies[r];
-      hi = b.x;
-      lo = b.y;
+// (body i, body j, p.y): the first sort, `bj` bits for body j (body_bits = 0:
+// p.y alone).
+struct PointGen {
+  const kdop_contact* rows;
+  const uint2* bodies;
+  int bj;
+  bool with_bodies;
+  __device__ uint64_t key(int64_t i) const {
+    const uint64_t y = ord_key(rows[i].p[1]);
+    if (!with_bodies) return y;
+    const uint2 b = bodies[i];
+    return ((((uint64_t)b.x << bj) | b.y) << 32) | y;
+  }
+  __device__ uint32_t val(int64_t i) const { return (uint32_t)i; }
+};
+// (body i, body j) after p.y, where both do not fit one key.
+struct BodyGen {
+  const uint2* bodies;
+  const uint32_t* perm;
+  __device__ uint64_t key(int64_t i) const {
+    const uint2 b = bodies[perm[i]];
+    return ((uint64_t)b.x << 32) | b.y;
+  }
+  __device__ uint32_t val(int64_t i) const { return perm[i]; }
+};
+// Field pairs of the rows of long runs, least significant first, then the run.
+// Values are positions in the first sort's order.
+struct LongGen {
+  const kdop_contact* rows;
+  const uint32_t* perm;  // first sort's order
+  const uint32_t* at;    // positions to sort
+  const uint32_t* run;   // run of a position
+  int pass;
+  __device__ uint64_t key(int64_t i) const {
+    const uint32_t k = at[i];
+    if (pass == 3) return run[k];
+    const kdop_contact& c = rows[perm[k]];
+    return pass == 0 ? two_keys(c.n[2], c.depth) : pass == 1 ? two_keys(c.n[1], c.n[0]) : two_keys(c.p[0], c.p[2]);
+  }
+  __device__ uint32_t val(int64_t i) const { return at[i]; }
+};
+
+__global__ void red_max_kernel(const uint2* __restrict__ bodies, int64_t n, unsigned* most) {
+  unsigned x = 0, y = 0;
+  for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
+    const uint2 b = bodies[i];
+    x = max(x, b.x);
+    y = max(y, b.y);
+  }
+  x = __reduce_max_sync(0xffffffffu, x);
+  y = __reduce_max_sync(0xffffffffu, y);
+  if ((threadIdx.x & 31) == 0) {
+    atomicMax(most, x);
+    atomicMax(most + 1, y);
+  }
+}
+
+struct ReduceArgs {
+  const kdop_contact* rows;
+  const uint2* bodies;
+  int64_t n;
+  const uint32_t* perm;   // rows in the first sort's order
+  uint32_t* run;          // run of a sorted position
+  uint32_t* starts;       // first position of a run; starts[runs] = n
+  uint32_t* order;        // rows in full order
+  Row* sorted;            // the same rows, copied
+  uint32_t* keep;
+  uint32_t* longs;        // positions in runs longer than kRankMax
+  kdop_contact* out;
+  uint2* out_bodies;
+  unsigned* head;         // ReduceHead words
+  unsigned long long* words_run;
+  unsigned long long* words_keep;
+};
+// Counters of a reduction, one device block read back as a whole.
+enum { H_ERR, H_TICKET_RUN, H_TICKET_KEEP, H_LONG, H_KEPT, H_MOST_I, H_MOST_J, H_WORDS = 8 };
+
+constexpr int RD_ITEMS = 4, RD_TILE = 256 * RD_ITEMS;
+
+// Runs of equal (bodies, p.y): a scan of their first rows.
+__global__ void __launch_bounds__(256) red_runs_kernel(ReduceArgs a) {
+  __shared__ unsigned s_tile;
+  if (threadIdx.x == 0) s_tile = atomicAdd(a.head + H_TICKET_RUN, 1u);
+  __syncthreads();
+  const unsigned tile = s_tile;
+  const int64_t base = (int64_t)tile * RD_TILE + (int64_t)threadIdx.x * RD_ITEMS;
+  uint32_t y_prev = 0;
+  uint2 b_prev = make_uint2(0u, 0u);
+  if (base > 0 && base <= a.n) {
+    const uint32_t r = a.perm[base - 1];
+    y_prev = ord_key(a.rows[r].p[1]);
+    b_prev = a.bodies[r];
+  }
+  uint32_t first = 0, sum = 0;  // bit j: item j starts a run
+#pragma unroll
+  for (int j = 0; j < RD_ITEMS; ++j) {
+    const int64_t k = base + j;
+    if (k >= a.n) continue;
+    const uint32_t r = a.perm[k];
+    const uint32_t y = ord_key(a.rows[r].p[1]);
+    const uint2 b = a.bodies[r];
+    if (k == 0 || y != y_prev || b.x != b_prev.x || b.y != b_prev.y) {
+      first |= 1u << j;
+      ++sum;
     }
+    y_prev = y;
+    b_prev = b;
   }
-  keys[i] = (hi << 32) | lo;
+  uint32_t total;
+  uint32_t at = block_scan<256, uint32_t>(sum, total);
+  at += tile_prefix(a.words_run, tile, total, a.head + H_ERR);
+#pragma unroll
+  for (int j = 0; j < RD_ITEMS; ++j) {
+    const int64_t k = base + j;
+    if (k >= a.n) continue;
+    if ((first >> j) & 1u) a.starts[at++] = (uint32_t)k;
+    a.run[k] = at - 1;
+    if (k == a.n - 1) a.starts[at] = (uint32_t)a.n;
+  }
 }
 
-// brk[i] = 1 where a segment starts (first row, new bodies, or a p.y gap
-// above the tolerance); brk[n] = 0 so a scan over n + 1 ends with the count.
-__global__ void red_breaks_kernel(const kdop_contact* __restrict__ rows, const uint2* __restrict__ bodies,
-                                  const uint32_t* __restrict__ perm, int64_t n, float eps, uint32_t* brk) {
-  int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (i > n) return;
-  uint32_t b = 0;
-  if (i == 0) {
-    b = 1;
-  } else if (i < n) {
-    const uint32_t r = perm[i], q = perm[i - 1];
-    const uint2 br = bodies[r], bq = bodies[q];
-    b = (br.x != bq.x || br.y != bq.y || fabsf(fsub(rows[r].p[1], rows[q].p[1])) > eps) ? 1u : 0u;
-  }
-  brk[i] = b;
+// Fields after p.y of two rows of a run, in the sort's order: -1, 0, 1.
+__device__ __forceinline__ int later_fields(const Row& x, const Row& y) {
+  const uint64_t p = two_keys(x.a.x, x.a.z), q = two_keys(y.a.x, y.a.z);
+  if (p != q) return p < q ? -1 : 1;
+  const uint64_t n = two_keys(x.b.x, x.a.w), m = two_keys(y.b.x, y.a.w);
+  if (n != m) return n < m ? -1 : 1;
+  const uint64_t d = two_keys(x.b.y, x.b.z), f = two_keys(y.b.y, y.b.z);
+  return d < f ? -1 : d > f ? 1 : 0;
 }
 
-__global__ void red_starts_kernel(const uint32_t* __restrict__ brk, const uint32_t* __restrict__ seg, int64_t n,
-                                  uint32_t* starts) {
-  int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (i < n && brk[i]) starts[seg[i]] = (uint32_t)i;
+// Each row to its place in the full order.  Neighbouring rows are mostly of one
+// run, so a warp's loads of the run's rows fall on one address.
+__global__ void __launch_bounds__(256) red_rank_kernel(ReduceArgs a) {
+  const int64_t k = (int64_t)blockIdx.x * 256 + threadIdx.x;
+  if (k >= a.n) return;
+  const uint32_t r = a.perm[k], g = a.run[k];
+  const uint32_t s = a.starts[g], e = a.starts[g + 1];
+  if (e - s > kRankMax) {
+    a.longs[k] = 1u;  // ordered by the radix sorts below
+    a.head[H_LONG] = 1u;
+    return;
+  }
+  a.longs[k] = 0u;
+  const Row x = load_row(a.rows, r);
+  uint32_t rank = 0;
+  for (uint32_t j = s; j < e; ++j) {
+    if (j == (uint32_t)k) continue;
+    const int c = later_fields(load_row(a.rows, a.perm[j]), x);
+    rank += (c < 0 || (c == 0 && j < (uint32_t)k)) ? 1u : 0u;  // equal rows keep their order
+  }
+  a.order[s + rank] = r;
+  a.sorted[s + rank] = x;
+}
+
+// Positions of the long runs' rows in increasing order: at[pos[k]] = k.
+__global__ void red_long_list_kernel(const uint32_t* __restrict__ flag, const uint32_t* __restrict__ pos, int64_t n,
+                                     uint32_t* at) {
+  const int64_t k = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  if (k < n && flag[k]) at[pos[k]] = (uint32_t)k;
+}
+// The i-th row of the long runs in sorted order goes to the i-th position.
+__global__ void red_long_place_kernel(ReduceArgs a, const uint32_t* __restrict__ at,
+                                      const uint32_t* __restrict__ sorted_at, int64_t m) {
+  const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= m) return;
+  const uint32_t r = a.perm[sorted_at[i]];
+  a.order[at[i]] = r;
+  a.sorted[at[i]] = load_row(a.rows, r);
 }
 
 // ContactPoint::operator== between the last kept row and a new one (bodies
 // equal within a segment): no component differs by more than eps.  A NaN
 // difference is not "more than eps", as in the reference.
-__device__ __forceinline__ bool same_point(const kdop_contact& k, const kdop_contact& c, float eps) {
-  return !(fabsf(fsub(c.p[1], k.p[1])) > eps) && !(fabsf(fsub(c.p[0], k.p[0])) > eps) &&
-         !(fabsf(fsub(c.p[2], k.p[2])) > eps) && !(fabsf(fsub(c.n[1], k.n[1])) > eps) &&
-         !(fabsf(fsub(c.n[0], k.n[0])) > eps) && !(fabsf(fsub(c.n[2], k.n[2])) > eps) &&
-         !(fabsf(fsub(c.depth, k.depth)) > eps);
+__device__ __forceinline__ bool same_point(const Row& k, const Row& c) {
+  return !(fabsf(fsub(c.a.y, k.a.y)) > kEps) && !(fabsf(fsub(c.a.x, k.a.x)) > kEps) &&
+         !(fabsf(fsub(c.a.z, k.a.z)) > kEps) && !(fabsf(fsub(c.b.x, k.b.x)) > kEps) &&
+         !(fabsf(fsub(c.a.w, k.a.w)) > kEps) && !(fabsf(fsub(c.b.y, k.b.y)) > kEps) &&
+         !(fabsf(fsub(c.b.z, k.b.z)) > kEps);
 }
 
-// Thread per segment: std::unique's walk (keep a row unless it equals the
-// last row kept).  keep[n] = 0 for the compaction scan.
-__global__ void red_walk_kernel(const kdop_contact* __restrict__ rows, const uint32_t* __restrict__ perm,
-                                const uint32_t* __restrict__ starts, int64_t n_seg, int64_t n, float eps,
-                                uint32_t* keep) {
-  int64_t s = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (s == 0) keep[n] = 0u;
-  if (s >= n_seg) return;
-  const int64_t a = starts[s], e = (s + 1 < n_seg) ? (int64_t)starts[s + 1] : n;
-  kdop_contact last = rows[perm[a]];
-  keep[a] = 1u;
-  for (int64_t j = a + 1; j < e; ++j) {
-    const kdop_contact c = rows[perm[j]];
-    const bool eq = same_point(last, c, eps);
-    keep[j] = eq ? 0u : 1u;
-    if (!eq) last = c;
+// Whether the first row of a run can equal no earlier row.
+__device__ __forceinline__ bool run_breaks(const ReduceArgs& a, uint32_t s) {
+  if (s == 0) return true;
+  const uint2 b = a.bodies[a.order[s]], q = a.bodies[a.order[s - 1]];
+  return b.x != q.x || b.y != q.y || fabsf(fsub(a.sorted[s].a.y, a.sorted[s - 1].a.y)) > kEps;
+}
+// Whether the row at position k starts a segment.
+__device__ __forceinline__ bool starts_segment(const ReduceArgs& a, uint32_t k) {
+  const uint32_t s = a.starts[a.run[k]];
+  if (s == k) return run_breaks(a, k);
+  // a gap in p.x inside a run that starts a segment (a NaN at its head would
+  // equal any row)
+  const float x = a.sorted[k].a.x, p = a.sorted[k - 1].a.x, x0 = a.sorted[s].a.x;
+  return fabsf(fsub(x, p)) > kEps && x0 == x0 && run_breaks(a, s);
+}
+
+constexpr uint32_t KEEP = 1u, SEGMENT = 2u;  // bits of keep[]
+
+__global__ void __launch_bounds__(256) red_segments_kernel(ReduceArgs a) {
+  const int64_t k = (int64_t)blockIdx.x * 256 + threadIdx.x;
+  if (k < a.n) a.keep[k] = starts_segment(a, (uint32_t)k) ? SEGMENT | KEEP : 0u;
+}
+
+// Thread per segment (its first row's): std::unique's walk -- a row is kept
+// unless it equals the last row kept.
+__global__ void __launch_bounds__(128) red_walk_kernel(ReduceArgs a) {
+  const int64_t k = (int64_t)blockIdx.x * 128 + threadIdx.x;
+  if (k >= a.n || !(a.keep[k] & SEGMENT)) return;
+  Row last = a.sorted[k];
+  for (int64_t j = k + 1; j < a.n; ++j) {
+    const uint32_t f = a.keep[j];
+    const Row c = a.sorted[j];
+    if (f & SEGMENT) break;
+    if (!same_point(last, c)) {
+      a.keep[j] = KEEP;
+      last = c;
+    }
   }
 }
 
-__global__ void red_write_kernel(const kdop_contact* __restrict__ rows, const uint2* __restrict__ bodies,
-                                 const uint32_t* __restrict__ perm, const uint32_t* __restrict__ keep,
-                                 const uint32_t* __restrict__ pos, int64_t n, kdop_contact* out, uint2* out_bodies) {
-  int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= n || !keep[i]) return;
-  const uint32_t r = perm[i];
-  out[pos[i]] = rows[r];
-  if (out_bodies) out_bodies[pos[i]] = bodies[r];
+__global__ void __launch_bounds__(256) red_write_kernel(ReduceArgs a) {
+  __shared__ unsigned s_tile;
+  if (threadIdx.x == 0) s_tile = atomicAdd(a.head + H_TICKET_KEEP, 1u);
+  __syncthreads();
+  const unsigned tile = s_tile;
+  // consecutive threads hold consecutive rows: one scan step per item
+  uint32_t keep[RD_ITEMS], pos[RD_ITEMS], sum = 0;
+#pragma unroll
+  for (int j = 0; j < RD_ITEMS; ++j) {
+    const int64_t k = (int64_t)tile * RD_TILE + j * 256 + threadIdx.x;
+    keep[j] = k < a.n ? a.keep[k] & KEEP : 0u;
+    uint32_t total;
+    pos[j] = sum + block_scan<256, uint32_t>(keep[j], total);
+    sum += total;
+  }
+  const uint32_t excl = tile_prefix(a.words_keep, tile, sum, a.head + H_ERR);
+#pragma unroll
+  for (int j = 0; j < RD_ITEMS; ++j) {
+    const int64_t k = (int64_t)tile * RD_TILE + j * 256 + threadIdx.x;
+    if (k == a.n - 1) a.head[H_KEPT] = excl + sum;
+    if (!keep[j]) continue;
+    const Row x = a.sorted[k];
+    float4* o = reinterpret_cast<float4*>(a.out + excl + pos[j]);
+    o[0] = x.a;
+    o[1] = x.b;
+    if (a.out_bodies) a.out_bodies[excl + pos[j]] = a.bodies[a.order[k]];
+  }
 }
 
 // Bodies (mesh of A, mesh of B) of each contact row of a scene: the row's
@@ -142,7 +325,8 @@ unsigned blocks_for(int64_t n, int t) { return (unsigned)((n + t - 1) / t); }
 
 // Work buffer of a reduction of n rows (256-byte aligned pieces).
 struct ReduceWork {
-  size_t keys, keys_tmp, perm, perm_tmp, radix, brk, seg, starts, keep, pos, scan, total;
+  size_t head, words_run, words_keep, keys, keys_tmp, perm, perm_tmp, radix, run, starts, order, sorted, keep, longs,
+      long_at, long_vals, scan, total;
   explicit ReduceWork(int64_t n) {
     size_t at = 0;
     auto take = [&](size_t b) {
@@ -150,18 +334,24 @@ struct ReduceWork {
       at += (b + 255) & ~(size_t)255;
       return o;
     };
-    const size_t m = (size_t)std::max<int64_t>(n, 1);
+    const size_t m = (size_t)std::max<int64_t>(n, 1), tiles = (m + RD_TILE - 1) / RD_TILE;
+    head = take(H_WORDS * 4);
+    words_run = take(tiles * 8);
+    words_keep = take(tiles * 8);
     keys = take(m * 8);
     keys_tmp = take(m * 8);
     perm = take(m * 4);
     perm_tmp = take(m * 4);
     radix = take(radix_scratch_words((int64_t)m) * 4);
-    brk = take((m + 1) * 4);
-    seg = take((m + 1) * 4);
-    starts = take(m * 4);
-    keep = take((m + 1) * 4);
-    pos = take((m + 1) * 4);
-    scan = take(scan_scratch_words((int64_t)m + 1) * 4);
+    run = take(m * 4);
+    starts = take((m + 1) * 4);
+    order = take(m * 4);
+    sorted = take(m * sizeof(Row));
+    keep = take(m * 4);
+    longs = take(m * 4);
+    long_at = take(m * 4);
+    long_vals = take(m * 4);
+    scan = take(scan_scratch_words((int64_t)m) * 4);
     total = at;
   }
 };
@@ -176,57 +366,100 @@ cudaError_t scene_contact_bodies(kdop_scene* s, int64_t n, uint2* bodies) {
   return cudaGetLastError();
 }
 
-// Reduces n rows (device) with their bodies (device); the kept rows go to out
-// (and their bodies to out_bodies, may be NULL) in the reduced order; *n_out
-// = rows kept.  Synchronises (the radix sort reads its key bits back).
-cudaError_t reduce_contact_rows(kdop_ctx* ctx, const kdop_contact* rows, const uint2* bodies, int64_t n, void* work,
-                                kdop_contact* out, uint2* out_bodies, int64_t* n_out) {
+// The rows of runs longer than kRankMax: (n.z, depth), (n.y, n.x), (p.x, p.z),
+// run, each a stable sort.  The first sort's keys, the half of its values that
+// does not hold the order, and keep[] are free here.
+static cudaError_t order_long_runs(kdop_ctx* ctx, const ReduceArgs& a, const ReduceWork& L, char* w,
+                                   const SortBuffers& first) {
+  cudaStream_t st = ctx->stream;
+  SortBuffers b{first.keys, first.keys_tmp, first.vals_tmp, reinterpret_cast<uint32_t*>(w + L.long_vals)};
+  uint32_t* pos = a.keep;
+  uint32_t* at = reinterpret_cast<uint32_t*>(w + L.long_at);
+  cudaError_t e;
+  if ((e = exclusive_scan_u32(a.longs, pos, a.n, reinterpret_cast<uint32_t*>(w + L.scan), st)) != cudaSuccess) return e;
+  uint32_t tail[2];
+  if ((e = cudaMemcpyAsync(&tail[0], pos + a.n - 1, 4, cudaMemcpyDeviceToHost, st)) != cudaSuccess) return e;
+  if ((e = cudaMemcpyAsync(&tail[1], a.longs + a.n - 1, 4, cudaMemcpyDeviceToHost, st)) != cudaSuccess) return e;
+  if ((e = cudaStreamSynchronize(st)) != cudaSuccess) return e;
+  const int64_t m = (int64_t)tail[0] + tail[1];
+  if (m == 0) return cudaSuccess;
+  red_long_list_kernel<<<blocks_for(a.n, 256), 256, 0, st>>>(a.longs, pos, a.n, at);
+  const uint32_t* from = at;
+  for (int pass = 0; pass < 4; ++pass) {
+    const int bits = pass < 3 ? 64 : bits_of((uint64_t)a.n);
+    e = radix_sort(LongGen{a.rows, a.perm, from, a.run, pass}, m, bits, b, w + L.radix, a.head + H_ERR, st,
+                   ctx->launches);
+    if (e != cudaSuccess) return e;
+    from = b.vals;
+  }
+  red_long_place_kernel<<<blocks_for(m, 256), 256, 0, st>>>(a, at, from, m);
+  ctx->launches += 2;
+  return cudaGetLastError();
+}
+
+// Reduces n rows (device) with their bodies (device, below n_bodies where that
+// is known, else n_bodies = 0); the kept rows go to out (and their bodies to
+// out_bodies, may be NULL) in the reduced order; *n_out = rows kept.
+// Synchronises.
+cudaError_t reduce_contact_rows(kdop_ctx* ctx, const kdop_contact* rows, const uint2* bodies, int64_t n,
+                                int64_t n_bodies, void* work, kdop_contact* out, uint2* out_bodies, int64_t* n_out) {
   cudaStream_t st = ctx->stream;
   *n_out = 0;
   if (n <= 0) return cudaSuccess;
   if (n >= ((int64_t)1 << 32) - 1) return cudaErrorInvalidValue;
   ReduceWork L(n);
   char* w = static_cast<char*>(work);
-  uint64_t* keys = reinterpret_cast<uint64_t*>(w + L.keys);
-  uint64_t* keys_tmp = reinterpret_cast<uint64_t*>(w + L.keys_tmp);
-  uint32_t* perm = reinterpret_cast<uint32_t*>(w + L.perm);
-  uint32_t* perm_tmp = reinterpret_cast<uint32_t*>(w + L.perm_tmp);
-  uint32_t* radix = reinterpret_cast<uint32_t*>(w + L.radix);
-  uint32_t* brk = reinterpret_cast<uint32_t*>(w + L.brk);
-  uint32_t* seg = reinterpret_cast<uint32_t*>(w + L.seg);
-  uint32_t* starts = reinterpret_cast<uint32_t*>(w + L.starts);
-  uint32_t* keep = reinterpret_cast<uint32_t*>(w + L.keep);
-  uint32_t* pos = reinterpret_cast<uint32_t*>(w + L.pos);
-  uint32_t* scan = reinterpret_cast<uint32_t*>(w + L.scan);
-  const float eps = 1.19209290e-07f * 10.0f;  // working_precision<float>()
-  const unsigned g = blocks_for(n, 256), g1 = blocks_for(n + 1, 256);
-  red_iota_kernel<<<g, 256, 0, st>>>(perm, n);
-  ctx->launches++;
+  ReduceArgs a;
+  a.rows = rows;
+  a.bodies = bodies;
+  a.n = n;
+  a.run = reinterpret_cast<uint32_t*>(w + L.run);
+  a.starts = reinterpret_cast<uint32_t*>(w + L.starts);
+  a.order = reinterpret_cast<uint32_t*>(w + L.order);
+  a.sorted = reinterpret_cast<Row*>(w + L.sorted);
+  a.keep = reinterpret_cast<uint32_t*>(w + L.keep);
+  a.longs = reinterpret_cast<uint32_t*>(w + L.longs);
+  a.out = out;
+  a.out_bodies = out_bodies;
+  a.head = reinterpret_cast<unsigned*>(w + L.head);
+  a.words_run = reinterpret_cast<unsigned long long*>(w + L.words_run);
+  a.words_keep = reinterpret_cast<unsigned long long*>(w + L.words_keep);
+  SortBuffers b{reinterpret_cast<uint64_t*>(w + L.keys), reinterpret_cast<uint64_t*>(w + L.keys_tmp),
+                reinterpret_cast<uint32_t*>(w + L.perm), reinterpret_cast<uint32_t*>(w + L.perm_tmp)};
+  unsigned h[H_WORDS];
   cudaError_t e;
-  for (int pass = 0; pass < 5; ++pass) {
-    red_keys_kernel<<<g, 256, 0, st>>>(rows, bodies, perm, n, pass, keys);
+  if ((e = cudaMemsetAsync(w + L.head, 0, L.keys - L.head, st)) != cudaSuccess) return e;
+  int bi = bits_of(n_bodies > 0 ? (uint64_t)n_bodies - 1 : 0), bj = bi;
+  if (n_bodies <= 0) {
+    red_max_kernel<<<(unsigned)std::min<int64_t>((n + 255) / 256, 592), 256, 0, st>>>(bodies, n, a.head + H_MOST_I);
     ctx->launches++;
-    if ((e = cudaGetLastError()) != cudaSuccess) return e;
-    if ((e = radix_sort_pairs(keys, perm, keys_tmp, perm_tmp, n, radix, st)) != cudaSuccess) return e;
+    if ((e = cudaMemcpyAsync(h, a.head, sizeof(h), cudaMemcpyDeviceToHost, st)) != cudaSuccess) return e;
+    if ((e = cudaStreamSynchronize(st)) != cudaSuccess) return e;
+    bi = bits_of(h[H_MOST_I]);
+    bj = bits_of(h[H_MOST_J]);
   }
-  red_breaks_kernel<<<g1, 256, 0, st>>>(rows, bodies, perm, n, eps, brk);
-  ctx->launches++;
-  if ((e = exclusive_scan_u32(brk, seg, n + 1, scan, st)) != cudaSuccess) return e;
-  red_starts_kernel<<<g, 256, 0, st>>>(brk, seg, n, starts);
-  ctx->launches++;
-  uint32_t n_seg = 0;
-  if ((e = cudaMemcpyAsync(&n_seg, seg + n, 4, cudaMemcpyDeviceToHost, st)) != cudaSuccess) return e;
+  const bool one = bi + bj <= 32;
+  e = radix_sort(PointGen{rows, bodies, bj, one}, n, 32 + (one ? bi + bj : 0), b, w + L.radix, a.head + H_ERR, st,
+                 ctx->launches);
+  if (e == cudaSuccess && !one)
+    e = radix_sort(BodyGen{bodies, b.vals}, n, 32 + bi, b, w + L.radix, a.head + H_ERR, st, ctx->launches);
+  if (e != cudaSuccess) return e;
+  a.perm = b.vals;
+  const unsigned tiles = blocks_for(n, RD_TILE);
+  red_runs_kernel<<<tiles, 256, 0, st>>>(a);
+  red_rank_kernel<<<blocks_for(n, 256), 256, 0, st>>>(a);
+  ctx->launches += 2;
+  if ((e = cudaMemcpyAsync(h, a.head, sizeof(h), cudaMemcpyDeviceToHost, st)) != cudaSuccess) return e;
   if ((e = cudaStreamSynchronize(st)) != cudaSuccess) return e;
-  red_walk_kernel<<<blocks_for(std::max<int64_t>(n_seg, 1), 128), 128, 0, st>>>(rows, perm, starts, n_seg, n, eps,
-                                                                                   keep);
-  ctx->launches++;
-  if ((e = exclusive_scan_u32(keep, pos, n + 1, scan, st)) != cudaSuccess) return e;
-  red_write_kernel<<<g, 256, 0, st>>>(rows, bodies, perm, keep, pos, n, out, out_bodies);
-  ctx->launches++;
-  uint32_t kept = 0;
-  if ((e = cudaMemcpyAsync(&kept, pos + n, 4, cudaMemcpyDeviceToHost, st)) != cudaSuccess) return e;
+  if (h[H_LONG] && (e = order_long_runs(ctx, a, L, w, b)) != cudaSuccess) return e;
+  red_segments_kernel<<<blocks_for(n, 256), 256, 0, st>>>(a);
+  red_walk_kernel<<<blocks_for(n, 128), 128, 0, st>>>(a);
+  red_write_kernel<<<tiles, 256, 0, st>>>(a);
+  ctx->launches += 3;
+  if ((e = cudaMemcpyAsync(h, a.head, sizeof(h), cudaMemcpyDeviceToHost, st)) != cudaSuccess) return e;
   if ((e = cudaStreamSynchronize(st)) != cudaSuccess) return e;
-  *n_out = kept;
+  if (h[H_ERR]) return cudaErrorLaunchTimeout;
+  *n_out = h[H_KEPT];
   return cudaGetLastError();
 }
 

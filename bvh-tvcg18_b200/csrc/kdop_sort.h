@@ -1,4 +1,5 @@
-// kdop_sort.h -- device radix sort and exclusive scan (kdop_sort.cu).
+// kdop_sort.h -- sizes of the device radix sort (kdop_sort.cuh), the exclusive
+// scan and the ordering of a traversal's results (kdop_sort.cu).
 #pragma once
 #include <cstddef>
 #include <cstdint>
@@ -6,14 +7,12 @@
 
 namespace kdop {
 
-// Words of scratch radix_sort_pairs needs for n keys.
+constexpr int64_t kSortTile = 2048, kSortTileLarge = 4096;  // keys per block and pass
+constexpr int64_t kLargeSort = 1 << 20;                     // from this many keys on, the large tile
+
+// Words of scratch a radix sort of n keys needs.
 size_t radix_scratch_words(int64_t n);
-// Stable ascending sort of (keys, vals), n < 2^32; keys_tmp / vals_tmp hold n
-// each; scratch radix_scratch_words(n) words (8-byte aligned).  Reads the
-// keys' common bits back to the host once (synchronises the stream).
-cudaError_t radix_sort_pairs(uint64_t* keys, uint32_t* vals, uint64_t* keys_tmp, uint32_t* vals_tmp, int64_t n,
-                             uint32_t* scratch, cudaStream_t st);
-// Words of scratch exclusive_scan_u32 needs for n counts.
+// Words of scratch exclusive_scan_u32 needs for n counts (8-byte aligned).
 size_t scan_scratch_words(int64_t n);
 // out[i] = in[0] + ... + in[i-1] (in == out allowed).
 cudaError_t exclusive_scan_u32(const uint32_t* in, uint32_t* out, int64_t n, uint32_t* scratch, cudaStream_t st);
@@ -24,7 +23,8 @@ struct kdop_scene;
 namespace kdop {
 // Sorts the last traversal's n candidate rows by (pair, tet of A, tet of B)
 // and, after kdop_contacts, regroups the n_contacts contact rows and the
-// records in that order.  work: sort_results_bytes(n, n_contacts) bytes.
+// records in that order.  work: sort_results_bytes(n, n_contacts) bytes.  A
+// bounded wait that gave up sets DEV_ERR_TIMEOUT in the scene's control block.
 cudaError_t sort_results(kdop_scene* s, int64_t n, int64_t n_contacts, void* work, cudaStream_t st);
 size_t sort_results_bytes(int64_t n, int64_t n_contacts);
 }  // namespace kdop

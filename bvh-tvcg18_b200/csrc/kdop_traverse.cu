@@ -36,7 +36,7 @@
 #include <mutex>
 
 #include "kdop_device.cuh"
-#include "kdop_sort.h"
+#include "kdop_sort.cuh"
 
 namespace kdop {
 
@@ -1077,18 +1077,18 @@ __global__ void frontier_final_kernel(unsigned* fs, unsigned cap) {
   }
 }
 
-__global__ void entry_keys_kernel(const uint4* __restrict__ f, unsigned n, uint64_t* keys, uint32_t* vals,
-                                  int by_pair) {
-  unsigned i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= n) return;
-  if (by_pair) {
-    keys[i] = f[vals[i]].z;
-  } else {
-    uint4 e = f[i];
-    keys[i] = ((uint64_t)e.x << 32) | e.y;
-    vals[i] = i;
-  }
-}
+// Frontier order: by (A, B) words, then, stably, by pair.
+struct EntryGen {
+  const uint4* f;
+  __device__ uint64_t key(int64_t i) const { return ((uint64_t)f[i].x << 32) | f[i].y; }
+  __device__ uint32_t val(int64_t i) const { return (uint32_t)i; }
+};
+struct EntryPairGen {
+  const uint4* f;
+  const uint32_t* order;
+  __device__ uint64_t key(int64_t i) const { return f[order[i]].z; }
+  __device__ uint32_t val(int64_t i) const { return order[i]; }
+};
 
 // this shard's entries: sorted positions rank, rank + n_ranks, ...
 __global__ void deal_kernel(const uint4* __restrict__ f, const uint32_t* __restrict__ order, unsigned n, int rank,
@@ -1155,11 +1155,8 @@ cudaError_t shard_impl(kdop_scene* s, int64_t n_pairs, const uint2* pairs, const
   ShardWork L(cap);
   unsigned* fs = reinterpret_cast<unsigned*>(w + L.fs);
   uint4* F[2] = {reinterpret_cast<uint4*>(w + L.f0), reinterpret_cast<uint4*>(w + L.f1)};
-  uint64_t* keys = reinterpret_cast<uint64_t*>(w + L.k);
-  uint64_t* ktmp = reinterpret_cast<uint64_t*>(w + L.kt);
-  uint32_t* vals = reinterpret_cast<uint32_t*>(w + L.v);
-  uint32_t* vtmp = reinterpret_cast<uint32_t*>(w + L.vt);
-  uint32_t* scratch = reinterpret_cast<uint32_t*>(w + L.sc);
+  SortBuffers b{reinterpret_cast<uint64_t*>(w + L.k), reinterpret_cast<uint64_t*>(w + L.kt),
+                reinterpret_cast<uint32_t*>(w + L.v), reinterpret_cast<uint32_t*>(w + L.vt)};
   uint4* mine = reinterpret_cast<uint4*>(w + L.mine);
   TravArgs a = frontier_args<K>(s, pairs, p);
   cudaError_t e;
@@ -1182,12 +1179,13 @@ cudaError_t shard_impl(kdop_scene* s, int64_t n_pairs, const uint2* pairs, const
   // deterministic order: by (A, B), then by pair
   if (n > 0) {
     const unsigned gn = (n + 255) / 256;
-    entry_keys_kernel<<<gn, 256, 0, st>>>(fin, n, keys, vals, 0);
-    if ((e = radix_sort_pairs(keys, vals, ktmp, vtmp, n, scratch, st)) != cudaSuccess) return e;
-    entry_keys_kernel<<<gn, 256, 0, st>>>(fin, n, keys, vals, 1);
-    if ((e = radix_sort_pairs(keys, vals, ktmp, vtmp, n, scratch, st)) != cudaSuccess) return e;
-    deal_kernel<<<gn, 256, 0, st>>>(fin, vals, n, rank, n_ranks, mine);
-    s->ctx->launches += 3;
+    unsigned* err = &s->ctl->error;
+    if ((e = radix_sort(EntryGen{fin}, n, 64, b, w + L.sc, err, st, s->ctx->launches)) != cudaSuccess) return e;
+    if ((e = radix_sort(EntryPairGen{fin, b.vals}, n, bits_of((uint64_t)std::max<int64_t>(n_pairs, 1) - 1), b, w + L.sc,
+                        err, st, s->ctx->launches)) != cudaSuccess)
+      return e;
+    deal_kernel<<<gn, 256, 0, st>>>(fin, b.vals, n, rank, n_ranks, mine);
+    s->ctx->launches += 1;
   }
   // the expansion's tests and leaf pairs belong to shard 0
   if (rank != 0) {
@@ -1196,17 +1194,17 @@ cudaError_t shard_impl(kdop_scene* s, int64_t n_pairs, const uint2* pairs, const
   }
   const int64_t m = n > (unsigned)rank ? ((int64_t)n - rank + n_ranks - 1) / n_ranks : 0;
   *n_entries = m;
-  TravBuffers b;
-  b.pairs = pairs;
-  b.order = nullptr;
-  b.entries = mine;
-  b.cand = s->cand;
-  b.cand_cap = s->cand_cap;
-  b.q_items = s->q_items;
-  b.q_tags = s->q_tags;
-  b.q_cap = s->queue_cap;
-  b.ctl = s->ctl;
-  return traverse_group<K>(s, m, b, p, 0);
+  TravBuffers t;
+  t.pairs = pairs;
+  t.order = nullptr;
+  t.entries = mine;
+  t.cand = s->cand;
+  t.cand_cap = s->cand_cap;
+  t.q_items = s->q_items;
+  t.q_tags = s->q_tags;
+  t.q_cap = s->queue_cap;
+  t.ctl = s->ctl;
+  return traverse_group<K>(s, m, t, p, 0);
 }
 
 }  // namespace
