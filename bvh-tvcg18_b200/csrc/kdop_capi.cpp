@@ -221,6 +221,9 @@ static void scene_free(kdop_scene* s) {
   if (s->root_dev) cudaFree(s->root_dev);
   s->root_dev = nullptr;
   dfree(s, &s->t_off_dev, s->n_meshes + 1);
+  dfree(s, &s->leaf_verts, s->nt);
+  dfree(s, &s->leaf_tet, s->nt);
+  dfree(s, &s->refit_blocks, s->refit_stage.empty() ? 0 : s->refit_stage.back());
   dfree(s, &s->quat, s->n_meshes);
   dfree(s, &s->pos, s->n_meshes);
   dfree(s, &s->lin_vel, s->n_meshes);
@@ -388,8 +391,9 @@ int kdop_scene_create_ex(kdop_ctx* ctx, int K, int n_meshes, const kdop_mesh_des
   kdop::ForestBuild fb;
   std::vector<int64_t> pre;
   std::vector<int32_t> lg;
-  int brc = build == KDOP_BUILD_HOST ? kdop::build_forest(xyz, nvs, tets, nts, orders, s->t_off, fb)
-                                     : kdop::forest_layout(nts, fb, pre, lg);
+  // node layout (the host build makes the same one and fills in the topology)
+  int brc = kdop::forest_layout(nts, fb, pre, lg);
+  if (brc == 0 && build == KDOP_BUILD_HOST) brc = kdop::build_forest(xyz, nvs, tets, nts, orders, s->t_off, fb);
   if (brc != 0) {
     delete box;
     return fail(ctx, KDOP_ERR_INVALID, "scene too large for 30-bit node indices");
@@ -444,6 +448,13 @@ int kdop_scene_create_ex(kdop_ctx* ctx, int K, int n_meshes, const kdop_mesh_des
     SC_TRY(dalloc(s, &s->t_off_dev, n_meshes + 1));
     std::vector<uint32_t> toff(s->t_off.begin(), s->t_off.end());
     SC_TRY(cudaMemcpyAsync(s->t_off_dev, toff.data(), toff.size() * 4, cudaMemcpyHostToDevice, st));
+    std::vector<kdop::RefitBlock> rblocks;
+    kdop::refit_blocks(fb, pre, lg, nts, s->t_off, rblocks, s->refit_stage);
+    SC_TRY(dalloc(s, &s->leaf_verts, nt));
+    SC_TRY(dalloc(s, &s->leaf_tet, nt));
+    SC_TRY(dalloc(s, &s->refit_blocks, (int64_t)rblocks.size()));
+    SC_TRY(cudaMemcpyAsync(s->refit_blocks, rblocks.data(), rblocks.size() * sizeof(kdop::RefitBlock),
+                           cudaMemcpyHostToDevice, st));
     SC_TRY(dalloc(s, &s->quat, n_meshes));
     SC_TRY(dalloc(s, &s->pos, n_meshes));
     SC_TRY(dalloc(s, &s->lin_vel, n_meshes));
@@ -496,6 +507,7 @@ int kdop_scene_create_ex(kdop_ctx* ctx, int K, int n_meshes, const kdop_mesh_des
       s->host_orders = (int)hm.size();
     }
     SC_TRY(kdop::launch_write_topology(s, topo_dev));
+    SC_TRY(kdop::launch_leaf_tables(s));
     // make_tree ends with a refit (kdop_make_tree.h:285)
     SC_TRY(kdop::launch_refit(s, KDOP_REFIT_VERTICES));
     s->refit_mode = KDOP_REFIT_VERTICES;

@@ -25,6 +25,19 @@ struct DirTable {
 // Columns of a scene's candidate buffer (each cand_cap uint32).
 constexpr int kCandCols = 5;
 
+// One block of a refit launch (kdop_refit.cu): up to 256 consecutive nodes of
+// one tree and the levels above them to their common ancestor.
+struct RefitBlock {
+  uint32_t first_leaf;  // its first tet in the leaf-order arrays
+  uint32_t tets;        // tets below its ancestor
+  uint32_t leaf_twin;   // first node of depth L + 1 below it (first launch)
+  int32_t levels;       // levels above its nodes (8, fewer in a small tree)
+  uint32_t node[9];     // first node of each of its levels, the ancestor's first
+  uint32_t pad_node;    // the root level's padding node, for the block that writes the root it repeats
+  uint32_t pad[2];
+};
+static_assert(sizeof(RefitBlock) == 64, "one 64-byte record per block");
+
 // Device-side control block of one traversal (+ contact generation).  The counters that every warp updates or polls
 // while the traversal runs sit on 128-byte lines of their own, so that atomics
 // and polls on one do not queue behind traffic on another in the same L2 slice.
@@ -111,6 +124,10 @@ struct kdop_scene {
   uint8_t* surf = nullptr;
   float4* nodes = nullptr;
   uint32_t* root_dev = nullptr;
+  uint4* leaf_verts = nullptr;     // global vertex indices of the tets in leaf order, mesh by mesh
+  uint32_t* leaf_tet = nullptr;    // tet | surface bit of the same
+  kdop::RefitBlock* refit_blocks = nullptr;  // blocks of the refit's launches, launch i from refit_stage[i] on
+  std::vector<int64_t> refit_stage;
   uint32_t* t_off_dev = nullptr;  // first tet of each mesh (n_meshes + 1)
   float4* quat = nullptr;
   float4* pos = nullptr;
@@ -217,6 +234,10 @@ void surface_map(int64_t n_tets, const uint32_t* tets, uint8_t* surf);
 
 // kernel launchers (return cudaGetLastError of the launches)
 cudaError_t launch_write_topology(kdop_scene* s, const uint32_t* topo_dev);
+void refit_blocks(const ForestBuild& fb, const std::vector<int64_t>& pre, const std::vector<int32_t>& lg,
+                  const std::vector<int64_t>& n_tets, const std::vector<int64_t>& t_off,
+                  std::vector<RefitBlock>& blocks, std::vector<int64_t>& stage);
+cudaError_t launch_leaf_tables(kdop_scene* s);  // leaf_verts, leaf_tet from the node records
 cudaError_t launch_refit(kdop_scene* s, int mode);
 cudaError_t launch_traverse(kdop_scene* s, int64_t n_pairs, const uint2* pairs, const TravParams& p, int plain);
 // broad phase (kdop_broad.cu)

@@ -7,140 +7,372 @@
 // 10-24).  The OpenCL back-end did one work-group per object with retry loops
 // (cl/kernels/kdop_cl_refit_tree.cl:17-168).
 //
-// Here the forest is stored level by level, so one launch refits one level of
-// every tree at once, deepest level first, one thread per node: a leaf poses
-// its four vertices once and projects them on all K/2 directions; an internal
-// node reads its children's twin record (2 NW consecutive float4, independent
-// loads in flight together).  Two sibling threads write the interleaved
-// chunks of one twin, so every store instruction fills whole 32-byte sectors.
+// Here one launch refits nine levels of every tree.  The index-median split
+// makes a tree over n tets complete down to depth L = floor(log2 n), where a
+// node holds one tet or two, so node i of depth d < L has the children 2 i and
+// 2 i + 1 of depth d + 1, and the nodes of one depth of one tree are
+// consecutive in memory.  A block takes 256 consecutive nodes of depth L: a
+// thread projects its node's one or two tets (written as leaves of depth L + 1
+// when there are two), and the block unites the 256 records in shared memory
+// up to their common ancestor and writes each level's records as one
+// consecutive range.  The next launch starts from the 1/256 as many ancestors.
 // In pose or deform mode the refit first poses every vertex once
 // (narrow_update_kdop_bvh.h:154-165 on the device, in the same call and the
 // same graph) into a scene-owned array the leaves read: posing inside the leaf
 // pass would transform each vertex once per tet that uses it (about 24 times
-// in a lattice).  The upper levels, too small to fill the GPU, are refitted by
-// one block that walks them with block barriers.
+// in a lattice).
+// Bound: the L1 data pipe (77 % of its peak at K = 14: the leaves' vertex
+// gathers, the shared-memory unions, the records' stores), then HBM (47 %).
+// Each node record is written once; a launch per level wrote every one, read it
+// again for its parent and gathered a leaf's tet through the record's topology
+// words, which now come from arrays in leaf order.  Steps before -> after: 64
+// deforming pairs of 384 k tets (K = 18) 5.00 -> 3.53 ms, one pair of 1.6 M
+// tets (K = 26) 1.66 -> 1.36 ms, 512 uneven pairs (K = 14) 13.2 -> 12.07 ms,
+// one pair of 6,000 tets 273 -> 202 us.  Not kept: block barriers between the
+// levels and a runtime walk over them (96 trees of 48,000 tets: 217 us against
+// 185), one block fewer per SM (208).
+#include <algorithm>
+
 #include "kdop_device.cuh"
 
 namespace kdop {
 
-// The record of one node: a leaf projects its tet's four (posed) vertices on
-// the K/2 directions (make_dop), an internal node takes the union of its two
-// children chunk by chunk (make_union); the topology words are kept.  Chunk
-// j of both children is one aligned 32-byte word of their twin record.
-template <int K, bool LDG>
-__device__ __forceinline__ void refit_node(float4* nodes, int64_t node, const uint4* __restrict__ tets,
-                                           const VertexSource& vs, const DirTable& dt) {
-  using L = NodeLayout<K>;
-  const float4 tc = LDG ? __ldg(nodes + L::at(node, L::TOPO_CHUNK)) : nodes[L::at(node, L::TOPO_CHUNK)];
-  const uint32_t w0 = L::word0(tc), w1 = L::word1(tc);
-  float w[4 * L::NW];
+__device__ __forceinline__ void stg256(float4* p, const float* a, const float* b) {
+  asm volatile("st.global.v8.f32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8};" ::"l"(p), "f"(a[0]), "f"(a[1]), "f"(a[2]),
+               "f"(a[3]), "f"(b[0]), "f"(b[1]), "f"(b[2]), "f"(b[3])
+               : "memory");
+}
+
+// Components of the unit corner and edge directions of the direction tables.
+struct DirScale {
+  float corner, edge;
+};
+
+// Projections of a point on the K/2 directions: dot3(d, p) = ((0 + d.x p.x) +
+// d.y p.y) + d.z p.z for the axes, (1, +-1, +-1) corner and edge directions of
+// the tables, with the products the directions share computed once (a product
+// with -c is the negative of that with c; x * 1 is x; products with 0 stay,
+// they carry infinities and NaN).  42 multiplications and additions become 20
+// at K = 14.
+template <int K>
+__device__ __forceinline__ void project(float4 q, DirScale ds, float* p) {
+  constexpr bool AXES = K == 6 || K == 14 || K == 18 || K == 26;
+  constexpr bool CORNERS = K == 8 || K == 14 || K == 20 || K == 26;
+  constexpr bool EDGES = K == 12 || K == 18 || K == 20 || K == 26;
+  const float zy = fmul(q.y, 0.f), zz = fmul(q.z, 0.f), z0 = fadd(0.f, fmul(q.x, 0.f));
+  int n = 0;
+  if (AXES) {
+    p[n++] = fadd(fadd(fadd(0.f, q.x), zy), zz);
+    p[n++] = fadd(fadd(z0, q.y), zz);
+    p[n++] = fadd(fadd(z0, zy), q.z);
+  }
+  if (CORNERS) {
+    const float x = fadd(0.f, fmul(q.x, ds.corner)), y = fmul(q.y, ds.corner), z = fmul(q.z, ds.corner);
+    const float a = fadd(x, y), b = fsub(x, y);
+    p[n++] = fadd(a, z);
+    p[n++] = fsub(a, z);
+    p[n++] = fadd(b, z);
+    p[n++] = fsub(b, z);
+  }
+  if (EDGES) {
+    const float ex = fmul(q.x, ds.edge), y = fmul(q.y, ds.edge), z = fmul(q.z, ds.edge);
+    const float x = fadd(0.f, ex);
+    p[n++] = fadd(fadd(x, y), zz);
+    p[n++] = fadd(fsub(x, y), zz);
+    p[n++] = fadd(fadd(x, zy), z);
+    p[n++] = fadd(fadd(z0, y), z);
+    p[n++] = fadd(fadd(fsub(0.f, ex), zy), z);
+    p[n++] = fadd(fsub(z0, y), z);
+  }
+}
+
+// Slabs of a tet with vertices v (make_dop).  A projection is a sum that
+// starts from +0, so it is never -0, and the running bounds start finite:
+// fminf / fmaxf (one instruction; a NaN operand is dropped) give the values
+// of the reference's std::min / std::max.
+template <int K>
+__device__ __forceinline__ void leaf_slabs(const float4* __restrict__ world, uint4 v, DirScale ds, float* w) {
+  const float4 q[4] = {__ldg(world + v.x), __ldg(world + v.y), __ldg(world + v.z), __ldg(world + v.w)};
+  float p[4][K / 2];
 #pragma unroll
-  for (int k = 0; k < 4 * L::NW; ++k) w[k] = 0.f;
-  if (w0 & LEAF_BIT) {
-    const uint4 t = __ldg(tets + w1);
-    const f3 p[4] = {world_vertex(vs, t.x), world_vertex(vs, t.y), world_vertex(vs, t.z), world_vertex(vs, t.w)};
+  for (int u = 0; u < 4; ++u) project<K>(q[u], ds, p[u]);
+  constexpr float big = 3.40282346638528859812e+38f;
 #pragma unroll
-    for (int s = 0; s < L::NS; ++s) {
-      const f3 d = mk3(dt.d[s][0], dt.d[s][1], dt.d[s][2]);
-      float lo = 3.40282346638528859812e+38f, hi = -3.40282346638528859812e+38f;
+  for (int s = 0; s < K / 2; ++s) {
+    w[2 * s] = fminf(fminf(fminf(big, p[0][s]), p[1][s]), fminf(p[2][s], p[3][s]));
+    w[2 * s + 1] = fmaxf(fmaxf(fmaxf(-big, p[0][s]), p[1][s]), fmaxf(p[2][s], p[3][s]));
+  }
+}
+
+constexpr int kRefitUp = 8;                    // levels a block unites above its nodes
+constexpr int kRefitSlots = 1 << kRefitUp;     // nodes a block starts from
+// Shared-memory row of one record word: the block's nodes in heap order (root
+// 1).  The stride keeps the words of a chunk and the nodes of eight twins on
+// different banks, and node pairs 8-byte aligned.
+constexpr int kRefitRow = 2 * kRefitSlots + 2;
+template <int K>
+constexpr size_t refit_smem() {
+  return (size_t)K * kRefitRow * 4 + kRefitSlots * 8;
+}
+
+struct RefitArgs {
+  float4* nodes;
+  const RefitBlock* blocks;
+  const uint4* leaf_verts;
+  const uint32_t* leaf_tet;
+  const float4* world;
+  DirScale ds;
+};
+
+// Slab x of node U of the block's heap: the union of its children (make_union;
+// slabs hold no NaN and no -0, so fminf / fmaxf are the reference's choices).
+__device__ __forceinline__ void unite_slab(float* T, uint32_t U, int x) {
+  float* row = T + 2 * x * kRefitRow;
+  const float2 lo = *reinterpret_cast<const float2*>(row + 2 * U);
+  const float2 hi = *reinterpret_cast<const float2*>(row + kRefitRow + 2 * U);
+  row[U] = fminf(lo.x, lo.y);
+  row[kRefitRow + U] = fmaxf(hi.x, hi.y);
+}
+// The 2^M nodes M levels below `root`, a slab of a node per lane.
+template <int K, int M>
+__device__ __forceinline__ void unite_level(float* T, uint32_t root, int lane) {
+  constexpr int N = (K / 2) << M;
 #pragma unroll
-      for (int v = 0; v < 4; ++v) {
-        const float pr = dot3(d, p[v]);
-        lo = smin(lo, pr);
-        hi = smax(hi, pr);
-      }
-      w[2 * s] = lo;
-      w[2 * s + 1] = hi;
-    }
-  } else {
-    const float4* c = nodes + L::at(w0, 0);  // chunk 0 of child w0; child w0 + 1 follows each chunk
+  for (int it = 0; it * 32 < N; ++it)
+    if ((it + 1) * 32 <= N || it * 32 + lane < N)
+      unite_slab(T, (root << M) + (uint32_t)(lane & ((1 << M) - 1)), (lane >> M) + it * (32 >> M));
+  __syncwarp();
+}
+
+// Chunk j of the twin of the children of heap node U to `to`; the topology
+// words of its two nodes are we, wo.
+template <int K>
+__device__ __forceinline__ void put_chunk(const float* T, uint32_t U, int j, uint2 we, uint2 wo, float4* to) {
+  const float* col = T + 4 * j * kRefitRow + 2 * U;
+  float e[4], o[4];
 #pragma unroll
-    for (int j = 0; j < L::NW; ++j) {
-      float4 a, b;
-      if (LDG) {
-        a = __ldg(c + 2 * j);
-        b = __ldg(c + 2 * j + 1);
-      } else {
-        a = c[2 * j];
-        b = c[2 * j + 1];
-      }
-      // lo: min(A.lo, B.lo) = (B < A) ? B : A ; hi: max(A.hi, B.hi) = (A < B) ? B : A
-      if (2 * j < L::NS) {
-        w[4 * j] = smin(a.x, b.x);
-        w[4 * j + 1] = smax(a.y, b.y);
-      }
-      if (2 * j + 1 < L::NS) {
-        w[4 * j + 2] = smin(a.z, b.z);
-        w[4 * j + 3] = smax(a.w, b.w);
-      }
+  for (int c = 0; c < 4; ++c) {
+    e[c] = o[c] = 0.f;
+    if (4 * j + c < K) {
+      const float2 x = *reinterpret_cast<const float2*>(col + c * kRefitRow);
+      e[c] = x.x;
+      o[c] = x.y;
     }
   }
-  w[L::TOPO_ZW ? 4 * L::TOPO_CHUNK + 2 : 4 * L::TOPO_CHUNK] = __uint_as_float(w0);
-  w[L::TOPO_ZW ? 4 * L::TOPO_CHUNK + 3 : 4 * L::TOPO_CHUNK + 1] = __uint_as_float(w1);
+  if (j == NodeLayout<K>::TOPO_CHUNK) {
+    constexpr int c = K % 4;
+    e[c] = __uint_as_float(we.x);
+    e[c + 1] = __uint_as_float(we.y);
+    o[c] = __uint_as_float(wo.x);
+    o[c + 1] = __uint_as_float(wo.y);
+  }
+  stg256(to, e, o);
+}
+// The twins of the children of the 2^M nodes M levels below heap node `root`,
+// which is the at-th of its level: consecutive records from node `first` on; a
+// chunk per lane, so that a warp writes 1 KB in a row.  kids: first child of
+// the first of them; words: their topology words instead, where they are the
+// block's own nodes.
+template <int K, int M>
+__device__ __forceinline__ void put_level(float4* nodes, const float* T, uint32_t root, uint32_t first, uint32_t kids,
+                                          const uint2* words, int lane) {
+  constexpr int NW = NodeLayout<K>::NW, N = NW << M;
+  float4* to = nodes + NodeLayout<K>::at(first, 0) + 2 * lane;
 #pragma unroll
-  for (int j = 0; j < L::NW; ++j)
-    nodes[L::at(node, j)] = make_float4(w[4 * j], w[4 * j + 1], w[4 * j + 2], w[4 * j + 3]);
+  for (int it = 0; it * 32 < N; ++it) {
+    if ((it + 1) * 32 > N && it * 32 + lane >= N) continue;
+    constexpr bool pow2 = (NW & (NW - 1)) == 0;
+    constexpr int sh = NW == 1 ? 0 : NW == 2 ? 1 : 2;
+    const int r = pow2 ? (lane >> sh) + it * (32 >> sh) : (it * 32 + lane) / NW;
+    const int j = pow2 ? lane & (NW - 1) : (it * 32 + lane) % NW;
+    const uint32_t k = kids + 4u * (uint32_t)r;
+    uint2 we = make_uint2(k, k + 1u), wo = make_uint2(k + 2u, k + 3u);
+    if (words) {
+      we = words[2 * r];
+      wo = words[2 * r + 1];
+    }
+    put_chunk<K>(T, (root << M) + (uint32_t)r, j, we, wo, to + 64 * it);
+  }
 }
 
-// One level of every tree, thread per node.
-template <int K>
-__global__ void __launch_bounds__(256) refit_level_kernel(float4* nodes, int64_t begin, int64_t count,
-                                                          const uint4* __restrict__ tets, VertexSource vs,
-                                                          DirTable dt) {
-  int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (t >= count) return;
-  refit_node<K, true>(nodes, begin + t, tets, vs, dt);
-}
-
-// Depths [0, top] of every tree: one block per tree.  The block lists its
-// tree's nodes of those depths top-down from the root (children from the
-// topology words), then refits them bottom-up, a block barrier per depth
-// (plain loads: the block reads records it wrote itself; the children of
-// depth `top` were refitted by the level launches before it).  One launch
-// replaces the per-level launches of the forest's small top levels, each of
-// which was bound by launch and load latency.  The padding node that may end
-// the root level (a copy of the first root's topology) is refitted by the
-// block of the tree rooted at node 0.
-constexpr int kTopDepth = 6;
-constexpr int kTopNodes = 2 << kTopDepth;  // >= 2^(kTopDepth + 1) - 1 nodes of a tree's top
-
-template <int K>
-__global__ void __launch_bounds__(256) refit_top_kernel(float4* nodes, const uint32_t* __restrict__ root, int top,
-                                                        uint32_t pad_node, const uint4* __restrict__ tets,
-                                                        VertexSource vs, DirTable dt) {
+// BOTTOM: from the tets of the nodes of depth L; else from the records of the
+// block's nodes, written by the launch before.  A warp unites its 32 nodes and
+// writes their levels by itself (no block barrier); the first warp does the
+// last levels from the warps' ancestors.
+template <int K, bool BOTTOM>
+__global__ void __launch_bounds__(kRefitSlots, K <= 8 ? 6 : K <= 14 ? 5 : K <= 20 ? 4 : 3)
+    refit_kernel(const __grid_constant__ RefitArgs a) {
   using L = NodeLayout<K>;
-  __shared__ uint32_t ids[kTopNodes];
-  __shared__ int lev[kTopDepth + 2];  // nodes of depth d: ids[lev[d] .. lev[d + 1])
-  __shared__ int fill;
-  const uint32_t r = root[blockIdx.x];
-  if (r == NO_NODE) return;  // empty mesh: the whole block leaves
-  if (threadIdx.x == 0) {
-    ids[0] = r;
-    lev[0] = 0;
-    lev[1] = 1;
-    fill = 1;
+  constexpr int NW = L::NW, NS = L::NS;
+  extern __shared__ float T[];  // T[w * kRefitRow + heap index]
+  uint2* slot_words = reinterpret_cast<uint2*>(T + K * kRefitRow);
+  const RefitBlock& b = a.blocks[blockIdx.x];
+  const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
+  const int hd = b.levels;             // levels above the block's nodes in this block
+  const int cnt = 1 << hd;             // its nodes
+  const int wl = min(hd, 5);           // levels within a warp
+  const int warps = cnt >> wl;         // warps with nodes
+  const uint32_t root = (uint32_t)(warps + wib);  // this warp's ancestor in the block's heap
+  if (wib < warps) {
+    const int t = (wib << wl) + lane;  // this thread's node of the block
+    if (BOTTOM) {
+      const bool act = lane < (1 << wl);
+      // The left half takes the odd tet at every split, so of 2^h nodes below
+      // an ancestor with r tets more than nodes the j-th in bit-reversed order
+      // holds two when j < r: the block's extra tets over its warps, then the
+      // warp's over its lanes.
+      const uint32_t extra = b.tets - (uint32_t)cnt;
+      const int wb = hd - wl;  // bits of a warp's number
+      uint32_t before = 0, mine = extra;
+      if (wb) {
+#pragma unroll
+        for (int w = 0; w < kRefitSlots / 32; ++w) {
+          const uint32_t x = (extra + (1u << wb) - 1u - (__brev((uint32_t)w) >> (32 - wb))) >> wb;
+          if (w < wib) before += x;
+          if (w == wib) mine = x;
+        }
+      }
+      const uint32_t rev = wl ? __brev((uint32_t)lane) >> (32 - wl) : 0u;
+      const bool two = act && rev < mine;
+      const unsigned twos = __ballot_sync(0xffffffffu, two);
+      before += __popc(twos & ((1u << lane) - 1u));  // two-tet nodes of the block before this one
+      if (act) {
+        // a node of one tet takes it twice (the union with itself)
+        const size_t at = (size_t)b.first_leaf + t + before;
+        const uint4 va = __ldg(a.leaf_verts + at), vb = __ldg(a.leaf_verts + at + (two ? 1 : 0));
+        const uint32_t t0 = __ldg(a.leaf_tet + at), t1 = __ldg(a.leaf_tet + at + (two ? 1 : 0));
+        float w[4 * NW], v[4 * NW];
+#pragma unroll
+        for (int c = 0; c < 4 * NW; ++c) w[c] = v[c] = 0.f;
+        leaf_slabs<K>(a.world, va, a.ds, w);
+        leaf_slabs<K>(a.world, vb, a.ds, v);
+        uint2 words = make_uint2(LEAF_BIT | (t0 & SURF_BIT) | (b.node[hd] + t), t0 & NODE_MASK);
+        if (two) {
+          // two leaves: their twin of depth L + 1
+          const uint32_t c = b.leaf_twin + 2u * before;
+          w[K] = __uint_as_float(LEAF_BIT | (t0 & SURF_BIT) | c);
+          w[K + 1] = __uint_as_float(t0 & NODE_MASK);
+          v[K] = __uint_as_float(LEAF_BIT | (t1 & SURF_BIT) | (c + 1u));
+          v[K + 1] = __uint_as_float(t1 & NODE_MASK);
+          float4* to = a.nodes + L::at(c, 0);
+#pragma unroll
+          for (int j = 0; j < NW; ++j) stg256(to + 2 * j, w + 4 * j, v + 4 * j);
+          words = make_uint2(c, c + 1u);
+        }
+        slot_words[t] = words;
+#pragma unroll
+        for (int k = 0; k < K; k += 2) {
+          T[k * kRefitRow + cnt + t] = fminf(w[k], v[k]);
+          T[(k + 1) * kRefitRow + cnt + t] = fmaxf(w[k + 1], v[k + 1]);
+        }
+      }
+    } else {
+      // records of the warp's 2^wl >= 2 consecutive nodes (whole twins)
+      const float4* from = a.nodes + L::at(b.node[hd] + (wib << wl), 0);
+      for (int q = lane; q < (NW << wl); q += 32) {
+        const float4 x = from[q];
+        const int i = (wib << wl) + 2 * (q / (2 * NW)) + (q & 1), j = (q % (2 * NW)) >> 1;
+        const float e[4] = {x.x, x.y, x.z, x.w};
+#pragma unroll
+        for (int c = 0; c < 4; ++c)
+          if (4 * j + c < K) T[(4 * j + c) * kRefitRow + cnt + i] = e[c];
+      }
+    }
+    __syncwarp();
+    if (wl == 5) {
+      unite_level<K, 4>(T, root, lane);
+      unite_level<K, 3>(T, root, lane);
+      unite_level<K, 2>(T, root, lane);
+      unite_level<K, 1>(T, root, lane);
+      unite_level<K, 0>(T, root, lane);
+      // levels from the block's own nodes up: those M + 1 levels below the
+      // warp's ancestor start at node 2^(M + 1) wib of their level
+      const uint32_t w = (uint32_t)wib;
+      if (BOTTOM)
+        put_level<K, 4>(a.nodes, T, root, b.node[hd] + 32u * w, 0u, slot_words + 32 * wib, lane);
+      put_level<K, 3>(a.nodes, T, root, b.node[hd - 1] + 16u * w, b.node[hd] + 32u * w, nullptr, lane);
+      put_level<K, 2>(a.nodes, T, root, b.node[hd - 2] + 8u * w, b.node[hd - 1] + 16u * w, nullptr, lane);
+      put_level<K, 1>(a.nodes, T, root, b.node[hd - 3] + 4u * w, b.node[hd - 2] + 8u * w, nullptr, lane);
+      put_level<K, 0>(a.nodes, T, root, b.node[hd - 4] + 2u * w, b.node[hd - 3] + 4u * w, nullptr, lane);
+    } else {
+      // a tree of fewer than 64 tets (or its last levels): one warp, level by level
+      for (int m = wl - 1; m >= 0; --m) {
+        for (int x = lane; x < (NS << m); x += 32) unite_slab(T, (1u << m) + (x & ((1 << m) - 1)), x >> m);
+        __syncwarp();
+      }
+      for (int m = BOTTOM ? wl - 1 : wl - 2; m >= 0; --m)
+        for (int q = lane; q < (NW << m); q += 32) {
+          const uint32_t r = (uint32_t)(q / NW);
+          const uint32_t k = m + 2 <= hd ? b.node[m + 2] + 4u * r : 0u;
+          uint2 we = make_uint2(k, k + 1u), wo = make_uint2(k + 2u, k + 3u);
+          if (m + 1 == hd) {
+            we = slot_words[2 * r];
+            wo = slot_words[2 * r + 1];
+          }
+          put_chunk<K>(T, (1u << m) + r, q % NW, we, wo, a.nodes + L::at(b.node[m + 1], 0) + 2 * q);
+        }
+    }
   }
   __syncthreads();
-  for (int d = 0; d < top; ++d) {
-    const int b = lev[d], e = lev[d + 1];
-    for (int i = b + (int)threadIdx.x; i < e; i += blockDim.x) {
-      const uint32_t w0 = L::word0(__ldg(nodes + L::at(ids[i], L::TOPO_CHUNK)));
-      if (!(w0 & LEAF_BIT)) {
-        const int at = atomicAdd(&fill, 2);
-        ids[at] = w0 & NODE_MASK;
-        ids[at + 1] = (w0 & NODE_MASK) + 1u;
-      }
-    }
-    __syncthreads();
-    if (threadIdx.x == 0) lev[d + 2] = fill;
-    __syncthreads();
+  if (wib > 0) return;
+  for (int n = warps >> 1; n >= 1; n >>= 1) {
+    for (int x = lane; x < n * NS; x += 32) unite_slab(T, (uint32_t)(n + x % n), x / n);
+    __syncwarp();
   }
-  for (int d = top; d >= 0; --d) {
-    for (int i = lev[d] + (int)threadIdx.x; i < lev[d + 1]; i += blockDim.x)
-      refit_node<K, false>(nodes, ids[i], tets, vs, dt);
-    if (d == 0 && r == 0u && pad_node != NO_NODE && threadIdx.x == blockDim.x - 1)
-      refit_node<K, false>(nodes, pad_node, tets, vs, dt);
-    __syncthreads();
+  for (int q = lane; q < (warps - 1) * NW; q += 32) {
+    // the twin below heap node U
+    const uint32_t U = (uint32_t)(q / NW) + 1u;
+    const int l = 32 - __clz(U);
+    const uint32_t i = 2 * U - (1u << l), k = b.node[l + 1] + 2u * i;
+    const int j = q % NW;
+    put_chunk<K>(T, U, j, make_uint2(k, k + 1u), make_uint2(k + 2u, k + 3u), a.nodes + L::at(b.node[l] + i, j));
+  }
+  // the common ancestor: one half of a twin
+  if (lane < NW) {
+    const uint2 words = (BOTTOM && hd == 0) ? slot_words[0] : make_uint2(b.node[1], b.node[1] + 1u);
+    float e[4];
+#pragma unroll
+    for (int c = 0; c < 4; ++c) {
+      const int w = 4 * lane + c;
+      e[c] = w < K ? T[w * kRefitRow + 1]
+                   : w == K ? __uint_as_float(words.x) : w == K + 1 ? __uint_as_float(words.y) : 0.f;
+    }
+    a.nodes[L::at(b.node[0], lane)] = make_float4(e[0], e[1], e[2], e[3]);
+    if (b.pad_node != NO_NODE) {
+      // the root level's padding node: the root again (a leaf under its own index)
+#pragma unroll
+      for (int c = 0; c < 4; ++c)
+        if (4 * lane + c == K && (words.x & LEAF_BIT))
+          e[c] = __uint_as_float((words.x & (LEAF_BIT | SURF_BIT)) | b.pad_node);
+      a.nodes[L::at(b.pad_node, lane)] = make_float4(e[0], e[1], e[2], e[3]);
+    }
+  }
+}
+
+// Tets in leaf order, from the topology words of the nodes of depth L and
+// L + 1: vertex indices, and the tet with its surface bit.  A block per block
+// of the refit's first launch.
+template <int K>
+__global__ void __launch_bounds__(kRefitSlots) leaf_table_kernel(const float4* __restrict__ nodes,
+                                                                 const RefitBlock* __restrict__ blocks,
+                                                                 const uint4* __restrict__ tets, uint4* leaf_verts,
+                                                                 uint32_t* leaf_tet) {
+  using L = NodeLayout<K>;
+  const RefitBlock& b = blocks[blockIdx.x];
+  if ((int)threadIdx.x >= (1 << b.levels)) return;
+  uint32_t f = 0, s = b.tets;
+  for (int k = b.levels - 1; k >= 0; --k) {
+    const uint32_t left = s - (s >> 1);
+    if ((threadIdx.x >> k) & 1u) f += left;
+    s = ((threadIdx.x >> k) & 1u) ? s >> 1 : left;
+  }
+  const float4 x = nodes[L::at(b.node[b.levels] + threadIdx.x, L::TOPO_CHUNK)];
+  const uint32_t node = L::word0(x) & NODE_MASK;  // a leaf's own index, or its first child
+  for (uint32_t c = 0; c < s; ++c) {
+    const float4 y = nodes[L::at(node + c, L::TOPO_CHUNK)];
+    const uint32_t tet = L::word1(y);
+    leaf_verts[(size_t)b.first_leaf + f + c] = tets[tet];
+    leaf_tet[(size_t)b.first_leaf + f + c] = tet | (L::word0(y) & SURF_BIT);
   }
 }
 
@@ -254,34 +486,116 @@ static VertexSource vertex_source(kdop_scene* s, int mode) {
 template <int K>
 static cudaError_t refit_impl(kdop_scene* s, int mode) {
   VertexSource vs = vertex_source(s, mode);
+  const float4* world = s->world;
   if (mode != KDOP_REFIT_VERTICES && s->nv > 0) {
     // pose (and deform) every vertex once; the leaves then read world
     // positions instead of transforming each vertex once per tet using it
     world_kernel<<<(unsigned)((s->nv + 255) / 256), 256, 0, s->ctx->stream>>>(s->nv, vs, s->posed);
     s->ctx->launches++;
-    vs = vertex_source(s, KDOP_REFIT_VERTICES);
-    vs.world = s->posed;
+    world = s->posed;
   }
-  int levels = (int)s->level_off.size() - 1;
-  if (levels <= 0) return cudaSuccess;
-  // depths [0, top] of every tree in one launch (a block per tree), the
-  // deeper levels one launch each, deepest first
-  const int top = std::min(kTopDepth, levels - 1);
-  for (int d = levels - 1; d > top; --d) {
-    int64_t b = s->level_off[d], n = s->level_off[d + 1] - b;
-    unsigned grid = (unsigned)((n + 255) / 256);
-    refit_level_kernel<K><<<grid, 256, 0, s->ctx->stream>>>(s->nodes, b, n, s->tets, vs, s->dirs);
+  // the direction tables list axes, corners, edges (K = 14: 3 axes, 4 corners)
+  constexpr int axes = (K == 6 || K == 14 || K == 18 || K == 26) ? 3 : 0;
+  constexpr int corners = (K == 8 || K == 14 || K == 20 || K == 26) ? 4 : 0;
+  RefitArgs a;
+  a.nodes = s->nodes;
+  a.leaf_verts = s->leaf_verts;
+  a.leaf_tet = s->leaf_tet;
+  a.world = world;
+  a.ds.corner = corners ? s->dirs.d[axes][0] : 0.f;
+  a.ds.edge = axes + corners < K / 2 ? s->dirs.d[axes + corners][0] : 0.f;
+  constexpr size_t smem = refit_smem<K>();
+  cudaError_t e = cudaFuncSetAttribute(refit_kernel<K, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  if (e == cudaSuccess)
+    e = cudaFuncSetAttribute(refit_kernel<K, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  if (e != cudaSuccess) return e;
+  for (size_t i = 0; i + 1 < s->refit_stage.size(); ++i) {
+    const unsigned n = (unsigned)(s->refit_stage[i + 1] - s->refit_stage[i]);
+    a.blocks = s->refit_blocks + s->refit_stage[i];
+    if (i == 0)
+      refit_kernel<K, true><<<n, kRefitSlots, smem, s->ctx->stream>>>(a);
+    else
+      refit_kernel<K, false><<<n, kRefitSlots, smem, s->ctx->stream>>>(a);
     s->ctx->launches++;
   }
+  return cudaGetLastError();
+}
+
+// Blocks of each launch of a refit (launch i: blocks stage[i] .. stage[i + 1]):
+// one per 256 nodes of depth L - 8 i of every tree.  pre: nodes of the trees
+// before m at depth d; t_off: first tet of a mesh.
+void refit_blocks(const ForestBuild& fb, const std::vector<int64_t>& pre, const std::vector<int32_t>& lg,
+                  const std::vector<int64_t>& n_tets, const std::vector<int64_t>& t_off,
+                  std::vector<RefitBlock>& blocks, std::vector<int64_t>& stage) {
+  blocks.clear();
+  stage.assign(1, 0);
+  const size_t nm = lg.size();
+  const int levels = (int)fb.level_off.size() - 1;
+  auto base = [&](size_t m, int d) -> uint32_t {
+    return d < levels ? (uint32_t)(fb.level_off[d] + pre[(size_t)d * (nm + 1) + m]) : 0u;
+  };
   // the root level holds one padding node after the real roots when their
-  // count is odd
+  // count is odd: the first tree's root again
   int64_t n_roots = 0;
-  for (int m = 0; m < s->n_meshes; ++m) n_roots += (s->t_off[m + 1] > s->t_off[m]) ? 1 : 0;
-  const uint32_t pad = (s->level_off[1] - s->level_off[0] > n_roots) ? (uint32_t)(s->level_off[1] - 1) : NO_NODE;
-  refit_top_kernel<K><<<(unsigned)s->n_meshes, 256, 0, s->ctx->stream>>>(s->nodes, s->root_dev, top, pad, s->tets,
-                                                                         vs, s->dirs);
+  for (size_t m = 0; m < nm; ++m) n_roots += lg[m] >= 0 ? 1 : 0;
+  uint32_t pad = NO_NODE;
+  if (n_roots > 0 && fb.level_off[1] - fb.level_off[0] > n_roots) pad = (uint32_t)(fb.level_off[1] - 1);
+  size_t first = 0;
+  while (first < nm && lg[first] < 0) ++first;
+  std::vector<std::pair<uint32_t, uint32_t>> range, next;  // tets [f, f + s) of the nodes of one depth
+  for (int i = 0;; ++i) {
+    for (size_t m = 0; m < nm; ++m) {
+      const int d = lg[m] - kRefitUp * i;  // depth 0 is done by the launch before, or is a single node
+      if (lg[m] < 0 || d < 0 || (i > 0 && d == 0)) continue;
+      const int hd = std::min(d, kRefitUp), d0 = d - hd;
+      range.assign(1, std::make_pair(0u, (uint32_t)n_tets[m]));
+      for (int k = 0; k < d0; ++k) {
+        next.clear();
+        for (const auto& r : range) {
+          const uint32_t left = r.second - (r.second >> 1);
+          next.push_back(std::make_pair(r.first, left));
+          next.push_back(std::make_pair(r.first + left, r.second - left));
+        }
+        range.swap(next);
+      }
+      for (size_t j = 0; j < range.size(); ++j) {
+        RefitBlock b;
+        b.first_leaf = (uint32_t)t_off[m] + range[j].first;
+        b.tets = range[j].second;
+        // two-tet nodes before the block's: its first tet less its first node
+        b.leaf_twin = base(m, lg[m] + 1) + 2u * (range[j].first - (uint32_t)(j << hd));
+        b.levels = hd;
+        for (int l = 0; l <= kRefitUp; ++l) b.node[l] = l <= hd ? base(m, d0 + l) + (uint32_t)(j << l) : 0u;
+        b.pad_node = (d0 == 0 && m == first) ? pad : NO_NODE;
+        b.pad[0] = b.pad[1] = 0;
+        blocks.push_back(b);
+      }
+    }
+    if ((int64_t)blocks.size() == stage.back()) break;
+    stage.push_back((int64_t)blocks.size());
+  }
+}
+
+template <int K>
+static cudaError_t leaf_tables_impl(kdop_scene* s) {
+  if (s->refit_stage.size() < 2) return cudaSuccess;
+  leaf_table_kernel<K><<<(unsigned)s->refit_stage[1], kRefitSlots, 0, s->ctx->stream>>>(
+      s->nodes, s->refit_blocks, s->tets, s->leaf_verts, s->leaf_tet);
   s->ctx->launches++;
   return cudaGetLastError();
+}
+
+cudaError_t launch_leaf_tables(kdop_scene* s) {
+  switch (s->K) {
+    case 6: return leaf_tables_impl<6>(s);
+    case 8: return leaf_tables_impl<8>(s);
+    case 12: return leaf_tables_impl<12>(s);
+    case 14: return leaf_tables_impl<14>(s);
+    case 18: return leaf_tables_impl<18>(s);
+    case 20: return leaf_tables_impl<20>(s);
+    case 26: return leaf_tables_impl<26>(s);
+  }
+  return cudaErrorInvalidValue;
 }
 
 cudaError_t launch_refit(kdop_scene* s, int mode) {
