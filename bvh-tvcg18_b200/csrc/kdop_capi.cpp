@@ -21,6 +21,7 @@ namespace {
 const int64_t kDefaultCand = 1 << 20;
 const int64_t kDefaultContacts = 1 << 20;
 const int64_t kDefaultQueue = 1 << 20;
+const int64_t kReadFloats = 16 << 20;  // words a read-back stages on the device at a time
 
 int fail(kdop_ctx* ctx, int status, const std::string& msg) {
   if (ctx) ctx->err = msg;
@@ -565,34 +566,22 @@ int kdop_read_tree(kdop_scene* s, int mesh, int64_t cap, float* vol, int64_t* te
   if (cap < *n_nodes) return fail(s->ctx, KDOP_ERR_CAPACITY, "tree read buffer too small");
   if (!vol || !tet) return KDOP_ERR_INVALID;
   cudaSetDevice(s->ctx->device);
-  std::vector<float> rec((size_t)(s->nn * s->NW * 4));
-  KDOP_CUDA(s->ctx, cudaMemcpyAsync(rec.data(), s->nodes, rec.size() * 4, cudaMemcpyDeviceToHost, s->ctx->stream));
-  KDOP_CUDA(s->ctx, cudaStreamSynchronize(s->ctx->stream));
-  const int tw = s->K;  // word index of `start`
-  std::vector<uint32_t> stack(1, s->root[mesh]);
-  int64_t k = 0;
-  while (!stack.empty()) {
-    uint32_t n = stack.back();
-    stack.pop_back();
-    // chunk j of node n sits at float4 2 NW (n / 2) + 2 j + n % 2 (twin records)
-    float r[32];  // NW <= 7 chunks
-    for (int j = 0; j < s->NW; ++j)
-      std::memcpy(r + 4 * j, &rec[4 * (size_t)((int64_t)(n >> 1) * 2 * s->NW + 2 * j + (n & 1))], 16);
-    // topology words: leaf (LEAF_BIT | flags | own index, tet), internal (c, c + 1)
-    uint32_t w0, w1;
-    std::memcpy(&w0, r + tw, 4);
-    std::memcpy(&w1, r + tw + 1, 4);
-    if (k >= *n_nodes) return fail(s->ctx, KDOP_ERR_STATE, "tree walk overran the node count");
-    std::memcpy(vol + k * s->K, r, (size_t)s->K * 4);
-    if (w0 & kdop::LEAF_BIT_HOST) {
-      tet[k] = (int64_t)w1 - s->t_off[mesh];
-    } else {
-      tet[k] = -1;
-      stack.push_back(w1);
-      stack.push_back(w0);
-    }
-    ++k;
+  // gathered in preorder on the device, a window at a time: tets (8-byte
+  // aligned), then slabs
+  const int64_t window = std::min<int64_t>(*n_nodes, kReadFloats / (s->K + 2));
+  cudaError_t e;
+  float* d = stage(s, window * (s->K + 2), &e);
+  if (!d) return cuda_fail(s->ctx, e, "staging alloc");
+  int64_t* d_tet = reinterpret_cast<int64_t*>(d);
+  float* d_vol = d + 2 * window;
+  for (int64_t at = 0; at < *n_nodes; at += window) {
+    const int64_t n = std::min(window, *n_nodes - at);
+    KDOP_CUDA(s->ctx, kdop::launch_preorder(s, mesh, at, n, d_vol, d_tet));
+    KDOP_CUDA(s->ctx, cudaMemcpyAsync(vol + at * s->K, d_vol, (size_t)n * s->K * 4, cudaMemcpyDeviceToHost,
+                                      s->ctx->stream));
+    KDOP_CUDA(s->ctx, cudaMemcpyAsync(tet + at, d_tet, (size_t)n * 8, cudaMemcpyDeviceToHost, s->ctx->stream));
   }
+  KDOP_CUDA(s->ctx, cudaStreamSynchronize(s->ctx->stream));
   return KDOP_OK;
 }
 
@@ -1001,19 +990,17 @@ int kdop_read_candidates(kdop_scene* s, uint32_t* rows, int64_t cap, int64_t* n_
   *n_rows = n;
   if (n > cap) return fail(s->ctx, KDOP_ERR_CAPACITY, "candidate read buffer too small");
   if (n == 0) return KDOP_OK;
-  std::vector<uint32_t> h(3 * (size_t)n);
-  for (int k = 0; k < 3; ++k)
-    KDOP_CUDA(s->ctx, cudaMemcpyAsync(h.data() + k * n, s->cand + k * s->cand_cap, (size_t)n * 4,
-                                      cudaMemcpyDeviceToHost, s->ctx->stream));
-  KDOP_CUDA(s->ctx, cudaStreamSynchronize(s->ctx->stream));
-  const std::vector<uint32_t>& ph = ext(s)->pairs_host;
-  for (int64_t i = 0; i < n; ++i) {
-    uint32_t p = h[2 * n + i];
-    uint32_t ma = ph[2 * p], mb = ph[2 * p + 1];
-    rows[3 * i] = p;
-    rows[3 * i + 1] = (uint32_t)((int64_t)h[i] - s->t_off[ma]);
-    rows[3 * i + 2] = (uint32_t)((int64_t)h[n + i] - s->t_off[mb]);
+  const int64_t window = std::min<int64_t>(n, kReadFloats / 3);
+  cudaError_t e;
+  float* d = stage(s, 3 * window, &e);
+  if (!d) return cuda_fail(s->ctx, e, "staging alloc");
+  for (int64_t at = 0; at < n; at += window) {
+    const int64_t m = std::min(window, n - at);
+    KDOP_CUDA(s->ctx, kdop::launch_candidate_rows(s, at, m, (int64_t)ext(s)->pairs_host.size() / 2,
+                                                  reinterpret_cast<uint32_t*>(d)));
+    KDOP_CUDA(s->ctx, cudaMemcpyAsync(rows + 3 * at, d, 3 * (size_t)m * 4, cudaMemcpyDeviceToHost, s->ctx->stream));
   }
+  KDOP_CUDA(s->ctx, cudaStreamSynchronize(s->ctx->stream));
   return KDOP_OK;
 }
 

@@ -239,6 +239,13 @@ void refit_blocks(const ForestBuild& fb, const std::vector<int64_t>& pre, const 
                   std::vector<RefitBlock>& blocks, std::vector<int64_t>& stage);
 cudaError_t launch_leaf_tables(kdop_scene* s);  // leaf_verts, leaf_tet from the node records
 cudaError_t launch_refit(kdop_scene* s, int mode);
+// Rows [first, first + count) of one tree in preorder (kdop_read_tree's rows)
+// into device memory.
+cudaError_t launch_preorder(kdop_scene* s, int mesh, int64_t first, int64_t count, float* vol, int64_t* tet);
+// The last traversal's candidates [first, first + n) as (pair, tet of A, tet
+// of B) rows with mesh-local tets, n_pairs = length of the pair list on the
+// device.
+cudaError_t launch_candidate_rows(kdop_scene* s, int64_t first, int64_t n, int64_t n_pairs, uint32_t* rows);
 cudaError_t launch_traverse(kdop_scene* s, int64_t n_pairs, const uint2* pairs, const TravParams& p, int plain);
 // broad phase (kdop_broad.cu)
 cudaError_t launch_mesh_radius(kdop_scene* s, unsigned* rbits);

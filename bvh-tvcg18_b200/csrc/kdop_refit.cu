@@ -405,6 +405,62 @@ __global__ void write_topology_kernel(float4* nodes, int64_t nn, const uint32_t*
   nodes[t] = o;
 }
 
+// One tree in the reference's preorder: thread per node h of depths 0 .. L in
+// heap numbering, which also takes the two leaves below a two-tet node.  The
+// left half of s tets fills 2 left - 1 places after its parent's.  Only the
+// places [first, first + count) are written (a window of the caller's buffer).
+struct TreeBase {
+  uint32_t base[32];  // first node of each depth
+};
+template <int K>
+__device__ __forceinline__ void put_node(const float4* __restrict__ nodes, uint32_t node, int64_t at, int64_t count,
+                                         uint32_t t_off, float* vol, int64_t* tet) {
+  using L = NodeLayout<K>;
+  if (at < 0 || at >= count) return;
+  uint32_t w0 = 0, w1 = 0;
+#pragma unroll
+  for (int j = 0; j < L::NW; ++j) {
+    const float4 x = nodes[L::at(node, j)];
+    const float e[4] = {x.x, x.y, x.z, x.w};
+#pragma unroll
+    for (int c = 0; c < 4; ++c)
+      if (4 * j + c < K) vol[at * K + 4 * j + c] = e[c];
+    if (j == L::TOPO_CHUNK) {
+      w0 = L::word0(x);
+      w1 = L::word1(x);
+    }
+  }
+  tet[at] = (w0 & LEAF_BIT) ? (int64_t)w1 - (int64_t)t_off : -1;
+}
+template <int K>
+__global__ void __launch_bounds__(256) preorder_kernel(const float4* __restrict__ nodes, TreeBase b, uint32_t n_tets,
+                                                       int depth, uint32_t t_off, int64_t first, int64_t count,
+                                                       float* vol, int64_t* tet) {
+  const uint32_t h = blockIdx.x * 256 + threadIdx.x + 1;
+  if (h >= (2u << depth)) return;
+  const int d = 31 - __clz(h);
+  uint32_t s = n_tets;
+  int64_t at = -first;
+  for (int k = d - 1; k >= 0; --k) {
+    const uint32_t left = s - (s >> 1);
+    if ((h >> k) & 1u) {
+      at += 2 * (int64_t)left;
+      s >>= 1;
+    } else {
+      at += 1;
+      s = left;
+    }
+  }
+  const uint32_t node = b.base[d] + (h - (1u << d));
+  put_node<K>(nodes, node, at, count, t_off, vol, tet);
+  if (d == depth && s == 2u) {
+    using L = NodeLayout<K>;
+    const uint32_t c = L::word0(nodes[L::at(node, L::TOPO_CHUNK)]);
+    put_node<K>(nodes, c, at + 1, count, t_off, vol, tet);
+    put_node<K>(nodes, c + 1, at + 2, count, t_off, vol, tet);
+  }
+}
+
 // World positions of all vertices (pose / deform modes), for read-back.
 __global__ void world_kernel(int64_t nv, VertexSource vs, float4* out) {
   int64_t v = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
@@ -583,6 +639,42 @@ static cudaError_t leaf_tables_impl(kdop_scene* s) {
       s->nodes, s->refit_blocks, s->tets, s->leaf_verts, s->leaf_tet);
   s->ctx->launches++;
   return cudaGetLastError();
+}
+
+template <int K>
+static cudaError_t preorder_impl(kdop_scene* s, int mesh, int64_t first, int64_t count, float* vol, int64_t* tet) {
+  // nodes of a tree at depth d: 2^d down to L = floor(log2 n), then two per
+  // two-tet node
+  TreeBase b;
+  int depth = 0;
+  const int64_t n = s->t_off[mesh + 1] - s->t_off[mesh];
+  while ((int64_t(2) << depth) <= n) ++depth;
+  for (int d = 0; d <= depth; ++d) {
+    int64_t at = s->level_off[d];
+    for (int m = 0; m < mesh; ++m) {
+      const int64_t k = s->t_off[m + 1] - s->t_off[m], full = int64_t(1) << d;
+      at += k >= full ? full : std::max<int64_t>(0, 2 * k - full);
+    }
+    b.base[d] = (uint32_t)at;
+  }
+  const unsigned threads = (2u << depth) - 1u;
+  preorder_kernel<K><<<(threads + 255) / 256, 256, 0, s->ctx->stream>>>(s->nodes, b, (uint32_t)n, depth,
+                                                                       (uint32_t)s->t_off[mesh], first, count, vol, tet);
+  s->ctx->launches++;
+  return cudaGetLastError();
+}
+
+cudaError_t launch_preorder(kdop_scene* s, int mesh, int64_t first, int64_t count, float* vol, int64_t* tet) {
+  switch (s->K) {
+    case 6: return preorder_impl<6>(s, mesh, first, count, vol, tet);
+    case 8: return preorder_impl<8>(s, mesh, first, count, vol, tet);
+    case 12: return preorder_impl<12>(s, mesh, first, count, vol, tet);
+    case 14: return preorder_impl<14>(s, mesh, first, count, vol, tet);
+    case 18: return preorder_impl<18>(s, mesh, first, count, vol, tet);
+    case 20: return preorder_impl<20>(s, mesh, first, count, vol, tet);
+    case 26: return preorder_impl<26>(s, mesh, first, count, vol, tet);
+  }
+  return cudaErrorInvalidValue;
 }
 
 cudaError_t launch_leaf_tables(kdop_scene* s) {

@@ -194,6 +194,27 @@ __global__ void __launch_bounds__(256) sort_apply_kernel(ApplyArgs a) {
   }
 }
 
+__global__ void __launch_bounds__(256) candidate_rows_kernel(const uint32_t* __restrict__ cA,
+                                                             const uint32_t* __restrict__ cB,
+                                                             const uint32_t* __restrict__ cP,
+                                                             const uint2* __restrict__ pairs, uint32_t n_pairs,
+                                                             const uint32_t* __restrict__ t_off, int64_t n,
+                                                             uint32_t* rows) {
+  // thread per row, then the block's 768 words in order
+  __shared__ uint32_t s[768];
+  const int64_t base = (int64_t)blockIdx.x * 256, i = base + threadIdx.x;
+  if (i < n) {
+    const uint32_t p = cP[i];
+    const uint2 m = p < n_pairs ? pairs[p] : make_uint2(0u, 0u);
+    s[3 * threadIdx.x] = p;
+    s[3 * threadIdx.x + 1] = cA[i] - t_off[m.x];
+    s[3 * threadIdx.x + 2] = cB[i] - t_off[m.y];
+  }
+  __syncthreads();
+  const int words = 3 * (int)min((int64_t)256, n - base);
+  for (int k = threadIdx.x; k < words; k += 256) rows[3 * base + k] = s[k];
+}
+
 // Contact rows of sorted candidate k to rows r.w ..: eight lanes a candidate,
 // 16 bytes a lane.
 __global__ void __launch_bounds__(256) contact_gather_kernel(int64_t n, const int4* __restrict__ rec,
@@ -213,6 +234,14 @@ __global__ void __launch_bounds__(256) contact_gather_kernel(int64_t n, const in
 }
 
 }  // namespace
+
+cudaError_t launch_candidate_rows(kdop_scene* s, int64_t first, int64_t n, int64_t n_pairs, uint32_t* rows) {
+  const uint32_t* c = s->cand + first;
+  candidate_rows_kernel<<<(unsigned)((n + 255) / 256), 256, 0, s->ctx->stream>>>(
+      c, c + s->cand_cap, c + 2 * s->cand_cap, s->pairs, (uint32_t)n_pairs, s->t_off_dev, n, rows);
+  s->ctx->launches++;
+  return cudaGetLastError();
+}
 
 // Work buffer of sort_results, every region 256-byte aligned.
 struct SortWork {
