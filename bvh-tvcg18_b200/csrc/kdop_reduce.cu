@@ -122,6 +122,7 @@ struct ReduceArgs {
   const uint2* bodies;
   int64_t n;
   const uint32_t* perm;   // rows in the first sort's order
+  uint64_t* next;         // (p.x, p.z) of the rows in that order
   uint32_t* run;          // run of a sorted position
   uint32_t* starts;       // first position of a run; starts[runs] = n
   uint32_t* order;        // rows in full order
@@ -159,8 +160,10 @@ __global__ void __launch_bounds__(256) red_runs_kernel(ReduceArgs a) {
     const int64_t k = base + j;
     if (k >= a.n) continue;
     const uint32_t r = a.perm[k];
-    const uint32_t y = ord_key(a.rows[r].p[1]);
+    const float4 p = reinterpret_cast<const float4*>(a.rows)[2 * (int64_t)r];
+    const uint32_t y = ord_key(p.y);
     const uint2 b = a.bodies[r];
+    a.next[k] = two_keys(p.x, p.z);
     if (k == 0 || y != y_prev || b.x != b_prev.x || b.y != b_prev.y) {
       first |= 1u << j;
       ++sum;
@@ -181,36 +184,47 @@ __global__ void __launch_bounds__(256) red_runs_kernel(ReduceArgs a) {
   }
 }
 
-// Fields after p.y of two rows of a run, in the sort's order: -1, 0, 1.
+// Fields after p of two rows, in the sort's order: -1, 0, 1.
 __device__ __forceinline__ int later_fields(const Row& x, const Row& y) {
-  const uint64_t p = two_keys(x.a.x, x.a.z), q = two_keys(y.a.x, y.a.z);
-  if (p != q) return p < q ? -1 : 1;
   const uint64_t n = two_keys(x.b.x, x.a.w), m = two_keys(y.b.x, y.a.w);
   if (n != m) return n < m ? -1 : 1;
   const uint64_t d = two_keys(x.b.y, x.b.z), f = two_keys(y.b.y, y.b.z);
   return d < f ? -1 : d > f ? 1 : 0;
 }
 
-// Each row to its place in the full order.  Neighbouring rows are mostly of one
-// run, so a warp's loads of the run's rows fall on one address.
+// Each row to its place in the full order: the rows of its run before it.  The
+// counting reads (p.x, p.z) keys laid out in the first sort's order --
+// neighbouring rows are mostly of one run, so a warp's loads fall on the same
+// addresses -- and whole rows only where those tie (reading whole rows through
+// the permutation took 399 us on 3.6 M rows).
 __global__ void __launch_bounds__(256) red_rank_kernel(ReduceArgs a) {
   const int64_t k = (int64_t)blockIdx.x * 256 + threadIdx.x;
   if (k >= a.n) return;
   const uint32_t r = a.perm[k], g = a.run[k];
   const uint32_t s = a.starts[g], e = a.starts[g + 1];
+  const Row x = load_row(a.rows, r);
   if (e - s > kRankMax) {
-    a.longs[k] = 1u;  // ordered by the radix sorts below
+    a.longs[k] = 1u;  // ordered by the radix sorts below, until then in the first sort's order
     a.head[H_LONG] = 1u;
+    a.order[k] = r;
+    a.sorted[k] = x;
     return;
   }
   a.longs[k] = 0u;
-  const Row x = load_row(a.rows, r);
-  uint32_t rank = 0;
+  const uint64_t mine = a.next[k];
+  uint32_t rank = 0, ties = 0;
+#pragma unroll 4
   for (uint32_t j = s; j < e; ++j) {
-    if (j == (uint32_t)k) continue;
-    const int c = later_fields(load_row(a.rows, a.perm[j]), x);
-    rank += (c < 0 || (c == 0 && j < (uint32_t)k)) ? 1u : 0u;  // equal rows keep their order
+    const uint64_t key = a.next[j];
+    rank += key < mine ? 1u : 0u;
+    ties += key == mine ? 1u : 0u;
   }
+  if (ties > 1)
+    for (uint32_t j = s; j < e; ++j) {
+      if (a.next[j] != mine || j == (uint32_t)k) continue;
+      const int c = later_fields(load_row(a.rows, a.perm[j]), x);
+      rank += (c < 0 || (c == 0 && j < (uint32_t)k)) ? 1u : 0u;  // equal rows keep their order
+    }
   a.order[s + rank] = r;
   a.sorted[s + rank] = x;
 }
@@ -325,7 +339,7 @@ unsigned blocks_for(int64_t n, int t) { return (unsigned)((n + t - 1) / t); }
 
 // Work buffer of a reduction of n rows (256-byte aligned pieces).
 struct ReduceWork {
-  size_t head, words_run, words_keep, keys, keys_tmp, perm, perm_tmp, radix, run, starts, order, sorted, keep, longs,
+  size_t head, words_run, words_keep, keys, keys_tmp, next, perm, perm_tmp, radix, run, starts, order, sorted, keep, longs,
       long_at, long_vals, scan, total;
   explicit ReduceWork(int64_t n) {
     size_t at = 0;
@@ -340,6 +354,7 @@ struct ReduceWork {
     words_keep = take(tiles * 8);
     keys = take(m * 8);
     keys_tmp = take(m * 8);
+    next = take(m * 8);
     perm = take(m * 4);
     perm_tmp = take(m * 4);
     radix = take(radix_scratch_words((int64_t)m) * 4);
@@ -413,6 +428,7 @@ cudaError_t reduce_contact_rows(kdop_ctx* ctx, const kdop_contact* rows, const u
   a.rows = rows;
   a.bodies = bodies;
   a.n = n;
+  a.next = reinterpret_cast<uint64_t*>(w + L.next);
   a.run = reinterpret_cast<uint32_t*>(w + L.run);
   a.starts = reinterpret_cast<uint32_t*>(w + L.starts);
   a.order = reinterpret_cast<uint32_t*>(w + L.order);
@@ -449,15 +465,20 @@ cudaError_t reduce_contact_rows(kdop_ctx* ctx, const kdop_contact* rows, const u
   red_runs_kernel<<<tiles, 256, 0, st>>>(a);
   red_rank_kernel<<<blocks_for(n, 256), 256, 0, st>>>(a);
   ctx->launches += 2;
-  if ((e = cudaMemcpyAsync(h, a.head, sizeof(h), cudaMemcpyDeviceToHost, st)) != cudaSuccess) return e;
-  if ((e = cudaStreamSynchronize(st)) != cudaSuccess) return e;
-  if (h[H_LONG] && (e = order_long_runs(ctx, a, L, w, b)) != cudaSuccess) return e;
-  red_segments_kernel<<<blocks_for(n, 256), 256, 0, st>>>(a);
-  red_walk_kernel<<<blocks_for(n, 128), 128, 0, st>>>(a);
-  red_write_kernel<<<tiles, 256, 0, st>>>(a);
-  ctx->launches += 3;
-  if ((e = cudaMemcpyAsync(h, a.head, sizeof(h), cudaMemcpyDeviceToHost, st)) != cudaSuccess) return e;
-  if ((e = cudaStreamSynchronize(st)) != cudaSuccess) return e;
+  // without waiting for the count of long runs: where there are some, they are
+  // ordered afterwards and the rest runs again
+  for (int round = 0;; ++round) {
+    red_segments_kernel<<<blocks_for(n, 256), 256, 0, st>>>(a);
+    red_walk_kernel<<<blocks_for(n, 128), 128, 0, st>>>(a);
+    red_write_kernel<<<tiles, 256, 0, st>>>(a);
+    ctx->launches += 3;
+    if ((e = cudaMemcpyAsync(h, a.head, sizeof(h), cudaMemcpyDeviceToHost, st)) != cudaSuccess) return e;
+    if ((e = cudaStreamSynchronize(st)) != cudaSuccess) return e;
+    if (round || !h[H_LONG]) break;
+    if ((e = order_long_runs(ctx, a, L, w, b)) != cudaSuccess) return e;
+    if ((e = cudaMemsetAsync(a.head + H_TICKET_KEEP, 0, 4, st)) != cudaSuccess) return e;
+    if ((e = cudaMemsetAsync(a.words_keep, 0, L.keys - L.words_keep, st)) != cudaSuccess) return e;
+  }
   if (h[H_ERR]) return cudaErrorLaunchTimeout;
   *n_out = h[H_KEPT];
   return cudaGetLastError();

@@ -34,7 +34,7 @@ namespace kdop {
 
 constexpr int kSortMaxPasses = 8;
 constexpr unsigned kSpinLimit = 1u << 23;  // polls of one published word
-constexpr int kSmallSort = 4096;           // keys one block sorts in shared memory
+constexpr int kSmallSort = 8192;           // keys one block sorts in shared memory
 
 __device__ __forceinline__ unsigned sort_digit(uint64_t key, int shift, unsigned mask) {
   return (unsigned)(key >> shift) & mask;
@@ -176,101 +176,6 @@ __global__ void __launch_bounds__(256) sort_keys_kernel(Gen gen, int64_t n, int 
   }
 }
 
-// One digit pass over tiles of 256 * ITEMS keys.  Items past n (last tile)
-// rank as digit 255 behind every key and are not written.
-template <int ITEMS>
-__global__ void __launch_bounds__(256) sort_pass_kernel(const uint64_t* __restrict__ kin,
-                                                        const uint32_t* __restrict__ vin, uint64_t* kout,
-                                                        uint32_t* vout, int64_t n, int shift,
-                                                        const uint32_t* __restrict__ hist, uint32_t* ticket,
-                                                        unsigned long long* words, unsigned epoch, unsigned* err) {
-  constexpr int TILE = 256 * ITEMS, WARPS = 8;
-  __shared__ uint32_t wc[WARPS][256];
-  __shared__ uint64_t ex[TILE];
-  __shared__ uint32_t gbase[256], lofs[256];
-  __shared__ unsigned s_tile;
-  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-  const unsigned lt = (1u << lane) - 1u;
-  if (threadIdx.x == 0) s_tile = atomicAdd(ticket, 1u);
-#pragma unroll
-  for (int j = 0; j < WARPS; ++j) wc[j][threadIdx.x] = 0;
-  __syncthreads();
-  const unsigned tile = s_tile;
-  const int64_t base = (int64_t)tile * TILE;
-  const int valid = (int)min((int64_t)TILE, n - base);
-  uint64_t k[ITEMS];
-  uint32_t v[ITEMS];
-  uint16_t rank[ITEMS];
-#pragma unroll
-  for (int r = 0; r < ITEMS; ++r) {
-    const int at = w * 32 * ITEMS + r * 32 + lane;
-    k[r] = at < valid ? kin[base + at] : ~0ull;
-    v[r] = at < valid ? vin[base + at] : 0u;
-  }
-  // ranks within the warp, in input order (warp w: 32 * ITEMS consecutive keys)
-#pragma unroll
-  for (int r = 0; r < ITEMS; ++r) {
-    const unsigned d = sort_digit(k[r], shift, 255u);
-    const unsigned peers = __match_any_sync(0xffffffffu, d);
-    const uint32_t c = wc[w][d];
-    rank[r] = (uint16_t)(c + __popc(peers & lt));
-    __syncwarp();
-    if ((peers & lt) == 0u) wc[w][d] = c + __popc(peers);
-    __syncwarp();
-  }
-  __syncthreads();
-  // digit threadIdx.x: the warps in order, then the tiles before this one
-  const unsigned d0 = threadIdx.x;
-  uint32_t count = 0;
-#pragma unroll
-  for (int j = 0; j < WARPS; ++j) {
-    const uint32_t c = wc[j][d0];
-    wc[j][d0] = count;
-    count += c;
-  }
-  unsigned long long* mine = words + (size_t)tile * 256 + d0;
-  publish(mine, count, tile == 0 ? 2u : 1u, epoch);
-  unsigned long long total;
-  const unsigned long long both = ((unsigned long long)hist[d0] << 16) | count;  // a tile holds < 2^16 keys
-  const unsigned long long before = block_scan<256, unsigned long long>(both, total);
-  const uint32_t local = (uint32_t)before & 0xFFFFu;
-  uint32_t excl = 0;
-  for (int64_t t = (int64_t)tile - 1; t >= 0; --t) {
-    uint32_t x;
-    const unsigned flag = await_word(words + (size_t)t * 256 + d0, epoch, x, err);
-    excl += x;
-    if (flag == 2u) break;
-  }
-  if (tile) publish(mine, excl + count, 2u, epoch);
-  lofs[d0] = local;
-  gbase[d0] = (uint32_t)(before >> 16) + excl - local;
-  __syncthreads();
-#pragma unroll
-  for (int r = 0; r < ITEMS; ++r) {
-    const unsigned d = sort_digit(k[r], shift, 255u);
-    rank[r] = (uint16_t)(lofs[d] + wc[w][d] + rank[r]);
-    ex[rank[r]] = k[r];
-  }
-  __syncthreads();
-  uint32_t to[ITEMS];
-#pragma unroll
-  for (int r = 0; r < ITEMS; ++r) {
-    const int at = r * 256 + threadIdx.x;
-    const uint64_t key = ex[at];
-    const uint32_t g = gbase[sort_digit(key, shift, 255u)] + (uint32_t)at;
-    to[r] = (at < valid && (int64_t)g < n) ? g : 0xFFFFFFFFu;
-    if (to[r] != 0xFFFFFFFFu) kout[g] = key;
-  }
-  __syncthreads();
-  uint32_t* exv = reinterpret_cast<uint32_t*>(ex);
-#pragma unroll
-  for (int r = 0; r < ITEMS; ++r) exv[rank[r]] = v[r];
-  __syncthreads();
-#pragma unroll
-  for (int r = 0; r < ITEMS; ++r)
-    if (to[r] != 0xFFFFFFFFu) vout[to[r]] = exv[r * 256 + threadIdx.x];
-}
-
 // Up to 1024 * ITEMS keys generated and sorted by one block.
 template <int ITEMS>
 constexpr size_t small_sort_smem() {
@@ -359,6 +264,10 @@ struct SortBuffers {
   uint32_t *vals, *vals_tmp;
 };
 
+// One digit pass from b's keys and values to its temporaries (kdop_sort.cu).
+cudaError_t launch_sort_pass(const SortBuffers& b, int64_t n, int shift, const uint32_t* hist, uint32_t* ticket,
+                             unsigned long long* words, unsigned epoch, unsigned* err, cudaStream_t st);
+
 // Stable ascending sort of the items 0 .. n-1 by gen.key(i), of which the low
 // `bits` bits vary (the others are equal in all keys), n < 2^32; the values
 // are gen.val(i).  gen may read b.vals at i (it is written at i only).
@@ -372,31 +281,30 @@ cudaError_t radix_sort(const Gen& gen, int64_t n, int bits, SortBuffers& b, void
   if (n <= kSmallSort) {
     if (n <= 1024) {
       small_sort_kernel<Gen, 1><<<1, 1024, small_sort_smem<1>(), st>>>(gen, (int)n, bits, b.keys, b.vals);
-    } else {
+    } else if (n <= 4096) {
       e = cudaFuncSetAttribute(small_sort_kernel<Gen, 4>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                (int)small_sort_smem<4>());
       if (e != cudaSuccess) return e;
       small_sort_kernel<Gen, 4><<<1, 1024, small_sort_smem<4>(), st>>>(gen, (int)n, bits, b.keys, b.vals);
+    } else {
+      e = cudaFuncSetAttribute(small_sort_kernel<Gen, 8>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                               (int)small_sort_smem<8>());
+      if (e != cudaSuccess) return e;
+      small_sort_kernel<Gen, 8><<<1, 1024, small_sort_smem<8>(), st>>>(gen, (int)n, bits, b.keys, b.vals);
     }
     launches += 1;
     return cudaGetLastError();
   }
   SortScratch s(scratch);
-  const bool large = n > kLargeSort;
-  const int64_t tile = large ? kSortTileLarge : kSortTile;
-  const int64_t tiles = (n + tile - 1) / tile;
+  const int64_t tiles = (n + kSortTile - 1) / kSortTile;
   if ((e = cudaMemsetAsync(scratch, 0, SortScratch::kHead + (size_t)tiles * 256 * 8, st)) != cudaSuccess) return e;
   sort_keys_kernel<<<(unsigned)std::min<int64_t>((n + 1023) / 1024, 1184), 256, 0, st>>>(gen, n, bits, b.keys, b.vals,
                                                                                         s.hist);
   launches += 1;
   unsigned epoch = 1;
   for (int p = 0; 8 * p < bits; ++p, ++epoch) {
-    if (large)
-      sort_pass_kernel<kSortTileLarge / 256><<<(unsigned)tiles, 256, 0, st>>>(
-          b.keys, b.vals, b.keys_tmp, b.vals_tmp, n, 8 * p, s.hist + 256 * p, s.ticket + p, s.words, epoch, err);
-    else
-      sort_pass_kernel<kSortTile / 256><<<(unsigned)tiles, 256, 0, st>>>(
-          b.keys, b.vals, b.keys_tmp, b.vals_tmp, n, 8 * p, s.hist + 256 * p, s.ticket + p, s.words, epoch, err);
+    e = launch_sort_pass(b, n, 8 * p, s.hist + 256 * p, s.ticket + p, s.words, epoch, err, st);
+    if (e != cudaSuccess) return e;
     launches += 1;
     std::swap(b.keys, b.keys_tmp);
     std::swap(b.vals, b.vals_tmp);

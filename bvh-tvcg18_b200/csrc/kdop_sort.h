@@ -7,8 +7,7 @@
 
 namespace kdop {
 
-constexpr int64_t kSortTile = 2048, kSortTileLarge = 4096;  // keys per block and pass
-constexpr int64_t kLargeSort = 1 << 20;                     // from this many keys on, the large tile
+constexpr int64_t kSortTile = 4096;  // keys per block and pass
 
 // Words of scratch a radix sort of n keys needs.
 size_t radix_scratch_words(int64_t n);
