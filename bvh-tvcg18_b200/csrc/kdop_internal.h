@@ -51,7 +51,8 @@ struct TravCtl {
   unsigned int n_seed;               // node pairs the first seed pass left for the second
   unsigned int n_surv;               // candidates past the contact pre-filter
   unsigned int n_mid;                // candidates past the face axes of the SAT test
-  unsigned int pad0[21];
+  unsigned int order_error;          // DEV_ERR_* of the sort that ordered the root pairs
+  unsigned int pad0[20];
   unsigned int n_cand;               // candidates emitted (may exceed capacity)
   unsigned int pad1[31];
   unsigned int init_head;            // root pairs claimed
@@ -112,6 +113,7 @@ struct kdop_scene {
   int64_t nv = 0, nt = 0, nn = 0;
   int depth = 0;
   std::vector<int64_t> v_off, t_off, level_off;
+  int64_t most_tets = 0;  // of any mesh
   std::vector<uint32_t> root;  // per mesh root node, 0xFFFFFFFF for an empty mesh
   kdop::DirTable dirs;
 
@@ -176,6 +178,9 @@ namespace kdop {
 // Entries (16 bytes each) the traversal's seed pass can leave for any list of
 // at most n pairs (kdop_traverse.cu).
 int64_t seed_entries(int sm_count, int64_t n);
+// pair_order of the scene's n pairs by decreasing size (most >= the tets of any
+// two meshes), in the seed pass's buffer.
+cudaError_t launch_pair_order(kdop_scene* s, int64_t n, uint32_t most);
 
 // fn(0 .. n-1) on up to 64 host threads
 template <typename F>

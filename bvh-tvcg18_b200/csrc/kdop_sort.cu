@@ -387,9 +387,7 @@ cudaError_t sort_results(kdop_scene* s, int64_t n, int64_t n_contacts, void* wor
   float4* rows_out = reinterpret_cast<float4*>(w + L.rows_out);
   uint32_t* cand_out = reinterpret_cast<uint32_t*>(w + L.cand_out);
   unsigned* err = &s->ctl->error;
-  int64_t most = 1;
-  for (int m = 0; m < s->n_meshes; ++m) most = std::max(most, s->t_off[m + 1] - s->t_off[m]);
-  CandGen gen{s->cand, s->cand + s->cand_cap, s->cand + 2 * s->cand_cap, s->pairs, s->t_off_dev, bits_of(most - 1)};
+  CandGen gen{s->cand, s->cand + s->cand_cap, s->cand + 2 * s->cand_cap, s->pairs, s->t_off_dev, bits_of(std::max<int64_t>(s->most_tets, 1) - 1)};
   const int pair_bits = bits_of((uint64_t)std::max<int64_t>(s->result_pairs, 1) - 1);
   const bool packed = s->pairs_current && pair_bits + 2 * gen.tb <= 64;
   cudaError_t e;

@@ -630,6 +630,54 @@ constexpr unsigned kSeedCap = 4 * kSeedStop;  // most a level of fewer than kSee
 constexpr int kSeedThreads = 512;
 constexpr int64_t kSeedTwiceMax = 64;
 
+// ---- order of the root pairs ----------------------------------------------------
+// Pairs by decreasing size (tets of both meshes), equal sizes in list order.
+struct PairSizeGen {
+  const uint2* pairs;
+  const uint32_t* t_off;
+  uint32_t most;  // tets of the two largest meshes at least
+  __device__ uint64_t key(int64_t i) const {
+    const uint2 m = pairs[i];
+    return most - (t_off[m.x + 1] - t_off[m.x]) - (t_off[m.y + 1] - t_off[m.y]);
+  }
+  __device__ uint32_t val(int64_t i) const { return (uint32_t)i; }
+};
+// Work of that sort, in the seed pass's buffer (free until the traversal).
+struct PairOrderWork {
+  size_t keys, keys_tmp, vals, vals_tmp, scratch, total;
+  explicit PairOrderWork(int64_t n) {
+    size_t at = 0;
+    auto take = [&](size_t b) {
+      size_t o = at;
+      at += (b + 255) & ~(size_t)255;
+      return o;
+    };
+    keys = take((size_t)n * 8);
+    keys_tmp = take((size_t)n * 8);
+    vals = take((size_t)n * 4);
+    vals_tmp = take((size_t)n * 4);
+    scratch = take(radix_scratch_words(n) * 4);
+    total = at;
+  }
+};
+
+cudaError_t launch_pair_order(kdop_scene* s, int64_t n, uint32_t most) {
+  char* w = reinterpret_cast<char*>(s->seeds);
+  const PairOrderWork L(n);
+  SortBuffers b{reinterpret_cast<uint64_t*>(w + L.keys), reinterpret_cast<uint64_t*>(w + L.keys_tmp),
+                reinterpret_cast<uint32_t*>(w + L.vals), reinterpret_cast<uint32_t*>(w + L.vals_tmp)};
+  // a sort wait that gave up leaves an incomplete order: every place starts as
+  // a valid pair index, and the traversals over this order report the error
+  cudaError_t e = cudaMemsetAsync(&s->ctl->order_error, 0, 4, s->ctx->stream);
+  if (e == cudaSuccess) e = cudaMemsetAsync(w + L.vals, 0, L.scratch - L.vals, s->ctx->stream);
+  if (e == cudaSuccess)
+    e = radix_sort(PairSizeGen{s->pairs, s->t_off_dev, most}, n, bits_of(most), b, w + L.scratch,
+                   &s->ctl->order_error, s->ctx->stream, s->ctx->launches);
+  if (e == cudaSuccess)
+    e = cudaMemcpyAsync(s->pair_order, b.vals, (size_t)n * 4, cudaMemcpyDeviceToDevice, s->ctx->stream);
+  return e;
+}
+
 // Pairs per block of the first pass: four blocks per SM until a group fills
 // a block's list.
 static int64_t seed_group(int sm_count, int64_t n_pairs) {
@@ -647,7 +695,8 @@ static int64_t seed_entries1(int sm_count, int64_t n) {
   return std::max(std::min<int64_t>(n, 4 * (int64_t)sm_count), (n + kSeedCap - 1) / kSeedCap) * kSeedCap;
 }
 int64_t seed_entries(int sm_count, int64_t n) {
-  return seed_entries1(sm_count, n) + (int64_t)seed_blocks2(sm_count, 1) * kSeedCap;
+  const int64_t seeds = seed_entries1(sm_count, n) + (int64_t)seed_blocks2(sm_count, 1) * kSeedCap;
+  return std::max(seeds, (int64_t)(PairOrderWork(n).total / sizeof(uint4)) + 1);  // the pair order's work, before
 }
 
 template <int K>
@@ -776,7 +825,7 @@ __global__ void trav_init_kernel(TravCtl* c, unsigned n_init, unsigned pair_base
     c->tests = 0;
     c->leaf_overlaps = 0;
     c->n_cand = 0;
-    c->error = 0;
+    c->error = c->order_error;
     c->n_seed = 0;
     c->n_contacts = 0;
   }
