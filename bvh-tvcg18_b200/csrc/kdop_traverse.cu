@@ -473,16 +473,14 @@ __global__ void __launch_bounds__(512, (C * S >= 4) ? 1 : 2) traverse_kernel(Tra
       float4 A0[S][C], A1[S][C], B0[S][C], B1[S][C];
 #pragma unroll
       for (int b = 0; b < S; ++b) {
-        const int i = b * E + ge;
-        eab[b] = make_uint2(0u, 0u);
-        if (i < n) eab[b] = sAB[(top + i) & MASK];
+        // a lane without an entry loads the last one's records again (no line
+        // of its own) and its verdicts are not used
+        eab[b] = sAB[(top + min(b * E + ge, n - 1)) & MASK];
         const float4* pa = nodes_q + (size_t)((eab[b].x & NODE_MASK) >> 1) * (2 * NW);
         const float4* pb = nodes_q + (size_t)((eab[b].y & NODE_MASK) >> 1) * (2 * NW);
 #pragma unroll
         for (int r = 0; r < C; ++r) {
           const int j = gq + Q * r;
-          // a lane without an entry (i >= n) loads the record of node 0's
-          // twin and its verdicts are never used: no zero fill
           if (j < NW) {
             ldg256(pa + 2 * Q * r, A0[b][r], A1[b][r]);
             ldg256(pb + 2 * Q * r, B0[b][r], B1[b][r]);
@@ -752,8 +750,8 @@ __global__ void __launch_bounds__(kSeedThreads) seed_kernel(TravArgs a, unsigned
       for (unsigned i0 = wib * E; i0 < c; i0 += nw * E) {
         const unsigned i = i0 + ge;
         const bool valid = i < c;
-        const uint2 x = valid ? AB[cur * kSeedCap + i] : make_uint2(0u, 0u);
-        const uint32_t pid = valid ? P[cur * kSeedCap + i] : 0u;
+        const uint2 x = AB[cur * kSeedCap + min(i, c - 1)];
+        const uint32_t pid = P[cur * kSeedCap + min(i, c - 1)];
         const float4* pa = nodes_q + (size_t)((x.x & NODE_MASK) >> 1) * (2 * NW);
         const float4* pb = nodes_q + (size_t)((x.y & NODE_MASK) >> 1) * (2 * NW);
         float4 A0[C], A1[C], B0[C], B1[C];
