@@ -66,7 +66,7 @@ void dfree(kdop_scene* s, T** p, int64_t n) {
 
 namespace kdop {
 cudaError_t launch_pack3(kdop_scene* s, const float* in, float4* out, int64_t n, int with_mesh_id);
-cudaError_t launch_pack4(kdop_scene* s, const float* in, float4* out, int64_t n);
+cudaError_t launch_pack_poses(kdop_scene* s, const float* quat, const float* pos);
 }  // namespace kdop
 
 struct kdop_scene_ext {
@@ -621,8 +621,7 @@ int kdop_set_poses(kdop_scene* s, const float* quat, const float* pos, int memor
     q = d;
     p = d + 4 * n;
   }
-  KDOP_CUDA(s->ctx, kdop::launch_pack4(s, q, s->quat, n));
-  KDOP_CUDA(s->ctx, kdop::launch_pack3(s, p, s->pos, n, -1));
+  KDOP_CUDA(s->ctx, kdop::launch_pack_poses(s, q, p));
   return KDOP_OK;
 }
 
@@ -806,6 +805,7 @@ static int upload_pairs(kdop_scene* s, int64_t n, const uint32_t* pairs, int mem
   if (n > kHostOrder) {
     KDOP_CUDA(s->ctx, kdop::launch_pair_order(s, n, (uint32_t)std::max<int64_t>(2 * s->most_tets, 1)));
     x->device_order = true;
+    s->pairs_tets = 2 * s->most_tets;  // a bound is enough for long lists
     return KDOP_OK;
   }
   if (x->device_order)
@@ -814,9 +814,11 @@ static int upload_pairs(kdop_scene* s, int64_t n, const uint32_t* pairs, int mem
   std::vector<uint32_t>& ord = x->order_host;
   ord.resize((size_t)n);
   std::vector<int64_t> size((size_t)n);
+  s->pairs_tets = 0;
   for (int64_t i = 0; i < n; ++i) {
     uint32_t a = x->pairs_host[2 * i], b = x->pairs_host[2 * i + 1];
     size[i] = (s->t_off[a + 1] - s->t_off[a]) + (s->t_off[b + 1] - s->t_off[b]);
+    s->pairs_tets += size[i];
     ord[i] = (uint32_t)i;
   }
   std::stable_sort(ord.begin(), ord.end(), [&](uint32_t i, uint32_t j) { return size[i] > size[j]; });

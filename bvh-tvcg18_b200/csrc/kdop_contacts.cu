@@ -220,13 +220,14 @@ __device__ __forceinline__ bool planes_oppose(const UPlane& pa, const UPlane& pb
 }
 
 // Appends the warp's kept candidates to a list (one atomic per warp).
-__device__ __forceinline__ void warp_append(bool keep, unsigned ci, unsigned* counter, uint32_t* list, int lane) {
+__device__ __forceinline__ void warp_append(bool keep, unsigned ci, unsigned* counter, uint32_t* list, unsigned cap,
+                                            int lane) {
   const unsigned m = __ballot_sync(0xffffffffu, keep);
   if (m) {
     unsigned at = 0;
     if (lane == 0) at = atomicAdd(counter, (unsigned)__popc(m));
-    at = __shfl_sync(0xffffffffu, at, 0);
-    if (keep) list[at + __popc(m & ((1u << lane) - 1u))] = ci;
+    at = __shfl_sync(0xffffffffu, at, 0) + __popc(m & ((1u << lane) - 1u));
+    if (keep && at < cap) list[at] = ci;
   }
 }
 
@@ -239,6 +240,9 @@ __global__ void __launch_bounds__(256) contacts_filter_kernel(ContactArgs a) {
   const int lane = threadIdx.x & 31;
   const unsigned n_cand = min(*(volatile unsigned*)&a.ctl->n_cand, a.cand_cap);
   const unsigned stride = gridDim.x * blockDim.x;
+  // counters of the later passes (n_mid, this pass's own, is zeroed by the
+  // traversal and by pass 3)
+  if (blockIdx.x == 0 && threadIdx.x == 0) a.ctl->n_surv = a.ctl->n_contacts = 0u;
   for (unsigned base = blockIdx.x * blockDim.x + (threadIdx.x & ~31u); base < n_cand; base += stride) {
     const unsigned ci = base + lane;
     bool keep = false;
@@ -267,7 +271,7 @@ __global__ void __launch_bounds__(256) contacts_filter_kernel(ContactArgs a) {
       }
       if (!keep) a.rec[ci] = make_int4(-1, -1, 0, 0);
     }
-    warp_append(keep, ci, &a.ctl->n_mid, a.mid, lane);
+    warp_append(keep, ci, &a.ctl->n_mid, a.mid, a.cand_cap, lane);
   }
 }
 
@@ -307,7 +311,7 @@ __device__ __forceinline__ bool stored_sat_test(int t, const PairStore& s) {
 __global__ void __launch_bounds__(256) contacts_edge_kernel(ContactArgs a) {
   __shared__ float store[8][24];
   const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
-  const unsigned n_mid = *(volatile unsigned*)&a.ctl->n_mid;
+  const unsigned n_mid = min(*(volatile unsigned*)&a.ctl->n_mid, a.cand_cap);
   if (n_mid <= kWarpCands) {
     const PairStore s{store[wib], 1};
     for (unsigned k = blockIdx.x * 8u + wib; k < n_mid; k += gridDim.x * 8u) {
@@ -342,7 +346,7 @@ __global__ void __launch_bounds__(256) contacts_edge_kernel(ContactArgs a) {
       keep = !sep;
       if (!keep) a.rec[ci] = make_int4(-1, -1, 0, 0);
     }
-    warp_append(keep, ci, &a.ctl->n_surv, a.surv, lane);
+    warp_append(keep, ci, &a.ctl->n_surv, a.surv, a.cand_cap, lane);
   }
 }
 
@@ -598,7 +602,8 @@ constexpr int CT_THREADS = 128;
 __global__ void __launch_bounds__(CT_THREADS, 6) contacts_thread_kernel(ContactArgs a) {
   __shared__ float store[kPairWords * CT_THREADS];
   const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
-  const unsigned n_surv = *(volatile unsigned*)&a.ctl->n_surv;
+  const unsigned n_surv = min(*(volatile unsigned*)&a.ctl->n_surv, a.cand_cap);
+  if (blockIdx.x == 0 && threadIdx.x == 0) a.ctl->n_mid = 0u;  // for the next call (pass 2 has read it)
   if (n_surv <= kWarpPairs) {
     float* mine = store + wib * (kPairWords + 3 * 56);
     for (unsigned k = blockIdx.x * (CT_THREADS / 32) + wib; k < n_surv; k += gridDim.x * (CT_THREADS / 32))
@@ -861,14 +866,6 @@ __global__ void __launch_bounds__(128) adjoint_kernel(AdjointArgs a) {
   }
 }
 
-__global__ void contacts_reset_kernel(TravCtl* c) {
-  if (threadIdx.x == 0) {
-    c->n_contacts = 0;
-    c->n_surv = 0;
-    c->n_mid = 0;
-  }
-}
-
 static VertexSource vsrc(kdop_scene* s) {
   VertexSource vs;
   vs.rest = s->rest;
@@ -902,12 +899,11 @@ cudaError_t launch_contacts(kdop_scene* s) {
   a.rec = s->records;
   a.out_cap = (unsigned)s->contact_cap;
   a.ctl = s->ctl;
-  contacts_reset_kernel<<<1, 32, 0, s->ctx->stream>>>(s->ctl);
   unsigned grid = (unsigned)s->ctx->sm_count * 8u;
   contacts_filter_kernel<<<grid, 256, 0, s->ctx->stream>>>(a);
   contacts_edge_kernel<<<grid, 256, 0, s->ctx->stream>>>(a);
   contacts_thread_kernel<<<grid * 2, 128, 0, s->ctx->stream>>>(a);
-  s->ctx->launches += 4;
+  s->ctx->launches += 3;
   return cudaGetLastError();
 }
 

@@ -114,6 +114,7 @@ struct kdop_scene {
   int depth = 0;
   std::vector<int64_t> v_off, t_off, level_off;
   int64_t most_tets = 0;  // of any mesh
+  int64_t pairs_tets = 0; // of the current pair list's meshes together
   std::vector<uint32_t> root;  // per mesh root node, 0xFFFFFFFF for an empty mesh
   kdop::DirTable dirs;
 

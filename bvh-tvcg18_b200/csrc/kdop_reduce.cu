@@ -213,7 +213,7 @@ __global__ void __launch_bounds__(256) red_rank_kernel(ReduceArgs a) {
   a.longs[k] = 0u;
   const uint64_t mine = a.next[k];
   uint32_t rank = 0, ties = 0;
-#pragma unroll 4
+#pragma unroll 8
   for (uint32_t j = s; j < e; ++j) {
     const uint64_t key = a.next[j];
     rank += key < mine ? 1u : 0u;
@@ -283,6 +283,7 @@ __global__ void __launch_bounds__(256) red_segments_kernel(ReduceArgs a) {
 __global__ void __launch_bounds__(128) red_walk_kernel(ReduceArgs a) {
   const int64_t k = (int64_t)blockIdx.x * 128 + threadIdx.x;
   if (k >= a.n || !(a.keep[k] & SEGMENT)) return;
+  if (k + 1 >= a.n || (a.keep[k + 1] & SEGMENT)) return;  // a segment of one row (most): kept
   Row last = a.sorted[k];
   for (int64_t j = k + 1; j < a.n; ++j) {
     const uint32_t f = a.keep[j];

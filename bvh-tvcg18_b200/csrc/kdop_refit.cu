@@ -506,10 +506,13 @@ __global__ void pack3_kernel(const float* __restrict__ in, float4* out, int64_t 
   float w = keep ? keep_w[i].w : 0.f;
   out[i] = make_float4(in[3 * i], in[3 * i + 1], in[3 * i + 2], w);
 }
-__global__ void pack4_kernel(const float* __restrict__ in, float4* out, int64_t n) {
+
+__global__ void pack_poses_kernel(const float* __restrict__ q, const float* __restrict__ p, float4* quat, float4* pos,
+                                  int64_t n) {
   int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n) return;
-  out[i] = make_float4(in[4 * i], in[4 * i + 1], in[4 * i + 2], in[4 * i + 3]);
+  quat[i] = make_float4(q[4 * i], q[4 * i + 1], q[4 * i + 2], q[4 * i + 3]);
+  pos[i] = make_float4(p[3 * i], p[3 * i + 1], p[3 * i + 2], 0.f);
 }
 
 cudaError_t launch_pack3(kdop_scene* s, const float* in, float4* out, int64_t n, int with_mesh_id) {
@@ -518,9 +521,10 @@ cudaError_t launch_pack3(kdop_scene* s, const float* in, float4* out, int64_t n,
   s->ctx->launches++;
   return cudaGetLastError();
 }
-cudaError_t launch_pack4(kdop_scene* s, const float* in, float4* out, int64_t n) {
+cudaError_t launch_pack_poses(kdop_scene* s, const float* quat, const float* pos) {
+  const int64_t n = s->n_meshes;
   if (n <= 0) return cudaSuccess;
-  pack4_kernel<<<(unsigned)((n + 255) / 256), 256, 0, s->ctx->stream>>>(in, out, n);
+  pack_poses_kernel<<<(unsigned)((n + 127) / 128), 128, 0, s->ctx->stream>>>(quat, pos, s->quat, s->pos, n);
   s->ctx->launches++;
   return cudaGetLastError();
 }

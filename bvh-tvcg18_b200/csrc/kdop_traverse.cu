@@ -626,7 +626,7 @@ __global__ void __launch_bounds__(512, (C * S >= 4) ? 1 : 2) traverse_kernel(Tra
 constexpr unsigned kSeedStop = 512;
 constexpr unsigned kSeedCap = 4 * kSeedStop;  // most a level of fewer than kSeedStop pairs leaves
 constexpr int kSeedThreads = 512;
-constexpr int64_t kSeedTwiceMax = 64;
+constexpr int64_t kSeedTwiceMax = 64, kSeedTwiceTets = 4096;
 
 // ---- order of the root pairs ----------------------------------------------------
 // Pairs by decreasing size (tets of both meshes), equal sizes in list order.
@@ -686,14 +686,18 @@ static int64_t seed_group(int sm_count, int64_t n_pairs) {
 // expanded once more, over two blocks per SM (one pair of 1.6 M tets 1,250 us
 // with one pass, 1,022 with two; 64 pairs 601 and 560 us, 256 pairs 455 and
 // 471 us, each against the same loop).
-static int seed_blocks2(int sm_count, int64_t n_pairs) { return n_pairs <= kSeedTwiceMax ? 2 * sm_count : 0; }
+// Pairs of fewer than kSeedTwiceTets tets in all end in the first pass or soon
+// after it.
+static int seed_blocks2(int sm_count, int64_t n_pairs, int64_t tets) {
+  return n_pairs <= kSeedTwiceMax && tets >= kSeedTwiceTets ? 2 * sm_count : 0;
+}
 
 // Entries the first pass can leave: kSeedCap per group of pairs.
 static int64_t seed_entries1(int sm_count, int64_t n) {
   return std::max(std::min<int64_t>(n, 4 * (int64_t)sm_count), (n + kSeedCap - 1) / kSeedCap) * kSeedCap;
 }
 int64_t seed_entries(int sm_count, int64_t n) {
-  const int64_t seeds = seed_entries1(sm_count, n) + (int64_t)seed_blocks2(sm_count, 1) * kSeedCap;
+  const int64_t seeds = seed_entries1(sm_count, n) + (int64_t)seed_blocks2(sm_count, 1, kSeedTwiceTets) * kSeedCap;
   return std::max(seeds, (int64_t)(PairOrderWork(n).total / sizeof(uint4)) + 1);  // the pair order's work, before
 }
 
@@ -826,6 +830,7 @@ __global__ void trav_init_kernel(TravCtl* c, unsigned n_init, unsigned pair_base
     c->error = c->order_error;
     c->n_seed = 0;
     c->n_contacts = 0;
+    c->n_mid = 0;
   }
   c->init_head = 0;
   c->q_head = 0;
@@ -913,7 +918,7 @@ static cudaError_t traverse_impl(kdop_scene* s, int64_t n_pairs, const TravBuffe
   if (b.seeds && !plain && p.wave_pairs <= 0 && n_pairs > 0) {
     const int sms = s->ctx->sm_count;
     const int64_t group = seed_group(sms, n_pairs), groups = (n_pairs + group - 1) / group;
-    const unsigned blocks2 = (unsigned)seed_blocks2(sms, n_pairs);
+    const unsigned blocks2 = (unsigned)seed_blocks2(sms, n_pairs, s->pairs_tets);
     constexpr size_t seed_smem = kSeedCap * 24;
     e = cudaFuncSetAttribute(seed_kernel<K>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)seed_smem);
     if (e != cudaSuccess) return e;
