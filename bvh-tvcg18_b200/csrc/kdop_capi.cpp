@@ -119,6 +119,29 @@ static float* stage(kdop_scene* s, int64_t nfloats, cudaError_t* err) {
   return x->stage;
 }
 
+// The control block's host copy holds what the device's does until the next
+// call that enqueues a change of it (a traversal, contacts, a graph step, a
+// sort): the counters are copied once per change, not once per call that reads
+// them (a step that reads statistics, sorts and reads contacts copied them five
+// times, 8 us each).  Work recorded into a capture can run again without a
+// call, so a scene that was ever captured into a caller's graph always copies.
+static void ctl_changes(kdop_scene* s) {
+  s->ctl_fresh = false;
+  cudaStreamCaptureStatus c = cudaStreamCaptureStatusNone;
+  if (cudaStreamIsCapturing(s->ctx->stream, &c) != cudaSuccess)
+    cudaGetLastError();
+  else if (c != cudaStreamCaptureStatusNone)
+    s->ctl_replayed = true;
+}
+// Synchronises and brings ctl_host up to date.
+static cudaError_t read_ctl(kdop_scene* s) {
+  if (s->ctl_fresh && !s->ctl_replayed) return cudaStreamSynchronize(s->ctx->stream);
+  cudaError_t e = cudaMemcpyAsync(s->ctl_host, s->ctl, sizeof(TravCtl), cudaMemcpyDeviceToHost, s->ctx->stream);
+  if (e == cudaSuccess) e = cudaStreamSynchronize(s->ctx->stream);
+  s->ctl_fresh = e == cudaSuccess;
+  return e;
+}
+
 extern "C" {
 
 int kdop_api_version(void) { return KDOP_API_VERSION; }
@@ -780,6 +803,7 @@ static int upload_pairs(kdop_scene* s, int64_t n, const uint32_t* pairs, int mem
   int rc = grow_pairs(s, std::max<int64_t>(n, 1));
   if (rc != KDOP_OK) return rc;
   s->pairs_current = false;  // until a traversal of this list is enqueued
+  ctl_changes(s);
   if (n == 0) {
     x->pairs_host.clear();
     return KDOP_OK;
@@ -927,8 +951,7 @@ int kdop_traverse_shard(kdop_scene* s, int64_t n_pairs, const uint32_t* pairs, i
 int kdop_get_stats(kdop_scene* s, kdop_stats* st) {
   if (!s || !st) return KDOP_ERR_INVALID;
   cudaSetDevice(s->ctx->device);
-  KDOP_CUDA(s->ctx, cudaMemcpyAsync(s->ctl_host, s->ctl, sizeof(TravCtl), cudaMemcpyDeviceToHost, s->ctx->stream));
-  KDOP_CUDA(s->ctx, cudaStreamSynchronize(s->ctx->stream));
+  KDOP_CUDA(s->ctx, read_ctl(s));
   const TravCtl& c = *s->ctl_host;
   std::memset(st, 0, sizeof(*st));
   st->n_pairs = s->last_pairs;
@@ -999,8 +1022,7 @@ int kdop_read_candidates(kdop_scene* s, uint32_t* rows, int64_t cap, int64_t* n_
   if (!s || !n_rows || (cap > 0 && !rows)) return KDOP_ERR_INVALID;
   if (!s->traversed) return fail(s->ctx, KDOP_ERR_STATE, "no traversal yet");
   cudaSetDevice(s->ctx->device);
-  KDOP_CUDA(s->ctx, cudaMemcpyAsync(s->ctl_host, s->ctl, sizeof(TravCtl), cudaMemcpyDeviceToHost, s->ctx->stream));
-  KDOP_CUDA(s->ctx, cudaStreamSynchronize(s->ctx->stream));
+  KDOP_CUDA(s->ctx, read_ctl(s));
   int64_t n = std::min<int64_t>((int64_t)s->ctl_host->n_cand, s->cand_cap);
   *n_rows = n;
   if (n > cap) return fail(s->ctx, KDOP_ERR_CAPACITY, "candidate read buffer too small");
@@ -1041,9 +1063,9 @@ int kdop_sort_results(kdop_scene* s) {
     x->sort_work_bytes = need;
     s->device_bytes += (int64_t)need;
   }
+  ctl_changes(s);
   KDOP_CUDA(s->ctx, kdop::sort_results(s, n, nc, x->sort_work, s->ctx->stream));
-  KDOP_CUDA(s->ctx, cudaMemcpyAsync(s->ctl_host, s->ctl, sizeof(TravCtl), cudaMemcpyDeviceToHost, s->ctx->stream));
-  KDOP_CUDA(s->ctx, cudaStreamSynchronize(s->ctx->stream));
+  KDOP_CUDA(s->ctx, read_ctl(s));
   if (s->ctl_host->error & kdop::DEV_ERR_TIMEOUT) return fail(s->ctx, KDOP_ERR_TIMEOUT, "sort wait timed out");
   return KDOP_OK;
 }
@@ -1053,6 +1075,7 @@ int kdop_contacts(kdop_scene* s) {
   if (!s->traversed) return fail(s->ctx, KDOP_ERR_STATE, "kdop_contacts before kdop_traverse");
   cudaSetDevice(s->ctx->device);
   KDOP_CUDA(s->ctx, ensure_posed(s));
+  ctl_changes(s);
   KDOP_CUDA(s->ctx, kdop::launch_contacts(s));
   s->contacted = true;
   return KDOP_OK;
@@ -1062,8 +1085,7 @@ int kdop_read_contacts(kdop_scene* s, kdop_contact* rows, int64_t cap, int64_t* 
   if (!s || !n_rows || (cap > 0 && !rows)) return KDOP_ERR_INVALID;
   if (!s->contacted) return fail(s->ctx, KDOP_ERR_STATE, "no contacts yet");
   cudaSetDevice(s->ctx->device);
-  KDOP_CUDA(s->ctx, cudaMemcpyAsync(s->ctl_host, s->ctl, sizeof(TravCtl), cudaMemcpyDeviceToHost, s->ctx->stream));
-  KDOP_CUDA(s->ctx, cudaStreamSynchronize(s->ctx->stream));
+  KDOP_CUDA(s->ctx, read_ctl(s));
   int64_t n = std::min<int64_t>((int64_t)s->ctl_host->n_contacts, s->contact_cap);
   *n_rows = n;
   if (n > cap) return fail(s->ctx, KDOP_ERR_CAPACITY, "contact read buffer too small");
@@ -1177,8 +1199,7 @@ int kdop_contacts_adjoint(kdop_scene* s, const float* dd, const float* dn, float
     KDOP_CUDA(s->ctx, kdop::launch_adjoint(s, dd, dn, grad));
     return KDOP_OK;
   }
-  KDOP_CUDA(s->ctx, cudaMemcpyAsync(s->ctl_host, s->ctl, sizeof(TravCtl), cudaMemcpyDeviceToHost, s->ctx->stream));
-  KDOP_CUDA(s->ctx, cudaStreamSynchronize(s->ctx->stream));
+  KDOP_CUDA(s->ctx, read_ctl(s));
   int64_t nc = std::min<int64_t>((int64_t)s->ctl_host->n_contacts, s->contact_cap);
   int64_t need = std::max<int64_t>(nc, 1) * 4 + 3 * s->nv;
   cudaError_t e;
@@ -1270,6 +1291,7 @@ int kdop_graph_launch(kdop_scene* s) {
   if (!s) return KDOP_ERR_INVALID;
   if (!s->graph_exec) return fail(s->ctx, KDOP_ERR_STATE, "no captured graph");
   cudaSetDevice(s->ctx->device);
+  ctl_changes(s);
   KDOP_CUDA(s->ctx, cudaGraphLaunch(s->graph_exec, s->ctx->stream));
   s->ctx->launches += ext(s)->graph_kernels;
   // the step just enqueued refits in the graph's mode: the contacts, the
@@ -1288,6 +1310,7 @@ int kdop_graph_launch(kdop_scene* s) {
 static float time_config(kdop_scene* s, int64_t n_pairs, const kdop::TravParams& p, int repeats,
                          std::vector<cudaEvent_t>& ev) {
   if (kdop::traverse_smem_bytes(p.block_warps, p.stack_cap) > s->ctx->smem_optin) return -1.f;
+  ctl_changes(s);
   if (kdop::launch_traverse(s, n_pairs, s->pairs, p, 0) != cudaSuccess) return -1.f;
   kdop_stats st;
   int r = kdop_get_stats(s, &st);
@@ -1295,10 +1318,12 @@ static float time_config(kdop_scene* s, int64_t n_pairs, const kdop::TravParams&
     int64_t nc = std::max<int64_t>(st.n_candidates + st.n_candidates / 4, s->cand_cap);
     int64_t nq = (st.device_error & kdop::DEV_ERR_QUEUE_FULL) ? std::max<int64_t>(2 * s->queue_cap, 2 * st.queue_used) : 0;
     if (kdop_reserve(s, nc, 0, nq) != KDOP_OK) return -1.f;
+    ctl_changes(s);
     if (kdop::launch_traverse(s, n_pairs, s->pairs, p, 0) != cudaSuccess) return -1.f;
     r = kdop_get_stats(s, &st);
   }
   if (r != KDOP_OK) return -1.f;
+  ctl_changes(s);
   cudaEventRecord(ev[0], s->ctx->stream);
   for (int k = 0; k < repeats; ++k) {
     kdop::launch_traverse(s, n_pairs, s->pairs, p, 0);

@@ -157,6 +157,8 @@ struct kdop_scene {
   int64_t queue_cap = 0;
   kdop::TravCtl* ctl = nullptr;
   kdop::TravCtl* ctl_host = nullptr;  // pinned
+  bool ctl_fresh = false;     // ctl_host holds what ctl does once the stream has run
+  bool ctl_replayed = false;  // calls were captured into a caller's graph, which changes ctl unseen
 
   int host_orders = 0;  // meshes whose leaf order came from the host (device build)
   int refit_mode = -1;
