@@ -246,21 +246,16 @@ static void scene_free(kdop_scene* s) {
   dfree(s, &s->nodes, s->nn * s->NW);
   if (s->root_dev) cudaFree(s->root_dev);
   s->root_dev = nullptr;
-  dfree(s, &s->t_off_dev, s->n_meshes + 1);
-  dfree(s, &s->leaf_verts, s->nt);
-  dfree(s, &s->leaf_tet, s->nt);
-  dfree(s, &s->refit_blocks, s->refit_stage.empty() ? 0 : s->refit_stage.back());
+  dfree(s, &s->tables, s->tables_bytes);
   dfree(s, &s->quat, s->n_meshes);
   dfree(s, &s->pos, s->n_meshes);
   dfree(s, &s->lin_vel, s->n_meshes);
   dfree(s, &s->ang_vel, s->n_meshes);
   dfree(s, &s->phase_dev, 1);
-  dfree(s, &s->pairs, s->pairs_cap);
-  dfree(s, &s->pair_order, s->pairs_cap);
+  dfree(s, &s->lists, s->lists_bytes);
   dfree(s, &s->cand, kdop::kCandCols * s->cand_cap);
   dfree(s, &s->contacts, s->contact_cap);
   dfree(s, &s->records, s->cand_cap);
-  dfree(s, &s->seeds, s->seeds_cap);
   dfree(s, &s->q_items, s->queue_cap);
   dfree(s, &s->q_tags, s->queue_cap);
   dfree(s, &s->ctl, 1);
@@ -336,15 +331,19 @@ static int grow_queue(kdop_scene* s, int64_t n) {
 
 static int grow_pairs(kdop_scene* s, int64_t n) {
   if (n <= s->pairs_cap) return KDOP_OK;
+  // one block: the seed pass's entries, the pairs, their order.  The old one is
+  // kept until the new one is there: the last results' pairs are read from it.
+  const int64_t seeds = kdop::seed_entries(s->ctx->sm_count, n) * (int64_t)sizeof(uint4);
+  const int64_t bytes = seeds + n * (int64_t)(sizeof(uint2) + sizeof(uint32_t));
+  char* lists = nullptr;
+  KDOP_CUDA(s->ctx, dalloc(s, &lists, bytes));
   drop_graph(s);
-  dfree(s, &s->pairs, s->pairs_cap);
-  dfree(s, &s->pair_order, s->pairs_cap);
-  dfree(s, &s->seeds, s->seeds_cap);
-  s->pairs_cap = s->seeds_cap = 0;
-  KDOP_CUDA(s->ctx, dalloc(s, &s->pair_order, n));
-  KDOP_CUDA(s->ctx, dalloc(s, &s->pairs, n));
-  KDOP_CUDA(s->ctx, dalloc(s, &s->seeds, kdop::seed_entries(s->ctx->sm_count, n)));
-  s->seeds_cap = kdop::seed_entries(s->ctx->sm_count, n);
+  dfree(s, &s->lists, s->lists_bytes);
+  s->lists = lists;
+  s->lists_bytes = bytes;
+  s->seeds = reinterpret_cast<uint4*>(s->lists);
+  s->pairs = reinterpret_cast<uint2*>(s->lists + seeds);
+  s->pair_order = reinterpret_cast<uint32_t*>(s->pairs + n);
   s->pairs_cap = n;
   return KDOP_OK;
 }
@@ -472,14 +471,20 @@ int kdop_scene_create_ex(kdop_ctx* ctx, int K, int n_meshes, const kdop_mesh_des
     size_t root_bytes = (size_t)n_meshes * 4;
     SC_TRY(cudaMalloc((void**)&s->root_dev, std::max<size_t>(root_bytes, 8)));
     s->device_bytes += (int64_t)root_bytes;
-    SC_TRY(dalloc(s, &s->t_off_dev, n_meshes + 1));
-    std::vector<uint32_t> toff(s->t_off.begin(), s->t_off.end());
-    SC_TRY(cudaMemcpyAsync(s->t_off_dev, toff.data(), toff.size() * 4, cudaMemcpyHostToDevice, st));
     std::vector<kdop::RefitBlock> rblocks;
     kdop::refit_blocks(fb, pre, lg, nts, s->t_off, rblocks, s->refit_stage);
-    SC_TRY(dalloc(s, &s->leaf_verts, nt));
-    SC_TRY(dalloc(s, &s->leaf_tet, nt));
-    SC_TRY(dalloc(s, &s->refit_blocks, (int64_t)rblocks.size()));
+    // one block of tables: the refit's blocks, vertices of the tets in leaf
+    // order, tets in leaf order, tet offsets
+    const size_t o_verts = rblocks.size() * sizeof(kdop::RefitBlock), o_tet = o_verts + (size_t)nt * sizeof(uint4),
+                 o_off = o_tet + (size_t)nt * 4;
+    s->tables_bytes = (int64_t)(o_off + ((size_t)n_meshes + 1) * 4);
+    SC_TRY(dalloc(s, &s->tables, s->tables_bytes));
+    s->refit_blocks = reinterpret_cast<kdop::RefitBlock*>(s->tables);
+    s->leaf_verts = reinterpret_cast<uint4*>(s->tables + o_verts);
+    s->leaf_tet = reinterpret_cast<uint32_t*>(s->tables + o_tet);
+    s->t_off_dev = reinterpret_cast<uint32_t*>(s->tables + o_off);
+    std::vector<uint32_t> toff(s->t_off.begin(), s->t_off.end());
+    SC_TRY(cudaMemcpyAsync(s->t_off_dev, toff.data(), toff.size() * 4, cudaMemcpyHostToDevice, st));
     SC_TRY(cudaMemcpyAsync(s->refit_blocks, rblocks.data(), rblocks.size() * sizeof(kdop::RefitBlock),
                            cudaMemcpyHostToDevice, st));
     SC_TRY(dalloc(s, &s->quat, n_meshes));

@@ -127,6 +127,8 @@ struct kdop_scene {
   uint8_t* surf = nullptr;
   float4* nodes = nullptr;
   uint32_t* root_dev = nullptr;
+  char* tables = nullptr;          // the next four, in one allocation
+  int64_t tables_bytes = 0;
   uint4* leaf_verts = nullptr;     // global vertex indices of the tets in leaf order, mesh by mesh
   uint32_t* leaf_tet = nullptr;    // tet | surface bit of the same
   kdop::RefitBlock* refit_blocks = nullptr;  // blocks of the refit's launches, launch i from refit_stage[i] on
@@ -141,6 +143,8 @@ struct kdop_scene {
   bool have_world = false;
 
   // traversal / contacts buffers
+  char* lists = nullptr;  // seeds, pairs and pair_order, in one allocation
+  int64_t lists_bytes = 0;
   uint2* pairs = nullptr;
   uint32_t* pair_order = nullptr;  // pair indices by decreasing size (tets of A + tets of B)
   int64_t pairs_cap = 0;
@@ -151,7 +155,6 @@ struct kdop_scene {
   int4* records = nullptr;  // per candidate: faces, candidate codes, count, first contact
   int64_t contact_cap = 0;
   uint4* seeds = nullptr;  // frontiers of the seed pass: seed_entries(pairs_cap)
-  int64_t seeds_cap = 0;
   uint4* q_items = nullptr;
   uint32_t* q_tags = nullptr;
   int64_t queue_cap = 0;
