@@ -34,7 +34,8 @@ struct RefitBlock {
   int32_t levels;       // levels above its nodes (8, fewer in a small tree)
   uint32_t node[9];     // first node of each of its levels, the ancestor's first
   uint32_t pad_node;    // the root level's padding node, for the block that writes the root it repeats
-  uint32_t pad[2];
+  uint32_t warps_alone; // its warps stop at their own ancestors, five levels up
+  uint32_t pad;
 };
 static_assert(sizeof(RefitBlock) == 64, "one 64-byte record per block");
 

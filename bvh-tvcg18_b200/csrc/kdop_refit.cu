@@ -106,13 +106,30 @@ __device__ __forceinline__ void leaf_slabs(const float4* __restrict__ world, uin
 
 constexpr int kRefitUp = 8;                    // levels a block unites above its nodes
 constexpr int kRefitSlots = 1 << kRefitUp;     // nodes a block starts from
+constexpr int64_t kWarpsAloneBlocks = 2048;    // from this many blocks on, warps of the first launch stop alone
 // Shared-memory row of one record word: the block's nodes in heap order (root
-// 1).  The stride keeps the words of a chunk and the nodes of eight twins on
-// different banks, and node pairs 8-byte aligned.
-constexpr int kRefitRow = 2 * kRefitSlots + 2;
+// 1).  Rows are 8 banks apart, so that two slabs a lane group apart in a union
+// fall on other halves of the banks, and a chunk's four rows are shifted by
+// chunk_skew banks more, so that the chunks of consecutive twins, which the
+// lanes of a store take, do not meet (rows of 514 words without the shift cost
+// 6.4 M of 43 M shared-memory passes at K = 18).
+constexpr int kRefitRow = 2 * kRefitSlots + 8;
+template <int K>
+__host__ __device__ constexpr int chunk_skew() {
+  constexpr int NW = NodeLayout<K>::NW;
+  return NW == 2 ? 16 : NW == 3 ? 10 : NW == 4 ? 8 : NW <= 6 ? 6 : 4;
+}
+template <int K>
+__device__ __forceinline__ float* word_row(float* T, int w) {
+  return T + w * kRefitRow + chunk_skew<K>() * (w >> 2);
+}
+template <int K>
+__host__ __device__ constexpr int refit_words() {
+  return (K * kRefitRow + chunk_skew<K>() * NodeLayout<K>::NW + 1) & ~1;  // slot_words follow, 8-byte aligned
+}
 template <int K>
 constexpr size_t refit_smem() {
-  return (size_t)K * kRefitRow * 4 + kRefitSlots * 8;
+  return (size_t)refit_words<K>() * 4 + kRefitSlots * 8;
 }
 
 struct RefitArgs {
@@ -126,8 +143,9 @@ struct RefitArgs {
 
 // Slab x of node U of the block's heap: the union of its children (make_union;
 // slabs hold no NaN and no -0, so fminf / fmaxf are the reference's choices).
+template <int K>
 __device__ __forceinline__ void unite_slab(float* T, uint32_t U, int x) {
-  float* row = T + 2 * x * kRefitRow;
+  float* row = word_row<K>(T, 2 * x);
   const float2 lo = *reinterpret_cast<const float2*>(row + 2 * U);
   const float2 hi = *reinterpret_cast<const float2*>(row + kRefitRow + 2 * U);
   row[U] = fminf(lo.x, lo.y);
@@ -140,7 +158,7 @@ __device__ __forceinline__ void unite_level(float* T, uint32_t root, int lane) {
 #pragma unroll
   for (int it = 0; it * 32 < N; ++it)
     if ((it + 1) * 32 <= N || it * 32 + lane < N)
-      unite_slab(T, (root << M) + (uint32_t)(lane & ((1 << M) - 1)), (lane >> M) + it * (32 >> M));
+      unite_slab<K>(T, (root << M) + (uint32_t)(lane & ((1 << M) - 1)), (lane >> M) + it * (32 >> M));
   __syncwarp();
 }
 
@@ -148,7 +166,7 @@ __device__ __forceinline__ void unite_level(float* T, uint32_t root, int lane) {
 // words of its two nodes are we, wo.
 template <int K>
 __device__ __forceinline__ void put_chunk(const float* T, uint32_t U, int j, uint2 we, uint2 wo, float4* to) {
-  const float* col = T + 4 * j * kRefitRow + 2 * U;
+  const float* col = T + j * (4 * kRefitRow + chunk_skew<K>()) + 2 * U;
   float e[4], o[4];
 #pragma unroll
   for (int c = 0; c < 4; ++c) {
@@ -167,6 +185,18 @@ __device__ __forceinline__ void put_chunk(const float* T, uint32_t U, int j, uin
     o[c + 1] = __uint_as_float(wo.y);
   }
   stg256(to, e, o);
+}
+// Chunk j of heap node U alone.
+template <int K>
+__device__ __forceinline__ float4 half_chunk(float* T, uint32_t U, int j, uint2 words) {
+  float e[4];
+#pragma unroll
+  for (int c = 0; c < 4; ++c) {
+    const int w = 4 * j + c;
+    e[c] = w < K ? word_row<K>(T, w)[U]
+                 : w == K ? __uint_as_float(words.x) : w == K + 1 ? __uint_as_float(words.y) : 0.f;
+  }
+  return make_float4(e[0], e[1], e[2], e[3]);
 }
 // The twins of the children of the 2^M nodes M levels below heap node `root`,
 // which is the at-th of its level: consecutive records from node `first` on; a
@@ -204,8 +234,8 @@ __global__ void __launch_bounds__(kRefitSlots, K <= 8 ? 6 : K <= 14 ? 5 : K <= 2
     refit_kernel(const __grid_constant__ RefitArgs a) {
   using L = NodeLayout<K>;
   constexpr int NW = L::NW, NS = L::NS;
-  extern __shared__ float T[];  // T[w * kRefitRow + heap index]
-  uint2* slot_words = reinterpret_cast<uint2*>(T + K * kRefitRow);
+  extern __shared__ float T[];  // word_row(T, w)[heap index]
+  uint2* slot_words = reinterpret_cast<uint2*>(T + refit_words<K>());
   const RefitBlock& b = a.blocks[blockIdx.x];
   const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
   const int hd = b.levels;             // levels above the block's nodes in this block
@@ -262,8 +292,8 @@ __global__ void __launch_bounds__(kRefitSlots, K <= 8 ? 6 : K <= 14 ? 5 : K <= 2
         slot_words[t] = words;
 #pragma unroll
         for (int k = 0; k < K; k += 2) {
-          T[k * kRefitRow + cnt + t] = fminf(w[k], v[k]);
-          T[(k + 1) * kRefitRow + cnt + t] = fmaxf(w[k + 1], v[k + 1]);
+          word_row<K>(T, k)[cnt + t] = fminf(w[k], v[k]);
+          word_row<K>(T, k + 1)[cnt + t] = fmaxf(w[k + 1], v[k + 1]);
         }
       }
     } else {
@@ -275,7 +305,7 @@ __global__ void __launch_bounds__(kRefitSlots, K <= 8 ? 6 : K <= 14 ? 5 : K <= 2
         const float e[4] = {x.x, x.y, x.z, x.w};
 #pragma unroll
         for (int c = 0; c < 4; ++c)
-          if (4 * j + c < K) T[(4 * j + c) * kRefitRow + cnt + i] = e[c];
+          if (4 * j + c < K) word_row<K>(T, 4 * j + c)[cnt + i] = e[c];
       }
     }
     __syncwarp();
@@ -294,10 +324,15 @@ __global__ void __launch_bounds__(kRefitSlots, K <= 8 ? 6 : K <= 14 ? 5 : K <= 2
       put_level<K, 2>(a.nodes, T, root, b.node[hd - 2] + 8u * w, b.node[hd - 1] + 16u * w, nullptr, lane);
       put_level<K, 1>(a.nodes, T, root, b.node[hd - 3] + 4u * w, b.node[hd - 2] + 8u * w, nullptr, lane);
       put_level<K, 0>(a.nodes, T, root, b.node[hd - 4] + 2u * w, b.node[hd - 3] + 4u * w, nullptr, lane);
+      if (b.warps_alone && lane < NW) {
+        // the next launch starts from the warps' ancestors
+        const uint32_t kids = b.node[hd - 4] + 2u * w;
+        a.nodes[L::at(b.node[hd - 5] + w, lane)] = half_chunk<K>(T, root, lane, make_uint2(kids, kids + 1u));
+      }
     } else {
       // a tree of fewer than 64 tets (or its last levels): one warp, level by level
       for (int m = wl - 1; m >= 0; --m) {
-        for (int x = lane; x < (NS << m); x += 32) unite_slab(T, (1u << m) + (x & ((1 << m) - 1)), x >> m);
+        for (int x = lane; x < (NS << m); x += 32) unite_slab<K>(T, (1u << m) + (x & ((1 << m) - 1)), x >> m);
         __syncwarp();
       }
       for (int m = BOTTOM ? wl - 1 : wl - 2; m >= 0; --m)
@@ -313,10 +348,11 @@ __global__ void __launch_bounds__(kRefitSlots, K <= 8 ? 6 : K <= 14 ? 5 : K <= 2
         }
     }
   }
+  if (b.warps_alone) return;
   __syncthreads();
   if (wib > 0) return;
   for (int n = warps >> 1; n >= 1; n >>= 1) {
-    for (int x = lane; x < n * NS; x += 32) unite_slab(T, (uint32_t)(n + x % n), x / n);
+    for (int x = lane; x < n * NS; x += 32) unite_slab<K>(T, (uint32_t)(n + x % n), x / n);
     __syncwarp();
   }
   for (int q = lane; q < (warps - 1) * NW; q += 32) {
@@ -330,21 +366,11 @@ __global__ void __launch_bounds__(kRefitSlots, K <= 8 ? 6 : K <= 14 ? 5 : K <= 2
   // the common ancestor: one half of a twin
   if (lane < NW) {
     const uint2 words = (BOTTOM && hd == 0) ? slot_words[0] : make_uint2(b.node[1], b.node[1] + 1u);
-    float e[4];
-#pragma unroll
-    for (int c = 0; c < 4; ++c) {
-      const int w = 4 * lane + c;
-      e[c] = w < K ? T[w * kRefitRow + 1]
-                   : w == K ? __uint_as_float(words.x) : w == K + 1 ? __uint_as_float(words.y) : 0.f;
-    }
-    a.nodes[L::at(b.node[0], lane)] = make_float4(e[0], e[1], e[2], e[3]);
+    a.nodes[L::at(b.node[0], lane)] = half_chunk<K>(T, 1u, lane, words);
     if (b.pad_node != NO_NODE) {
       // the root level's padding node: the root again (a leaf under its own index)
-#pragma unroll
-      for (int c = 0; c < 4; ++c)
-        if (4 * lane + c == K && (words.x & LEAF_BIT))
-          e[c] = __uint_as_float((words.x & (LEAF_BIT | SURF_BIT)) | b.pad_node);
-      a.nodes[L::at(b.pad_node, lane)] = make_float4(e[0], e[1], e[2], e[3]);
+      const uint32_t own = (words.x & LEAF_BIT) ? (words.x & (LEAF_BIT | SURF_BIT)) | b.pad_node : words.x;
+      a.nodes[L::at(b.pad_node, lane)] = half_chunk<K>(T, 1u, lane, make_uint2(own, words.y));
     }
   }
 }
@@ -582,8 +608,13 @@ static cudaError_t refit_impl(kdop_scene* s, int mode) {
 }
 
 // Blocks of each launch of a refit (launch i: blocks stage[i] .. stage[i + 1]):
-// one per 256 nodes of depth L - 8 i of every tree.  pre: nodes of the trees
-// before m at depth d; t_off: first tet of a mesh.
+// one per 256 nodes of depth L of every tree, then of depth L - 8, L - 16 and so
+// on.  In a large forest the first launch's warps stop at their own ancestors
+// and the depths are L, L - 5, L - 13, ...: its blocks then have no barrier and
+// no last levels that one warp works on while the other seven's place stays
+// taken (96 trees of 48,000 tets, 12,288 blocks, K = 18: 222 -> 211 us, K = 26: 307 -> 287); in a small
+// one the launch that this can add costs more.  pre: nodes of the trees before
+// m at depth d; t_off: first tet of a mesh.
 void refit_blocks(const ForestBuild& fb, const std::vector<int64_t>& pre, const std::vector<int32_t>& lg,
                   const std::vector<int64_t>& n_tets, const std::vector<int64_t>& t_off,
                   std::vector<RefitBlock>& blocks, std::vector<int64_t>& stage) {
@@ -602,10 +633,14 @@ void refit_blocks(const ForestBuild& fb, const std::vector<int64_t>& pre, const 
   if (n_roots > 0 && fb.level_off[1] - fb.level_off[0] > n_roots) pad = (uint32_t)(fb.level_off[1] - 1);
   size_t first = 0;
   while (first < nm && lg[first] < 0) ++first;
+  int64_t bottom = 0;
+  for (size_t m = 0; m < nm; ++m) bottom += lg[m] >= 0 ? int64_t(1) << std::max(lg[m] - kRefitUp, 0) : 0;
+  const bool alone = bottom >= kWarpsAloneBlocks;
   std::vector<std::pair<uint32_t, uint32_t>> range, next;  // tets [f, f + s) of the nodes of one depth
   for (int i = 0;; ++i) {
+    const int above = kRefitUp * i - (alone && i > 0 ? kRefitUp - 5 : 0);
     for (size_t m = 0; m < nm; ++m) {
-      const int d = lg[m] - kRefitUp * i;  // depth 0 is done by the launch before, or is a single node
+      const int d = lg[m] - above;  // depth 0 is done by the launch before, or is a single node
       if (lg[m] < 0 || d < 0 || (i > 0 && d == 0)) continue;
       const int hd = std::min(d, kRefitUp), d0 = d - hd;
       range.assign(1, std::make_pair(0u, (uint32_t)n_tets[m]));
@@ -627,7 +662,8 @@ void refit_blocks(const ForestBuild& fb, const std::vector<int64_t>& pre, const 
         b.levels = hd;
         for (int l = 0; l <= kRefitUp; ++l) b.node[l] = l <= hd ? base(m, d0 + l) + (uint32_t)(j << l) : 0u;
         b.pad_node = (d0 == 0 && m == first) ? pad : NO_NODE;
-        b.pad[0] = b.pad[1] = 0;
+        b.warps_alone = alone && i == 0 && hd > 5;
+        b.pad = 0;
         blocks.push_back(b);
       }
     }

@@ -95,3 +95,34 @@ def test_refit_in_three_launches(ctx, oracle, n):
     ds = kd.DeviceScene(ctx, 18, [mesh, scenes.lattice(2, 0.1, rng)])
     assert mesh.n_tets > 1 << 16
     check(oracle, ds, mesh, 0, 18, mesh.xyz)
+
+
+@pytest.mark.parametrize("K", [14, 18, 26])
+def test_refit_of_a_large_forest(ctx, oracle, K):
+    # above 2,048 blocks of 256 nodes the first launch's warps stop on their own
+    rng = np.random.default_rng(K)
+    big = scenes.lattice(46, 0.2, rng)  # 584,016 tets: 2^19 nodes of depth 19
+    meshes = [soup(n, rng) for n in (1, 31, 32, 33, 64, 65, 130, 300, 5000)] + [big]
+    meshes += [soup(2, rng)] * (1 - len(meshes) % 2)
+    ds = kd.DeviceScene(ctx, K, meshes)
+    worlds = [(m.xyz + rng.uniform(-0.1, 0.1, m.xyz.shape)).astype(np.float32) for m in meshes]
+    ds.set_vertices(np.concatenate(worlds))
+    ds.refit(kd.REFIT_VERTICES)
+    for i, m in enumerate(meshes):
+        if m is not big:
+            check(oracle, ds, m, i, K, worlds[i])
+            continue
+        vol, tet = ds.read_tree(i)
+        leaf = tet >= 0
+        assert np.array_equal(np.sort(tet[leaf]), np.arange(m.n_tets))
+        assert np.array_equal(vol[leaf], oracle.leaf_dops(K, worlds[i], m.tets)[tet[leaf]])
+        at, size = np.array([0]), np.array([m.n_tets])
+        while len(at):  # a level's nodes against their children
+            at, size = at[size > 1], size[size > 1]
+            left = size - size // 2
+            a, b = at + 1, at + 2 * left
+            assert not leaf[at].any()
+            assert np.array_equal(vol[at, 0::2], np.minimum(vol[a, 0::2], vol[b, 0::2]))
+            assert np.array_equal(vol[at, 1::2], np.maximum(vol[a, 1::2], vol[b, 1::2]))
+            at = np.stack([a, b], 1).ravel()
+            size = np.stack([left, size - left], 1).ravel()
