@@ -359,15 +359,23 @@ int kdop_scene_create_ex(kdop_ctx* ctx, int K, int n_meshes, const kdop_mesh_des
   *out = nullptr;
   if (!valid_K(K)) return fail(ctx, KDOP_ERR_INVALID, "K must be one of 6, 8, 12, 14, 18, 20, 26");
   if (n_meshes < 0 || (n_meshes > 0 && !meshes)) return fail(ctx, KDOP_ERR_INVALID, "bad mesh list");
+  // meshes with a vertex index out of range
+  std::vector<char> bad_index((size_t)n_meshes, 0);
+  kdop::parallel_for(n_meshes, [&](int m) {
+    const kdop_mesh_desc& d = meshes[m];
+    if (d.n_verts < 0 || d.n_tets <= 0 || !d.tets) return;
+    uint32_t most = 0;
+    for (int64_t i = 0; i < 4 * d.n_tets; ++i) most = std::max(most, d.tets[i]);
+    bad_index[m] = (int64_t)most >= d.n_verts;
+  });
   int64_t nv = 0, nt = 0;
   for (int m = 0; m < n_meshes; ++m) {
     const kdop_mesh_desc& d = meshes[m];
     if (d.n_verts < 0 || d.n_tets < 0) return fail(ctx, KDOP_ERR_INVALID, "negative mesh size");
     if ((d.n_verts > 0 && !d.xyz) || (d.n_tets > 0 && !d.tets))
       return fail(ctx, KDOP_ERR_INVALID, "null mesh array");
-    for (int64_t i = 0; i < 4 * d.n_tets; ++i)
-      if ((int64_t)d.tets[i] >= d.n_verts)
-        return fail(ctx, KDOP_ERR_INVALID, "tet vertex index out of range in mesh " + std::to_string(m));
+    if (bad_index[m])
+      return fail(ctx, KDOP_ERR_INVALID, "tet vertex index out of range in mesh " + std::to_string(m));
     if (d.leaf_order) {
       std::vector<char> seen((size_t)d.n_tets, 0);
       for (int64_t i = 0; i < d.n_tets; ++i) {
