@@ -15,7 +15,7 @@
 // -- the sorted list without a sort.
 // Bound: latency.  Count and write passes of a thread per body left the GPU
 // idle (12 blocks for 1,500 bodies, each thread a chain of 1,500 loads): 281 us
-// with the scan between them, now one launch of 16 us.
+// with the scan between them, now one launch of 17 us.
 #include <algorithm>
 
 #include "kdop_device.cuh"

@@ -837,7 +837,7 @@ static int upload_pairs(kdop_scene* s, int64_t n, const uint32_t* pairs, int mem
     KDOP_CUDA(s->ctx, cudaMemcpyAsync(s->pairs, pairs, (size_t)n * 8, cudaMemcpyDeviceToDevice, s->ctx->stream));
   }
   // largest pairs first: the traversal takes root pairs in this order.  Sorted
-  // on the device above kHostOrder pairs (18,000 pairs: 0.6 ms on the host, 25
+  // on the device above kHostOrder pairs (18,000 pairs: 1.1 ms on the host, 22
   // us there; up to 256 the host's sort costs less than the sort's launches).
   if (n > kHostOrder) {
     KDOP_CUDA(s->ctx, kdop::launch_pair_order(s, n, (uint32_t)std::max<int64_t>(2 * s->most_tets, 1)));

@@ -21,16 +21,17 @@
 // same graph) into a scene-owned array the leaves read: posing inside the leaf
 // pass would transform each vertex once per tet that uses it (about 24 times
 // in a lattice).
-// Bound: the L1 data pipe (77 % of its peak at K = 14: the leaves' vertex
-// gathers, the shared-memory unions, the records' stores), then HBM (47 %).
-// Each node record is written once; a launch per level wrote every one, read it
+// Bound: the L1 data pipe (73 to 77 % of its peak at K = 14 and 18: the leaves'
+// vertex gathers, the shared-memory unions, the records' stores), then HBM (47
+// %).  Each node record is written once; a launch per level wrote every one, read it
 // again for its parent and gathered a leaf's tet through the record's topology
 // words, which now come from arrays in leaf order.  Steps before -> after: 64
-// deforming pairs of 384 k tets (K = 18) 5.00 -> 3.53 ms, one pair of 1.6 M
-// tets (K = 26) 1.66 -> 1.36 ms, 512 uneven pairs (K = 14) 13.2 -> 12.07 ms,
-// one pair of 6,000 tets 273 -> 202 us.  Not kept: block barriers between the
-// levels and a runtime walk over them (96 trees of 48,000 tets: 217 us against
-// 185), one block fewer per SM (208).
+// deforming pairs of 384 k tets (K = 18) 5.00 -> 3.53 ms (3.15 since the warps
+// of large forests stop alone), one pair of 1.6 M tets (K = 26) 1.66 -> 1.36
+// ms, 512 uneven pairs (K = 14) 13.2 -> 12.07 ms, one pair of 6,000 tets 273 ->
+// 202 us.  Not kept: block barriers between the levels and a runtime walk over
+// them (96 trees of 48,000 tets: 217 us against 185), one block fewer per SM
+// (208).
 #include <algorithm>
 
 #include "kdop_device.cuh"
@@ -106,7 +107,12 @@ __device__ __forceinline__ void leaf_slabs(const float4* __restrict__ world, uin
 
 constexpr int kRefitUp = 8;                    // levels a block unites above its nodes
 constexpr int kRefitSlots = 1 << kRefitUp;     // nodes a block starts from
-constexpr int64_t kWarpsAloneBlocks = 2048;    // from this many blocks on, warps of the first launch stop alone
+// From this many blocks on, the first launch's warps each stop at the ancestor
+// of their own 32 nodes: a block's last three levels and its barrier keep seven
+// of its eight warps' places taken while one works (96 trees of 48,000 tets: K =
+// 18 222 -> 211 us, K = 20 251 -> 229, K = 26 313 -> 287).
+// Smaller forests keep the block's join, which saves levels of the next launch.
+constexpr int64_t kWarpsAloneBlocks = 2048;
 // Shared-memory row of one record word: the block's nodes in heap order (root
 // 1).  Rows are 8 banks apart, so that two slabs a lane group apart in a union
 // fall on other halves of the banks, and a chunk's four rows are shifted by

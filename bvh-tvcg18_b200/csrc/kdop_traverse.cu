@@ -298,12 +298,14 @@ __device__ __forceinline__ unsigned claim_size(unsigned left, unsigned warps) {
 // The lane tests its slabs for the four child pairs; a ballot over the
 // entry's lanes combines the verdicts; the lane holding the topology chunk
 // broadcasts the children's word 0; lane q then handles child pairs q, q + Q.
-// Bound: instruction issue and the L1 data pipe.  A deque holding one pair
+// Bound: the L1 data pipe (82 % of its peak at k = 14; a 256-bit load passes
+// each 128-byte line it touches twice), then the ALU pipe (56 %); 3.1 warp
+// instructions per node-pair test, 4.6 before.  A deque holding one pair
 // only (no pair index beside its entries: 8 instead of 12 bytes of shared
 // memory, the rest of the array caches records), verdicts combined by ballots
 // instead of shuffles, and the refill, root test and donation polls outside
 // the step took the batched workload (1.96 G tests, k = 14) from 11.28 to 9.6
-// ms.
+// ms, and to 9.4 with the lanes beyond the last entry repeating its loads.
 // S sub-batches are loaded together per step, and one compaction per step
 // packs the pushes of all of them.
 template <int K, int C, int S>
@@ -687,7 +689,8 @@ static int64_t seed_group(int sm_count, int64_t n_pairs) {
 // with one pass, 1,022 with two; 64 pairs 601 and 560 us, 256 pairs 455 and
 // 471 us, each against the same loop).
 // Pairs of fewer than kSeedTwiceTets tets in all end in the first pass or soon
-// after it.
+// after it (a touching pair of 384 tets 198 -> 187 us without the second launch
+// and with the poses packed by one).
 static int seed_blocks2(int sm_count, int64_t n_pairs, int64_t tets) {
   return n_pairs <= kSeedTwiceMax && tets >= kSeedTwiceTets ? 2 * sm_count : 0;
 }

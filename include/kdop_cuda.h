@@ -166,7 +166,8 @@ typedef struct {
                              overlapping leaf pair */
   int32_t block_warps;    /* warps per block (0: tuned default) */
   int32_t stack_cap;      /* node-pair entries per warp stack, power of two (0: default) */
-  int32_t init_chunk;     /* root pairs taken per queue claim (0: default) */
+  int32_t init_chunk;     /* root pairs taken per queue claim, and the least number of
+                             seeded frontier entries per claim (0: default) */
   int32_t donate_min;     /* stack size from which a warp gives work to idle warps (0: default) */
   int32_t timeout_ms;     /* bound of every device-side wait (0: 5000) */
   int32_t load_group;     /* expansion shape (0: default 4): 1 = one 32-byte chunk pair per lane
