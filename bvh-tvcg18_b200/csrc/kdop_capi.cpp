@@ -83,6 +83,7 @@ struct kdop_scene_ext {
   int64_t broad_cap = 0;
   float* broad_pos = nullptr;
   std::vector<uint32_t> pairs_host;  // last traversed mesh pairs
+  std::vector<uint32_t> pairs_next;  // a list on its way in
   std::vector<uint32_t> order_host;  // their order of processing
   bool device_order = false;         // made on the device
   int64_t graph_kernels = 0;
@@ -331,18 +332,29 @@ static int grow_queue(kdop_scene* s, int64_t n) {
 
 static int grow_pairs(kdop_scene* s, int64_t n) {
   if (n <= s->pairs_cap) return KDOP_OK;
-  // one block: the seed pass's entries, the pairs, their order.  The old one is
-  // kept until the new one is there: the last results' pairs are read from it.
+  // one block: the seed pass's entries, the pairs, their order.  The pairs are
+  // carried over: the last results' meshes are read from them until the next
+  // list is there.
   const int64_t seeds = kdop::seed_entries(s->ctx->sm_count, n) * (int64_t)sizeof(uint4);
   const int64_t bytes = seeds + n * (int64_t)(sizeof(uint2) + sizeof(uint32_t));
   char* lists = nullptr;
   KDOP_CUDA(s->ctx, dalloc(s, &lists, bytes));
+  uint2* pairs = reinterpret_cast<uint2*>(lists + seeds);
+  cudaError_t e = cudaSuccess;
+  if (s->pairs_cap > 0)
+    e = cudaMemcpyAsync(pairs, s->pairs, (size_t)s->pairs_cap * sizeof(uint2), cudaMemcpyDeviceToDevice,
+                        s->ctx->stream);
+  if (e == cudaSuccess && s->pairs_cap > 0) e = cudaStreamSynchronize(s->ctx->stream);
+  if (e != cudaSuccess) {
+    dfree(s, &lists, bytes);
+    return cuda_fail(s->ctx, e, "pair list copy");
+  }
   drop_graph(s);
   dfree(s, &s->lists, s->lists_bytes);
   s->lists = lists;
   s->lists_bytes = bytes;
   s->seeds = reinterpret_cast<uint4*>(s->lists);
-  s->pairs = reinterpret_cast<uint2*>(s->lists + seeds);
+  s->pairs = pairs;
   s->pair_order = reinterpret_cast<uint32_t*>(s->pairs + n);
   s->pairs_cap = n;
   return KDOP_OK;
@@ -813,29 +825,29 @@ int kdop_traverse_opts_default(const kdop_scene* s, kdop_traverse_opts* o) {
 
 static int upload_pairs(kdop_scene* s, int64_t n, const uint32_t* pairs, int memory) {
   kdop_scene_ext* x = ext(s);
+  // The list is checked before anything of the scene changes: after a refused
+  // one the last results are still there, with the list they came from.
+  std::vector<uint32_t>& list = x->pairs_next;
+  if (memory == KDOP_HOST) {
+    list.assign(pairs, pairs + 2 * n);
+  } else {
+    list.assign((size_t)(2 * n), 0);
+    if (n > 0) {
+      KDOP_CUDA(s->ctx, cudaMemcpyAsync(list.data(), pairs, (size_t)n * 8, cudaMemcpyDeviceToHost, s->ctx->stream));
+      KDOP_CUDA(s->ctx, cudaStreamSynchronize(s->ctx->stream));
+    }
+  }
+  for (uint32_t m : list)
+    if ((int64_t)m >= s->n_meshes) return fail(s->ctx, KDOP_ERR_INVALID, "mesh index out of range in pairs");
   int rc = grow_pairs(s, std::max<int64_t>(n, 1));
   if (rc != KDOP_OK) return rc;
   s->pairs_current = false;  // until a traversal of this list is enqueued
   ctl_changes(s);
-  if (n == 0) {
-    x->pairs_host.clear();
-    return KDOP_OK;
-  }
-  if (memory == KDOP_HOST) {
-    for (int64_t i = 0; i < 2 * n; ++i)
-      if ((int64_t)pairs[i] >= s->n_meshes) return fail(s->ctx, KDOP_ERR_INVALID, "mesh index out of range in pairs");
-    x->pairs_host.assign(pairs, pairs + 2 * n);
-    KDOP_CUDA(s->ctx, cudaMemcpyAsync(s->pairs, pairs, (size_t)n * 8, cudaMemcpyHostToDevice, s->ctx->stream));
-  } else {
-    x->pairs_host.assign((size_t)(2 * n), 0);
-    KDOP_CUDA(s->ctx, cudaMemcpyAsync(x->pairs_host.data(), pairs, (size_t)n * 8, cudaMemcpyDeviceToHost,
-                                      s->ctx->stream));
-    KDOP_CUDA(s->ctx, cudaStreamSynchronize(s->ctx->stream));
-    for (int64_t i = 0; i < 2 * n; ++i)
-      if ((int64_t)x->pairs_host[i] >= s->n_meshes)
-        return fail(s->ctx, KDOP_ERR_INVALID, "mesh index out of range in pairs");
-    KDOP_CUDA(s->ctx, cudaMemcpyAsync(s->pairs, pairs, (size_t)n * 8, cudaMemcpyDeviceToDevice, s->ctx->stream));
-  }
+  x->pairs_host.swap(list);
+  if (n == 0) return KDOP_OK;
+  KDOP_CUDA(s->ctx, cudaMemcpyAsync(s->pairs, pairs, (size_t)n * 8,
+                                    memory == KDOP_HOST ? cudaMemcpyHostToDevice : cudaMemcpyDeviceToDevice,
+                                    s->ctx->stream));
   // largest pairs first: the traversal takes root pairs in this order.  Sorted
   // on the device above kHostOrder pairs (18,000 pairs: 1.1 ms on the host, 22
   // us there; up to 256 the host's sort costs less than the sort's launches).
@@ -1046,8 +1058,7 @@ int kdop_read_candidates(kdop_scene* s, uint32_t* rows, int64_t cap, int64_t* n_
   if (!d) return cuda_fail(s->ctx, e, "staging alloc");
   for (int64_t at = 0; at < n; at += window) {
     const int64_t m = std::min(window, n - at);
-    KDOP_CUDA(s->ctx, kdop::launch_candidate_rows(s, at, m, (int64_t)ext(s)->pairs_host.size() / 2,
-                                                  reinterpret_cast<uint32_t*>(d)));
+    KDOP_CUDA(s->ctx, kdop::launch_candidate_rows(s, at, m, reinterpret_cast<uint32_t*>(d)));
     KDOP_CUDA(s->ctx, cudaMemcpyAsync(rows + 3 * at, d, 3 * (size_t)m * 4, cudaMemcpyDeviceToHost, s->ctx->stream));
   }
   KDOP_CUDA(s->ctx, cudaStreamSynchronize(s->ctx->stream));

@@ -255,9 +255,8 @@ cudaError_t launch_refit(kdop_scene* s, int mode);
 // into device memory.
 cudaError_t launch_preorder(kdop_scene* s, int mesh, int64_t first, int64_t count, float* vol, int64_t* tet);
 // The last traversal's candidates [first, first + n) as (pair, tet of A, tet
-// of B) rows with mesh-local tets, n_pairs = length of the pair list on the
-// device.
-cudaError_t launch_candidate_rows(kdop_scene* s, int64_t first, int64_t n, int64_t n_pairs, uint32_t* rows);
+// of B) rows with mesh-local tets.
+cudaError_t launch_candidate_rows(kdop_scene* s, int64_t first, int64_t n, uint32_t* rows);
 cudaError_t launch_traverse(kdop_scene* s, int64_t n_pairs, const uint2* pairs, const TravParams& p, int plain);
 // broad phase (kdop_broad.cu)
 cudaError_t launch_mesh_radius(kdop_scene* s, unsigned* rbits);

@@ -342,10 +342,11 @@ __global__ void __launch_bounds__(256) contact_gather_kernel(int64_t n, const in
 
 }  // namespace
 
-cudaError_t launch_candidate_rows(kdop_scene* s, int64_t first, int64_t n, int64_t n_pairs, uint32_t* rows) {
+cudaError_t launch_candidate_rows(kdop_scene* s, int64_t first, int64_t n, uint32_t* rows) {
   const uint32_t* c = s->cand + first;
+  // the results' pair indices run over the list on the device, which is as long
   candidate_rows_kernel<<<(unsigned)((n + 255) / 256), 256, 0, s->ctx->stream>>>(
-      c, c + s->cand_cap, c + 2 * s->cand_cap, s->pairs, (uint32_t)n_pairs, s->t_off_dev, n, rows);
+      c, c + s->cand_cap, c + 2 * s->cand_cap, s->pairs, (uint32_t)s->result_pairs, s->t_off_dev, n, rows);
   s->ctx->launches++;
   return cudaGetLastError();
 }
