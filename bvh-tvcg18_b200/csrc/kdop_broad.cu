@@ -62,7 +62,7 @@ constexpr int BR_WARPS = 8;  // bodies per block
 // and not written; total gets the number found.
 __global__ void __launch_bounds__(32 * BR_WARPS) broad_kernel(BoxArgs a, uint2* out, unsigned cap, unsigned* ticket,
                                                               unsigned long long* words, unsigned* total,
-                                                              unsigned* err) {
+                                                              WaitLimit lim) {
   __shared__ unsigned s_tile, s_count[BR_WARPS];
   if (threadIdx.x == 0) s_tile = atomicAdd(ticket, 1u);
   __syncthreads();
@@ -89,7 +89,7 @@ __global__ void __launch_bounds__(32 * BR_WARPS) broad_kernel(BoxArgs a, uint2* 
     if (k < w) before += s_count[k];
     sum += s_count[k];
   }
-  const unsigned first = tile_prefix(words, tile, sum, err);
+  const unsigned first = tile_prefix(words, tile, sum, lim);
   if (threadIdx.x == 0 && (int)(tile + 1) * BR_WARPS >= a.n) *total = first + sum;
   if (n == 0) return;
   unsigned at = first + before;
@@ -167,9 +167,10 @@ cudaError_t broad_phase(kdop_scene* s, const unsigned* rbits, const float* pos_d
   } else {
     a.pos = s->pos;
   }
-  broad_kernel<<<(unsigned)((n + BR_WARPS - 1) / BR_WARPS), 32 * BR_WARPS, 0, st>>>(
-      a, pairs, (unsigned)std::min<int64_t>(cap, 0xFFFFFFFFll), head + 2,
-      reinterpret_cast<unsigned long long*>(w + L.words), head, head + 1);
+  const unsigned blocks = tile_blocks(s->ctx, STUCK_SCAN, head + 2, (unsigned)((n + BR_WARPS - 1) / BR_WARPS));
+  broad_kernel<<<blocks, 32 * BR_WARPS, 0, st>>>(a, pairs, (unsigned)std::min<int64_t>(cap, 0xFFFFFFFFll), head + 2,
+                                                 reinterpret_cast<unsigned long long*>(w + L.words), head,
+                                                 WaitLimit{head + 1, s->ctx->wait_ns});
   s->ctx->launches += pos_dev ? 2 : 1;
   unsigned h[2];
   if ((e = cudaMemcpyAsync(h, head, sizeof(h), cudaMemcpyDeviceToHost, st)) != cudaSuccess) return e;

@@ -139,9 +139,9 @@ struct MeshGen {
 // equal neighbouring codes within a mesh
 __global__ void ties_kernel(const uint4* __restrict__ tets, const float4* __restrict__ rest,
                             const uint32_t* __restrict__ vals, const uint64_t* __restrict__ codes, int64_t nt,
-                            uint32_t* tied) {
+                            uint32_t* tied, const unsigned* err) {
   int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (i < 1 || i >= nt) return;
+  if (i < 1 || i >= nt || gave_up(err)) return;  // the order may be incomplete
   uint32_t a = vals[i - 1], b = vals[i];
   int ma = mesh_of(rest, __ldg(tets + a).x), mb = mesh_of(rest, __ldg(tets + b).x);
   if (ma == mb && codes[a] == codes[b]) tied[ma] = 1u;
@@ -302,16 +302,16 @@ cudaError_t device_morton_perm(kdop_scene* s, uint32_t* perm, std::vector<char>&
         cudaSuccess)
       break;
     if ((e = cudaMemsetAsync(tied, 0, (size_t)nm * 4 + 4, st)) != cudaSuccess) break;
-    if ((e = radix_sort(CodeGen{s->tets, s->rest, prm, codes}, nt, 63, b, w + o_rad, err, st, s->ctx->launches)) !=
-        cudaSuccess)
+    const WaitLimit lim{err, s->ctx->wait_ns};
+    if ((e = radix_sort(s->ctx, CodeGen{s->tets, s->rest, prm, codes}, nt, 63, b, w + o_rad, lim)) != cudaSuccess)
       break;
-    if ((e = radix_sort(MeshGen{s->tets, s->rest, b.vals}, nt, bits_of(nm - 1), b, w + o_rad, err, st,
-                        s->ctx->launches)) != cudaSuccess)
+    if ((e = radix_sort(s->ctx, MeshGen{s->tets, s->rest, b.vals}, nt, bits_of(nm - 1), b, w + o_rad, lim)) !=
+        cudaSuccess)
       break;
     if (b.vals != perm &&
         (e = cudaMemcpyAsync(perm, b.vals, (size_t)nt * 4, cudaMemcpyDeviceToDevice, st)) != cudaSuccess)
       break;
-    ties_kernel<<<g, 256, 0, st>>>(s->tets, s->rest, perm, codes, nt, tied);
+    ties_kernel<<<g, 256, 0, st>>>(s->tets, s->rest, perm, codes, nt, tied, err);
     std::vector<uint32_t> ht((size_t)nm + 1);
     if ((e = cudaMemcpyAsync(ht.data(), tied, (size_t)nm * 4 + 4, cudaMemcpyDeviceToHost, st)) != cudaSuccess) break;
     if ((e = cudaStreamSynchronize(st)) != cudaSuccess) break;

@@ -32,7 +32,8 @@ int fail(kdop_ctx* ctx, int status, const std::string& msg) {
 int cuda_fail(kdop_ctx* ctx, cudaError_t e, const char* where) {
   std::string m = std::string(where) + ": " + cudaGetErrorString(e);
   cudaGetLastError();
-  return fail(ctx, KDOP_ERR_CUDA, m);
+  // (also how the launchers report a device-side wait that gave up)
+  return fail(ctx, e == cudaErrorLaunchTimeout ? KDOP_ERR_TIMEOUT : KDOP_ERR_CUDA, m);
 }
 
 #define KDOP_CUDA(ctx, call)                                   \
@@ -101,6 +102,8 @@ struct SceneBox {
   kdop_scene_ext x;
 };
 static kdop_scene_ext* ext(kdop_scene* s) { return &reinterpret_cast<SceneBox*>(s)->x; }
+
+static int lost(kdop_scene* s) { return fail(s->ctx, KDOP_ERR_STATE, "results lost: a wait of their sort timed out"); }
 
 static float* stage(kdop_scene* s, int64_t nfloats, cudaError_t* err) {
   kdop_scene_ext* x = ext(s);
@@ -223,6 +226,13 @@ int kdop_ctx_set_stream(kdop_ctx* ctx, void* stream) {
 }
 
 void* kdop_ctx_stream(const kdop_ctx* ctx) { return ctx ? (void*)ctx->stream : nullptr; }
+
+int kdop_ctx_set_wait_limit(kdop_ctx* ctx, int timeout_ms, int test_stuck) {
+  if (!ctx || timeout_ms < 0 || test_stuck < 0 || test_stuck > 3) return KDOP_ERR_INVALID;
+  ctx->wait_ns = (long long)(timeout_ms > 0 ? timeout_ms : 5000) * 1000000ll;
+  ctx->test_stuck = test_stuck;
+  return KDOP_OK;
+}
 
 int kdop_ctx_synchronize(kdop_ctx* ctx) {
   if (!ctx) return KDOP_ERR_INVALID;
@@ -823,7 +833,7 @@ int kdop_traverse_opts_default(const kdop_scene* s, kdop_traverse_opts* o) {
   return KDOP_OK;
 }
 
-static int upload_pairs(kdop_scene* s, int64_t n, const uint32_t* pairs, int memory) {
+static int upload_pairs(kdop_scene* s, int64_t n, const uint32_t* pairs, int memory, long long wait_ns) {
   kdop_scene_ext* x = ext(s);
   // The list is checked before anything of the scene changes: after a refused
   // one the last results are still there, with the list they came from.
@@ -852,7 +862,7 @@ static int upload_pairs(kdop_scene* s, int64_t n, const uint32_t* pairs, int mem
   // on the device above kHostOrder pairs (18,000 pairs: 1.1 ms on the host, 22
   // us there; up to 256 the host's sort costs less than the sort's launches).
   if (n > kHostOrder) {
-    KDOP_CUDA(s->ctx, kdop::launch_pair_order(s, n, (uint32_t)std::max<int64_t>(2 * s->most_tets, 1)));
+    KDOP_CUDA(s->ctx, kdop::launch_pair_order(s, n, (uint32_t)std::max<int64_t>(2 * s->most_tets, 1), wait_ns));
     x->device_order = true;
     s->pairs_tets = 2 * s->most_tets;  // a bound is enough for long lists
     return KDOP_OK;
@@ -882,13 +892,14 @@ int kdop_traverse(kdop_scene* s, int64_t n_pairs, const uint32_t* pairs, int mem
   kdop::TravParams p;
   int mode = 0;
   if (kdop_resolve_traverse_opts(s, opts, p, mode) != KDOP_OK) return fail(s->ctx, KDOP_ERR_INVALID, "bad traversal options");
-  int rc = upload_pairs(s, n_pairs, pairs, memory);
+  int rc = upload_pairs(s, n_pairs, pairs, memory, p.timeout_ns);
   if (rc != KDOP_OK) return rc;
   KDOP_CUDA(s->ctx, kdop::launch_traverse(s, n_pairs, s->pairs, p, mode == KDOP_TRAVERSE_PLAIN));
   s->traversed = true;
   s->contacted = false;
   s->last_pairs = s->result_pairs = n_pairs;
   s->pairs_current = true;
+  s->results_lost = false;
   s->last_mode = mode;
   s->last_params = p;
   return KDOP_OK;
@@ -955,7 +966,7 @@ int kdop_traverse_shard(kdop_scene* s, int64_t n_pairs, const uint32_t* pairs, i
   int mode = 0;
   if (kdop_resolve_traverse_opts(s, opts, p, mode) != KDOP_OK || mode != KDOP_TRAVERSE_BATCHED)
     return fail(s->ctx, KDOP_ERR_INVALID, "bad traversal options (shards are batched)");
-  int rc = upload_pairs(s, n_pairs, pairs, memory);
+  int rc = upload_pairs(s, n_pairs, pairs, memory, p.timeout_ns);
   if (rc != KDOP_OK) return rc;
   int64_t ne = 0;
   kdop_scene_ext* x = ext(s);
@@ -968,6 +979,7 @@ int kdop_traverse_shard(kdop_scene* s, int64_t n_pairs, const uint32_t* pairs, i
   s->contacted = false;
   s->last_pairs = s->result_pairs = n_pairs;
   s->pairs_current = true;
+  s->results_lost = false;
   s->last_mode = mode;
   s->last_params = p;
   return KDOP_OK;
@@ -1046,6 +1058,7 @@ int kdop_set_capacity(kdop_scene* s, int64_t candidates, int64_t contacts, int64
 int kdop_read_candidates(kdop_scene* s, uint32_t* rows, int64_t cap, int64_t* n_rows) {
   if (!s || !n_rows || (cap > 0 && !rows)) return KDOP_ERR_INVALID;
   if (!s->traversed) return fail(s->ctx, KDOP_ERR_STATE, "no traversal yet");
+  if (s->results_lost) return lost(s);
   cudaSetDevice(s->ctx->device);
   KDOP_CUDA(s->ctx, read_ctl(s));
   int64_t n = std::min<int64_t>((int64_t)s->ctl_host->n_cand, s->cand_cap);
@@ -1068,6 +1081,7 @@ int kdop_read_candidates(kdop_scene* s, uint32_t* rows, int64_t cap, int64_t* n_
 int kdop_sort_results(kdop_scene* s) {
   if (!s) return KDOP_ERR_INVALID;
   if (!s->traversed) return fail(s->ctx, KDOP_ERR_STATE, "kdop_sort_results before kdop_traverse");
+  if (s->results_lost) return lost(s);
   kdop_stats st;
   int rc = kdop_get_stats(s, &st);  // synchronises; reports overflow and device errors
   if (rc != KDOP_OK) return rc;
@@ -1088,15 +1102,19 @@ int kdop_sort_results(kdop_scene* s) {
     s->device_bytes += (int64_t)need;
   }
   ctl_changes(s);
-  KDOP_CUDA(s->ctx, kdop::sort_results(s, n, nc, x->sort_work, s->ctx->stream));
+  KDOP_CUDA(s->ctx, kdop::sort_results(s, n, nc, x->sort_work));
   KDOP_CUDA(s->ctx, read_ctl(s));
-  if (s->ctl_host->error & kdop::DEV_ERR_TIMEOUT) return fail(s->ctx, KDOP_ERR_TIMEOUT, "sort wait timed out");
+  if (s->ctl_host->error & kdop::DEV_ERR_TIMEOUT) {
+    s->results_lost = true;
+    return fail(s->ctx, KDOP_ERR_TIMEOUT, "sort wait timed out");
+  }
   return KDOP_OK;
 }
 
 int kdop_contacts(kdop_scene* s) {
   if (!s) return KDOP_ERR_INVALID;
   if (!s->traversed) return fail(s->ctx, KDOP_ERR_STATE, "kdop_contacts before kdop_traverse");
+  if (s->results_lost) return lost(s);
   cudaSetDevice(s->ctx->device);
   KDOP_CUDA(s->ctx, ensure_posed(s));
   ctl_changes(s);
@@ -1108,6 +1126,7 @@ int kdop_contacts(kdop_scene* s) {
 int kdop_read_contacts(kdop_scene* s, kdop_contact* rows, int64_t cap, int64_t* n_rows) {
   if (!s || !n_rows || (cap > 0 && !rows)) return KDOP_ERR_INVALID;
   if (!s->contacted) return fail(s->ctx, KDOP_ERR_STATE, "no contacts yet");
+  if (s->results_lost) return lost(s);
   cudaSetDevice(s->ctx->device);
   KDOP_CUDA(s->ctx, read_ctl(s));
   int64_t n = std::min<int64_t>((int64_t)s->ctl_host->n_contacts, s->contact_cap);
@@ -1198,6 +1217,7 @@ int kdop_reduce_contact_rows(kdop_ctx* ctx, const kdop_contact* rows, const uint
 int kdop_reduce_contacts(kdop_scene* s, kdop_contact* out, uint32_t* out_bodies, int64_t cap, int64_t* n_out) {
   if (!s || !n_out || (cap > 0 && !out)) return KDOP_ERR_INVALID;
   if (!s->contacted) return fail(s->ctx, KDOP_ERR_STATE, "kdop_reduce_contacts before kdop_contacts");
+  if (s->results_lost) return lost(s);
   kdop_stats st;
   int rc = kdop_get_stats(s, &st);  // synchronises; reports overflow and device errors
   if (rc != KDOP_OK) return rc;
@@ -1217,6 +1237,7 @@ int kdop_reduce_contacts(kdop_scene* s, kdop_contact* out, uint32_t* out_bodies,
 int kdop_contacts_adjoint(kdop_scene* s, const float* dd, const float* dn, float* grad, int memory) {
   if (!s || !dd || !grad) return KDOP_ERR_INVALID;
   if (!s->contacted) return fail(s->ctx, KDOP_ERR_STATE, "adjoint before kdop_contacts");
+  if (s->results_lost) return lost(s);
   cudaSetDevice(s->ctx->device);
   KDOP_CUDA(s->ctx, ensure_posed(s));
   if (memory == KDOP_DEVICE) {
@@ -1260,7 +1281,7 @@ int kdop_graph_capture(kdop_scene* s, int refit_mode, int64_t n_pairs, const uin
   int mode = 0;
   if (kdop_resolve_traverse_opts(s, opts, p, mode) != KDOP_OK) return fail(s->ctx, KDOP_ERR_INVALID, "bad traversal options");
   kdop_graph_release(s);
-  int rc = upload_pairs(s, n_pairs, pairs, memory);
+  int rc = upload_pairs(s, n_pairs, pairs, memory, p.timeout_ns);
   if (rc != KDOP_OK) return rc;
   // settle function attributes outside the capture
   KDOP_CUDA(s->ctx, kdop::traverse_prepare(s->K, kdop::traverse_smem_bytes(p.block_warps, p.stack_cap)));
@@ -1323,6 +1344,7 @@ int kdop_graph_launch(kdop_scene* s) {
   s->refit_mode = ext(s)->graph_refit_mode;
   s->result_pairs = ext(s)->graph_pairs;
   s->pairs_current = true;
+  s->results_lost = false;
   if (s->refit_mode != KDOP_REFIT_VERTICES) s->posed_valid = true;
   return KDOP_OK;
 }
@@ -1367,11 +1389,12 @@ int kdop_autotune(kdop_scene* s, int64_t n_pairs, const uint32_t* pairs, int mem
   cudaSetDevice(s->ctx->device);
   // at least five timed runs per configuration, odd so the median is a run
   repeats = std::max(repeats, 5) | 1;
-  int rc = upload_pairs(s, n_pairs, pairs, memory);
+  int rc = upload_pairs(s, n_pairs, pairs, memory, s->ctx->wait_ns);
   if (rc != KDOP_OK) return rc;
   // the timed traversals leave their results in the scene
   s->result_pairs = n_pairs;
   s->pairs_current = true;
+  s->results_lost = false;
   std::vector<cudaEvent_t> ev((size_t)repeats + 1, nullptr);
   for (auto& e : ev) {
     cudaError_t ce = cudaEventCreate(&e);

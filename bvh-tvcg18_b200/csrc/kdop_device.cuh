@@ -19,6 +19,12 @@ constexpr uint32_t SURF_BIT = 0x40000000u;   // leaf word: the tet has a boundar
 constexpr uint32_t NODE_MASK = 0x3FFFFFFFu;  // node index bits of a word
 constexpr uint32_t NO_NODE = 0xFFFFFFFFu;
 
+__device__ __forceinline__ unsigned long long global_ns() {
+  unsigned long long t;
+  asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
+  return t;
+}
+
 // ---- node record ------------------------------------------------------------
 // K floats of slabs (lo_s, hi_s interleaved, s = 0..K/2-1, in direction-table
 // order), then two topology words, padded to whole float4 chunks.  The words

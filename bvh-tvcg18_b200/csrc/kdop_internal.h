@@ -104,6 +104,10 @@ struct kdop_ctx {
   // grow-only device scratch of the contact reduction, freed with the context
   char* scratch = nullptr;
   size_t scratch_bytes = 0;
+  // bound of the device-side waits of the calls that take no options, and the
+  // test hook (kdop_ctx_set_wait_limit)
+  long long wait_ns = 5000000000ll;
+  int test_stuck = 0;
 };
 
 struct kdop_scene {
@@ -168,6 +172,7 @@ struct kdop_scene {
   int refit_mode = -1;
   bool traversed = false;
   bool contacted = false;
+  bool results_lost = false;  // a sort of the results gave up in the middle; cleared by the next traversal
   int64_t last_pairs = 0;
   int64_t result_pairs = 0;    // pairs the last results' pair indices run over
   bool pairs_current = false;  // `pairs` is the list the last results came from
@@ -187,7 +192,7 @@ namespace kdop {
 int64_t seed_entries(int sm_count, int64_t n);
 // pair_order of the scene's n pairs by decreasing size (most >= the tets of any
 // two meshes), in the seed pass's buffer.
-cudaError_t launch_pair_order(kdop_scene* s, int64_t n, uint32_t most);
+cudaError_t launch_pair_order(kdop_scene* s, int64_t n, uint32_t most, long long wait_ns);
 
 // fn(0 .. n-1) on up to 64 host threads
 template <typename F>

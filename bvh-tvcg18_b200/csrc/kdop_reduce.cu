@@ -132,6 +132,7 @@ struct ReduceArgs {
   kdop_contact* out;
   uint2* out_bodies;
   unsigned* head;         // ReduceHead words
+  long long wait_ns;
   unsigned long long* words_run;
   unsigned long long* words_keep;
 };
@@ -143,9 +144,11 @@ constexpr int RD_ITEMS = 4, RD_TILE = 256 * RD_ITEMS;
 // Runs of equal (bodies, p.y): a scan of their first rows.
 __global__ void __launch_bounds__(256) red_runs_kernel(ReduceArgs a) {
   __shared__ unsigned s_tile;
-  if (threadIdx.x == 0) s_tile = atomicAdd(a.head + H_TICKET_RUN, 1u);
+  const WaitLimit lim{a.head + H_ERR, a.wait_ns};
+  if (threadIdx.x == 0) s_tile = take_tile(a.head + H_TICKET_RUN, lim);
   __syncthreads();
   const unsigned tile = s_tile;
+  if (tile == kNoTile) return;
   const int64_t base = (int64_t)tile * RD_TILE + (int64_t)threadIdx.x * RD_ITEMS;
   uint32_t y_prev = 0;
   uint2 b_prev = make_uint2(0u, 0u);
@@ -173,7 +176,7 @@ __global__ void __launch_bounds__(256) red_runs_kernel(ReduceArgs a) {
   }
   uint32_t total;
   uint32_t at = block_scan<256, uint32_t>(sum, total);
-  at += tile_prefix(a.words_run, tile, total, a.head + H_ERR);
+  at += tile_prefix(a.words_run, tile, total, lim);
 #pragma unroll
   for (int j = 0; j < RD_ITEMS; ++j) {
     const int64_t k = base + j;
@@ -201,6 +204,7 @@ __global__ void __launch_bounds__(256) red_rank_kernel(ReduceArgs a) {
   const int64_t k = (int64_t)blockIdx.x * 256 + threadIdx.x;
   if (k >= a.n) return;
   const uint32_t r = a.perm[k], g = a.run[k];
+  if (gave_up(a.head + H_ERR)) return;  // the order or the runs are incomplete
   const uint32_t s = a.starts[g], e = a.starts[g + 1];
   const Row x = load_row(a.rows, r);
   if (e - s > kRankMax) {
@@ -232,6 +236,7 @@ __global__ void __launch_bounds__(256) red_rank_kernel(ReduceArgs a) {
 // Positions of the long runs' rows in increasing order: at[pos[k]] = k.
 __global__ void red_long_list_kernel(const uint32_t* __restrict__ flag, const uint32_t* __restrict__ pos, int64_t n,
                                      uint32_t* at) {
+  // (launched by a host that has seen no wait give up)
   const int64_t k = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (k < n && flag[k]) at[pos[k]] = (uint32_t)k;
 }
@@ -240,7 +245,9 @@ __global__ void red_long_place_kernel(ReduceArgs a, const uint32_t* __restrict__
                                       const uint32_t* __restrict__ sorted_at, int64_t m) {
   const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= m) return;
-  const uint32_t r = a.perm[sorted_at[i]];
+  const uint32_t from = sorted_at[i];
+  if (gave_up(a.head + H_ERR)) return;
+  const uint32_t r = a.perm[from];
   a.order[at[i]] = r;
   a.sorted[at[i]] = load_row(a.rows, r);
 }
@@ -275,14 +282,14 @@ constexpr uint32_t KEEP = 1u, SEGMENT = 2u;  // bits of keep[]
 
 __global__ void __launch_bounds__(256) red_segments_kernel(ReduceArgs a) {
   const int64_t k = (int64_t)blockIdx.x * 256 + threadIdx.x;
-  if (k < a.n) a.keep[k] = starts_segment(a, (uint32_t)k) ? SEGMENT | KEEP : 0u;
+  if (k < a.n && !gave_up(a.head + H_ERR)) a.keep[k] = starts_segment(a, (uint32_t)k) ? SEGMENT | KEEP : 0u;
 }
 
 // Thread per segment (its first row's): std::unique's walk -- a row is kept
 // unless it equals the last row kept.
 __global__ void __launch_bounds__(128) red_walk_kernel(ReduceArgs a) {
   const int64_t k = (int64_t)blockIdx.x * 128 + threadIdx.x;
-  if (k >= a.n || !(a.keep[k] & SEGMENT)) return;
+  if (k >= a.n || !(a.keep[k] & SEGMENT) || gave_up(a.head + H_ERR)) return;
   if (k + 1 >= a.n || (a.keep[k + 1] & SEGMENT)) return;  // a segment of one row (most): kept
   Row last = a.sorted[k];
   for (int64_t j = k + 1; j < a.n; ++j) {
@@ -298,9 +305,11 @@ __global__ void __launch_bounds__(128) red_walk_kernel(ReduceArgs a) {
 
 __global__ void __launch_bounds__(256) red_write_kernel(ReduceArgs a) {
   __shared__ unsigned s_tile;
-  if (threadIdx.x == 0) s_tile = atomicAdd(a.head + H_TICKET_KEEP, 1u);
+  const WaitLimit lim{a.head + H_ERR, a.wait_ns};
+  if (threadIdx.x == 0) s_tile = take_tile(a.head + H_TICKET_KEEP, lim);
   __syncthreads();
   const unsigned tile = s_tile;
+  if (tile == kNoTile) return;
   // consecutive threads hold consecutive rows: one scan step per item
   uint32_t keep[RD_ITEMS], pos[RD_ITEMS], sum = 0;
 #pragma unroll
@@ -311,7 +320,7 @@ __global__ void __launch_bounds__(256) red_write_kernel(ReduceArgs a) {
     pos[j] = sum + block_scan<256, uint32_t>(keep[j], total);
     sum += total;
   }
-  const uint32_t excl = tile_prefix(a.words_keep, tile, sum, a.head + H_ERR);
+  const uint32_t excl = tile_prefix(a.words_keep, tile, sum, lim);
 #pragma unroll
   for (int j = 0; j < RD_ITEMS; ++j) {
     const int64_t k = (int64_t)tile * RD_TILE + j * 256 + threadIdx.x;
@@ -403,8 +412,8 @@ static cudaError_t order_long_runs(kdop_ctx* ctx, const ReduceArgs& a, const Red
   const uint32_t* from = at;
   for (int pass = 0; pass < 4; ++pass) {
     const int bits = pass < 3 ? 64 : bits_of((uint64_t)a.n);
-    e = radix_sort(LongGen{a.rows, a.perm, from, a.run, pass}, m, bits, b, w + L.radix, a.head + H_ERR, st,
-                   ctx->launches);
+    e = radix_sort(ctx, LongGen{a.rows, a.perm, from, a.run, pass}, m, bits, b, w + L.radix,
+                   WaitLimit{a.head + H_ERR, ctx->wait_ns});
     if (e != cudaSuccess) return e;
     from = b.vals;
   }
@@ -439,6 +448,7 @@ cudaError_t reduce_contact_rows(kdop_ctx* ctx, const kdop_contact* rows, const u
   a.out = out;
   a.out_bodies = out_bodies;
   a.head = reinterpret_cast<unsigned*>(w + L.head);
+  a.wait_ns = ctx->wait_ns;
   a.words_run = reinterpret_cast<unsigned long long*>(w + L.words_run);
   a.words_keep = reinterpret_cast<unsigned long long*>(w + L.words_keep);
   SortBuffers b{reinterpret_cast<uint64_t*>(w + L.keys), reinterpret_cast<uint64_t*>(w + L.keys_tmp),
@@ -456,14 +466,13 @@ cudaError_t reduce_contact_rows(kdop_ctx* ctx, const kdop_contact* rows, const u
     bj = bits_of(h[H_MOST_J]);
   }
   const bool one = bi + bj <= 32;
-  e = radix_sort(PointGen{rows, bodies, bj, one}, n, 32 + (one ? bi + bj : 0), b, w + L.radix, a.head + H_ERR, st,
-                 ctx->launches);
-  if (e == cudaSuccess && !one)
-    e = radix_sort(BodyGen{bodies, b.vals}, n, 32 + bi, b, w + L.radix, a.head + H_ERR, st, ctx->launches);
+  const WaitLimit lim{a.head + H_ERR, ctx->wait_ns};
+  e = radix_sort(ctx, PointGen{rows, bodies, bj, one}, n, 32 + (one ? bi + bj : 0), b, w + L.radix, lim);
+  if (e == cudaSuccess && !one) e = radix_sort(ctx, BodyGen{bodies, b.vals}, n, 32 + bi, b, w + L.radix, lim);
   if (e != cudaSuccess) return e;
   a.perm = b.vals;
   const unsigned tiles = blocks_for(n, RD_TILE);
-  red_runs_kernel<<<tiles, 256, 0, st>>>(a);
+  red_runs_kernel<<<tile_blocks(ctx, STUCK_SCAN, a.head + H_TICKET_RUN, tiles), 256, 0, st>>>(a);
   red_rank_kernel<<<blocks_for(n, 256), 256, 0, st>>>(a);
   ctx->launches += 2;
   // without waiting for the count of long runs: where there are some, they are
@@ -471,11 +480,11 @@ cudaError_t reduce_contact_rows(kdop_ctx* ctx, const kdop_contact* rows, const u
   for (int round = 0;; ++round) {
     red_segments_kernel<<<blocks_for(n, 256), 256, 0, st>>>(a);
     red_walk_kernel<<<blocks_for(n, 128), 128, 0, st>>>(a);
-    red_write_kernel<<<tiles, 256, 0, st>>>(a);
+    red_write_kernel<<<tile_blocks(ctx, STUCK_SCAN, a.head + H_TICKET_KEEP, tiles), 256, 0, st>>>(a);
     ctx->launches += 3;
     if ((e = cudaMemcpyAsync(h, a.head, sizeof(h), cudaMemcpyDeviceToHost, st)) != cudaSuccess) return e;
     if ((e = cudaStreamSynchronize(st)) != cudaSuccess) return e;
-    if (round || !h[H_LONG]) break;
+    if (round || h[H_ERR] || !h[H_LONG]) break;
     if ((e = order_long_runs(ctx, a, L, w, b)) != cudaSuccess) return e;
     if ((e = cudaMemsetAsync(a.head + H_TICKET_KEEP, 0, 4, st)) != cudaSuccess) return e;
     if ((e = cudaMemsetAsync(a.words_keep, 0, L.keys - L.words_keep, st)) != cudaSuccess) return e;

@@ -25,7 +25,7 @@ constexpr size_t kPassSmem = (size_t)kSortTile * 12 + SP_WARPS * 256 * 4;
 __global__ void __launch_bounds__(SP_THREADS, 1280 / SP_THREADS)
     sort_pass_kernel(const uint64_t* __restrict__ kin, const uint32_t* __restrict__ vin, uint64_t* kout,
                      uint32_t* vout, int64_t n, int shift, const uint32_t* __restrict__ hist, uint32_t* ticket,
-                     unsigned long long* words, unsigned epoch, unsigned* err) {
+                     unsigned long long* words, unsigned epoch, WaitLimit lim) {
   constexpr int TILE = (int)kSortTile, ITEMS = SP_ITEMS, WARPS = SP_WARPS;
   extern __shared__ uint64_t ex[];                         // TILE keys in digit order
   uint32_t* exv = reinterpret_cast<uint32_t*>(ex + TILE);  // and their values
@@ -82,7 +82,7 @@ __global__ void __launch_bounds__(SP_THREADS, 1280 / SP_THREADS)
     uint32_t excl = 0;
     for (int64_t t = (int64_t)tile - 1; t >= 0; --t) {
       uint32_t c;
-      const unsigned flag = await_word(words + (size_t)t * 256 + d0, epoch, c, err);
+      const unsigned flag = await_word(words + (size_t)t * 256 + d0, epoch, c, lim);
       excl += c;
       if (flag == 2u) break;
     }
@@ -183,13 +183,14 @@ cudaError_t exclusive_scan_u32(const uint32_t* in, uint32_t* out, int64_t n, uin
   return cudaGetLastError();
 }
 
-cudaError_t launch_sort_pass(const SortBuffers& b, int64_t n, int shift, const uint32_t* hist, uint32_t* ticket,
-                             unsigned long long* words, unsigned epoch, unsigned* err, cudaStream_t st) {
+cudaError_t launch_sort_pass(const kdop_ctx* ctx, const SortBuffers& b, int64_t n, int shift, const uint32_t* hist,
+                             uint32_t* ticket, unsigned long long* words, unsigned epoch, WaitLimit lim) {
   const cudaError_t e =
       cudaFuncSetAttribute(sort_pass_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kPassSmem);
   if (e != cudaSuccess) return e;
-  sort_pass_kernel<<<(unsigned)((n + kSortTile - 1) / kSortTile), SP_THREADS, kPassSmem, st>>>(
-      b.keys, b.vals, b.keys_tmp, b.vals_tmp, n, shift, hist, ticket, words, epoch, err);
+  const unsigned blocks = tile_blocks(ctx, STUCK_SORT, ticket, (unsigned)((n + kSortTile - 1) / kSortTile));
+  sort_pass_kernel<<<blocks, SP_THREADS, kPassSmem, ctx->stream>>>(b.keys, b.vals, b.keys_tmp, b.vals_tmp, n, shift,
+                                                                   hist, ticket, words, epoch, lim);
   return cudaGetLastError();
 }
 
@@ -246,18 +247,20 @@ struct ApplyArgs {
   uint32_t* src;         // first contact row of a sorted candidate before the sort
   uint32_t* ticket;
   unsigned long long* words;
-  unsigned* err;
+  WaitLimit lim;
 };
 
 constexpr int AP_ITEMS = 4, AP_TILE = 256 * AP_ITEMS;
 
 // Candidate rows in sorted order and, with contacts, their records with the
-// rows' new places (a scan of the contact counts in the same pass).
+// rows' new places (a scan of the contact counts in the same pass).  Nothing
+// after a wait that gave up: the order may be incomplete.
 __global__ void __launch_bounds__(256) sort_apply_kernel(ApplyArgs a) {
   __shared__ unsigned s_tile;
-  if (threadIdx.x == 0) s_tile = a.rec ? atomicAdd(a.ticket, 1u) : blockIdx.x;
+  if (threadIdx.x == 0) s_tile = a.rec ? take_tile(a.ticket, a.lim) : gave_up(a.lim.err) ? kNoTile : blockIdx.x;
   __syncthreads();
   const unsigned tile = s_tile;
+  if (tile == kNoTile) return;
   const int64_t base = (int64_t)tile * AP_TILE + (int64_t)threadIdx.x * AP_ITEMS;
   int4 r[AP_ITEMS];
   uint32_t sum = 0;
@@ -287,7 +290,7 @@ __global__ void __launch_bounds__(256) sort_apply_kernel(ApplyArgs a) {
   if (!a.rec) return;
   uint32_t total;
   uint32_t run = block_scan<256, uint32_t>(sum, total);
-  run += tile_prefix(a.words, tile, total, a.err);
+  run += tile_prefix(a.words, tile, total, a.lim);
 #pragma unroll
   for (int j = 0; j < AP_ITEMS; ++j) {
     const int64_t k = base + j;
@@ -326,11 +329,12 @@ __global__ void __launch_bounds__(256) candidate_rows_kernel(const uint32_t* __r
 // 16 bytes a lane.
 __global__ void __launch_bounds__(256) contact_gather_kernel(int64_t n, const int4* __restrict__ rec,
                                                              const uint32_t* __restrict__ src,
-                                                             const float4* __restrict__ rows, float4* rows_out) {
+                                                             const float4* __restrict__ rows, float4* rows_out,
+                                                             const unsigned* err) {
   const int64_t k = ((int64_t)blockIdx.x * 256 + threadIdx.x) >> 3;
   if (k >= n) return;
   const int4 r = rec[k];
-  if (r.z <= 0) return;
+  if (gave_up(err) || r.z <= 0) return;  // the records may be incomplete
   const float4* from = rows + 2 * (size_t)src[k];
   float4* to = rows_out + 2 * (size_t)(uint32_t)r.w;
   for (int c = threadIdx.x & 7; c < 2 * r.z; c += 8) {
@@ -378,7 +382,8 @@ struct SortWork {
   }
 };
 
-cudaError_t sort_results(kdop_scene* s, int64_t n, int64_t n_contacts, void* work, cudaStream_t st) {
+cudaError_t sort_results(kdop_scene* s, int64_t n, int64_t n_contacts, void* work) {
+  cudaStream_t st = s->ctx->stream;
   if (n <= 0) return cudaSuccess;
   char* w = static_cast<char*>(work);
   SortWork L(n, n_contacts);
@@ -387,18 +392,17 @@ cudaError_t sort_results(kdop_scene* s, int64_t n, int64_t n_contacts, void* wor
   int4* rec_out = reinterpret_cast<int4*>(w + L.rec_out);
   float4* rows_out = reinterpret_cast<float4*>(w + L.rows_out);
   uint32_t* cand_out = reinterpret_cast<uint32_t*>(w + L.cand_out);
-  unsigned* err = &s->ctl->error;
+  const WaitLimit lim{&s->ctl->error, s->ctx->wait_ns};
   CandGen gen{s->cand, s->cand + s->cand_cap, s->cand + 2 * s->cand_cap, s->pairs, s->t_off_dev, bits_of(std::max<int64_t>(s->most_tets, 1) - 1)};
   const int pair_bits = bits_of((uint64_t)std::max<int64_t>(s->result_pairs, 1) - 1);
   const bool packed = s->pairs_current && pair_bits + 2 * gen.tb <= 64;
   cudaError_t e;
   if (packed) {
-    e = radix_sort(gen, n, pair_bits + 2 * gen.tb, b, w + L.scratch, err, st, s->ctx->launches);
+    e = radix_sort(s->ctx, gen, n, pair_bits + 2 * gen.tb, b, w + L.scratch, lim);
   } else {
     const int tb = bits_of(s->nt > 0 ? s->nt - 1 : 0);  // at most 30
-    e = radix_sort(TetGen{gen.cA, gen.cB, tb}, n, 2 * tb, b, w + L.scratch, err, st, s->ctx->launches);
-    if (e == cudaSuccess)
-      e = radix_sort(PairGen{gen.cP, b.vals}, n, 32, b, w + L.scratch, err, st, s->ctx->launches);
+    e = radix_sort(s->ctx, TetGen{gen.cA, gen.cB, tb}, n, 2 * tb, b, w + L.scratch, lim);
+    if (e == cudaSuccess) e = radix_sort(s->ctx, PairGen{gen.cP, b.vals}, n, 32, b, w + L.scratch, lim);
   }
   if (e != cudaSuccess) return e;
   const bool with_contacts = s->contacted;
@@ -416,9 +420,10 @@ cudaError_t sort_results(kdop_scene* s, int64_t n, int64_t n_contacts, void* wor
   a.src = reinterpret_cast<uint32_t*>(w + L.src);
   a.ticket = reinterpret_cast<uint32_t*>(w + L.head);
   a.words = reinterpret_cast<unsigned long long*>(w + L.words);
-  a.err = err;
+  a.lim = lim;
   if (with_contacts && (e = cudaMemsetAsync(w + L.head, 0, L.keys - L.head, st)) != cudaSuccess) return e;
-  sort_apply_kernel<<<(unsigned)L.tiles, 256, 0, st>>>(a);
+  const unsigned tiles = with_contacts ? tile_blocks(s->ctx, STUCK_SCAN, a.ticket, (unsigned)L.tiles) : (unsigned)L.tiles;
+  sort_apply_kernel<<<tiles, 256, 0, st>>>(a);
   s->ctx->launches++;
   if (!packed)
     for (int k = 0; k < 3; ++k) {
@@ -427,7 +432,7 @@ cudaError_t sort_results(kdop_scene* s, int64_t n, int64_t n_contacts, void* wor
     }
   if (with_contacts) {
     contact_gather_kernel<<<(unsigned)((n + 31) / 32), 256, 0, st>>>(
-        n, rec_out, a.src, reinterpret_cast<const float4*>(s->contacts), rows_out);
+        n, rec_out, a.src, reinterpret_cast<const float4*>(s->contacts), rows_out, lim.err);
     s->ctx->launches++;
     e = cudaMemcpyAsync(s->records, rec_out, (size_t)n * sizeof(int4), cudaMemcpyDeviceToDevice, st);
     if (e == cudaSuccess && n_contacts > 0)

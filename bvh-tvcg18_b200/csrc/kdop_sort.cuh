@@ -14,8 +14,10 @@
 //     known), and writes the keys in digit order through shared memory, so
 //     that a warp's stores fall on consecutive addresses.  Tiles come off the
 //     ticket in order, so a block waits only for blocks already running; the
-//     wait is bounded all the same (kSpinLimit polls, then the sort's error
-//     word is set and the block goes on).
+//     wait is bounded all the same (WaitLimit).  A block whose wait gave up
+//     goes on with the counts it has: places stay within the output, but not
+//     every place is written, so whatever reads the output as indices looks at
+//     the error word first (gave_up) and returns.
 //   * Up to kSmallSort keys are generated and sorted by one block in shared
 //     memory, in one launch.
 // Bound: latency below about 1 M keys (a launch per pass), memory above.  The
@@ -27,17 +29,27 @@
 #include <cstdint>
 #include <cuda_runtime.h>
 
-#include "kdop_internal.h"
+#include "kdop_device.cuh"
 #include "kdop_sort.h"
 
 namespace kdop {
 
 constexpr int kSortMaxPasses = 8;
-constexpr unsigned kSpinLimit = 1u << 23;  // polls of one published word
 constexpr int kSmallSort = 8192;           // keys one block sorts in shared memory
 
 __device__ __forceinline__ unsigned sort_digit(uint64_t key, int shift, unsigned mask) {
   return (unsigned)(key >> shift) & mask;
+}
+
+// ---- bounded waits --------------------------------------------------------------
+// A wait ends after `ns`, or as soon as another one of the same error word gave
+// up: a launch whose waits fail takes `ns` once, not once per word.
+struct WaitLimit {
+  unsigned* err;  // device word that gets DEV_ERR_TIMEOUT
+  long long ns;
+};
+__device__ __forceinline__ bool gave_up(const unsigned* err) {
+  return (*(const volatile unsigned*)err & (unsigned)DEV_ERR_TIMEOUT) != 0u;
 }
 
 // ---- published tile words -----------------------------------------------------
@@ -49,24 +61,39 @@ __device__ __forceinline__ void publish(unsigned long long* w, uint32_t v, unsig
 }
 // Waits for the word (bounded); its flag, and its value in v.
 __device__ __forceinline__ unsigned await_word(const unsigned long long* w, unsigned epoch, uint32_t& v,
-                                               unsigned* err) {
-  for (unsigned it = 0; it < kSpinLimit; ++it) {
+                                               WaitLimit lim) {
+  unsigned long long t0 = 0;
+  for (unsigned it = 1;; ++it) {
     const unsigned long long x = *(const volatile unsigned long long*)w;
     if ((unsigned)(x >> 34) == epoch) {
       v = (uint32_t)x;
       return (unsigned)(x >> 32) & 3u;
     }
+    if (it & 63u) continue;
+    if (gave_up(lim.err)) break;
+    const unsigned long long now = global_ns();
+    if (it == 64u) t0 = now;
+    if ((long long)(now - t0) > lim.ns) {
+      atomicOr(lim.err, (unsigned)DEV_ERR_TIMEOUT);
+      break;
+    }
   }
-  atomicOr(err, (unsigned)DEV_ERR_TIMEOUT);
   v = 0;
   return 2u;
+}
+// A block's tile: the next one off the ticket, or kNoTile when a wait of this or
+// an earlier kernel gave up (its input may be incomplete).  Thread 0's.
+constexpr unsigned kNoTile = 0xFFFFFFFFu;
+__device__ __forceinline__ unsigned take_tile(unsigned* ticket, WaitLimit lim) {
+  const unsigned tile = atomicAdd(ticket, 1u);
+  return gave_up(lim.err) ? kNoTile : tile;
 }
 
 // Exclusive prefix of a block's total over the blocks before it (tiles in
 // ticket order); called by the whole block, the result in every thread.
 // words: one per tile, zeroed before the launch.
 __device__ __forceinline__ uint32_t tile_prefix(unsigned long long* words, unsigned tile, uint32_t total,
-                                                unsigned* err) {
+                                                WaitLimit lim) {
   __shared__ uint32_t s_excl;
   if (threadIdx.x < 32) {
     const int lane = threadIdx.x;
@@ -76,7 +103,7 @@ __device__ __forceinline__ uint32_t tile_prefix(unsigned long long* words, unsig
       // 32 tiles at once, the nearest on lane 0
       uint32_t v = 0;
       unsigned flag = 2u;
-      if (at - lane >= 0) flag = await_word(words + (at - lane), 1u, v, err);
+      if (at - lane >= 0) flag = await_word(words + (at - lane), 1u, v, lim);
       const unsigned sums = __ballot_sync(0xffffffffu, flag == 2u);
       const int last = sums ? __ffs(sums) - 1 : 31;  // nearest tile whose sum is known
       uint32_t x = lane <= last ? v : 0u;
@@ -141,11 +168,13 @@ struct SortScratch {
 
 // Keys (and values) of every item and, for the passes over `bits` bits, the
 // digit counts.  A digit that a whole warp shares (the high bits, mostly) is
-// counted by one lane.
+// counted by one lane.  Nothing after a wait that gave up: gen may read indices
+// an earlier sort left incomplete.
 template <class Gen>
 __global__ void __launch_bounds__(256) sort_keys_kernel(Gen gen, int64_t n, int bits, uint64_t* keys, uint32_t* vals,
-                                                        uint32_t* hist) {
+                                                        uint32_t* hist, const unsigned* err) {
   __shared__ uint32_t h[kSortMaxPasses][256];
+  if (gave_up(err)) return;  // no wait in this kernel: all its threads read the same
   const int passes = (bits + 7) / 8;
   for (int i = threadIdx.x; i < kSortMaxPasses * 256; i += 256) (&h[0][0])[i] = 0;
   __syncthreads();
@@ -182,7 +211,9 @@ constexpr size_t small_sort_smem() {
   return (size_t)1024 * ITEMS * 8 + 32 * 257 * 4;
 }
 template <class Gen, int ITEMS>
-__global__ void __launch_bounds__(1024) small_sort_kernel(Gen gen, int n, int bits, uint64_t* keys, uint32_t* vals) {
+__global__ void __launch_bounds__(1024) small_sort_kernel(Gen gen, int n, int bits, uint64_t* keys, uint32_t* vals,
+                                                          const unsigned* err) {
+  if (gave_up(err)) return;  // as sort_keys_kernel
   extern __shared__ uint64_t ex[];                                      // 1024 * ITEMS
   uint32_t* wc = reinterpret_cast<uint32_t*>(ex + 1024 * ITEMS);        // [32 warps][256 digits], a row 257 words
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
@@ -264,33 +295,46 @@ struct SortBuffers {
   uint32_t *vals, *vals_tmp;
 };
 
+// Test hook (kdop_ctx_set_wait_limit): the kinds of wait that a block nobody
+// runs is to leave without an end.
+enum : int { STUCK_SORT = 1, STUCK_SCAN = 2 };
+// Blocks to launch for `blocks` tiles off `ticket`: all of them, or with the hook
+// one less, whose tile (the first) nobody takes.
+inline unsigned tile_blocks(const kdop_ctx* ctx, int kind, uint32_t* ticket, unsigned blocks) {
+  if (!(ctx->test_stuck & kind) || blocks < 2u) return blocks;
+  return cudaMemsetAsync(ticket, 1, 1, ctx->stream) == cudaSuccess ? blocks - 1u : blocks;
+}
+
 // One digit pass from b's keys and values to its temporaries (kdop_sort.cu).
-cudaError_t launch_sort_pass(const SortBuffers& b, int64_t n, int shift, const uint32_t* hist, uint32_t* ticket,
-                             unsigned long long* words, unsigned epoch, unsigned* err, cudaStream_t st);
+cudaError_t launch_sort_pass(const kdop_ctx* ctx, const SortBuffers& b, int64_t n, int shift, const uint32_t* hist,
+                             uint32_t* ticket, unsigned long long* words, unsigned epoch, WaitLimit lim);
 
 // Stable ascending sort of the items 0 .. n-1 by gen.key(i), of which the low
 // `bits` bits vary (the others are equal in all keys), n < 2^32; the values
 // are gen.val(i).  gen may read b.vals at i (it is written at i only).
-// scratch: radix_scratch_words(n) words, 8-byte aligned.  *err (device) gets
-// DEV_ERR_TIMEOUT when a bounded wait gave up; the caller clears and reads it.
+// scratch: radix_scratch_words(n) words, 8-byte aligned.  *lim.err gets
+// DEV_ERR_TIMEOUT when a bounded wait gave up (the sorted keys and values are
+// then incomplete); the caller clears and reads it.  On the context's stream.
 template <class Gen>
-cudaError_t radix_sort(const Gen& gen, int64_t n, int bits, SortBuffers& b, void* scratch, unsigned* err,
-                       cudaStream_t st, long long& launches) {
+cudaError_t radix_sort(kdop_ctx* ctx, const Gen& gen, int64_t n, int bits, SortBuffers& b, void* scratch,
+                       WaitLimit lim) {
   if (n <= 0) return cudaSuccess;
+  cudaStream_t st = ctx->stream;
+  long long& launches = ctx->launches;
   cudaError_t e;
   if (n <= kSmallSort) {
     if (n <= 1024) {
-      small_sort_kernel<Gen, 1><<<1, 1024, small_sort_smem<1>(), st>>>(gen, (int)n, bits, b.keys, b.vals);
+      small_sort_kernel<Gen, 1><<<1, 1024, small_sort_smem<1>(), st>>>(gen, (int)n, bits, b.keys, b.vals, lim.err);
     } else if (n <= 4096) {
       e = cudaFuncSetAttribute(small_sort_kernel<Gen, 4>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                (int)small_sort_smem<4>());
       if (e != cudaSuccess) return e;
-      small_sort_kernel<Gen, 4><<<1, 1024, small_sort_smem<4>(), st>>>(gen, (int)n, bits, b.keys, b.vals);
+      small_sort_kernel<Gen, 4><<<1, 1024, small_sort_smem<4>(), st>>>(gen, (int)n, bits, b.keys, b.vals, lim.err);
     } else {
       e = cudaFuncSetAttribute(small_sort_kernel<Gen, 8>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                (int)small_sort_smem<8>());
       if (e != cudaSuccess) return e;
-      small_sort_kernel<Gen, 8><<<1, 1024, small_sort_smem<8>(), st>>>(gen, (int)n, bits, b.keys, b.vals);
+      small_sort_kernel<Gen, 8><<<1, 1024, small_sort_smem<8>(), st>>>(gen, (int)n, bits, b.keys, b.vals, lim.err);
     }
     launches += 1;
     return cudaGetLastError();
@@ -299,11 +343,11 @@ cudaError_t radix_sort(const Gen& gen, int64_t n, int bits, SortBuffers& b, void
   const int64_t tiles = (n + kSortTile - 1) / kSortTile;
   if ((e = cudaMemsetAsync(scratch, 0, SortScratch::kHead + (size_t)tiles * 256 * 8, st)) != cudaSuccess) return e;
   sort_keys_kernel<<<(unsigned)std::min<int64_t>((n + 1023) / 1024, 1184), 256, 0, st>>>(gen, n, bits, b.keys, b.vals,
-                                                                                        s.hist);
+                                                                                        s.hist, lim.err);
   launches += 1;
   unsigned epoch = 1;
   for (int p = 0; 8 * p < bits; ++p, ++epoch) {
-    e = launch_sort_pass(b, n, 8 * p, s.hist + 256 * p, s.ticket + p, s.words, epoch, err, st);
+    e = launch_sort_pass(ctx, b, n, 8 * p, s.hist + 256 * p, s.ticket + p, s.words, epoch, lim);
     if (e != cudaSuccess) return e;
     launches += 1;
     std::swap(b.keys, b.keys_tmp);

@@ -23,7 +23,8 @@ namespace kdop {
 // Sorts the last traversal's n candidate rows by (pair, tet of A, tet of B)
 // and, after kdop_contacts, regroups the n_contacts contact rows and the
 // records in that order.  work: sort_results_bytes(n, n_contacts) bytes.  A
-// bounded wait that gave up sets DEV_ERR_TIMEOUT in the scene's control block.
-cudaError_t sort_results(kdop_scene* s, int64_t n, int64_t n_contacts, void* work, cudaStream_t st);
+// bounded wait that gave up sets DEV_ERR_TIMEOUT in the scene's control block;
+// the results are then lost.
+cudaError_t sort_results(kdop_scene* s, int64_t n, int64_t n_contacts, void* work);
 size_t sort_results_bytes(int64_t n, int64_t n_contacts);
 }  // namespace kdop

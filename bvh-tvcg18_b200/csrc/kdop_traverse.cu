@@ -81,11 +81,6 @@ struct TravBuffers {
   uint4* seeds = nullptr;  // room for the seed pass's entries (seed_entries), or NULL: start from the root pairs
 };
 
-__device__ __forceinline__ unsigned long long global_ns() {
-  unsigned long long t;
-  asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
-  return t;
-}
 // 256-bit read-only load of two consecutive float4 chunks (p 32-byte aligned).
 __device__ __forceinline__ void ldg256(const float4* p, float4& x, float4& y) {
   asm("ld.global.nc.v8.f32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
@@ -329,6 +324,7 @@ __global__ void __launch_bounds__(512, (C * S >= 4) ? 1 : 2) traverse_kernel(Tra
   uint2* sAB = reinterpret_cast<uint2*>(smem) + (size_t)wib * CAP;  // this warp's deque
   TravCtl* ctl = a.ctl;
   if (a.seeded && ctl->n_init == 0u && a.stuck == 0) return;  // the seed pass finished every pair
+  if (a.entries && !a.seeded && gave_up(&ctl->error)) return;  // the frontier's order gave up: no entries
   if (lane == 0) s_claim[wib] = make_uint2(0u, 0u);
   __syncwarp();
 
@@ -661,7 +657,7 @@ struct PairOrderWork {
   }
 };
 
-cudaError_t launch_pair_order(kdop_scene* s, int64_t n, uint32_t most) {
+cudaError_t launch_pair_order(kdop_scene* s, int64_t n, uint32_t most, long long wait_ns) {
   char* w = reinterpret_cast<char*>(s->seeds);
   const PairOrderWork L(n);
   SortBuffers b{reinterpret_cast<uint64_t*>(w + L.keys), reinterpret_cast<uint64_t*>(w + L.keys_tmp),
@@ -671,8 +667,8 @@ cudaError_t launch_pair_order(kdop_scene* s, int64_t n, uint32_t most) {
   cudaError_t e = cudaMemsetAsync(&s->ctl->order_error, 0, 4, s->ctx->stream);
   if (e == cudaSuccess) e = cudaMemsetAsync(w + L.vals, 0, L.scratch - L.vals, s->ctx->stream);
   if (e == cudaSuccess)
-    e = radix_sort(PairSizeGen{s->pairs, s->t_off_dev, most}, n, bits_of(most), b, w + L.scratch,
-                   &s->ctl->order_error, s->ctx->stream, s->ctx->launches);
+    e = radix_sort(s->ctx, PairSizeGen{s->pairs, s->t_off_dev, most}, n, bits_of(most), b, w + L.scratch,
+                   WaitLimit{&s->ctl->order_error, wait_ns});
   if (e == cudaSuccess)
     e = cudaMemcpyAsync(s->pair_order, b.vals, (size_t)n * 4, cudaMemcpyDeviceToDevice, s->ctx->stream);
   return e;
@@ -1147,10 +1143,10 @@ struct EntryPairGen {
 
 // this shard's entries: sorted positions rank, rank + n_ranks, ...
 __global__ void deal_kernel(const uint4* __restrict__ f, const uint32_t* __restrict__ order, unsigned n, int rank,
-                            int n_ranks, uint4* mine) {
+                            int n_ranks, uint4* mine, const unsigned* err) {
   unsigned j = blockIdx.x * blockDim.x + threadIdx.x;
   unsigned src = (unsigned)rank + j * (unsigned)n_ranks;
-  if (src < n) mine[j] = f[order[src]];
+  if (src < n && !gave_up(err)) mine[j] = f[order[src]];  // the order may be incomplete
 }
 
 __global__ void clear_totals_kernel(TravCtl* c) {
@@ -1234,12 +1230,12 @@ cudaError_t shard_impl(kdop_scene* s, int64_t n_pairs, const uint2* pairs, const
   // deterministic order: by (A, B), then by pair
   if (n > 0) {
     const unsigned gn = (n + 255) / 256;
-    unsigned* err = &s->ctl->error;
-    if ((e = radix_sort(EntryGen{fin}, n, 64, b, w + L.sc, err, st, s->ctx->launches)) != cudaSuccess) return e;
-    if ((e = radix_sort(EntryPairGen{fin, b.vals}, n, bits_of((uint64_t)std::max<int64_t>(n_pairs, 1) - 1), b, w + L.sc,
-                        err, st, s->ctx->launches)) != cudaSuccess)
+    const WaitLimit lim{&s->ctl->error, p.timeout_ns};
+    if ((e = radix_sort(s->ctx, EntryGen{fin}, n, 64, b, w + L.sc, lim)) != cudaSuccess) return e;
+    if ((e = radix_sort(s->ctx, EntryPairGen{fin, b.vals}, n, bits_of((uint64_t)std::max<int64_t>(n_pairs, 1) - 1), b,
+                        w + L.sc, lim)) != cudaSuccess)
       return e;
-    deal_kernel<<<gn, 256, 0, st>>>(fin, b.vals, n, rank, n_ranks, mine);
+    deal_kernel<<<gn, 256, 0, st>>>(fin, b.vals, n, rank, n_ranks, mine, lim.err);
     s->ctx->launches += 1;
   }
   // the expansion's tests and leaf pairs belong to shard 0

@@ -95,6 +95,7 @@ def load_library():
         "kdop_ctx_set_stream": ([vp, vp], i32),
         "kdop_ctx_stream": ([vp], vp),
         "kdop_ctx_synchronize": ([vp], i32),
+        "kdop_ctx_set_wait_limit": ([vp, i32, i32], i32),
         "kdop_ctx_launch_count": ([vp], i64),
         "kdop_scene_create": ([vp, i32, i32, C.POINTER(MeshDesc), C.POINTER(vp)], i32),
         "kdop_scene_create_ex": ([vp, i32, i32, C.POINTER(MeshDesc), i32, C.POINTER(vp)], i32),
@@ -206,6 +207,10 @@ class Context:
 
     def synchronize(self):
         self._check(self.lib.kdop_ctx_synchronize(self.h))
+
+    def set_wait_limit(self, timeout_ms: int = 0, test_stuck: int = 0):
+        self._check(self.lib.kdop_ctx_set_wait_limit(self.h, int(timeout_ms), int(test_stuck)),
+                    "kdop_ctx_set_wait_limit")
 
     @property
     def launches(self) -> int:

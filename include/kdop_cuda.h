@@ -78,6 +78,14 @@ int kdop_ctx_destroy(kdop_ctx* ctx);
 int kdop_ctx_set_stream(kdop_ctx* ctx, void* cuda_stream);
 void* kdop_ctx_stream(const kdop_ctx* ctx);
 int kdop_ctx_synchronize(kdop_ctx* ctx);
+/* Bound of the device-side waits of the calls that take no traversal options
+ * (sorting, reduction, broad phase, tree build, autotuning): timeout_ms, 0:
+ * 5000.  A call whose wait gave up returns KDOP_ERR_TIMEOUT, and a later
+ * kdop_get_stats where the wait was a traversal's; results that
+ * kdop_sort_results gave up on are lost (KDOP_ERR_STATE until the next
+ * traversal).  test_stuck is a test hook: 0, or a sum of 1 (the passes of long
+ * sorts) and 2 (one-pass scans), whose waits then have no end of their own. */
+int kdop_ctx_set_wait_limit(kdop_ctx* ctx, int timeout_ms, int test_stuck);
 
 /* ---- scene: meshes + trees (replaces mesh_reorder + make_tree) ------------ */
 typedef struct {
