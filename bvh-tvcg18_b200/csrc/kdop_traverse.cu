@@ -313,6 +313,7 @@ __global__ void __launch_bounds__(512, (C * S >= 4) ? 1 : 2) traverse_kernel(Tra
   constexpr int CBITS = SLOTS <= 1 ? 1 : SLOTS <= 3 ? 2 : 3;  // bits of a lane's push count
   extern __shared__ uint32_t smem[];
   __shared__ uint2 s_claim[16];  // per warp: claimed initial work not yet taken [x, y)
+  __shared__ unsigned s_first;
   const int lane = threadIdx.x & 31;
   const int wib = threadIdx.x >> 5;
   const int ge = lane / Q, gq = lane % Q;  // entry and chunk lane of this lane
@@ -325,12 +326,29 @@ __global__ void __launch_bounds__(512, (C * S >= 4) ? 1 : 2) traverse_kernel(Tra
   TravCtl* ctl = a.ctl;
   if (a.seeded && ctl->n_init == 0u && a.stuck == 0) return;  // the seed pass finished every pair
   if (a.entries && !a.seeded && gave_up(&ctl->error)) return;  // the frontier's order gave up: no entries
-  if (lane == 0) s_claim[wib] = make_uint2(0u, 0u);
+  // A block that starts takes a first claim of the seeded entries for each of its
+  // warps at once (an atomic per block, not per warp).  All claims come off the
+  // one counter, so that entries belong to running warps only: a block that
+  // waits for a place on an SM another stream uses owns nothing the running ones
+  // would wait for.
+  auto first_claim = [&](unsigned n_init) {
+    return max(claim_size(n_init, gridDim.x * (blockDim.x >> 5)), (unsigned)a.init_chunk);
+  };
+  uint2 own = make_uint2(0u, 0u);
+  bool init_done = false;
+  if (a.seeded) {
+    const unsigned n_init = ctl->n_init, first = first_claim(n_init);
+    if (threadIdx.x == 0) s_first = atomicAdd(&ctl->init_head, first * (blockDim.x >> 5));
+    __syncthreads();
+    own.x = min(s_first + (unsigned)wib * first, n_init);
+    own.y = min(own.x + first, n_init);
+    init_done = own.x >= n_init;
+  }
+  if (lane == 0) s_claim[wib] = own;
   __syncwarp();
 
   int top = 0, bot = 0;  // deque [bot, top) in virtual positions
   int release = 0;       // work units taken and not yet released
-  bool init_done = false;
   unsigned claim = 0xFFFFFFFFu;
   // per-lane counts, added to the control block's 64-bit totals every 1024
   // steps and at the end (at most 4 per lane and step: no overflow)
@@ -367,21 +385,15 @@ __global__ void __launch_bounds__(512, (C * S >= 4) ? 1 : 2) traverse_kernel(Tra
         uint2 r = s_claim[wib];
         __syncwarp();
         if (r.x == r.y) {
-          // a warp's first claim of seeded entries is its own share, later
-          // ones (and all claims of root pairs) come off the common counter
-          const unsigned n_init = ctl->n_init, warps = gridDim.x * (blockDim.x >> 5);
-          const unsigned first = a.seeded ? max(claim_size(n_init, warps), (unsigned)a.init_chunk) : 0u;
-          unsigned base, chunk;
-          if (a.seeded && r.y == 0u) {
-            chunk = first;
-            base = min((blockIdx.x * (blockDim.x >> 5) + wib) * first, n_init);
-          } else {
-            chunk = (unsigned)a.init_chunk;
-            if (a.seeded) chunk = max(chunk, claim_size(n_init - min(n_init, max(r.y, warps * first)), warps));
-            base = 0;
-            if (lane == 0) base = atomicAdd(&ctl->init_head, chunk);
-            base = min(__shfl_sync(0xffffffffu, base, 0) + warps * first, n_init);
+          const unsigned n_init = ctl->n_init;
+          unsigned base = 0, chunk = (unsigned)a.init_chunk;
+          if (a.seeded) {
+            // what is left when every block has its first claim, at most
+            const unsigned warps = gridDim.x * (blockDim.x >> 5);
+            chunk = max(chunk, claim_size(n_init - min(n_init, max(r.y, warps * first_claim(n_init))), warps));
           }
+          if (lane == 0) base = atomicAdd(&ctl->init_head, chunk);
+          base = min(__shfl_sync(0xffffffffu, base, 0), n_init);
           init_done = base >= n_init;
           r = make_uint2(base, min(base + chunk, n_init));
         }
