@@ -170,7 +170,7 @@ cudaError_t broad_phase(kdop_scene* s, const unsigned* rbits, const float* pos_d
   const unsigned blocks = tile_blocks(s->ctx, STUCK_SCAN, head + 2, (unsigned)((n + BR_WARPS - 1) / BR_WARPS));
   broad_kernel<<<blocks, 32 * BR_WARPS, 0, st>>>(a, pairs, (unsigned)std::min<int64_t>(cap, 0xFFFFFFFFll), head + 2,
                                                  reinterpret_cast<unsigned long long*>(w + L.words), head,
-                                                 WaitLimit{head + 1, s->ctx->wait_ns});
+                                                 WaitLimit(head + 1, s->ctx->wait_ns));
   s->ctx->launches += pos_dev ? 2 : 1;
   unsigned h[2];
   if ((e = cudaMemcpyAsync(h, head, sizeof(h), cudaMemcpyDeviceToHost, st)) != cudaSuccess) return e;

@@ -132,17 +132,20 @@ struct MeshGen {
   const uint4* tets;
   const float4* rest;
   const uint32_t* order;
-  __device__ uint64_t key(int64_t i) const { return (uint64_t)(uint32_t)mesh_of(rest, __ldg(tets + order[i]).x); }
+  int64_t n;
+  __device__ uint64_t key(int64_t i) const {
+    return (uint64_t)(uint32_t)mesh_of(rest, __ldg(tets + bounded(order[i], n)).x);
+  }
   __device__ uint32_t val(int64_t i) const { return order[i]; }
 };
 
 // equal neighbouring codes within a mesh
 __global__ void ties_kernel(const uint4* __restrict__ tets, const float4* __restrict__ rest,
                             const uint32_t* __restrict__ vals, const uint64_t* __restrict__ codes, int64_t nt,
-                            uint32_t* tied, const unsigned* err) {
+                            uint32_t* tied) {
   int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (i < 1 || i >= nt || gave_up(err)) return;  // the order may be incomplete
-  uint32_t a = vals[i - 1], b = vals[i];
+  if (i < 1 || i >= nt) return;
+  uint32_t a = bounded(vals[i - 1], nt), b = bounded(vals[i], nt);
   int ma = mesh_of(rest, __ldg(tets + a).x), mb = mesh_of(rest, __ldg(tets + b).x);
   if (ma == mb && codes[a] == codes[b]) tied[ma] = 1u;
 }
@@ -302,16 +305,16 @@ cudaError_t device_morton_perm(kdop_scene* s, uint32_t* perm, std::vector<char>&
         cudaSuccess)
       break;
     if ((e = cudaMemsetAsync(tied, 0, (size_t)nm * 4 + 4, st)) != cudaSuccess) break;
-    const WaitLimit lim{err, s->ctx->wait_ns};
+    const WaitLimit lim(err, s->ctx->wait_ns);
     if ((e = radix_sort(s->ctx, CodeGen{s->tets, s->rest, prm, codes}, nt, 63, b, w + o_rad, lim)) != cudaSuccess)
       break;
-    if ((e = radix_sort(s->ctx, MeshGen{s->tets, s->rest, b.vals}, nt, bits_of(nm - 1), b, w + o_rad, lim)) !=
+    if ((e = radix_sort(s->ctx, MeshGen{s->tets, s->rest, b.vals, nt}, nt, bits_of(nm - 1), b, w + o_rad, lim)) !=
         cudaSuccess)
       break;
     if (b.vals != perm &&
         (e = cudaMemcpyAsync(perm, b.vals, (size_t)nt * 4, cudaMemcpyDeviceToDevice, st)) != cudaSuccess)
       break;
-    ties_kernel<<<g, 256, 0, st>>>(s->tets, s->rest, perm, codes, nt, tied, err);
+    ties_kernel<<<g, 256, 0, st>>>(s->tets, s->rest, perm, codes, nt, tied);
     std::vector<uint32_t> ht((size_t)nm + 1);
     if ((e = cudaMemcpyAsync(ht.data(), tied, (size_t)nm * 4 + 4, cudaMemcpyDeviceToHost, st)) != cudaSuccess) break;
     if ((e = cudaStreamSynchronize(st)) != cudaSuccess) break;

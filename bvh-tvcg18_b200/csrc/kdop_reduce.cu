@@ -79,8 +79,9 @@ struct PointGen {
 struct BodyGen {
   const uint2* bodies;
   const uint32_t* perm;
+  int64_t n;
   __device__ uint64_t key(int64_t i) const {
-    const uint2 b = bodies[perm[i]];
+    const uint2 b = bodies[bounded(perm[i], n)];
     return ((uint64_t)b.x << 32) | b.y;
   }
   __device__ uint32_t val(int64_t i) const { return perm[i]; }
@@ -93,8 +94,9 @@ struct LongGen {
   const uint32_t* at;    // positions to sort
   const uint32_t* run;   // run of a position
   int pass;
+  int64_t n;
   __device__ uint64_t key(int64_t i) const {
-    const uint32_t k = at[i];
+    const uint32_t k = bounded(at[i], n);
     if (pass == 3) return run[k];
     const kdop_contact& c = rows[perm[k]];
     return pass == 0 ? two_keys(c.n[2], c.depth) : pass == 1 ? two_keys(c.n[1], c.n[0]) : two_keys(c.p[0], c.p[2]);
@@ -132,7 +134,7 @@ struct ReduceArgs {
   kdop_contact* out;
   uint2* out_bodies;
   unsigned* head;         // ReduceHead words
-  long long wait_ns;
+  WaitLimit lim;
   unsigned long long* words_run;
   unsigned long long* words_keep;
 };
@@ -144,16 +146,14 @@ constexpr int RD_ITEMS = 4, RD_TILE = 256 * RD_ITEMS;
 // Runs of equal (bodies, p.y): a scan of their first rows.
 __global__ void __launch_bounds__(256) red_runs_kernel(ReduceArgs a) {
   __shared__ unsigned s_tile;
-  const WaitLimit lim{a.head + H_ERR, a.wait_ns};
-  if (threadIdx.x == 0) s_tile = take_tile(a.head + H_TICKET_RUN, lim);
+  if (threadIdx.x == 0) s_tile = atomicAdd(a.head + H_TICKET_RUN, 1u);
   __syncthreads();
   const unsigned tile = s_tile;
-  if (tile == kNoTile) return;
   const int64_t base = (int64_t)tile * RD_TILE + (int64_t)threadIdx.x * RD_ITEMS;
   uint32_t y_prev = 0;
   uint2 b_prev = make_uint2(0u, 0u);
   if (base > 0 && base <= a.n) {
-    const uint32_t r = a.perm[base - 1];
+    const uint32_t r = bounded(a.perm[base - 1], a.n);
     y_prev = ord_key(a.rows[r].p[1]);
     b_prev = a.bodies[r];
   }
@@ -162,7 +162,7 @@ __global__ void __launch_bounds__(256) red_runs_kernel(ReduceArgs a) {
   for (int j = 0; j < RD_ITEMS; ++j) {
     const int64_t k = base + j;
     if (k >= a.n) continue;
-    const uint32_t r = a.perm[k];
+    const uint32_t r = bounded(a.perm[k], a.n);
     const float4 p = reinterpret_cast<const float4*>(a.rows)[2 * (int64_t)r];
     const uint32_t y = ord_key(p.y);
     const uint2 b = a.bodies[r];
@@ -176,7 +176,7 @@ __global__ void __launch_bounds__(256) red_runs_kernel(ReduceArgs a) {
   }
   uint32_t total;
   uint32_t at = block_scan<256, uint32_t>(sum, total);
-  at += tile_prefix(a.words_run, tile, total, lim);
+  at += tile_prefix(a.words_run, tile, total, a.lim);
 #pragma unroll
   for (int j = 0; j < RD_ITEMS; ++j) {
     const int64_t k = base + j;
@@ -203,9 +203,8 @@ __device__ __forceinline__ int later_fields(const Row& x, const Row& y) {
 __global__ void __launch_bounds__(256) red_rank_kernel(ReduceArgs a) {
   const int64_t k = (int64_t)blockIdx.x * 256 + threadIdx.x;
   if (k >= a.n) return;
-  const uint32_t r = a.perm[k], g = a.run[k];
-  if (gave_up(a.head + H_ERR)) return;  // the order or the runs are incomplete
-  const uint32_t s = a.starts[g], e = a.starts[g + 1];
+  const uint32_t r = bounded(a.perm[k], a.n), g = bounded(a.run[k], a.n);
+  const uint32_t s = bounded(a.starts[g], a.n), e = min(a.starts[g + 1], (uint32_t)a.n);
   const Row x = load_row(a.rows, r);
   if (e - s > kRankMax) {
     a.longs[k] = 1u;  // ordered by the radix sorts below, until then in the first sort's order
@@ -226,17 +225,17 @@ __global__ void __launch_bounds__(256) red_rank_kernel(ReduceArgs a) {
   if (ties > 1)
     for (uint32_t j = s; j < e; ++j) {
       if (a.next[j] != mine || j == (uint32_t)k) continue;
-      const int c = later_fields(load_row(a.rows, a.perm[j]), x);
+      const int c = later_fields(load_row(a.rows, bounded(a.perm[j], a.n)), x);
       rank += (c < 0 || (c == 0 && j < (uint32_t)k)) ? 1u : 0u;  // equal rows keep their order
     }
-  a.order[s + rank] = r;
-  a.sorted[s + rank] = x;
+  const uint32_t at = bounded(s + rank, a.n);
+  a.order[at] = r;
+  a.sorted[at] = x;
 }
 
 // Positions of the long runs' rows in increasing order: at[pos[k]] = k.
 __global__ void red_long_list_kernel(const uint32_t* __restrict__ flag, const uint32_t* __restrict__ pos, int64_t n,
                                      uint32_t* at) {
-  // (launched by a host that has seen no wait give up)
   const int64_t k = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (k < n && flag[k]) at[pos[k]] = (uint32_t)k;
 }
@@ -245,9 +244,7 @@ __global__ void red_long_place_kernel(ReduceArgs a, const uint32_t* __restrict__
                                       const uint32_t* __restrict__ sorted_at, int64_t m) {
   const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= m) return;
-  const uint32_t from = sorted_at[i];
-  if (gave_up(a.head + H_ERR)) return;
-  const uint32_t r = a.perm[from];
+  const uint32_t r = bounded(a.perm[bounded(sorted_at[i], a.n)], a.n);
   a.order[at[i]] = r;
   a.sorted[at[i]] = load_row(a.rows, r);
 }
@@ -265,13 +262,13 @@ __device__ __forceinline__ bool same_point(const Row& k, const Row& c) {
 // Whether the first row of a run can equal no earlier row.
 __device__ __forceinline__ bool run_breaks(const ReduceArgs& a, uint32_t s) {
   if (s == 0) return true;
-  const uint2 b = a.bodies[a.order[s]], q = a.bodies[a.order[s - 1]];
+  const uint2 b = a.bodies[bounded(a.order[s], a.n)], q = a.bodies[bounded(a.order[s - 1], a.n)];
   return b.x != q.x || b.y != q.y || fabsf(fsub(a.sorted[s].a.y, a.sorted[s - 1].a.y)) > kEps;
 }
 // Whether the row at position k starts a segment.
 __device__ __forceinline__ bool starts_segment(const ReduceArgs& a, uint32_t k) {
-  const uint32_t s = a.starts[a.run[k]];
-  if (s == k) return run_breaks(a, k);
+  const uint32_t s = bounded(a.starts[bounded(a.run[k], a.n)], a.n);
+  if (s == k || k == 0) return run_breaks(a, k);
   // a gap in p.x inside a run that starts a segment (a NaN at its head would
   // equal any row)
   const float x = a.sorted[k].a.x, p = a.sorted[k - 1].a.x, x0 = a.sorted[s].a.x;
@@ -282,14 +279,14 @@ constexpr uint32_t KEEP = 1u, SEGMENT = 2u;  // bits of keep[]
 
 __global__ void __launch_bounds__(256) red_segments_kernel(ReduceArgs a) {
   const int64_t k = (int64_t)blockIdx.x * 256 + threadIdx.x;
-  if (k < a.n && !gave_up(a.head + H_ERR)) a.keep[k] = starts_segment(a, (uint32_t)k) ? SEGMENT | KEEP : 0u;
+  if (k < a.n) a.keep[k] = starts_segment(a, (uint32_t)k) ? SEGMENT | KEEP : 0u;
 }
 
 // Thread per segment (its first row's): std::unique's walk -- a row is kept
 // unless it equals the last row kept.
 __global__ void __launch_bounds__(128) red_walk_kernel(ReduceArgs a) {
   const int64_t k = (int64_t)blockIdx.x * 128 + threadIdx.x;
-  if (k >= a.n || !(a.keep[k] & SEGMENT) || gave_up(a.head + H_ERR)) return;
+  if (k >= a.n || !(a.keep[k] & SEGMENT)) return;
   if (k + 1 >= a.n || (a.keep[k + 1] & SEGMENT)) return;  // a segment of one row (most): kept
   Row last = a.sorted[k];
   for (int64_t j = k + 1; j < a.n; ++j) {
@@ -305,11 +302,9 @@ __global__ void __launch_bounds__(128) red_walk_kernel(ReduceArgs a) {
 
 __global__ void __launch_bounds__(256) red_write_kernel(ReduceArgs a) {
   __shared__ unsigned s_tile;
-  const WaitLimit lim{a.head + H_ERR, a.wait_ns};
-  if (threadIdx.x == 0) s_tile = take_tile(a.head + H_TICKET_KEEP, lim);
+  if (threadIdx.x == 0) s_tile = atomicAdd(a.head + H_TICKET_KEEP, 1u);
   __syncthreads();
   const unsigned tile = s_tile;
-  if (tile == kNoTile) return;
   // consecutive threads hold consecutive rows: one scan step per item
   uint32_t keep[RD_ITEMS], pos[RD_ITEMS], sum = 0;
 #pragma unroll
@@ -320,7 +315,7 @@ __global__ void __launch_bounds__(256) red_write_kernel(ReduceArgs a) {
     pos[j] = sum + block_scan<256, uint32_t>(keep[j], total);
     sum += total;
   }
-  const uint32_t excl = tile_prefix(a.words_keep, tile, sum, lim);
+  const uint32_t excl = tile_prefix(a.words_keep, tile, sum, a.lim);
 #pragma unroll
   for (int j = 0; j < RD_ITEMS; ++j) {
     const int64_t k = (int64_t)tile * RD_TILE + j * 256 + threadIdx.x;
@@ -330,7 +325,7 @@ __global__ void __launch_bounds__(256) red_write_kernel(ReduceArgs a) {
     float4* o = reinterpret_cast<float4*>(a.out + excl + pos[j]);
     o[0] = x.a;
     o[1] = x.b;
-    if (a.out_bodies) a.out_bodies[excl + pos[j]] = a.bodies[a.order[k]];
+    if (a.out_bodies) a.out_bodies[excl + pos[j]] = a.bodies[bounded(a.order[k], a.n)];
   }
 }
 
@@ -412,8 +407,7 @@ static cudaError_t order_long_runs(kdop_ctx* ctx, const ReduceArgs& a, const Red
   const uint32_t* from = at;
   for (int pass = 0; pass < 4; ++pass) {
     const int bits = pass < 3 ? 64 : bits_of((uint64_t)a.n);
-    e = radix_sort(ctx, LongGen{a.rows, a.perm, from, a.run, pass}, m, bits, b, w + L.radix,
-                   WaitLimit{a.head + H_ERR, ctx->wait_ns});
+    e = radix_sort(ctx, LongGen{a.rows, a.perm, from, a.run, pass, a.n}, m, bits, b, w + L.radix, a.lim);
     if (e != cudaSuccess) return e;
     from = b.vals;
   }
@@ -448,7 +442,7 @@ cudaError_t reduce_contact_rows(kdop_ctx* ctx, const kdop_contact* rows, const u
   a.out = out;
   a.out_bodies = out_bodies;
   a.head = reinterpret_cast<unsigned*>(w + L.head);
-  a.wait_ns = ctx->wait_ns;
+  a.lim = WaitLimit(a.head + H_ERR, ctx->wait_ns);
   a.words_run = reinterpret_cast<unsigned long long*>(w + L.words_run);
   a.words_keep = reinterpret_cast<unsigned long long*>(w + L.words_keep);
   SortBuffers b{reinterpret_cast<uint64_t*>(w + L.keys), reinterpret_cast<uint64_t*>(w + L.keys_tmp),
@@ -466,9 +460,8 @@ cudaError_t reduce_contact_rows(kdop_ctx* ctx, const kdop_contact* rows, const u
     bj = bits_of(h[H_MOST_J]);
   }
   const bool one = bi + bj <= 32;
-  const WaitLimit lim{a.head + H_ERR, ctx->wait_ns};
-  e = radix_sort(ctx, PointGen{rows, bodies, bj, one}, n, 32 + (one ? bi + bj : 0), b, w + L.radix, lim);
-  if (e == cudaSuccess && !one) e = radix_sort(ctx, BodyGen{bodies, b.vals}, n, 32 + bi, b, w + L.radix, lim);
+  e = radix_sort(ctx, PointGen{rows, bodies, bj, one}, n, 32 + (one ? bi + bj : 0), b, w + L.radix, a.lim);
+  if (e == cudaSuccess && !one) e = radix_sort(ctx, BodyGen{bodies, b.vals, n}, n, 32 + bi, b, w + L.radix, a.lim);
   if (e != cudaSuccess) return e;
   a.perm = b.vals;
   const unsigned tiles = blocks_for(n, RD_TILE);

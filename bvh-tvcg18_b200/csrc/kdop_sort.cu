@@ -232,7 +232,8 @@ struct TetGen {
 };
 struct PairGen {
   const uint32_t *cP, *perm;
-  __device__ uint64_t key(int64_t i) const { return cP[perm[i]]; }
+  int64_t n;
+  __device__ uint64_t key(int64_t i) const { return cP[bounded(perm[i], n)]; }
   __device__ uint32_t val(int64_t i) const { return perm[i]; }
 };
 
@@ -241,6 +242,7 @@ struct ApplyArgs {
   const uint64_t* keys;  // sorted keys, or NULL: rows are gathered by perm
   const uint32_t* perm;
   CandGen c;
+  int64_t n_pairs;
   uint32_t *oA, *oB, *oP;
   const int4* rec;       // NULL without contacts
   int4* rec_out;
@@ -253,14 +255,12 @@ struct ApplyArgs {
 constexpr int AP_ITEMS = 4, AP_TILE = 256 * AP_ITEMS;
 
 // Candidate rows in sorted order and, with contacts, their records with the
-// rows' new places (a scan of the contact counts in the same pass).  Nothing
-// after a wait that gave up: the order may be incomplete.
+// rows' new places (a scan of the contact counts in the same pass).
 __global__ void __launch_bounds__(256) sort_apply_kernel(ApplyArgs a) {
   __shared__ unsigned s_tile;
-  if (threadIdx.x == 0) s_tile = a.rec ? take_tile(a.ticket, a.lim) : gave_up(a.lim.err) ? kNoTile : blockIdx.x;
+  if (threadIdx.x == 0) s_tile = a.rec ? atomicAdd(a.ticket, 1u) : blockIdx.x;
   __syncthreads();
   const unsigned tile = s_tile;
-  if (tile == kNoTile) return;
   const int64_t base = (int64_t)tile * AP_TILE + (int64_t)threadIdx.x * AP_ITEMS;
   int4 r[AP_ITEMS];
   uint32_t sum = 0;
@@ -271,19 +271,19 @@ __global__ void __launch_bounds__(256) sort_apply_kernel(ApplyArgs a) {
     if (k >= a.n) continue;
     if (a.keys) {
       const uint64_t key = a.keys[k];
-      const uint32_t p = (uint32_t)(key >> (2 * a.c.tb)), m = (1u << a.c.tb) - 1u;
+      const uint32_t p = bounded((uint32_t)(key >> (2 * a.c.tb)), a.n_pairs), m = (1u << a.c.tb) - 1u;
       const uint2 mp = a.c.pairs[p];
       a.oA[k] = a.c.t_off[mp.x] + ((uint32_t)(key >> a.c.tb) & m);
       a.oB[k] = a.c.t_off[mp.y] + ((uint32_t)key & m);
       a.oP[k] = p;
     } else {
-      const uint32_t o = a.perm[k];
+      const uint32_t o = bounded(a.perm[k], a.n);
       a.oA[k] = a.c.cA[o];
       a.oB[k] = a.c.cB[o];
       a.oP[k] = a.c.cP[o];
     }
     if (a.rec) {
-      r[j] = a.rec[a.perm[k]];
+      r[j] = a.rec[bounded(a.perm[k], a.n)];
       sum += (uint32_t)max(r[j].z, 0);
     }
   }
@@ -392,7 +392,7 @@ cudaError_t sort_results(kdop_scene* s, int64_t n, int64_t n_contacts, void* wor
   int4* rec_out = reinterpret_cast<int4*>(w + L.rec_out);
   float4* rows_out = reinterpret_cast<float4*>(w + L.rows_out);
   uint32_t* cand_out = reinterpret_cast<uint32_t*>(w + L.cand_out);
-  const WaitLimit lim{&s->ctl->error, s->ctx->wait_ns};
+  const WaitLimit lim(&s->ctl->error, s->ctx->wait_ns);
   CandGen gen{s->cand, s->cand + s->cand_cap, s->cand + 2 * s->cand_cap, s->pairs, s->t_off_dev, bits_of(std::max<int64_t>(s->most_tets, 1) - 1)};
   const int pair_bits = bits_of((uint64_t)std::max<int64_t>(s->result_pairs, 1) - 1);
   const bool packed = s->pairs_current && pair_bits + 2 * gen.tb <= 64;
@@ -402,7 +402,7 @@ cudaError_t sort_results(kdop_scene* s, int64_t n, int64_t n_contacts, void* wor
   } else {
     const int tb = bits_of(s->nt > 0 ? s->nt - 1 : 0);  // at most 30
     e = radix_sort(s->ctx, TetGen{gen.cA, gen.cB, tb}, n, 2 * tb, b, w + L.scratch, lim);
-    if (e == cudaSuccess) e = radix_sort(s->ctx, PairGen{gen.cP, b.vals}, n, 32, b, w + L.scratch, lim);
+    if (e == cudaSuccess) e = radix_sort(s->ctx, PairGen{gen.cP, b.vals, n}, n, 32, b, w + L.scratch, lim);
   }
   if (e != cudaSuccess) return e;
   const bool with_contacts = s->contacted;
@@ -411,6 +411,7 @@ cudaError_t sort_results(kdop_scene* s, int64_t n, int64_t n_contacts, void* wor
   a.keys = packed ? b.keys : nullptr;
   a.perm = b.vals;
   a.c = gen;
+  a.n_pairs = std::max<int64_t>(s->result_pairs, 1);
   // the sorted keys hold the rows: they go straight to the scene's columns
   a.oA = packed ? s->cand : cand_out;
   a.oB = packed ? s->cand + s->cand_cap : cand_out + n;

@@ -325,7 +325,6 @@ __global__ void __launch_bounds__(512, (C * S >= 4) ? 1 : 2) traverse_kernel(Tra
   uint2* sAB = reinterpret_cast<uint2*>(smem) + (size_t)wib * CAP;  // this warp's deque
   TravCtl* ctl = a.ctl;
   if (a.seeded && ctl->n_init == 0u && a.stuck == 0) return;  // the seed pass finished every pair
-  if (a.entries && !a.seeded && gave_up(&ctl->error)) return;  // the frontier's order gave up: no entries
   // A block that starts takes a first claim of the seeded entries for each of its
   // warps at once (an atomic per block, not per warp).  All claims come off the
   // one counter, so that entries belong to running warps only: a block that
@@ -680,7 +679,7 @@ cudaError_t launch_pair_order(kdop_scene* s, int64_t n, uint32_t most, long long
   if (e == cudaSuccess) e = cudaMemsetAsync(w + L.vals, 0, L.scratch - L.vals, s->ctx->stream);
   if (e == cudaSuccess)
     e = radix_sort(s->ctx, PairSizeGen{s->pairs, s->t_off_dev, most}, n, bits_of(most), b, w + L.scratch,
-                   WaitLimit{&s->ctl->order_error, wait_ns});
+                   WaitLimit(&s->ctl->order_error, wait_ns));
   if (e == cudaSuccess)
     e = cudaMemcpyAsync(s->pair_order, b.vals, (size_t)n * 4, cudaMemcpyDeviceToDevice, s->ctx->stream);
   return e;
@@ -1149,16 +1148,17 @@ struct EntryGen {
 struct EntryPairGen {
   const uint4* f;
   const uint32_t* order;
-  __device__ uint64_t key(int64_t i) const { return f[order[i]].z; }
+  int64_t n;
+  __device__ uint64_t key(int64_t i) const { return f[bounded(order[i], n)].z; }
   __device__ uint32_t val(int64_t i) const { return order[i]; }
 };
 
 // this shard's entries: sorted positions rank, rank + n_ranks, ...
 __global__ void deal_kernel(const uint4* __restrict__ f, const uint32_t* __restrict__ order, unsigned n, int rank,
-                            int n_ranks, uint4* mine, const unsigned* err) {
+                            int n_ranks, uint4* mine) {
   unsigned j = blockIdx.x * blockDim.x + threadIdx.x;
   unsigned src = (unsigned)rank + j * (unsigned)n_ranks;
-  if (src < n && !gave_up(err)) mine[j] = f[order[src]];  // the order may be incomplete
+  if (src < n) mine[j] = f[bounded(order[src], n)];
 }
 
 __global__ void clear_totals_kernel(TravCtl* c) {
@@ -1242,12 +1242,12 @@ cudaError_t shard_impl(kdop_scene* s, int64_t n_pairs, const uint2* pairs, const
   // deterministic order: by (A, B), then by pair
   if (n > 0) {
     const unsigned gn = (n + 255) / 256;
-    const WaitLimit lim{&s->ctl->error, p.timeout_ns};
+    const WaitLimit lim(&s->ctl->error, p.timeout_ns);
     if ((e = radix_sort(s->ctx, EntryGen{fin}, n, 64, b, w + L.sc, lim)) != cudaSuccess) return e;
-    if ((e = radix_sort(s->ctx, EntryPairGen{fin, b.vals}, n, bits_of((uint64_t)std::max<int64_t>(n_pairs, 1) - 1), b,
+    if ((e = radix_sort(s->ctx, EntryPairGen{fin, b.vals, n}, n, bits_of((uint64_t)std::max<int64_t>(n_pairs, 1) - 1), b,
                         w + L.sc, lim)) != cudaSuccess)
       return e;
-    deal_kernel<<<gn, 256, 0, st>>>(fin, b.vals, n, rank, n_ranks, mine, lim.err);
+    deal_kernel<<<gn, 256, 0, st>>>(fin, b.vals, n, rank, n_ranks, mine);
     s->ctx->launches += 1;
   }
   // the expansion's tests and leaf pairs belong to shard 0
