@@ -61,7 +61,6 @@ struct TravArgs {
   unsigned n_meshes;
   const uint32_t* __restrict__ order;  // root pair i -> pair index (NULL: identity)
   const uint4* __restrict__ entries;   // when set: initial work = these deque entries (A, B, pair)
-  int seeded;          // entries come from the seed pass (their count is known on the device only)
   int stuck;           // test hook: outstanding work units nobody completes
   unsigned poll_mask;  // queue counters polled on steps with (step & poll_mask) == 0
 };
@@ -250,22 +249,20 @@ __device__ __forceinline__ void put_candidate(const TravArgs& a, unsigned at, ui
 // traversal's own test of the root pair (:42), both counted as the reference
 // does.  True when the pair is to be expanded (wa, wb its entry).
 template <int K>
-__device__ __forceinline__ bool root_pair(const TravArgs& a, uint32_t pid, bool count, uint32_t& wa, uint32_t& wb,
+__device__ __forceinline__ bool root_pair(const TravArgs& a, uint32_t pid, uint32_t& wa, uint32_t& wb,
                                           unsigned& tests32, unsigned& lo32) {
   const uint2 mp = a.pairs[pid];
   if (mp.x >= a.n_meshes || mp.y >= a.n_meshes) {
-    if (count) atomicOr(&a.ctl->error, DEV_ERR_BAD_INDEX);
+    atomicOr(&a.ctl->error, DEV_ERR_BAD_INDEX);
     return false;
   }
   const uint32_t ra = a.root[mp.x], rb = a.root[mp.y];
   if (ra == NO_NODE || rb == NO_NODE) return false;
   const bool ov = node_overlap<K>(a.nodes, ra, rb, wa, wb);
-  if (count) tests32 += ov ? 2u : 1u;
+  tests32 += ov ? 2u : 1u;
   if (!ov || !(wa & wb & LEAF_BIT)) return ov;
-  if (count) {
-    lo32 += 1u;
-    if (!a.surface_filter || (wa & wb & SURF_BIT)) put_candidate<K>(a, atomicAdd(&a.ctl->n_cand, 1u), wa, wb, pid);
-  }
+  lo32 += 1u;
+  if (!a.surface_filter || (wa & wb & SURF_BIT)) put_candidate<K>(a, atomicAdd(&a.ctl->n_cand, 1u), wa, wb, pid);
   return false;
 }
 
@@ -303,7 +300,15 @@ __device__ __forceinline__ unsigned claim_size(unsigned left, unsigned warps) {
 // ms, and to 9.4 with the lanes beyond the last entry repeating its loads.
 // S sub-batches are loaded together per step, and one compaction per step
 // packs the pushes of all of them.
-template <int K, int C, int S>
+//
+// SEEDED: starts from the seed pass's entries.  Otherwise a warp claims
+// init_chunk root pairs (tested one per lane) or entries of a caller's frontier
+// at a time.  They lie at the bottom of its deque, each with a pair index of its
+// own beside it, until they are begun, so that waiting warps can be given them
+// like any other entry.  (Held back one by one instead, a claim of 32 took 64
+// touching pairs of 6,000 tets from 213 to 1,322 us, and used up the queue of
+// the call that cannot grow it.)
+template <int K, int C, int S, bool SEEDED>
 __global__ void __launch_bounds__(512, (C * S >= 4) ? 1 : 2) traverse_kernel(TravArgs a) {
   using L = NodeLayout<K>;
   using CP = Coop<K, C>;
@@ -312,8 +317,9 @@ __global__ void __launch_bounds__(512, (C * S >= 4) ? 1 : 2) traverse_kernel(Tra
   constexpr int SLOTS = PM * S;                     // pushes per lane per step
   constexpr int CBITS = SLOTS <= 1 ? 1 : SLOTS <= 3 ? 2 : 3;  // bits of a lane's push count
   extern __shared__ uint32_t smem[];
-  __shared__ uint2 s_claim[16];  // per warp: claimed initial work not yet taken [x, y)
+  __shared__ uint2 s_claim[SEEDED ? 16 : 1];  // per warp: claimed initial work not yet taken [x, y)
   __shared__ unsigned s_first;
+  __shared__ uint32_t s_pair[SEEDED ? 1 : 16 * 32];  // per warp: pairs of the claimed entries, by deque position
   const int lane = threadIdx.x & 31;
   const int wib = threadIdx.x >> 5;
   const int ge = lane / Q, gq = lane % Q;  // entry and chunk lane of this lane
@@ -324,7 +330,7 @@ __global__ void __launch_bounds__(512, (C * S >= 4) ? 1 : 2) traverse_kernel(Tra
   const int MASK = CAP - 1;
   uint2* sAB = reinterpret_cast<uint2*>(smem) + (size_t)wib * CAP;  // this warp's deque
   TravCtl* ctl = a.ctl;
-  if (a.seeded && ctl->n_init == 0u && a.stuck == 0) return;  // the seed pass finished every pair
+  if (SEEDED && ctl->n_init == 0u && a.stuck == 0) return;  // the seed pass finished every pair
   // A block that starts takes a first claim of the seeded entries for each of its
   // warps at once (an atomic per block, not per warp).  All claims come off the
   // one counter, so that entries belong to running warps only: a block that
@@ -333,20 +339,19 @@ __global__ void __launch_bounds__(512, (C * S >= 4) ? 1 : 2) traverse_kernel(Tra
   auto first_claim = [&](unsigned n_init) {
     return max(claim_size(n_init, gridDim.x * (blockDim.x >> 5)), (unsigned)a.init_chunk);
   };
-  uint2 own = make_uint2(0u, 0u);
   bool init_done = false;
-  if (a.seeded) {
+  if (SEEDED) {
     const unsigned n_init = ctl->n_init, first = first_claim(n_init);
     if (threadIdx.x == 0) s_first = atomicAdd(&ctl->init_head, first * (blockDim.x >> 5));
     __syncthreads();
-    own.x = min(s_first + (unsigned)wib * first, n_init);
-    own.y = min(own.x + first, n_init);
-    init_done = own.x >= n_init;
+    const unsigned own = min(s_first + (unsigned)wib * first, n_init);
+    if (lane == 0) s_claim[wib] = make_uint2(own, min(own + first, n_init));
+    __syncwarp();
+    init_done = own >= n_init;
   }
-  if (lane == 0) s_claim[wib] = own;
-  __syncwarp();
 
   int top = 0, bot = 0;  // deque [bot, top) in virtual positions
+  int begun = 0;         // not SEEDED: [bot, begun) are claimed entries of a pair each
   int release = 0;       // work units taken and not yet released
   unsigned claim = 0xFFFFFFFFu;
   // per-lane counts, added to the control block's 64-bit totals every 1024
@@ -365,14 +370,16 @@ __global__ void __launch_bounds__(512, (C * S >= 4) ? 1 : 2) traverse_kernel(Tra
     }
     tests32 = lo32 = 0;
   };
-  // Pair index of the deque's entries.  A deque is filled from one root pair,
-  // one queue item or frontier entries of one pair, and entries inherit their
-  // parent's pair, so it holds a single pair at any time (warp-uniform).
+  // Pair index of the deque's entries (from `begun` on).  A deque is filled from
+  // one root pair, one queue item or frontier entries of one pair, and entries
+  // inherit their parent's pair, so it holds a single pair at any time
+  // (warp-uniform).
   uint32_t curP = 0;
   const uint32_t need = a.surface_filter ? SURF_BIT : 0u;  // word bits an emitted leaf pair has to share
 
   unsigned step = 0;
   for (;;) {
+    if (!SEEDED) ++step;
     if (top == bot) {
       // Work handed to the queue was counted before it was published, so the
       // release needs no fence.
@@ -380,51 +387,67 @@ __global__ void __launch_bounds__(512, (C * S >= 4) ? 1 : 2) traverse_kernel(Tra
         if (lane == 0) atomicSub(&ctl->work, release);
         release = 0;
       }
-      if (!init_done) {
+      if (SEEDED && !init_done) {
         uint2 r = s_claim[wib];
         __syncwarp();
         if (r.x == r.y) {
-          const unsigned n_init = ctl->n_init;
-          unsigned base = 0, chunk = (unsigned)a.init_chunk;
-          if (a.seeded) {
-            // what is left when every block has its first claim, at most
-            const unsigned warps = gridDim.x * (blockDim.x >> 5);
-            chunk = max(chunk, claim_size(n_init - min(n_init, max(r.y, warps * first_claim(n_init))), warps));
-          }
+          // what is left when every block has its first claim, at most
+          const unsigned n_init = ctl->n_init, warps = gridDim.x * (blockDim.x >> 5);
+          const unsigned left = n_init - min(n_init, max(r.y, warps * first_claim(n_init)));
+          const unsigned chunk = max((unsigned)a.init_chunk, claim_size(left, warps));
+          unsigned base = 0;
           if (lane == 0) base = atomicAdd(&ctl->init_head, chunk);
           base = min(__shfl_sync(0xffffffffu, base, 0), n_init);
           init_done = base >= n_init;
           r = make_uint2(base, min(base + chunk, n_init));
         }
         if (!init_done) {
-          if (a.entries) {
-            // pending node pairs of a frontier (their tests are counted
-            // already): the claim's leading run of one pair
-            const bool in = r.x + lane < r.y;
-            uint4 e = make_uint4(0u, 0u, 0u, 0u);
-            if (in) e = a.entries[r.x + lane];
-            curP = __shfl_sync(0xffffffffu, e.z, 0);
-            const unsigned same = __ballot_sync(0xffffffffu, in && e.z == curP);
-            const int run = (same == 0xffffffffu) ? 32 : __ffs(~same) - 1;
-            if (lane < run) sAB[(top + lane) & MASK] = make_uint2(e.x, e.y);
-            top += run;
-            release += run;
-            r.x += (unsigned)run;
-          } else {
-            // a root pair: the whole warp tests it, lane 0 counts and writes
-            uint32_t pid = ctl->pair_base + r.x;
-            if (a.order) pid = a.order[pid];
-            uint32_t wa = 0, wb = 0;
-            const bool expand = root_pair<K>(a, pid, lane == 0, wa, wb, tests32, lo32);
-            curP = pid;
-            release += 1;
-            r.x += 1u;
-            if (expand) {
-              if (lane == 0) sAB[top & MASK] = make_uint2(wa, wb);
-              top += 1;
-            }
-          }
+          // pending node pairs of a frontier (their tests are counted already):
+          // the claim's leading run of one pair
+          const bool in = r.x + lane < r.y;
+          uint4 e = make_uint4(0u, 0u, 0u, 0u);
+          if (in) e = a.entries[r.x + lane];
+          curP = __shfl_sync(0xffffffffu, e.z, 0);
+          const unsigned same = __ballot_sync(0xffffffffu, in && e.z == curP);
+          const int run = (same == 0xffffffffu) ? 32 : __ffs(~same) - 1;
+          if (lane < run) sAB[(top + lane) & MASK] = make_uint2(e.x, e.y);
+          top += run;
+          release += run;
+          r.x += (unsigned)run;
           if (lane == 0) s_claim[wib] = r;
+          __syncwarp();
+          continue;
+        }
+      }
+      if (!SEEDED && !init_done) {
+        unsigned first = 0;
+        if (lane == 0) first = atomicAdd(&ctl->init_head, (unsigned)a.init_chunk);
+        first = __shfl_sync(0xffffffffu, first, 0);
+        const unsigned n_init = ctl->n_init;
+        init_done = first >= n_init;
+        if (!init_done) {
+          const int n = (int)min((unsigned)a.init_chunk, n_init - first);
+          uint32_t wa = 0, wb = 0, pid = 0;
+          bool there = lane < n;
+          if (there && a.entries) {
+            const uint4 e = a.entries[first + lane];
+            wa = e.x;
+            wb = e.y;
+            pid = e.z;
+          } else if (there) {
+            pid = ctl->pair_base + first + lane;
+            if (a.order) pid = a.order[pid];
+            there = root_pair<K>(a, pid, wa, wb, tests32, lo32);
+          }
+          const unsigned m = __ballot_sync(0xffffffffu, there);
+          if (there) {
+            const int at = top + __popc(m & lt_mask);
+            sAB[at & MASK] = make_uint2(wa, wb);
+            s_pair[wib * 32 + (at & 31)] = pid;
+          }
+          release += n;
+          top += __popc(m);
+          begun = top;
           __syncwarp();
           continue;
         }
@@ -475,8 +498,10 @@ __global__ void __launch_bounds__(512, (C * S >= 4) ? 1 : 2) traverse_kernel(Tra
     // this step's pushes (entry words) and emitted leaf pairs (node words)
     bool push[SLOTS], emit[SLOTS];
     uint32_t pushA[SLOTS], pushB[SLOTS];
+    const bool had_two = SEEDED || top - bot >= 2;
     {
-      const int n = min(E * S, top - bot);
+      if (!SEEDED && top == begun) curP = s_pair[wib * 32 + (--begun & 31)];
+      const int n = min(E * S, top - (SEEDED ? bot : begun));
       top -= n;
       uint2 eab[S];
       float4 A0[S][C], A1[S][C], B0[S][C], B1[S][C];
@@ -574,11 +599,11 @@ __global__ void __launch_bounds__(512, (C * S >= 4) ? 1 : 2) traverse_kernel(Tra
     // The queue counters are polled on every (poll_mask + 1)-th step.  A deep
     // deque gives to any waiting warp; while many warps wait (the tail of the
     // traversal) any deque with two or more entries gives half.
-    ++step;
+    if (SEEDED) ++step;
     if ((step & a.poll_mask) == 0u) {
       if ((step & 1023u) == 0u) fold_counts();
       const int depth = top - bot;
-      if (depth >= 2) {
+      if (depth >= 2 && had_two) {
         int waiting = 0;
         if (lane == 0) {
           const unsigned q_h = ld_volatile(&ctl->q_head), q_t = ld_volatile(&ctl->q_tail);
@@ -597,13 +622,15 @@ __global__ void __launch_bounds__(512, (C * S >= 4) ? 1 : 2) traverse_kernel(Tra
           __syncwarp();
           if (lane < room) {
             uint2 ab = sAB[(bot + lane) & MASK];
-            a.q_items[t0 + lane] = make_uint4(ab.x, ab.y, curP, 0u);
+            const uint32_t pid = SEEDED || bot + lane >= begun ? curP : s_pair[wib * 32 + ((bot + lane) & 31)];
+            a.q_items[t0 + lane] = make_uint4(ab.x, ab.y, pid, 0u);
           }
           __threadfence();
           __syncwarp();
           if (lane < room) atomicExch(&a.q_tags[t0 + lane], 1u);
           // entries that found no room stay lost only with DEV_ERR_QUEUE_FULL set
           bot += d;
+          begun = max(begun, bot);
         }
       }
     }
@@ -750,7 +777,7 @@ __global__ void __launch_bounds__(kSeedThreads) seed_kernel(TravArgs a, unsigned
       } else {
         const uint32_t pid = a.order[base + i];
         uint32_t wa = 0, wb = 0;
-        if (root_pair<K>(a, pid, true, wa, wb, tests32, lo32)) {
+        if (root_pair<K>(a, pid, wa, wb, tests32, lo32)) {
           const unsigned at = atomicAdd(&cnt[0], 1u);
           AB[at] = make_uint2(wa, wb);
           P[at] = pid;
@@ -855,15 +882,20 @@ size_t traverse_smem_bytes(int block_warps, int stack_cap) {
   return (size_t)block_warps * (size_t)stack_cap * sizeof(uint2);
 }
 
+template <int K, int C, int S>
+static cudaError_t prepare_shape(size_t smem) {
+  cudaError_t e = cudaFuncSetAttribute(traverse_kernel<K, C, S, true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                       (int)smem);
+  if (e == cudaSuccess)
+    e = cudaFuncSetAttribute(traverse_kernel<K, C, S, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  return e;
+}
 template <int K>
 static cudaError_t prepare_k(size_t smem) {
-  cudaError_t e = cudaFuncSetAttribute(traverse_kernel<K, 1, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-  if (e == cudaSuccess)
-    e = cudaFuncSetAttribute(traverse_kernel<K, 1, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-  if (e == cudaSuccess)
-    e = cudaFuncSetAttribute(traverse_kernel<K, 2, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-  if (e == cudaSuccess)
-    e = cudaFuncSetAttribute(traverse_kernel<K, 2, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  cudaError_t e = prepare_shape<K, 1, 1>(smem);
+  if (e == cudaSuccess) e = prepare_shape<K, 1, 2>(smem);
+  if (e == cudaSuccess) e = prepare_shape<K, 2, 1>(smem);
+  if (e == cudaSuccess) e = prepare_shape<K, 2, 2>(smem);
   return e;
 }
 
@@ -886,13 +918,15 @@ static cudaError_t traverse_impl(kdop_scene* s, int64_t n_pairs, const TravBuffe
   cudaStream_t st = s->ctx->stream;
   int threads = traverse_block_threads(p.block_warps);
   size_t smem = traverse_smem_bytes(p.block_warps, p.stack_cap);
-  cudaError_t e = cudaFuncSetAttribute(traverse_kernel<K, C, S>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  const bool seeded = b.seeds && !plain && p.wave_pairs <= 0 && n_pairs > 0;
+  const auto kernel = seeded ? traverse_kernel<K, C, S, true> : traverse_kernel<K, C, S, false>;
+  cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   if (e != cudaSuccess) return e;
-  e = cudaFuncSetAttribute(traverse_kernel<K, C, S>, cudaFuncAttributePreferredSharedMemoryCarveout,
+  e = cudaFuncSetAttribute(kernel, cudaFuncAttributePreferredSharedMemoryCarveout,
                            p.smem_carveout > 0 ? p.smem_carveout : -1);
   if (e != cudaSuccess) return e;
   int per_sm = 0;
-  e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, traverse_kernel<K, C, S>, threads, smem);
+  e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, threads, smem);
   if (e != cudaSuccess) return e;
   if (per_sm < 1) return cudaErrorInvalidConfiguration;
   unsigned grid = (unsigned)(per_sm * s->ctx->sm_count);
@@ -923,9 +957,8 @@ static cudaError_t traverse_impl(kdop_scene* s, int64_t n_pairs, const TravBuffe
   // waiting for donations and polls every 4th step (config 3, one launch per
   // pair: 88 ms vs 103 ms every 16th).
   a.poll_mask = plain ? 3u : 15u;
-  a.seeded = 0;
   a.stuck = p.stuck_work;
-  if (b.seeds && !plain && p.wave_pairs <= 0 && n_pairs > 0) {
+  if (seeded) {
     const int sms = s->ctx->sm_count;
     const int64_t group = seed_group(sms, n_pairs), groups = (n_pairs + group - 1) / group;
     const unsigned blocks2 = (unsigned)seed_blocks2(sms, n_pairs, s->pairs_tets);
@@ -941,15 +974,14 @@ static cudaError_t traverse_impl(kdop_scene* s, int64_t n_pairs, const TravBuffe
       seed_kernel<K><<<blocks2, kSeedThreads, seed_smem, st>>>(a, 0u, 0u, b.seeds, &b.ctl->n_seed, seeds2,
                                                               &b.ctl->n_init);
     a.entries = blocks2 ? seeds2 : b.seeds;
-    a.seeded = 1;
-    traverse_kernel<K, C, S><<<grid, threads, smem, st>>>(a);
+    kernel<<<grid, threads, smem, st>>>(a);
     s->ctx->launches += blocks2 ? 4 : 3;
     return cudaGetLastError();
   }
   if (b.entries) {
     // seeded by a frontier: its tests and leaf pairs are in the totals already
     trav_init_kernel<<<1, 32, 0, st>>>(b.ctl, (unsigned)n_pairs, 0u, 0, p.stuck_work);
-    traverse_kernel<K, C, S><<<grid, threads, smem, st>>>(a);
+    kernel<<<grid, threads, smem, st>>>(a);
     s->ctx->launches += 2;
   } else if (!plain) {
     // waves of wave_pairs root pairs (largest first), or all at once
@@ -959,14 +991,14 @@ static cudaError_t traverse_impl(kdop_scene* s, int64_t n_pairs, const TravBuffe
       int64_t n = std::min<int64_t>(wave, n_pairs - off);
       trav_init_kernel<<<1, 32, 0, st>>>(b.ctl, (unsigned)std::max<int64_t>(n, 0), (unsigned)off, off == 0,
                                          p.stuck_work);
-      traverse_kernel<K, C, S><<<grid, threads, smem, st>>>(a);
+      kernel<<<grid, threads, smem, st>>>(a);
       s->ctx->launches += 2;
       if (n_pairs == 0) break;
     }
   } else {
     for (int64_t i = 0; i < n_pairs; ++i) {
       trav_init_kernel<<<1, 32, 0, st>>>(b.ctl, 1u, (unsigned)i, i == 0 ? 1 : 0, p.stuck_work);
-      traverse_kernel<K, C, S><<<grid, threads, smem, st>>>(a);
+      kernel<<<grid, threads, smem, st>>>(a);
       s->ctx->launches += 2;
     }
     if (n_pairs == 0) {
