@@ -326,16 +326,19 @@ __global__ void __launch_bounds__(256) candidate_rows_kernel(const uint32_t* __r
 }
 
 // Contact rows of sorted candidate k to rows r.w ..: eight lanes a candidate,
-// 16 bytes a lane.
+// 16 bytes a lane.  Records a timed-out sort left incomplete may name rows past
+// the n_rows there are: nothing is copied for them.
 __global__ void __launch_bounds__(256) contact_gather_kernel(int64_t n, const int4* __restrict__ rec,
                                                              const uint32_t* __restrict__ src,
                                                              const float4* __restrict__ rows, float4* rows_out,
-                                                             const unsigned* err) {
+                                                             int64_t n_rows) {
   const int64_t k = ((int64_t)blockIdx.x * 256 + threadIdx.x) >> 3;
   if (k >= n) return;
   const int4 r = rec[k];
-  if (gave_up(err) || r.z <= 0) return;  // the records may be incomplete
-  const float4* from = rows + 2 * (size_t)src[k];
+  if (r.z <= 0) return;
+  const uint32_t first = src[k];
+  if ((int64_t)max(first, (uint32_t)r.w) + r.z > n_rows) return;
+  const float4* from = rows + 2 * (size_t)first;
   float4* to = rows_out + 2 * (size_t)(uint32_t)r.w;
   for (int c = threadIdx.x & 7; c < 2 * r.z; c += 8) {
     float4 x = from[c];
@@ -433,7 +436,7 @@ cudaError_t sort_results(kdop_scene* s, int64_t n, int64_t n_contacts, void* wor
     }
   if (with_contacts) {
     contact_gather_kernel<<<(unsigned)((n + 31) / 32), 256, 0, st>>>(
-        n, rec_out, a.src, reinterpret_cast<const float4*>(s->contacts), rows_out, lim.err);
+        n, rec_out, a.src, reinterpret_cast<const float4*>(s->contacts), rows_out, n_contacts);
     s->ctx->launches++;
     e = cudaMemcpyAsync(s->records, rec_out, (size_t)n * sizeof(int4), cudaMemcpyDeviceToDevice, st);
     if (e == cudaSuccess && n_contacts > 0)
