@@ -42,7 +42,10 @@ class ContactGeometry(torch.autograd.Function):
         scene.read_contacts_into(rows)  # synchronises
         ctx.scene = scene
         ctx.n_verts, ctx.n_contacts = xyz.shape[0], n
-        return rows[:, 6].contiguous(), rows[:, 3:6].contiguous()
+        # copies for any n: of at most one row a slice is contiguous as it is, and
+        # an output that is a view may not be written in place by the caller
+        return (rows[:, 6].clone(memory_format=torch.contiguous_format),
+                rows[:, 3:6].clone(memory_format=torch.contiguous_format))
 
     @staticmethod
     def backward(ctx, g_depth, g_normal):
