@@ -10,6 +10,7 @@ forward pass (contact face, extreme candidates) held fixed.
 """
 from __future__ import annotations
 
+import numpy as np
 import torch
 
 from . import lib as kd
@@ -31,7 +32,9 @@ class ContactGeometry(torch.autograd.Function):
         if not xyz.is_cuda or xyz.dtype != torch.float32:
             raise TypeError("xyz must be a float32 CUDA tensor")
         work, current = _scene_stream(scene, xyz.device)
+        # conversions run on the current stream: before the scene's waits for it
         x = xyz.detach().contiguous()
+        pairs = kd._arg(pairs, np.uint32)
         work.wait_stream(current)
         scene.set_vertices(x)
         scene.refit(kd.REFIT_VERTICES)
