@@ -23,6 +23,7 @@ const int64_t kDefaultContacts = 1 << 20;
 const int64_t kDefaultQueue = 1 << 20;
 const int64_t kHostOrder = 256;        // pairs up to which the host orders them
 const int64_t kReadFloats = 16 << 20;  // words a read-back stages on the device at a time
+const int64_t kReadLeast = 4096;       // items it stages when the device has no room for more
 
 int fail(kdop_ctx* ctx, int status, const std::string& msg) {
   if (ctx) ctx->err = msg;
@@ -71,8 +72,10 @@ cudaError_t launch_pack_poses(kdop_scene* s, const float* quat, const float* pos
 }  // namespace kdop
 
 struct kdop_scene_ext {
-  float* stage = nullptr;
+  float* stage = nullptr;  // host arrays on their way in
   int64_t stage_n = 0;
+  float* read_stage = nullptr;  // rows and nodes on their way out
+  int64_t read_n = 0;
   void* sort_work = nullptr;  // kdop_sort_results scratch
   size_t sort_work_bytes = 0;
   void* shard_work = nullptr;  // kdop_traverse_shard scratch
@@ -105,22 +108,36 @@ static kdop_scene_ext* ext(kdop_scene* s) { return &reinterpret_cast<SceneBox*>(
 
 static int lost(kdop_scene* s) { return fail(s->ctx, KDOP_ERR_STATE, "results lost: a wait of their sort timed out"); }
 
-static float* stage(kdop_scene* s, int64_t nfloats, cudaError_t* err) {
-  kdop_scene_ext* x = ext(s);
+static float* grow_stage(kdop_scene* s, float** buf, int64_t* have, int64_t nfloats, cudaError_t* err) {
   *err = cudaSuccess;
-  if (x->stage_n < nfloats) {
-    if (x->stage) {
-      cudaFree(x->stage);
-      s->device_bytes -= x->stage_n * 4;
+  if (*have < nfloats) {
+    if (*buf) {
+      cudaFree(*buf);
+      s->device_bytes -= *have * 4;
     }
-    x->stage = nullptr;
-    x->stage_n = 0;
-    *err = cudaMalloc((void**)&x->stage, (size_t)std::max<int64_t>(nfloats, 1) * 4);
+    *buf = nullptr;
+    *have = 0;
+    *err = cudaMalloc((void**)buf, (size_t)std::max<int64_t>(nfloats, 1) * 4);
     if (*err != cudaSuccess) return nullptr;
-    x->stage_n = std::max<int64_t>(nfloats, 1);
-    s->device_bytes += x->stage_n * 4;
+    *have = std::max<int64_t>(nfloats, 1);
+    s->device_bytes += *have * 4;
   }
-  return x->stage;
+  return *buf;
+}
+static float* stage(kdop_scene* s, int64_t nfloats, cudaError_t* err) {
+  return grow_stage(s, &ext(s)->stage, &ext(s)->stage_n, nfloats, err);
+}
+// Room for `window` items of `words` words each to be read back.  A buffer
+// apart from the uploads': a graph the caller captured may hold a host upload
+// through that one, so a read-back leaves it where it is.  Fewer items at a
+// time where the device has no room for them (`window` says how many).
+static float* read_stage(kdop_scene* s, int64_t words, int64_t* window, cudaError_t* err) {
+  for (;;) {
+    float* d = grow_stage(s, &ext(s)->read_stage, &ext(s)->read_n, words * *window, err);
+    if (d || *err != cudaErrorMemoryAllocation || *window <= kReadLeast) return d;
+    cudaGetLastError();
+    *window = std::max((*window + 1) / 2, kReadLeast);
+  }
 }
 
 // The control block's host copy holds what the device's does until the next
@@ -274,6 +291,8 @@ static void scene_free(kdop_scene* s) {
   s->ctl_host = nullptr;
   if (x->stage) cudaFree(x->stage);
   x->stage = nullptr;
+  if (x->read_stage) cudaFree(x->read_stage);
+  x->read_stage = nullptr;
   if (x->sort_work) cudaFree(x->sort_work);
   x->sort_work = nullptr;
   x->sort_work_bytes = 0;
@@ -629,9 +648,9 @@ int kdop_read_tree(kdop_scene* s, int mesh, int64_t cap, float* vol, int64_t* te
   cudaSetDevice(s->ctx->device);
   // gathered in preorder on the device, a window at a time: tets (8-byte
   // aligned), then slabs
-  const int64_t window = std::min<int64_t>(*n_nodes, kReadFloats / (s->K + 2));
+  int64_t window = std::min<int64_t>(*n_nodes, kReadFloats / (s->K + 2));
   cudaError_t e;
-  float* d = stage(s, window * (s->K + 2), &e);
+  float* d = read_stage(s, s->K + 2, &window, &e);
   if (!d) return cuda_fail(s->ctx, e, "staging alloc");
   int64_t* d_tet = reinterpret_cast<int64_t*>(d);
   float* d_vol = d + 2 * window;
@@ -1065,9 +1084,9 @@ int kdop_read_candidates(kdop_scene* s, uint32_t* rows, int64_t cap, int64_t* n_
   *n_rows = n;
   if (n > cap) return fail(s->ctx, KDOP_ERR_CAPACITY, "candidate read buffer too small");
   if (n == 0) return KDOP_OK;
-  const int64_t window = std::min<int64_t>(n, kReadFloats / 3);
+  int64_t window = std::min<int64_t>(n, kReadFloats / 3);
   cudaError_t e;
-  float* d = stage(s, 3 * window, &e);
+  float* d = read_stage(s, 3, &window, &e);
   if (!d) return cuda_fail(s->ctx, e, "staging alloc");
   for (int64_t at = 0; at < n; at += window) {
     const int64_t m = std::min(window, n - at);
