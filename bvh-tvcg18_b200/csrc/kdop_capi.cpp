@@ -359,15 +359,24 @@ static int grow_queue(kdop_scene* s, int64_t n) {
   return KDOP_OK;
 }
 
-static int grow_pairs(kdop_scene* s, int64_t n) {
-  if (n <= s->pairs_cap) return KDOP_OK;
+static int grow_pairs(kdop_scene* s, int64_t need) {
+  if (need <= s->pairs_cap) return KDOP_OK;
   // one block: the seed pass's entries, the pairs, their order.  The pairs are
   // carried over: the last results' meshes are read from them until the next
-  // list is there.
-  const int64_t seeds = kdop::seed_entries(s->ctx->sm_count, n) * (int64_t)sizeof(uint4);
-  const int64_t bytes = seeds + n * (int64_t)(sizeof(uint2) + sizeof(uint32_t));
+  // list is there.  A list longer than the scene was made for gets room for the
+  // next ones, so that one that grows from step to step does not take a new
+  // block (up to 29 MB) every step: 20 to 120 pairs of 162 tets 763 -> 117 us a
+  // step.
+  int64_t n = s->pairs_cap > 0 ? need + need / 4 + 16 : need, seeds, bytes;
   char* lists = nullptr;
-  KDOP_CUDA(s->ctx, dalloc(s, &lists, bytes));
+  for (;; n = need) {
+    seeds = kdop::seed_entries(s->ctx->sm_count, n) * (int64_t)sizeof(uint4);
+    bytes = seeds + n * (int64_t)(sizeof(uint2) + sizeof(uint32_t));
+    const cudaError_t e = dalloc(s, &lists, bytes);
+    if (e == cudaSuccess) break;
+    if (n == need) return cuda_fail(s->ctx, e, "pair list alloc");
+    cudaGetLastError();
+  }
   uint2* pairs = reinterpret_cast<uint2*>(lists + seeds);
   cudaError_t e = cudaSuccess;
   if (s->pairs_cap > 0)

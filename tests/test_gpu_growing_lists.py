@@ -1,0 +1,34 @@
+"""Steps whose lists grow a little each time take new device memory only now and
+then, and give what a scene made for the last list gives."""
+import numpy as np
+import pytest
+
+import kdop_b200 as kd
+from conftest import sorted_rows
+from kdop_b200 import scenes
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("bodies, first, steps", [(2, 1, 40), (20, 20, 100), (40, 250, 40)])
+def test_pair_list_grows_by_one(ctx, bodies, first, steps):
+    sc = scenes.config5(n_pairs=bodies // 2, n=3)
+    rng = np.random.default_rng(bodies)
+    pairs = rng.integers(0, bodies, (first + steps, 2)).astype(np.uint32)
+    ds = kd.DeviceScene(ctx, sc.K, sc.meshes)
+    ds.set_poses(sc.quat, sc.pos)
+    ds.refit(kd.REFIT_POSE)
+    ds.traverse_sync(pairs[:first])
+    held = set()
+    for n in range(first + 1, first + steps + 1):
+        st = ds.traverse_sync(pairs[:n])
+        held.add(ds.info()["device_bytes"])
+    # a block holds a quarter and 16 pairs more than the list it was made for
+    assert len(held) <= 6
+    other = kd.DeviceScene(ctx, sc.K, sc.meshes)
+    other.set_poses(sc.quat, sc.pos)
+    other.refit(kd.REFIT_POSE)
+    assert other.traverse_sync(pairs).n_tests == st.n_tests
+    assert np.array_equal(sorted_rows(ds.candidates()), sorted_rows(other.candidates()))
+    ds.close()
+    other.close()
