@@ -140,6 +140,14 @@ static float* read_stage(kdop_scene* s, int64_t words, int64_t* window, cudaErro
   }
 }
 
+// Whether the scene's stream is being captured into a graph of the caller's.
+static bool capturing(kdop_scene* s) {
+  cudaStreamCaptureStatus c = cudaStreamCaptureStatusNone;
+  if (cudaStreamIsCapturing(s->ctx->stream, &c) == cudaSuccess) return c != cudaStreamCaptureStatusNone;
+  cudaGetLastError();
+  return false;
+}
+
 // The control block's host copy holds what the device's does until the next
 // call that enqueues a change of it (a traversal, contacts, a graph step, a
 // sort): the counters are copied once per change, not once per call that reads
@@ -148,11 +156,7 @@ static float* read_stage(kdop_scene* s, int64_t words, int64_t* window, cudaErro
 // call, so a scene that was ever captured into a caller's graph always copies.
 static void ctl_changes(kdop_scene* s) {
   s->ctl_fresh = false;
-  cudaStreamCaptureStatus c = cudaStreamCaptureStatusNone;
-  if (cudaStreamIsCapturing(s->ctx->stream, &c) != cudaSuccess)
-    cudaGetLastError();
-  else if (c != cudaStreamCaptureStatusNone)
-    s->ctl_replayed = true;
+  if (capturing(s)) s->ctl_replayed = true;
 }
 // Synchronises and brings ctl_host up to date.
 static cudaError_t read_ctl(kdop_scene* s) {
@@ -379,10 +383,19 @@ static int grow_pairs(kdop_scene* s, int64_t need) {
   }
   uint2* pairs = reinterpret_cast<uint2*>(lists + seeds);
   cudaError_t e = cudaSuccess;
-  if (s->pairs_cap > 0)
+  if (capturing(s)) {
+    // nothing runs on the scene's stream now: valid mesh indices instead, for
+    // reads before the captured traversal has run
+    cudaStream_t side = nullptr;
+    e = cudaStreamCreateWithFlags(&side, cudaStreamNonBlocking);
+    if (e == cudaSuccess) e = cudaMemsetAsync(pairs, 0, (size_t)n * sizeof(uint2), side);
+    if (e == cudaSuccess) e = cudaStreamSynchronize(side);
+    if (side) cudaStreamDestroy(side);
+  } else if (s->pairs_cap > 0) {
     e = cudaMemcpyAsync(pairs, s->pairs, (size_t)s->pairs_cap * sizeof(uint2), cudaMemcpyDeviceToDevice,
                         s->ctx->stream);
-  if (e == cudaSuccess && s->pairs_cap > 0) e = cudaStreamSynchronize(s->ctx->stream);
+    if (e == cudaSuccess) e = cudaStreamSynchronize(s->ctx->stream);
+  }
   if (e != cudaSuccess) {
     dfree(s, &lists, bytes);
     return cuda_fail(s->ctx, e, "pair list copy");

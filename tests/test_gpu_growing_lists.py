@@ -7,6 +7,7 @@ import kdop_b200 as kd
 from conftest import sorted_rows
 from kdop_b200 import scenes
 
+torch = pytest.importorskip("torch")
 pytestmark = pytest.mark.gpu
 
 
@@ -32,3 +33,28 @@ def test_pair_list_grows_by_one(ctx, bodies, first, steps):
     assert np.array_equal(sorted_rows(ds.candidates()), sorted_rows(other.candidates()))
     ds.close()
     other.close()
+
+
+@pytest.mark.parametrize("n_pairs", [21, 200, 300])
+def test_longer_list_inside_a_callers_capture(n_pairs):
+    stream = torch.cuda.Stream()
+    ctx = kd.Context(0, stream=stream.cuda_stream)
+    sc = scenes.config5(n_pairs=10, n=3)
+    rng = np.random.default_rng(n_pairs)
+    pairs = rng.integers(0, 20, (n_pairs, 2)).astype(np.uint32)
+    ds = kd.DeviceScene(ctx, sc.K, sc.meshes)
+    ds.set_poses(sc.quat, sc.pos)
+    ds.refit(kd.REFIT_POSE)
+    ds.traverse_sync(pairs[:20])
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph, stream=stream, capture_error_mode="relaxed"):
+        ds.traverse(pairs)
+    ds.candidates()  # of the traversal before, the list already the next one's: any rows, no fault
+    with torch.cuda.stream(stream):
+        graph.replay()
+    other = kd.DeviceScene(ctx, sc.K, sc.meshes)
+    other.set_poses(sc.quat, sc.pos)
+    other.refit(kd.REFIT_POSE)
+    assert ds.stats().n_tests == other.traverse_sync(pairs).n_tests
+    assert np.array_equal(sorted_rows(ds.candidates()), sorted_rows(other.candidates()))
+    del graph
