@@ -382,19 +382,17 @@ static int grow_pairs(kdop_scene* s, int64_t need) {
     cudaGetLastError();
   }
   uint2* pairs = reinterpret_cast<uint2*>(lists + seeds);
-  cudaError_t e = cudaSuccess;
-  if (capturing(s)) {
-    // nothing runs on the scene's stream now: valid mesh indices instead, for
-    // reads before the captured traversal has run
-    cudaStream_t side = nullptr;
-    e = cudaStreamCreateWithFlags(&side, cudaStreamNonBlocking);
-    if (e == cudaSuccess) e = cudaMemsetAsync(pairs, 0, (size_t)n * sizeof(uint2), side);
-    if (e == cudaSuccess) e = cudaStreamSynchronize(side);
-    if (side) cudaStreamDestroy(side);
-  } else if (s->pairs_cap > 0) {
-    e = cudaMemcpyAsync(pairs, s->pairs, (size_t)s->pairs_cap * sizeof(uint2), cudaMemcpyDeviceToDevice,
-                        s->ctx->stream);
-    if (e == cudaSuccess) e = cudaStreamSynchronize(s->ctx->stream);
+  // every place holds valid mesh indices at any time; nothing runs on the
+  // scene's stream while it is being captured
+  cudaStream_t st = s->ctx->stream;
+  const bool side = capturing(s);
+  cudaError_t e = side ? cudaStreamCreateWithFlags(&st, cudaStreamNonBlocking) : cudaSuccess;
+  if (e == cudaSuccess) {
+    e = cudaMemsetAsync(pairs, 0, (size_t)n * sizeof(uint2), st);
+    if (e == cudaSuccess && !side && s->pairs_cap > 0)
+      e = cudaMemcpyAsync(pairs, s->pairs, (size_t)s->pairs_cap * sizeof(uint2), cudaMemcpyDeviceToDevice, st);
+    if (e == cudaSuccess && (side || s->pairs_cap > 0)) e = cudaStreamSynchronize(st);
+    if (side) cudaStreamDestroy(st);
   }
   if (e != cudaSuccess) {
     dfree(s, &lists, bytes);

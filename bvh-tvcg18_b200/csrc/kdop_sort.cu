@@ -223,7 +223,8 @@ struct CandGen {
 };
 // The same order in two sorts, least significant first, for keys wider than 64
 // bits and for results whose pair list the scene no longer holds: tets by their
-// global numbers, then pair indices.
+// global numbers, then pair indices (also where a replayed graph of the caller's
+// may have put another list there).
 struct TetGen {
   const uint32_t *cA, *cB;
   int tb;
@@ -351,9 +352,12 @@ __global__ void __launch_bounds__(256) contact_gather_kernel(int64_t n, const in
 
 cudaError_t launch_candidate_rows(kdop_scene* s, int64_t first, int64_t n, uint32_t* rows) {
   const uint32_t* c = s->cand + first;
-  // the results' pair indices run over the list on the device, which is as long
+  // the results' pair indices run over the list on the device, which is as long;
+  // the library knows no more than its room when a replayed graph of the
+  // caller's may have put another one there
+  const int64_t n_pairs = s->ctl_replayed ? s->pairs_cap : s->result_pairs;
   candidate_rows_kernel<<<(unsigned)((n + 255) / 256), 256, 0, s->ctx->stream>>>(
-      c, c + s->cand_cap, c + 2 * s->cand_cap, s->pairs, (uint32_t)s->result_pairs, s->t_off_dev, n, rows);
+      c, c + s->cand_cap, c + 2 * s->cand_cap, s->pairs, (uint32_t)n_pairs, s->t_off_dev, n, rows);
   s->ctx->launches++;
   return cudaGetLastError();
 }
@@ -398,7 +402,7 @@ cudaError_t sort_results(kdop_scene* s, int64_t n, int64_t n_contacts, void* wor
   const WaitLimit lim(&s->ctl->error, s->ctx->wait_ns);
   CandGen gen{s->cand, s->cand + s->cand_cap, s->cand + 2 * s->cand_cap, s->pairs, s->t_off_dev, bits_of(std::max<int64_t>(s->most_tets, 1) - 1)};
   const int pair_bits = bits_of((uint64_t)std::max<int64_t>(s->result_pairs, 1) - 1);
-  const bool packed = s->pairs_current && pair_bits + 2 * gen.tb <= 64;
+  const bool packed = s->pairs_current && !s->ctl_replayed && pair_bits + 2 * gen.tb <= 64;
   cudaError_t e;
   if (packed) {
     e = radix_sort(s->ctx, gen, n, pair_bits + 2 * gen.tb, b, w + L.scratch, lim);

@@ -58,3 +58,35 @@ def test_longer_list_inside_a_callers_capture(n_pairs):
     assert ds.stats().n_tests == other.traverse_sync(pairs).n_tests
     assert np.array_equal(sorted_rows(ds.candidates()), sorted_rows(other.candidates()))
     del graph
+
+
+@pytest.mark.parametrize("n_pairs, between", [(300, 10), (40, 400)])
+def test_replay_of_a_list_after_another(n_pairs, between):
+    """The results are those of the graph's list, whatever list a call had in between."""
+    stream = torch.cuda.Stream()
+    ctx = kd.Context(0, stream=stream.cuda_stream)
+    sc = scenes.config5(n_pairs=10, n=3)
+    rng = np.random.default_rng(n_pairs)
+    pairs = rng.integers(0, 20, (n_pairs, 2)).astype(np.uint32)
+    ds = kd.DeviceScene(ctx, sc.K, sc.meshes)
+    ds.set_poses(sc.quat, sc.pos)
+    ds.refit(kd.REFIT_POSE)
+    ds.traverse_sync(rng.integers(0, 20, (max(n_pairs, between), 2)).astype(np.uint32))
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph, stream=stream, capture_error_mode="relaxed"):
+        ds.traverse(pairs)
+        ds.contacts()
+    ds.traverse_sync(rng.integers(0, 20, (between, 2)).astype(np.uint32), contacts=True)
+    with torch.cuda.stream(stream):
+        graph.replay()
+    other = kd.DeviceScene(ctx, sc.K, sc.meshes)
+    other.set_poses(sc.quat, sc.pos)
+    other.refit(kd.REFIT_POSE)
+    other.traverse_sync(pairs, contacts=True)
+    for scene in (ds, other):
+        scene.sort_results()
+    assert np.array_equal(ds.candidates(), other.candidates())
+    assert ds.read_contacts().tobytes() == other.read_contacts().tobytes()
+    for got, want in zip(ds.reduce_contacts(), other.reduce_contacts()):
+        assert got.tobytes() == want.tobytes()
+    del graph
