@@ -132,8 +132,16 @@ static float* stage(kdop_scene* s, int64_t nfloats, cudaError_t* err) {
 // through that one, so a read-back leaves it where it is.  Fewer items at a
 // time where the device has no room for them (`window` says how many).
 static float* read_stage(kdop_scene* s, int64_t words, int64_t* window, cudaError_t* err) {
+  kdop_scene_ext* x = ext(s);
+  // results that grow from step to step do not take a new buffer every step
+  const int64_t need = words * *window;
+  if (x->read_n > 0 && x->read_n < need) {
+    float* d = grow_stage(s, &x->read_stage, &x->read_n, need + need / 4, err);
+    if (d) return d;
+    cudaGetLastError();
+  }
   for (;;) {
-    float* d = grow_stage(s, &ext(s)->read_stage, &ext(s)->read_n, words * *window, err);
+    float* d = grow_stage(s, &x->read_stage, &x->read_n, words * *window, err);
     if (d || *err != cudaErrorMemoryAllocation || *window <= kReadLeast) return d;
     cudaGetLastError();
     *window = std::max((*window + 1) / 2, kReadLeast);

@@ -90,3 +90,22 @@ def test_replay_of_a_list_after_another(n_pairs, between):
     for got, want in zip(ds.reduce_contacts(), other.reduce_contacts()):
         assert got.tobytes() == want.tobytes()
     del graph
+
+
+def test_candidates_grow_from_step_to_step(ctx):
+    sc = scenes.touching_pair(n=8, seed=0, K=14)
+    ds = kd.DeviceScene(ctx, sc.K, sc.meshes)
+    axis = sc.pos[1] - sc.pos[0]
+    held, counts = set(), []
+    for k in range(60):
+        pos = sc.pos.copy()
+        pos[1] -= np.float32(0.01 * k) * axis
+        ds.set_poses(sc.quat, pos)
+        ds.refit(kd.REFIT_POSE)
+        ds.traverse_sync(sc.pairs)
+        counts.append(len(ds.candidates()))
+        held.add(ds.info()["device_bytes"])
+    assert counts[-1] > 2 * counts[0] and len(set(counts)) > 30
+    # a quarter more room each time it runs out
+    assert len(held) <= 3 + np.log(max(counts) / min(counts)) / np.log(1.25)
+    ds.close()
