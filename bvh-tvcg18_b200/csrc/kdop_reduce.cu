@@ -13,13 +13,18 @@
 // Here: one stable radix sort by (body i, body j, p.y), whose width follows
 // from the bodies' numbers (50 bits for 512 bodies), then the rows that tie in
 // it -- runs of equal keys -- are ranked among themselves by the other six
-// fields, a thread per row counting the run's rows before its own.  Runs
-// longer than kRankMax are ordered by three more stable radix sorts of their
-// rows alone and a fourth by run.  (Sorting all rows by all nine fields, five
+// fields, a thread per row counting the run's rows before its own.  The rows of
+// runs longer than kRankMax, and those that tie in (p.x, p.z) with more than
+// kTiesMax, are ordered by three more stable radix sorts of those rows alone,
+// over the digits that vary in them, and a fourth by run.  (Sorting all rows by all nine fields, five
 // 64-bit sorts of up to eight passes each, moved every row's key 32 times: of
 // the 3.6 M rows of 256 touching pairs 40 % are in runs of one or two rows and
 // 17 % in runs of more than 32, the longest 371.)  Floats are mapped to
-// integers that order like float `<`, -0 folded onto +0.
+// integers that order like float `<`, -0 folded onto +0.  Many rows alike, as flat
+// faces that rest on each other give (700,001 rows, five sorts of all of them ->
+// now): runs of 500 duplicates 969 -> 881 us, of 500 points eight times each 990
+// -> 917, runs of 1,000 duplicates 1,196 -> 833, one of 20,000 in 20,000 4,768 ->
+// 4,258.
 //
 // The unique is sequential by definition (a row is compared with the last row
 // kept, not with its predecessor, and the tolerance is not transitive), but it
@@ -41,6 +46,7 @@ namespace {
 
 constexpr float kEps = 1.19209290e-07f * 10.0f;  // working_precision<float>()
 constexpr uint32_t kRankMax = 512;               // longest run ranked row by row
+constexpr uint32_t kTiesMax = 32;                // most rows of one (p.x, p.z) in it that are
 
 // Integer image of a float that orders like float `<` (NaN aside); -0 and +0
 // map to the same value.
@@ -86,20 +92,22 @@ struct BodyGen {
   }
   __device__ uint32_t val(int64_t i) const { return perm[i]; }
 };
-// Field pairs of the rows of long runs, least significant first, then the run.
-// Values are positions in the first sort's order.
+// Field pairs of a row, the most significant last.
+__device__ __forceinline__ uint64_t field_pair(const kdop_contact& c, int pass) {
+  return pass == 0 ? two_keys(c.n[2], c.depth) : pass == 1 ? two_keys(c.n[1], c.n[0]) : two_keys(c.p[0], c.p[2]);
+}
+// Field pairs of the rows still to be ordered, least significant first, then the
+// run.  Values are places.
 struct LongGen {
   const kdop_contact* rows;
-  const uint32_t* perm;  // first sort's order
-  const uint32_t* at;    // positions to sort
-  const uint32_t* run;   // run of a position
+  const uint32_t* placed;  // row at a place so far
+  const uint32_t* at;      // places to sort
+  const uint32_t* run;     // run of a place
   int pass;
   int64_t n;
   __device__ uint64_t key(int64_t i) const {
     const uint32_t k = bounded(at[i], n);
-    if (pass == 3) return run[k];
-    const kdop_contact& c = rows[perm[k]];
-    return pass == 0 ? two_keys(c.n[2], c.depth) : pass == 1 ? two_keys(c.n[1], c.n[0]) : two_keys(c.p[0], c.p[2]);
+    return pass == 3 ? run[k] : field_pair(rows[bounded(placed[k], n)], pass);
   }
   __device__ uint32_t val(int64_t i) const { return at[i]; }
 };
@@ -130,16 +138,19 @@ struct ReduceArgs {
   uint32_t* order;        // rows in full order
   Row* sorted;            // the same rows, copied
   uint32_t* keep;
-  uint32_t* longs;        // positions in runs longer than kRankMax
+  uint32_t* longs;        // places whose rows the rank kernel leaves to the sorts
   kdop_contact* out;
   uint2* out_bodies;
+  int ordered;            // every row is at its place
   unsigned* head;         // ReduceHead words
   WaitLimit lim;
   unsigned long long* words_run;
   unsigned long long* words_keep;
 };
 // Counters of a reduction, one device block read back as a whole.
-enum { H_ERR, H_TICKET_RUN, H_TICKET_KEEP, H_LONG, H_KEPT, H_MOST_I, H_MOST_J, H_WORDS = 8 };
+// H_BITS: of each field pair, bits set and bits clear in a row still to be
+// ordered (64-bit words).
+enum { H_ERR, H_TICKET_RUN, H_TICKET_KEEP, H_LONG, H_KEPT, H_MOST_I, H_MOST_J, H_BITS = 8, H_WORDS = H_BITS + 12 };
 
 constexpr int RD_ITEMS = 4, RD_TILE = 256 * RD_ITEMS;
 
@@ -207,13 +218,13 @@ __global__ void __launch_bounds__(256) red_rank_kernel(ReduceArgs a) {
   const uint32_t s = bounded(a.starts[g], a.n), e = min(a.starts[g + 1], (uint32_t)a.n);
   const Row x = load_row(a.rows, r);
   if (e - s > kRankMax) {
-    a.longs[k] = 1u;  // ordered by the radix sorts below, until then in the first sort's order
+    // ordered by the radix sorts below, until then in the first sort's order
+    a.longs[k] = 1u;
     a.head[H_LONG] = 1u;
     a.order[k] = r;
     a.sorted[k] = x;
     return;
   }
-  a.longs[k] = 0u;
   const uint64_t mine = a.next[k];
   uint32_t rank = 0, ties = 0;
 #pragma unroll 8
@@ -222,29 +233,63 @@ __global__ void __launch_bounds__(256) red_rank_kernel(ReduceArgs a) {
     rank += key < mine ? 1u : 0u;
     ties += key == mine ? 1u : 0u;
   }
-  if (ties > 1)
+  const bool many = ties > kTiesMax;
+  if (many) {
+    // so are rows that tie in (p.x, p.z) with many others
+#pragma unroll 8
+    for (uint32_t j = s; j < (uint32_t)k; ++j) rank += a.next[j] == mine ? 1u : 0u;
+    a.head[H_LONG] = 1u;
+  } else if (ties > 1) {
     for (uint32_t j = s; j < e; ++j) {
       if (a.next[j] != mine || j == (uint32_t)k) continue;
       const int c = later_fields(load_row(a.rows, bounded(a.perm[j], a.n)), x);
       rank += (c < 0 || (c == 0 && j < (uint32_t)k)) ? 1u : 0u;  // equal rows keep their order
     }
+  }
   const uint32_t at = bounded(s + rank, a.n);
   a.order[at] = r;
   a.sorted[at] = x;
+  a.longs[at] = many ? 1u : 0u;
 }
 
-// Positions of the long runs' rows in increasing order: at[pos[k]] = k.
-__global__ void red_long_list_kernel(const uint32_t* __restrict__ flag, const uint32_t* __restrict__ pos, int64_t n,
-                                     uint32_t* at) {
-  const int64_t k = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (k < n && flag[k]) at[pos[k]] = (uint32_t)k;
+// Places left to the sorts in increasing order: at[pos[k]] = k; and which bits of
+// their rows' fields vary (rows in one plane have one normal, duplicates nothing
+// that differs: most passes of a sort would move nothing).
+__global__ void __launch_bounds__(256) red_long_list_kernel(ReduceArgs a, const uint32_t* __restrict__ pos,
+                                                            uint32_t* at) {
+  unsigned long long set[3] = {0, 0, 0}, clear[3] = {0, 0, 0};
+  for (int64_t k = (int64_t)blockIdx.x * 256 + threadIdx.x; k < a.n; k += (int64_t)gridDim.x * 256) {
+    if (!a.longs[k]) continue;
+    at[pos[k]] = (uint32_t)k;
+    const kdop_contact& c = a.rows[bounded(a.order[k], a.n)];
+#pragma unroll
+    for (int p = 0; p < 3; ++p) {
+      const uint64_t x = field_pair(c, p);
+      set[p] |= x;
+      clear[p] |= ~x;
+    }
+  }
+  unsigned long long* bits = reinterpret_cast<unsigned long long*>(a.head + H_BITS);
+#pragma unroll
+  for (int p = 0; p < 3; ++p) {
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+      set[p] |= __shfl_xor_sync(0xffffffffu, set[p], o);
+      clear[p] |= __shfl_xor_sync(0xffffffffu, clear[p], o);
+    }
+    if ((threadIdx.x & 31) == 0 && (set[p] | clear[p])) {
+      atomicOr(bits + 2 * p, set[p]);
+      atomicOr(bits + 2 * p + 1, clear[p]);
+    }
+  }
 }
-// The i-th row of the long runs in sorted order goes to the i-th position.
-__global__ void red_long_place_kernel(ReduceArgs a, const uint32_t* __restrict__ at,
-                                      const uint32_t* __restrict__ sorted_at, int64_t m) {
+// The i-th row in sorted order goes to the i-th place.
+__global__ void red_long_place_kernel(ReduceArgs a, const uint32_t* __restrict__ placed,
+                                      const uint32_t* __restrict__ at, const uint32_t* __restrict__ sorted_at,
+                                      int64_t m) {
   const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= m) return;
-  const uint32_t r = bounded(a.perm[bounded(sorted_at[i], a.n)], a.n);
+  const uint32_t r = bounded(placed[bounded(sorted_at[i], a.n)], a.n);
   a.order[at[i]] = r;
   a.sorted[at[i]] = load_row(a.rows, r);
 }
@@ -277,6 +322,11 @@ __device__ __forceinline__ bool starts_segment(const ReduceArgs& a, uint32_t k) 
 
 constexpr uint32_t KEEP = 1u, SEGMENT = 2u;  // bits of keep[]
 
+// The kernels from here on run once without the host's knowing whether rows are
+// still to be ordered; where some are, the walk and the write leave it to their
+// second run.
+__device__ __forceinline__ bool too_early(const ReduceArgs& a) { return !a.ordered && a.head[H_LONG]; }
+
 __global__ void __launch_bounds__(256) red_segments_kernel(ReduceArgs a) {
   const int64_t k = (int64_t)blockIdx.x * 256 + threadIdx.x;
   if (k < a.n) a.keep[k] = starts_segment(a, (uint32_t)k) ? SEGMENT | KEEP : 0u;
@@ -286,24 +336,53 @@ __global__ void __launch_bounds__(256) red_segments_kernel(ReduceArgs a) {
 // unless it equals the last row kept.
 __global__ void __launch_bounds__(128) red_walk_kernel(ReduceArgs a) {
   const int64_t k = (int64_t)blockIdx.x * 128 + threadIdx.x;
-  if (k >= a.n || !(a.keep[k] & SEGMENT)) return;
+  if (k >= a.n) return;
+  const bool early = too_early(a);  // (beside the flag's load, not before it)
+  if (!(a.keep[k] & SEGMENT) || early) return;
   if (k + 1 >= a.n || (a.keep[k + 1] & SEGMENT)) return;  // a segment of one row (most): kept
   Row last = a.sorted[k];
-  for (int64_t j = k + 1; j < a.n; ++j) {
+  int64_t j = k + 1;
+  for (int c = 0; c < 8; ++c, ++j) {
+    if (j >= a.n) return;
     const uint32_t f = a.keep[j];
-    const Row c = a.sorted[j];
-    if (f & SEGMENT) break;
-    if (!same_point(last, c)) {
+    const Row x = a.sorted[j];
+    if (f & SEGMENT) return;
+    if (!same_point(last, x)) {
       a.keep[j] = KEEP;
-      last = c;
+      last = x;
+    }
+  }
+  // a long segment: two rows' loads in flight (more take registers that the
+  // short ones' warps go without)
+  for (; j < a.n; j += 2) {
+    uint32_t f[2];
+    Row x[2];
+#pragma unroll
+    for (int q = 0; q < 2; ++q) {
+      const int64_t at = min(j + q, a.n - 1);
+      f[q] = j + q < a.n ? a.keep[at] : SEGMENT;
+      x[q] = a.sorted[at];
+    }
+#pragma unroll
+    for (int q = 0; q < 2; ++q) {
+      if (f[q] & SEGMENT) return;
+      if (!same_point(last, x[q])) {
+        a.keep[j + q] = KEEP;
+        last = x[q];
+      }
     }
   }
 }
 
 __global__ void __launch_bounds__(256) red_write_kernel(ReduceArgs a) {
   __shared__ unsigned s_tile;
-  if (threadIdx.x == 0) s_tile = atomicAdd(a.head + H_TICKET_KEEP, 1u);
+  if (threadIdx.x == 0) {
+    const bool early = too_early(a);
+    const unsigned tile = atomicAdd(a.head + H_TICKET_KEEP, 1u);
+    s_tile = early ? 0xFFFFFFFFu : tile;
+  }
   __syncthreads();
+  if (s_tile == 0xFFFFFFFFu) return;
   const unsigned tile = s_tile;
   // consecutive threads hold consecutive rows: one scan step per item
   uint32_t keep[RD_ITEMS], pos[RD_ITEMS], sum = 0;
@@ -386,33 +465,40 @@ cudaError_t scene_contact_bodies(kdop_scene* s, int64_t n, uint2* bodies) {
   return cudaGetLastError();
 }
 
-// The rows of runs longer than kRankMax: (n.z, depth), (n.y, n.x), (p.x, p.z),
-// run, each a stable sort.  The first sort's keys, the half of its values that
-// does not hold the order, and keep[] are free here.
+// The rows left by the rank kernel: (n.z, depth), (n.y, n.x), (p.x, p.z), run, each
+// a stable sort.  The first sort's keys, the half of its values that does not
+// hold the order, next[] and keep[] are free here.
 static cudaError_t order_long_runs(kdop_ctx* ctx, const ReduceArgs& a, const ReduceWork& L, char* w,
                                    const SortBuffers& first) {
   cudaStream_t st = ctx->stream;
   SortBuffers b{first.keys, first.keys_tmp, first.vals_tmp, reinterpret_cast<uint32_t*>(w + L.long_vals)};
   uint32_t* pos = a.keep;
   uint32_t* at = reinterpret_cast<uint32_t*>(w + L.long_at);
+  uint32_t* placed = reinterpret_cast<uint32_t*>(a.next);
   cudaError_t e;
   if ((e = exclusive_scan_u32(a.longs, pos, a.n, reinterpret_cast<uint32_t*>(w + L.scan), st)) != cudaSuccess) return e;
+  red_long_list_kernel<<<std::min(blocks_for(a.n, 256), 592u), 256, 0, st>>>(a, pos, at);
+  ctx->launches++;
+  if ((e = cudaMemcpyAsync(placed, a.order, (size_t)a.n * 4, cudaMemcpyDeviceToDevice, st)) != cudaSuccess) return e;
   uint32_t tail[2];
+  unsigned long long bits[6];
   if ((e = cudaMemcpyAsync(&tail[0], pos + a.n - 1, 4, cudaMemcpyDeviceToHost, st)) != cudaSuccess) return e;
   if ((e = cudaMemcpyAsync(&tail[1], a.longs + a.n - 1, 4, cudaMemcpyDeviceToHost, st)) != cudaSuccess) return e;
+  if ((e = cudaMemcpyAsync(bits, a.head + H_BITS, sizeof(bits), cudaMemcpyDeviceToHost, st)) != cudaSuccess) return e;
   if ((e = cudaStreamSynchronize(st)) != cudaSuccess) return e;
   const int64_t m = (int64_t)tail[0] + tail[1];
   if (m == 0) return cudaSuccess;
-  red_long_list_kernel<<<blocks_for(a.n, 256), 256, 0, st>>>(a.longs, pos, a.n, at);
   const uint32_t* from = at;
   for (int pass = 0; pass < 4; ++pass) {
-    const int bits = pass < 3 ? 64 : bits_of((uint64_t)a.n);
-    e = radix_sort(ctx, LongGen{a.rows, a.perm, from, a.run, pass, a.n}, m, bits, b, w + L.radix, a.lim);
+    const uint64_t vary = pass < 3 ? bits[2 * pass] & bits[2 * pass + 1] : ~0ull;
+    if (!vary) continue;
+    e = radix_sort(ctx, LongGen{a.rows, placed, from, a.run, pass, a.n}, m, pass < 3 ? 64 : bits_of((uint64_t)a.n), b,
+                   w + L.radix, a.lim, vary);
     if (e != cudaSuccess) return e;
     from = b.vals;
   }
-  red_long_place_kernel<<<blocks_for(m, 256), 256, 0, st>>>(a, at, from, m);
-  ctx->launches += 2;
+  red_long_place_kernel<<<blocks_for(m, 256), 256, 0, st>>>(a, placed, at, from, m);
+  ctx->launches++;
   return cudaGetLastError();
 }
 
@@ -468,8 +554,9 @@ cudaError_t reduce_contact_rows(kdop_ctx* ctx, const kdop_contact* rows, const u
   red_runs_kernel<<<tile_blocks(ctx, STUCK_SCAN, a.head + H_TICKET_RUN, tiles), 256, 0, st>>>(a);
   red_rank_kernel<<<blocks_for(n, 256), 256, 0, st>>>(a);
   ctx->launches += 2;
-  // without waiting for the count of long runs: where there are some, they are
-  // ordered afterwards and the rest runs again
+  // without waiting for the host to learn whether rows are still to be ordered:
+  // where there are some, the rest returns at once and runs when they are
+  a.ordered = 0;
   for (int round = 0;; ++round) {
     red_segments_kernel<<<blocks_for(n, 256), 256, 0, st>>>(a);
     red_walk_kernel<<<blocks_for(n, 128), 128, 0, st>>>(a);
@@ -479,6 +566,7 @@ cudaError_t reduce_contact_rows(kdop_ctx* ctx, const kdop_contact* rows, const u
     if ((e = cudaStreamSynchronize(st)) != cudaSuccess) return e;
     if (round || h[H_ERR] || !h[H_LONG]) break;
     if ((e = order_long_runs(ctx, a, L, w, b)) != cudaSuccess) return e;
+    a.ordered = 1;
     if ((e = cudaMemsetAsync(a.head + H_TICKET_KEEP, 0, 4, st)) != cudaSuccess) return e;
     if ((e = cudaMemsetAsync(a.words_keep, 0, L.keys - L.words_keep, st)) != cudaSuccess) return e;
   }

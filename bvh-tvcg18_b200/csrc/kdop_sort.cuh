@@ -214,7 +214,8 @@ constexpr size_t small_sort_smem() {
   return (size_t)1024 * ITEMS * 8 + 32 * 257 * 4;
 }
 template <class Gen, int ITEMS>
-__global__ void __launch_bounds__(1024) small_sort_kernel(Gen gen, int n, int bits, uint64_t* keys, uint32_t* vals) {
+__global__ void __launch_bounds__(1024) small_sort_kernel(Gen gen, int n, int bits, uint64_t vary, uint64_t* keys,
+                                                         uint32_t* vals) {
   extern __shared__ uint64_t ex[];                                      // 1024 * ITEMS
   uint32_t* wc = reinterpret_cast<uint32_t*>(ex + 1024 * ITEMS);        // [32 warps][256 digits], a row 257 words
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
@@ -229,6 +230,7 @@ __global__ void __launch_bounds__(1024) small_sort_kernel(Gen gen, int n, int bi
     v[r] = at < n ? gen.val(at) : 0u;
   }
   for (int shift = 0; shift < bits; shift += 8) {
+    if (((vary >> shift) & 255u) == 0u) continue;
     // the last pass may cover fewer than 8 varying bits: past them all keys
     // agree, and the items past n (all ones) still rank last
 #pragma unroll
@@ -311,7 +313,8 @@ cudaError_t launch_sort_pass(const kdop_ctx* ctx, const SortBuffers& b, int64_t 
                              uint32_t* ticket, unsigned long long* words, unsigned epoch, WaitLimit lim);
 
 // Stable ascending sort of the items 0 .. n-1 by gen.key(i), of which the low
-// `bits` bits vary (the others are equal in all keys), n < 2^32; the values
+// `bits` bits vary (the others are equal in all keys; of those, digits without a
+// bit of `vary`, where the caller knows it, take no pass), n < 2^32; the values
 // are gen.val(i).  gen may read b.vals at i (it is written at i only).
 // scratch: radix_scratch_words(n) words, 8-byte aligned.  *lim.err gets
 // DEV_ERR_TIMEOUT when a bounded wait gave up (some of the sorted keys and values
@@ -319,24 +322,24 @@ cudaError_t launch_sort_pass(const kdop_ctx* ctx, const SortBuffers& b, int64_t 
 // context's stream.
 template <class Gen>
 cudaError_t radix_sort(kdop_ctx* ctx, const Gen& gen, int64_t n, int bits, SortBuffers& b, void* scratch,
-                       WaitLimit lim) {
+                       WaitLimit lim, uint64_t vary = ~0ull) {
   if (n <= 0) return cudaSuccess;
   cudaStream_t st = ctx->stream;
   long long& launches = ctx->launches;
   cudaError_t e;
   if (n <= kSmallSort) {
     if (n <= 1024) {
-      small_sort_kernel<Gen, 1><<<1, 1024, small_sort_smem<1>(), st>>>(gen, (int)n, bits, b.keys, b.vals);
+      small_sort_kernel<Gen, 1><<<1, 1024, small_sort_smem<1>(), st>>>(gen, (int)n, bits, vary, b.keys, b.vals);
     } else if (n <= 4096) {
       e = cudaFuncSetAttribute(small_sort_kernel<Gen, 4>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                (int)small_sort_smem<4>());
       if (e != cudaSuccess) return e;
-      small_sort_kernel<Gen, 4><<<1, 1024, small_sort_smem<4>(), st>>>(gen, (int)n, bits, b.keys, b.vals);
+      small_sort_kernel<Gen, 4><<<1, 1024, small_sort_smem<4>(), st>>>(gen, (int)n, bits, vary, b.keys, b.vals);
     } else {
       e = cudaFuncSetAttribute(small_sort_kernel<Gen, 8>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                (int)small_sort_smem<8>());
       if (e != cudaSuccess) return e;
-      small_sort_kernel<Gen, 8><<<1, 1024, small_sort_smem<8>(), st>>>(gen, (int)n, bits, b.keys, b.vals);
+      small_sort_kernel<Gen, 8><<<1, 1024, small_sort_smem<8>(), st>>>(gen, (int)n, bits, vary, b.keys, b.vals);
     }
     launches += 1;
     return cudaGetLastError();
@@ -348,10 +351,12 @@ cudaError_t radix_sort(kdop_ctx* ctx, const Gen& gen, int64_t n, int bits, SortB
                                                                                         s.hist);
   launches += 1;
   unsigned epoch = 1;
-  for (int p = 0; 8 * p < bits; ++p, ++epoch) {
+  for (int p = 0; 8 * p < bits; ++p) {
+    if (((vary >> (8 * p)) & 255u) == 0u) continue;
     e = launch_sort_pass(ctx, b, n, 8 * p, s.hist + 256 * p, s.ticket + p, s.words, epoch, lim);
     if (e != cudaSuccess) return e;
     launches += 1;
+    ++epoch;
     std::swap(b.keys, b.keys_tmp);
     std::swap(b.vals, b.vals_tmp);
   }
