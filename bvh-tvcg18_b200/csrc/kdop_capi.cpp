@@ -23,6 +23,11 @@ const int64_t kDefaultContacts = 1 << 20;
 const int64_t kDefaultQueue = 1 << 20;
 const int64_t kHostOrder = 256;        // pairs up to which the host orders them
 const int64_t kReadFloats = 16 << 20;  // words a read-back stages on the device at a time
+// Bytes of a tree that the gather writes to pinned host memory itself: up to 10 KB
+// 17 to 22 us, at 49 KB 37, where two copies to the caller's arrays took 31 and 48
+// (all of the scene's nodes at once 17 to 29 and 43, of a scene of one tree).  At
+// 84 KB the two copies take 51.
+const int64_t kReadPinned = 64 << 10;
 const int64_t kReadLeast = 4096;       // items it stages when the device has no room for more
 
 int fail(kdop_ctx* ctx, int status, const std::string& msg) {
@@ -570,7 +575,7 @@ int kdop_scene_create_ex(kdop_ctx* ctx, int K, int n_meshes, const kdop_mesh_des
     SC_TRY(dalloc(s, &s->ang_vel, n_meshes));
     SC_TRY(dalloc(s, &s->phase_dev, 1));
     SC_TRY(dalloc(s, &s->ctl, 1));
-    SC_TRY(cudaMallocHost((void**)&s->ctl_host, sizeof(TravCtl)));
+    SC_TRY(cudaMallocHost((void**)&s->ctl_host, sizeof(TravCtl) + kReadPinned));
     std::memset(s->ctl_host, 0, sizeof(TravCtl));
     SC_TRY(cudaMemcpyAsync(s->rest, rest.data(), (size_t)nv * sizeof(float4), cudaMemcpyHostToDevice, st));
     SC_TRY(cudaMemcpyAsync(s->world, rest.data(), (size_t)nv * sizeof(float4), cudaMemcpyHostToDevice, st));
@@ -674,6 +679,16 @@ int kdop_read_tree(kdop_scene* s, int mesh, int64_t cap, float* vol, int64_t* te
   if (cap < *n_nodes) return fail(s->ctx, KDOP_ERR_CAPACITY, "tree read buffer too small");
   if (!vol || !tet) return KDOP_ERR_INVALID;
   cudaSetDevice(s->ctx->device);
+  const int64_t bytes = *n_nodes * (s->K + 2) * 4;
+  if (bytes <= kReadPinned) {
+    int64_t* h_tet = reinterpret_cast<int64_t*>(s->ctl_host + 1);  // behind the counters' host copy
+    float* h_vol = reinterpret_cast<float*>(h_tet + *n_nodes);
+    KDOP_CUDA(s->ctx, kdop::launch_preorder(s, mesh, 0, *n_nodes, h_vol, h_tet));
+    KDOP_CUDA(s->ctx, cudaStreamSynchronize(s->ctx->stream));
+    std::memcpy(tet, h_tet, (size_t)*n_nodes * 8);
+    std::memcpy(vol, h_vol, (size_t)*n_nodes * s->K * 4);
+    return KDOP_OK;
+  }
   // gathered in preorder on the device, a window at a time: tets (8-byte
   // aligned), then slabs
   int64_t window = std::min<int64_t>(*n_nodes, kReadFloats / (s->K + 2));

@@ -80,3 +80,38 @@ def test_read_backs_on_a_full_device(ctx):
     assert np.array_equal(sorted_rows(got), sorted_rows(rows))
     assert np.array_equal(vol2, vol) and np.array_equal(tet2, tet)
     ds.close()
+
+
+def preorder(slabs, tets):
+    """The tree over leaves `tets` in order, split at the index median, in preorder."""
+    vol, tet = [], []
+
+    def walk(f, n):
+        at = len(vol)
+        vol.append(None)
+        tet.append(int(tets[f]) if n == 1 else -1)
+        if n == 1:
+            vol[at] = slabs[tets[f]]
+            return vol[at]
+        left = n - n // 2
+        a, b = walk(f, left), walk(f + left, n - left)
+        vol[at] = np.where(np.arange(slabs.shape[1]) % 2, np.maximum(a, b), np.minimum(a, b))
+        return vol[at]
+
+    walk(0, len(tets))
+    return np.array(vol), np.array(tet)
+
+
+# a node takes 4 K + 8 bytes: trees around the 64 KB that are read through pinned memory
+@pytest.mark.parametrize("K,n_tets", [(6, 1), (6, 2), (6, 512), (14, 7), (14, 512), (14, 513), (26, 292), (26, 293)])
+def test_small_trees(ctx, oracle, K, n_tets):
+    rng = np.random.default_rng(n_tets)
+    whole = scenes.lattice(5, 0.1, rng)
+    mesh = scenes.Mesh(whole.xyz, whole.tets[:n_tets], whole.surf[:n_tets])
+    ds = kd.DeviceScene(ctx, K, [scenes.lattice(1), mesh, whole])
+    for m in (mesh, whole, mesh):  # the buffer of one read is another's
+        vol, tet = ds.read_tree(1 if m is mesh else 2)
+        want_vol, want_tet = preorder(oracle.leaf_dops(K, m.xyz, m.tets), tet[tet >= 0])
+        assert np.array_equal(np.sort(tet[tet >= 0]), np.arange(m.n_tets))
+        assert np.array_equal(tet, want_tet) and np.array_equal(vol, want_vol)
+    ds.close()
