@@ -113,29 +113,37 @@ constexpr int kRefitSlots = 1 << kRefitUp;     // nodes a block starts from
 // 18 222 -> 211 us, K = 20 251 -> 229, K = 26 313 -> 287).
 // Smaller forests keep the block's join, which saves levels of the next launch.
 constexpr int64_t kWarpsAloneBlocks = 2048;
+// Forests of trees smaller than this have blocks of one warp with the shared
+// memory of 32 nodes: of 256 threads seven warps had nothing to do (20,000 trees
+// of one tet, K = 26: 74 -> 20 us, a launch per level 52; 3,000 of 63, K = 14: 21 ->
+// 11, 3,000 of 64 with blocks of 256 threads 22).
+constexpr int64_t kTinyTets = 64;
 // Shared-memory row of one record word: the block's nodes in heap order (root
 // 1).  Rows are 8 banks apart, so that two slabs a lane group apart in a union
 // fall on other halves of the banks, and a chunk's four rows are shifted by
 // chunk_skew banks more, so that the chunks of consecutive twins, which the
 // lanes of a store take, do not meet (rows of 514 words without the shift cost
 // 6.4 M of 43 M shared-memory passes at K = 18).
-constexpr int kRefitRow = 2 * kRefitSlots + 8;
+template <int SLOTS>
+__host__ __device__ constexpr int refit_row() {
+  return 2 * SLOTS + 8;
+}
 template <int K>
 __host__ __device__ constexpr int chunk_skew() {
   constexpr int NW = NodeLayout<K>::NW;
   return NW == 2 ? 16 : NW == 3 ? 10 : NW == 4 ? 8 : NW <= 6 ? 6 : 4;
 }
-template <int K>
+template <int K, int SLOTS>
 __device__ __forceinline__ float* word_row(float* T, int w) {
-  return T + w * kRefitRow + chunk_skew<K>() * (w >> 2);
+  return T + w * refit_row<SLOTS>() + chunk_skew<K>() * (w >> 2);
 }
-template <int K>
+template <int K, int SLOTS>
 __host__ __device__ constexpr int refit_words() {
-  return (K * kRefitRow + chunk_skew<K>() * NodeLayout<K>::NW + 1) & ~1;  // slot_words follow, 8-byte aligned
+  return (K * refit_row<SLOTS>() + chunk_skew<K>() * NodeLayout<K>::NW + 1) & ~1;  // slot_words follow, 8-byte aligned
 }
-template <int K>
+template <int K, int SLOTS>
 constexpr size_t refit_smem() {
-  return (size_t)refit_words<K>() * 4 + kRefitSlots * 8;
+  return (size_t)refit_words<K, SLOTS>() * 4 + SLOTS * 8;
 }
 
 struct RefitArgs {
@@ -149,36 +157,36 @@ struct RefitArgs {
 
 // Slab x of node U of the block's heap: the union of its children (make_union;
 // slabs hold no NaN and no -0, so fminf / fmaxf are the reference's choices).
-template <int K>
+template <int K, int SLOTS>
 __device__ __forceinline__ void unite_slab(float* T, uint32_t U, int x) {
-  float* row = word_row<K>(T, 2 * x);
+  float* row = word_row<K, SLOTS>(T, 2 * x);
   const float2 lo = *reinterpret_cast<const float2*>(row + 2 * U);
-  const float2 hi = *reinterpret_cast<const float2*>(row + kRefitRow + 2 * U);
+  const float2 hi = *reinterpret_cast<const float2*>(row + refit_row<SLOTS>() + 2 * U);
   row[U] = fminf(lo.x, lo.y);
-  row[kRefitRow + U] = fmaxf(hi.x, hi.y);
+  row[refit_row<SLOTS>() + U] = fmaxf(hi.x, hi.y);
 }
 // The 2^M nodes M levels below `root`, a slab of a node per lane.
-template <int K, int M>
+template <int K, int SLOTS, int M>
 __device__ __forceinline__ void unite_level(float* T, uint32_t root, int lane) {
   constexpr int N = (K / 2) << M;
 #pragma unroll
   for (int it = 0; it * 32 < N; ++it)
     if ((it + 1) * 32 <= N || it * 32 + lane < N)
-      unite_slab<K>(T, (root << M) + (uint32_t)(lane & ((1 << M) - 1)), (lane >> M) + it * (32 >> M));
+      unite_slab<K, SLOTS>(T, (root << M) + (uint32_t)(lane & ((1 << M) - 1)), (lane >> M) + it * (32 >> M));
   __syncwarp();
 }
 
 // Chunk j of the twin of the children of heap node U to `to`; the topology
 // words of its two nodes are we, wo.
-template <int K>
+template <int K, int SLOTS>
 __device__ __forceinline__ void put_chunk(const float* T, uint32_t U, int j, uint2 we, uint2 wo, float4* to) {
-  const float* col = T + j * (4 * kRefitRow + chunk_skew<K>()) + 2 * U;
+  const float* col = T + j * (4 * refit_row<SLOTS>() + chunk_skew<K>()) + 2 * U;
   float e[4], o[4];
 #pragma unroll
   for (int c = 0; c < 4; ++c) {
     e[c] = o[c] = 0.f;
     if (4 * j + c < K) {
-      const float2 x = *reinterpret_cast<const float2*>(col + c * kRefitRow);
+      const float2 x = *reinterpret_cast<const float2*>(col + c * refit_row<SLOTS>());
       e[c] = x.x;
       o[c] = x.y;
     }
@@ -193,13 +201,13 @@ __device__ __forceinline__ void put_chunk(const float* T, uint32_t U, int j, uin
   stg256(to, e, o);
 }
 // Chunk j of heap node U alone.
-template <int K>
+template <int K, int SLOTS>
 __device__ __forceinline__ float4 half_chunk(float* T, uint32_t U, int j, uint2 words) {
   float e[4];
 #pragma unroll
   for (int c = 0; c < 4; ++c) {
     const int w = 4 * j + c;
-    e[c] = w < K ? word_row<K>(T, w)[U]
+    e[c] = w < K ? word_row<K, SLOTS>(T, w)[U]
                  : w == K ? __uint_as_float(words.x) : w == K + 1 ? __uint_as_float(words.y) : 0.f;
   }
   return make_float4(e[0], e[1], e[2], e[3]);
@@ -209,7 +217,7 @@ __device__ __forceinline__ float4 half_chunk(float* T, uint32_t U, int j, uint2 
 // chunk per lane, so that a warp writes 1 KB in a row.  kids: first child of
 // the first of them; words: their topology words instead, where they are the
 // block's own nodes.
-template <int K, int M>
+template <int K, int SLOTS, int M>
 __device__ __forceinline__ void put_level(float4* nodes, const float* T, uint32_t root, uint32_t first, uint32_t kids,
                                           const uint2* words, int lane) {
   constexpr int NW = NodeLayout<K>::NW, N = NW << M;
@@ -227,7 +235,7 @@ __device__ __forceinline__ void put_level(float4* nodes, const float* T, uint32_
       we = words[2 * r];
       wo = words[2 * r + 1];
     }
-    put_chunk<K>(T, (root << M) + (uint32_t)r, j, we, wo, to + 64 * it);
+    put_chunk<K, SLOTS>(T, (root << M) + (uint32_t)r, j, we, wo, to + 64 * it);
   }
 }
 
@@ -235,13 +243,13 @@ __device__ __forceinline__ void put_level(float4* nodes, const float* T, uint32_
 // block's nodes, written by the launch before.  A warp unites its 32 nodes and
 // writes their levels by itself (no block barrier); the first warp does the
 // last levels from the warps' ancestors.
-template <int K, bool BOTTOM>
-__global__ void __launch_bounds__(kRefitSlots, K <= 8 ? 6 : K <= 14 ? 5 : K <= 20 ? 4 : 3)
+template <int K, bool BOTTOM, int SLOTS>
+__global__ void __launch_bounds__(SLOTS, SLOTS == 32 ? (K <= 20 ? 32 : 24) : K <= 8 ? 6 : K <= 14 ? 5 : K <= 20 ? 4 : 3)
     refit_kernel(const __grid_constant__ RefitArgs a) {
   using L = NodeLayout<K>;
   constexpr int NW = L::NW, NS = L::NS;
   extern __shared__ float T[];  // word_row(T, w)[heap index]
-  uint2* slot_words = reinterpret_cast<uint2*>(T + refit_words<K>());
+  uint2* slot_words = reinterpret_cast<uint2*>(T + refit_words<K, SLOTS>());
   const RefitBlock& b = a.blocks[blockIdx.x];
   const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
   const int hd = b.levels;             // levels above the block's nodes in this block
@@ -262,7 +270,7 @@ __global__ void __launch_bounds__(kRefitSlots, K <= 8 ? 6 : K <= 14 ? 5 : K <= 2
       uint32_t before = 0, mine = extra;
       if (wb) {
 #pragma unroll
-        for (int w = 0; w < kRefitSlots / 32; ++w) {
+        for (int w = 0; w < SLOTS / 32; ++w) {
           const uint32_t x = (extra + (1u << wb) - 1u - (__brev((uint32_t)w) >> (32 - wb))) >> wb;
           if (w < wib) before += x;
           if (w == wib) mine = x;
@@ -298,8 +306,8 @@ __global__ void __launch_bounds__(kRefitSlots, K <= 8 ? 6 : K <= 14 ? 5 : K <= 2
         slot_words[t] = words;
 #pragma unroll
         for (int k = 0; k < K; k += 2) {
-          word_row<K>(T, k)[cnt + t] = fminf(w[k], v[k]);
-          word_row<K>(T, k + 1)[cnt + t] = fmaxf(w[k + 1], v[k + 1]);
+          word_row<K, SLOTS>(T, k)[cnt + t] = fminf(w[k], v[k]);
+          word_row<K, SLOTS>(T, k + 1)[cnt + t] = fmaxf(w[k + 1], v[k + 1]);
         }
       }
     } else {
@@ -311,34 +319,34 @@ __global__ void __launch_bounds__(kRefitSlots, K <= 8 ? 6 : K <= 14 ? 5 : K <= 2
         const float e[4] = {x.x, x.y, x.z, x.w};
 #pragma unroll
         for (int c = 0; c < 4; ++c)
-          if (4 * j + c < K) word_row<K>(T, 4 * j + c)[cnt + i] = e[c];
+          if (4 * j + c < K) word_row<K, SLOTS>(T, 4 * j + c)[cnt + i] = e[c];
       }
     }
     __syncwarp();
     if (wl == 5) {
-      unite_level<K, 4>(T, root, lane);
-      unite_level<K, 3>(T, root, lane);
-      unite_level<K, 2>(T, root, lane);
-      unite_level<K, 1>(T, root, lane);
-      unite_level<K, 0>(T, root, lane);
+      unite_level<K, SLOTS, 4>(T, root, lane);
+      unite_level<K, SLOTS, 3>(T, root, lane);
+      unite_level<K, SLOTS, 2>(T, root, lane);
+      unite_level<K, SLOTS, 1>(T, root, lane);
+      unite_level<K, SLOTS, 0>(T, root, lane);
       // levels from the block's own nodes up: those M + 1 levels below the
       // warp's ancestor start at node 2^(M + 1) wib of their level
       const uint32_t w = (uint32_t)wib;
       if (BOTTOM)
-        put_level<K, 4>(a.nodes, T, root, b.node[hd] + 32u * w, 0u, slot_words + 32 * wib, lane);
-      put_level<K, 3>(a.nodes, T, root, b.node[hd - 1] + 16u * w, b.node[hd] + 32u * w, nullptr, lane);
-      put_level<K, 2>(a.nodes, T, root, b.node[hd - 2] + 8u * w, b.node[hd - 1] + 16u * w, nullptr, lane);
-      put_level<K, 1>(a.nodes, T, root, b.node[hd - 3] + 4u * w, b.node[hd - 2] + 8u * w, nullptr, lane);
-      put_level<K, 0>(a.nodes, T, root, b.node[hd - 4] + 2u * w, b.node[hd - 3] + 4u * w, nullptr, lane);
+        put_level<K, SLOTS, 4>(a.nodes, T, root, b.node[hd] + 32u * w, 0u, slot_words + 32 * wib, lane);
+      put_level<K, SLOTS, 3>(a.nodes, T, root, b.node[hd - 1] + 16u * w, b.node[hd] + 32u * w, nullptr, lane);
+      put_level<K, SLOTS, 2>(a.nodes, T, root, b.node[hd - 2] + 8u * w, b.node[hd - 1] + 16u * w, nullptr, lane);
+      put_level<K, SLOTS, 1>(a.nodes, T, root, b.node[hd - 3] + 4u * w, b.node[hd - 2] + 8u * w, nullptr, lane);
+      put_level<K, SLOTS, 0>(a.nodes, T, root, b.node[hd - 4] + 2u * w, b.node[hd - 3] + 4u * w, nullptr, lane);
       if (b.warps_alone && lane < NW) {
         // the next launch starts from the warps' ancestors
         const uint32_t kids = b.node[hd - 4] + 2u * w;
-        a.nodes[L::at(b.node[hd - 5] + w, lane)] = half_chunk<K>(T, root, lane, make_uint2(kids, kids + 1u));
+        a.nodes[L::at(b.node[hd - 5] + w, lane)] = half_chunk<K, SLOTS>(T, root, lane, make_uint2(kids, kids + 1u));
       }
     } else {
       // a tree of fewer than 64 tets (or its last levels): one warp, level by level
       for (int m = wl - 1; m >= 0; --m) {
-        for (int x = lane; x < (NS << m); x += 32) unite_slab<K>(T, (1u << m) + (x & ((1 << m) - 1)), x >> m);
+        for (int x = lane; x < (NS << m); x += 32) unite_slab<K, SLOTS>(T, (1u << m) + (x & ((1 << m) - 1)), x >> m);
         __syncwarp();
       }
       for (int m = BOTTOM ? wl - 1 : wl - 2; m >= 0; --m)
@@ -350,7 +358,7 @@ __global__ void __launch_bounds__(kRefitSlots, K <= 8 ? 6 : K <= 14 ? 5 : K <= 2
             we = slot_words[2 * r];
             wo = slot_words[2 * r + 1];
           }
-          put_chunk<K>(T, (1u << m) + r, q % NW, we, wo, a.nodes + L::at(b.node[m + 1], 0) + 2 * q);
+          put_chunk<K, SLOTS>(T, (1u << m) + r, q % NW, we, wo, a.nodes + L::at(b.node[m + 1], 0) + 2 * q);
         }
     }
   }
@@ -358,7 +366,7 @@ __global__ void __launch_bounds__(kRefitSlots, K <= 8 ? 6 : K <= 14 ? 5 : K <= 2
   __syncthreads();
   if (wib > 0) return;
   for (int n = warps >> 1; n >= 1; n >>= 1) {
-    for (int x = lane; x < n * NS; x += 32) unite_slab<K>(T, (uint32_t)(n + x % n), x / n);
+    for (int x = lane; x < n * NS; x += 32) unite_slab<K, SLOTS>(T, (uint32_t)(n + x % n), x / n);
     __syncwarp();
   }
   for (int q = lane; q < (warps - 1) * NW; q += 32) {
@@ -367,16 +375,16 @@ __global__ void __launch_bounds__(kRefitSlots, K <= 8 ? 6 : K <= 14 ? 5 : K <= 2
     const int l = 32 - __clz(U);
     const uint32_t i = 2 * U - (1u << l), k = b.node[l + 1] + 2u * i;
     const int j = q % NW;
-    put_chunk<K>(T, U, j, make_uint2(k, k + 1u), make_uint2(k + 2u, k + 3u), a.nodes + L::at(b.node[l] + i, j));
+    put_chunk<K, SLOTS>(T, U, j, make_uint2(k, k + 1u), make_uint2(k + 2u, k + 3u), a.nodes + L::at(b.node[l] + i, j));
   }
   // the common ancestor: one half of a twin
   if (lane < NW) {
     const uint2 words = (BOTTOM && hd == 0) ? slot_words[0] : make_uint2(b.node[1], b.node[1] + 1u);
-    a.nodes[L::at(b.node[0], lane)] = half_chunk<K>(T, 1u, lane, words);
+    a.nodes[L::at(b.node[0], lane)] = half_chunk<K, SLOTS>(T, 1u, lane, words);
     if (b.pad_node != NO_NODE) {
       // the root level's padding node: the root again (a leaf under its own index)
       const uint32_t own = (words.x & LEAF_BIT) ? (words.x & (LEAF_BIT | SURF_BIT)) | b.pad_node : words.x;
-      a.nodes[L::at(b.pad_node, lane)] = half_chunk<K>(T, 1u, lane, make_uint2(own, words.y));
+      a.nodes[L::at(b.pad_node, lane)] = half_chunk<K, SLOTS>(T, 1u, lane, make_uint2(own, words.y));
     }
   }
 }
@@ -596,18 +604,30 @@ static cudaError_t refit_impl(kdop_scene* s, int mode) {
   a.world = world;
   a.ds.corner = corners ? s->dirs.d[axes][0] : 0.f;
   a.ds.edge = axes + corners < K / 2 ? s->dirs.d[axes + corners][0] : 0.f;
-  constexpr size_t smem = refit_smem<K>();
-  cudaError_t e = cudaFuncSetAttribute(refit_kernel<K, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  if (s->most_tets < kTinyTets) {
+    // one launch: no tree has more than 32 nodes of depth L
+    const unsigned n = s->refit_stage.size() > 1 ? (unsigned)s->refit_stage[1] : 0u;
+    a.blocks = s->refit_blocks;
+    if (n) {
+      refit_kernel<K, true, 32><<<n, 32, refit_smem<K, 32>(), s->ctx->stream>>>(a);
+      s->ctx->launches++;
+    }
+    return cudaGetLastError();
+  }
+  constexpr size_t smem = refit_smem<K, kRefitSlots>();
+  cudaError_t e =
+      cudaFuncSetAttribute(refit_kernel<K, true, kRefitSlots>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   if (e == cudaSuccess)
-    e = cudaFuncSetAttribute(refit_kernel<K, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    e = cudaFuncSetAttribute(refit_kernel<K, false, kRefitSlots>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                             (int)smem);
   if (e != cudaSuccess) return e;
   for (size_t i = 0; i + 1 < s->refit_stage.size(); ++i) {
     const unsigned n = (unsigned)(s->refit_stage[i + 1] - s->refit_stage[i]);
     a.blocks = s->refit_blocks + s->refit_stage[i];
     if (i == 0)
-      refit_kernel<K, true><<<n, kRefitSlots, smem, s->ctx->stream>>>(a);
+      refit_kernel<K, true, kRefitSlots><<<n, kRefitSlots, smem, s->ctx->stream>>>(a);
     else
-      refit_kernel<K, false><<<n, kRefitSlots, smem, s->ctx->stream>>>(a);
+      refit_kernel<K, false, kRefitSlots><<<n, kRefitSlots, smem, s->ctx->stream>>>(a);
     s->ctx->launches++;
   }
   return cudaGetLastError();
