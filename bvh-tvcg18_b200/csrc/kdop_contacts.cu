@@ -129,7 +129,6 @@ __device__ __forceinline__ bool sat_test(int t, const f3* A, const f3* B) {
 struct ContactArgs {
   const uint32_t* candA;
   const uint32_t* candB;
-  const uint32_t* candP;
   uint32_t* surv;  // candidates that overlap and have an admissible face pair (n_surv of them)
   uint32_t* mid;   // candidates with an admissible face pair (n_mid of them)
   unsigned cand_cap;
@@ -888,7 +887,6 @@ cudaError_t launch_contacts(kdop_scene* s) {
   ContactArgs a;
   a.candA = s->cand;
   a.candB = s->cand + s->cand_cap;
-  a.candP = s->cand + 2 * s->cand_cap;
   a.surv = s->cand + 3 * s->cand_cap;
   a.mid = s->cand + 4 * s->cand_cap;
   a.cand_cap = (unsigned)s->cand_cap;

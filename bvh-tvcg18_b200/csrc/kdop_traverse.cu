@@ -42,7 +42,6 @@ namespace kdop {
 
 struct TravArgs {
   const float4* __restrict__ nodes;
-  const uint8_t* __restrict__ surf;
   const uint32_t* __restrict__ root;
   const uint2* __restrict__ pairs;
   uint32_t* candA;
@@ -932,7 +931,6 @@ static cudaError_t traverse_impl(kdop_scene* s, int64_t n_pairs, const TravBuffe
   unsigned grid = (unsigned)(per_sm * s->ctx->sm_count);
   TravArgs a;
   a.nodes = s->nodes;
-  a.surf = s->surf;
   a.root = s->root_dev;
   a.pairs = b.pairs;
   a.order = b.order;
@@ -1206,7 +1204,6 @@ TravArgs frontier_args(kdop_scene* s, const uint2* pairs, const TravParams& p) {
   TravArgs a;
   std::memset(&a, 0, sizeof(a));
   a.nodes = s->nodes;
-  a.surf = s->surf;
   a.root = s->root_dev;
   a.pairs = pairs;
   a.candA = s->cand;
