@@ -18,7 +18,10 @@ from . import lib as kd
 
 def _scene_stream(scene, device):
     """The scene's stream and torch's current one on `device`."""
-    return torch.cuda.ExternalStream(scene.ctx.stream, device=device), torch.cuda.current_stream(device)
+    handle = scene.ctx.stream
+    # cudaStreamLegacy (1) is the stream torch calls the default one, and no ExternalStream's
+    work = torch.cuda.default_stream(device) if handle == 1 else torch.cuda.ExternalStream(handle, device=device)
+    return work, torch.cuda.current_stream(device)
 
 
 class ContactGeometry(torch.autograd.Function):
