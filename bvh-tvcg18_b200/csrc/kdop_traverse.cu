@@ -314,7 +314,7 @@ __global__ void __launch_bounds__(512, (C * S >= 4) ? 1 : 2) traverse_kernel(Tra
   constexpr int NW = L::NW;
   constexpr int Q = CP::Q, E = CP::E, PM = CP::PM;
   constexpr int SLOTS = PM * S;                     // pushes per lane per step
-  constexpr int CBITS = SLOTS <= 1 ? 1 : SLOTS <= 3 ? 2 : 3;  // bits of a lane's push count
+  constexpr int CBITS = SLOTS <= 1 ? 1 : SLOTS <= 3 ? 2 : SLOTS <= 7 ? 3 : 4;  // bits of a lane's emit count
   extern __shared__ uint32_t smem[];
   __shared__ uint2 s_claim[SEEDED ? 16 : 1];  // per warp: claimed initial work not yet taken [x, y)
   __shared__ unsigned s_first;
