@@ -60,7 +60,7 @@ def test_longer_list_inside_a_callers_capture(n_pairs):
     del graph
 
 
-@pytest.mark.parametrize("n_pairs, between", [(300, 10), (40, 400)])
+@pytest.mark.parametrize("n_pairs, between", [(300, 10), (40, 400), (40, 250), (1, 256)])
 def test_replay_of_a_list_after_another(n_pairs, between):
     """The results are those of the graph's list, whatever list a call had in between."""
     stream = torch.cuda.Stream()
