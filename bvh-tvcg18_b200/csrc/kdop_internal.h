@@ -51,7 +51,7 @@ struct TravCtl {
   unsigned int pair_base;            // pair index of the first root pair
   unsigned int n_seed;               // node pairs the first seed pass left for the second
   unsigned int n_surv;               // candidates past the contact pre-filter
-  unsigned int n_mid;                // candidates past the face axes of the SAT test
+  unsigned int n_mid;                // candidates with an admissible face pair
   unsigned int order_error;          // DEV_ERR_* of the sort that ordered the root pairs
   unsigned int pad0[20];
   unsigned int n_cand;               // candidates emitted (may exceed capacity)
@@ -154,7 +154,7 @@ struct kdop_scene {
   uint32_t* pair_order = nullptr;  // pair indices by decreasing size (tets of A + tets of B)
   int64_t pairs_cap = 0;
   uint32_t* cand = nullptr;  // kCandCols * cand_cap: A tets | B tets | pair ids | pre-filter survivors |
-                             // candidates past the face axes of the SAT test
+                             // candidates with an admissible face pair
   int64_t cand_cap = 0;
   kdop_contact* contacts = nullptr;
   int4* records = nullptr;  // per candidate: faces, candidate codes, count, first contact

@@ -109,8 +109,8 @@ constexpr int kRefitUp = 8;                    // levels a block unites above it
 constexpr int kRefitSlots = 1 << kRefitUp;     // nodes a block starts from
 // From this many blocks on, the first launch's warps each stop at the ancestor
 // of their own 32 nodes: a block's last three levels and its barrier keep seven
-// of its eight warps' places taken while one works (96 trees of 48,000 tets: K =
-// 18 222 -> 211 us, K = 20 251 -> 229, K = 26 313 -> 287).
+// of its eight warps' places taken while one works (96 trees of 48,000 tets,
+// 12,288 blocks: K = 18 222 -> 211 us, K = 20 251 -> 229, K = 26 313 -> 287).
 // Smaller forests keep the block's join, which saves levels of the next launch.
 constexpr int64_t kWarpsAloneBlocks = 2048;
 // Forests of trees smaller than this have blocks of one warp with the shared
@@ -638,7 +638,7 @@ static cudaError_t refit_impl(kdop_scene* s, int mode) {
 // on.  In a large forest the first launch's warps stop at their own ancestors
 // and the depths are L, L - 5, L - 13, ...: its blocks then have no barrier and
 // no last levels that one warp works on while the other seven's place stays
-// taken (96 trees of 48,000 tets, 12,288 blocks, K = 18: 222 -> 211 us, K = 26: 307 -> 287); in a small
+// taken (12,288 blocks: kWarpsAloneBlocks); in a small
 // one the launch that this can add costs more.  pre: nodes of the trees before
 // m at depth d; t_off: first tet of a mesh.
 void refit_blocks(const ForestBuild& fb, const std::vector<int64_t>& pre, const std::vector<int32_t>& lg,
