@@ -1354,7 +1354,7 @@ int kdop_graph_capture(kdop_scene* s, int refit_mode, int64_t n_pairs, const uin
   int rc = upload_pairs(s, n_pairs, pairs, memory, p.timeout_ns);
   if (rc != KDOP_OK) return rc;
   // settle function attributes outside the capture
-  KDOP_CUDA(s->ctx, kdop::traverse_prepare(s->K, kdop::traverse_smem_bytes(p.block_warps, p.stack_cap)));
+  KDOP_CUDA(s->ctx, kdop::traverse_prepare(s->K, kdop::traverse_smem_limit(s->ctx->smem_optin)));
   KDOP_CUDA(s->ctx, cudaStreamSynchronize(s->ctx->stream));
   long long before = s->ctx->launches;
   // the captured contact kernels take their vertex source from the refit

@@ -292,6 +292,7 @@ int kdop_resolve_traverse_opts(const kdop_scene* s, const kdop_traverse_opts* o,
 
 namespace kdop {
 size_t traverse_smem_bytes(int block_warps, int stack_cap);
+size_t traverse_smem_limit(size_t smem_optin);
 cudaError_t traverse_prepare(int K, size_t smem);
 
 }  // namespace kdop

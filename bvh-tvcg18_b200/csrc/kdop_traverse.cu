@@ -880,6 +880,10 @@ int traverse_block_threads(int block_warps) { return 32 * block_warps; }
 size_t traverse_smem_bytes(int block_warps, int stack_cap) {
   return (size_t)block_warps * (size_t)stack_cap * sizeof(uint2);
 }
+// The kernels' limit, one for every shape: the attribute is the function's, and a
+// host thread that set a shape's own could lower it between another thread's
+// setting and its launch.  Options allow no shape above it.
+size_t traverse_smem_limit(size_t smem_optin) { return smem_optin / 12 * sizeof(uint2); }
 
 template <int K, int C, int S>
 static cudaError_t prepare_shape(size_t smem) {
@@ -919,7 +923,8 @@ static cudaError_t traverse_impl(kdop_scene* s, int64_t n_pairs, const TravBuffe
   size_t smem = traverse_smem_bytes(p.block_warps, p.stack_cap);
   const bool seeded = b.seeds && !plain && p.wave_pairs <= 0 && n_pairs > 0;
   const auto kernel = seeded ? traverse_kernel<K, C, S, true> : traverse_kernel<K, C, S, false>;
-  cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                       (int)traverse_smem_limit(s->ctx->smem_optin));
   if (e != cudaSuccess) return e;
   e = cudaFuncSetAttribute(kernel, cudaFuncAttributePreferredSharedMemoryCarveout,
                            p.smem_carveout > 0 ? p.smem_carveout : -1);
