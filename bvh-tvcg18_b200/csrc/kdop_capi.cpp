@@ -1011,9 +1011,11 @@ int kdop_broad_phase(kdop_scene* s, const float* positions, int memory, uint32_t
   if (total > x->broad_cap) {
     if (x->broad_pairs) cudaFree(x->broad_pairs);
     x->broad_pairs = nullptr;
+    s->device_bytes -= x->broad_cap * (int64_t)sizeof(uint2);
+    x->broad_cap = 0;  // no room until the allocation has succeeded: a query writes what it has room for
     int64_t c = total + total / 4 + 256;
     KDOP_CUDA(s->ctx, cudaMalloc((void**)&x->broad_pairs, (size_t)c * sizeof(uint2)));
-    s->device_bytes += (c - x->broad_cap) * (int64_t)sizeof(uint2);
+    s->device_bytes += c * (int64_t)sizeof(uint2);
     x->broad_cap = c;
     KDOP_CUDA(s->ctx, kdop::broad_phase(s, x->radius_bits, pos, x->broad_work, x->broad_pairs, x->broad_cap, &total));
   }
