@@ -167,9 +167,12 @@ static bool capturing(kdop_scene* s) {
 // them (a step that reads statistics, sorts and reads contacts copied them five
 // times, 8 us each).  Work recorded into a capture can run again without a
 // call, so a scene that was ever captured into a caller's graph always copies.
-static void ctl_changes(kdop_scene* s) {
+// Says whether the scene's stream is being captured.
+static bool ctl_changes(kdop_scene* s) {
   s->ctl_fresh = false;
-  if (capturing(s)) s->ctl_replayed = true;
+  const bool c = capturing(s);
+  if (c) s->ctl_replayed = true;
+  return c;
 }
 // Synchronises and brings ctl_host up to date.
 static cudaError_t read_ctl(kdop_scene* s) {
@@ -914,7 +917,7 @@ static int upload_pairs(kdop_scene* s, int64_t n, const uint32_t* pairs, int mem
   int rc = grow_pairs(s, std::max<int64_t>(n, 1));
   if (rc != KDOP_OK) return rc;
   s->pairs_current = false;  // until a traversal of this list is enqueued
-  ctl_changes(s);
+  const bool captured = ctl_changes(s);
   x->pairs_host.swap(list);
   if (n == 0) return KDOP_OK;
   KDOP_CUDA(s->ctx, cudaMemcpyAsync(s->pairs, pairs, (size_t)n * 8,
@@ -935,7 +938,7 @@ static int upload_pairs(kdop_scene* s, int64_t n, const uint32_t* pairs, int mem
     s->pairs_tets = 0;
     for (int64_t i = 0; i < n; ++i) s->pairs_tets += tets(i);
   }
-  if (n > kHostOrder || capturing(s)) {
+  if (n > kHostOrder || captured) {
     KDOP_CUDA(s->ctx, kdop::launch_pair_order(s, n, (uint32_t)std::max<int64_t>(2 * s->most_tets, 1), wait_ns));
     x->device_order = true;
     return KDOP_OK;
