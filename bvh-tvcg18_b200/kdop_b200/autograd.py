@@ -61,6 +61,8 @@ class ContactGeometry(torch.autograd.Function):
         gd = (g_depth if g_depth is not None else torch.zeros(n, device=dev)).float().contiguous()
         gn = (g_normal if g_normal is not None else torch.zeros((n, 3), device=dev)).float().contiguous()
         grad = torch.zeros((ctx.n_verts, 3), dtype=torch.float32, device=dev)
+        if n == 0:  # nothing to carry back, and no addresses for the adjoint
+            return grad, None, None, None
         work, current = _scene_stream(scene, dev)
         work.wait_stream(current)
         scene.adjoint(gd, gn, grad)
